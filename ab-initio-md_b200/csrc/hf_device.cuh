@@ -31,18 +31,11 @@ __host__ __device__ constexpr int ncon_cap(int l) { return l == 0 ? 2 : 1; }
 __host__ __device__ constexpr int hidx(int t, int u, int v) {
     return nherm(t + u + v - 1) + (u + v) * (u + v + 1) / 2 + v;
 }
-// Cartesian component i of angular momentum l in PySCF order.
-__host__ __device__ constexpr int cart_x(int l, int i) {
-    int n = 0;
-    for (int lx = l; lx >= 0; --lx)
-        for (int ly = l - lx; ly >= 0; --ly) { if (n == i) return lx; ++n; }
-    return 0;
-}
+// Cartesian component i of angular momentum l <= 2 in PySCF order
+// (s; x y z; xx xy xz yy yz zz).
+__host__ __device__ constexpr int cart_x(int l, int i) { return l == 0 ? 0 : (l == 1 ? (i == 0) : (i == 0 ? 2 : (i < 3))); }
 __host__ __device__ constexpr int cart_y(int l, int i) {
-    int n = 0;
-    for (int lx = l; lx >= 0; --lx)
-        for (int ly = l - lx; ly >= 0; --ly) { if (n == i) return ly; ++n; }
-    return 0;
+    return l == 0 ? 0 : (l == 1 ? (i == 1) : (i == 3 ? 2 : (i == 1 || i == 4)));
 }
 __host__ __device__ constexpr int cart_z(int l, int i) { return l - cart_x(l, i) - cart_y(l, i); }
 
@@ -62,11 +55,14 @@ __host__ __device__ inline int npp_bucket(int npp) {
     return b;
 }
 
-// Normalisation of Cartesian component (lx, ly, lz) relative to x^l:
-// sqrt((2l-1)!! / ((2lx-1)!! (2ly-1)!! (2lz-1)!!)).
-__host__ __device__ constexpr double dfact_odd(int n) { double r = 1.0; for (int k = n; k > 1; k -= 2) r *= k; return r; }
-__host__ __device__ inline double cart_norm(int lx, int ly, int lz) {
-    return sqrt(dfact_odd(2 * (lx + ly + lz) - 1) / (dfact_odd(2 * lx - 1) * dfact_odd(2 * ly - 1) * dfact_odd(2 * lz - 1)));
+// the component with powers (l - y - z, y, z)
+__host__ __device__ constexpr int cart_index(int y, int z) { return (y + z) * (y + z + 1) / 2 + z; }
+
+// Normalisation of Cartesian component (lx, ly, lz) relative to x^l,
+// sqrt((2l-1)!! / ((2lx-1)!! (2ly-1)!! (2lz-1)!!)), for l <= 2: sqrt(3) for
+// xy, xz and yz, 1 for the others.
+__host__ __device__ constexpr double cart_norm(int lx, int ly, int lz) {
+    return lx + ly + lz == 2 && lx != 2 && ly != 2 && lz != 2 ? 1.7320508075688772935 : 1.0;
 }
 
 // ---------------------------------------------------------------- accumulation
@@ -86,6 +82,21 @@ __device__ __forceinline__ facc to_fixed(double v, double scale) {
     return static_cast<facc>(__double2ll_rn(v * scale));
 }
 __device__ __forceinline__ void fadd(facc* p, double v, double scale) { atomicAdd(p, to_fixed(v, scale)); }
+// The same sum in shared memory, held as two 32-bit planes (lo, hi): a 64-bit
+// shared atomicAdd is a compare-and-swap loop, while the 32-bit ones are
+// native, so the low word is added first and its carry goes into the high
+// word. The pair of planes equals the 64-bit sum modulo 2^64 once every add
+// has finished. Measured (one B200, 256 threads per SM, random addresses in
+// 7200 words): 13 against 23 cycles a warp; 21 against 114 where eight lanes
+// share an address.
+__device__ __forceinline__ void sadd(unsigned* lo, unsigned* hi, double v, double scale) {
+    const facc x = to_fixed(v, scale);
+    const unsigned l = static_cast<unsigned>(x);
+    const unsigned old = atomicAdd(lo, l);
+    const unsigned h = static_cast<unsigned>(x >> 32) + (old + l < old ? 1u : 0u);
+    if (h) atomicAdd(hi, h);
+}
+__device__ __forceinline__ facc join_planes(unsigned lo, unsigned hi) { return (static_cast<facc>(hi) << 32) | lo; }
 __host__ __device__ __forceinline__ double from_fixed(facc u, double scale) {
     return static_cast<double>(static_cast<long long>(u)) / scale;
 }
@@ -291,6 +302,43 @@ __device__ __forceinline__ void hermite_e(RT pa, RT pb, RT oo2p, RT e00, RT (&e)
                 if (t + 1 <= i - 1 + j) v += (t + 1) * e[i - 1][j][t + 1];
                 if (t > 0) v += oo2p * e[i - 1][j][t - 1];
                 e[i][j][t] = v;
+            }
+}
+
+// de[i][j][t] = dE^{ij}_t / dX for X = A - B, at fixed exponents (E depends on
+// the centres through X alone: P - A = -(b/p) X, P - B = (a/p) X,
+// E^{00}_0 ~ exp(-mu X^2)), by differentiating the recursions of hermite_e;
+// e holds E, bp = b/p, ap = a/p, x2mu = 2 mu X.
+template <int IM, int JM, typename RT>
+__device__ __forceinline__ void hermite_de(RT pa, RT pb, RT oo2p, RT bp, RT ap, RT x2mu,
+                                           const RT (&e)[IM + 1][JM + 1][IM + JM + 1],
+                                           RT (&de)[IM + 1][JM + 1][IM + JM + 1]) {
+#pragma unroll
+    for (int i = 0; i <= IM; ++i)
+#pragma unroll
+        for (int j = 0; j <= JM; ++j)
+#pragma unroll
+            for (int t = 0; t <= IM + JM; ++t) de[i][j][t] = RT(0);
+    de[0][0][0] = -x2mu * e[0][0][0];
+#pragma unroll
+    for (int j = 1; j <= JM; ++j)
+#pragma unroll
+        for (int t = 0; t <= j; ++t) {
+            RT v = t <= j - 1 ? pb * de[0][j - 1][t] + ap * e[0][j - 1][t] : RT(0);
+            if (t + 1 <= j - 1) v += (t + 1) * de[0][j - 1][t + 1];
+            if (t > 0) v += oo2p * de[0][j - 1][t - 1];
+            de[0][j][t] = v;
+        }
+#pragma unroll
+    for (int i = 1; i <= IM; ++i)
+#pragma unroll
+        for (int j = 0; j <= JM; ++j)
+#pragma unroll
+            for (int t = 0; t <= i + j; ++t) {
+                RT v = t <= i - 1 + j ? pa * de[i - 1][j][t] - bp * e[i - 1][j][t] : RT(0);
+                if (t + 1 <= i - 1 + j) v += (t + 1) * de[i - 1][j][t + 1];
+                if (t > 0) v += oo2p * de[i - 1][j][t - 1];
+                de[i][j][t] = v;
             }
 }
 

@@ -74,6 +74,18 @@ struct BraStageT {
 };
 using BraStage = BraStageT<double>;
 
+template <typename RT>
+__device__ __forceinline__ void stage_bra_scalars(const BraStageT<RT>& st) {
+    for (int ib = threadIdx.x; ib < st.nbp; ib += blockDim.x) {
+        const double* b = st.rec + (size_t)ib * PPW;
+        RT* o = st.SB + (size_t)ib * SBW;
+        const double p = b[0] + b[1];
+        const double vals[SBW] = {p, 1.0 / p, b[3], b[4], b[5], b[0], b[1], 0.0, b[12], b[13], b[14], b[15]};
+#pragma unroll
+        for (int i = 0; i < SBW; ++i) o[i] = static_cast<RT>(vals[i]);
+    }
+}
+
 // Fill the shared stage (E tables and scalars) for all bra primitives.
 template <int LA, int LB, int G, typename RT>
 __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
@@ -92,14 +104,7 @@ __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
 #pragma unroll
                 for (int t = 0; t < LA + LB + 1 + 2 * G; ++t) out[BE::at(d, i, j, t)] = static_cast<RT>(e[i][j][t]);
     }
-    for (int ib = threadIdx.x; ib < st.nbp; ib += blockDim.x) {
-        const double* b = st.rec + (size_t)ib * PPW;
-        RT* o = st.SB + (size_t)ib * SBW;
-        const double p = b[0] + b[1];
-        const double vals[SBW] = {p, 1.0 / p, b[3], b[4], b[5], b[0], b[1], 0.0, b[12], b[13], b[14], b[15]};
-#pragma unroll
-        for (int i = 0; i < SBW; ++i) o[i] = static_cast<RT>(vals[i]);
-    }
+    stage_bra_scalars(st);
 }
 
 // One primitive-pair record of a ket pair (16 doubles, 128-byte aligned),
@@ -867,6 +872,134 @@ __device__ __forceinline__ void ket_items(int nper, int j0, int64_t cnt, Queue& 
     }
 }
 
+// ---- Flat items
+// The column items of one chunk, over all segments of its ket class, are one
+// list: item i belongs to the segment sub with pre[sub] <= i < pre[sub + 1],
+// and within it to ket pair (i - pre[sub]) % cnt[sub] (column-major:
+// neighbouring lanes take the same column of different ket pairs, so that the
+// column's box conditions are warp-uniform). Threads walk the list with stride
+// blockDim.x and meet no barrier on the way. One list per segment, with a
+// barrier after each, left threads idle: at (H2O)32 a bra pair has some 50 ket
+// pairs in a segment, and 128 threads share them.
+// Where ket pairs are tested (difference builds, gradients), the list runs
+// over the pairs that passed, queued LQ_CAP at a time.
+constexpr int LQ_CAP = 1024;
+template <typename T>
+__device__ __forceinline__ T warp_incl(T v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const T u = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += u;
+    }
+    return v;
+}
+struct FlatItems {
+    int64_t pre[NSUB + 1];      // items before each segment of the class (of the queued pairs)
+    int cnt[NSUB];              // ket pairs of the chunk's window in each segment (of the queued ones)
+    int j0[NSUB];               // sorted position (queue slot) of the first of them
+    int kcnt[NSUB], kj0[NSUB];  // the whole window: pairs and first sorted position
+    int kpre[NSUB + 1];         // pairs before each segment
+    int nper[NSUB];             // items per ket pair
+    int wsum[32];
+};
+
+// The window of chunk j of nch of bra position spos (warp 0 calls it, one lane
+// per segment): kcnt, kj0, kpre, nper, and the item list over the whole window.
+template <int CX, int CY, typename RT>
+__device__ __forceinline__ void plan_window(const QuartetArgs& q, int spos, int nbp, int j, int nch, int ncols,
+                                            int nkg, int nsp, FlatItems& f) {
+    const int sub = threadIdx.x & 31;
+    int64_t kb = 0, len = 0, wk = 1;
+    if (sub < NSUB) {
+        int64_t ke;
+        ket_range<RT>(q, CY * NSUB + sub, spos, kb, ke);
+        len = ke > kb ? ke - kb : 0;
+        wk = ket_work<CX, CY>(sub) * nbp;
+    }
+    const int64_t incl = warp_incl(len * wk), W = __shfl_sync(0xffffffffu, incl, 31);
+    int64_t k0 = 0, k1 = 0;
+    if (len > 0)
+        window_kets(chunk_edge(W, j, nch), chunk_edge(W, j + 1, nch), incl - len * wk, wk, len, k0, k1);
+    const int cnt = k1 > k0 ? static_cast<int>(k1 - k0) : 0;
+    const int nper = ncols * nkg * nsp;
+    const int kincl = warp_incl(cnt);
+    const int64_t iincl = warp_incl(static_cast<int64_t>(cnt) * nper);
+    if (sub < NSUB) {
+        f.cnt[sub] = f.kcnt[sub] = cnt;
+        f.j0[sub] = f.kj0[sub] = q.seg_start[CY * NSUB + sub] + static_cast<int>(kb + k0);
+        f.nper[sub] = nper;
+        f.kpre[sub + 1] = kincl;
+        f.pre[sub + 1] = iincl;
+    }
+    if (sub == 0) {
+        f.kpre[0] = 0;
+        f.pre[0] = 0;
+    }
+}
+
+// Every item of the window: work(sub, pos, r) with pos the ket's sorted
+// position and r < nper[sub]. QUEUED: only the ket pairs that pass keep(pos)
+// (kept in order, so that items, threads and partial sums are the same on
+// every run); queue holds LQ_CAP ints. All threads of the CTA call this.
+template <typename Keep, typename Work>
+__device__ __forceinline__ void flat_items(FlatItems& f, bool queued, int* queue, Keep keep, Work work) {
+    constexpr int PER = LQ_CAP / 128;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int total = f.kpre[NSUB];
+    for (int base = 0; base < total; base += queued ? LQ_CAP : total) {
+        if (queued) {
+            if (threadIdx.x < NSUB) f.cnt[threadIdx.x] = 0;
+            // PER consecutive pairs a thread
+            unsigned mask = 0;
+            int s = 0, pos[PER];
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const int i = base + static_cast<int>(threadIdx.x) * PER + k;
+                if (i >= total) continue;
+                while (i >= f.kpre[s + 1]) ++s;
+                pos[k] = f.kj0[s] + i - f.kpre[s];
+                if (keep(pos[k])) mask |= 1u << k;
+            }
+            const int c = __popc(mask), incl = warp_incl(c);
+            if (lane == 31) f.wsum[warp] = incl;
+            __syncthreads();
+            int slot = incl - c;
+            for (int w = 0; w < warp; ++w) slot += f.wsum[w];
+            s = 0;
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                const int i = base + static_cast<int>(threadIdx.x) * PER + k;
+                if (!(mask >> k & 1u)) continue;
+                while (i >= f.kpre[s + 1]) ++s;
+                queue[slot++] = pos[k];
+                atomicAdd(&f.cnt[s], 1);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const int n = lane < NSUB ? f.cnt[lane] : 0;
+                const int ni = warp_incl(n);
+                const int64_t ii = warp_incl(static_cast<int64_t>(n) * (lane < NSUB ? f.nper[lane] : 0));
+                if (lane < NSUB) {
+                    f.j0[lane] = ni - n;
+                    f.pre[lane + 1] = ii;
+                }
+            }
+            __syncthreads();
+        }
+        const int64_t items = f.pre[NSUB];
+        int s = 0;
+        for (int64_t it = threadIdx.x; it < items; it += blockDim.x) {
+            while (it >= f.pre[s + 1]) ++s;
+            const unsigned loc = static_cast<unsigned>(it - f.pre[s]), nq = f.cnt[s];
+            const unsigned r = loc / nq;
+            const int at = f.j0[s] + static_cast<int>(loc - r * nq);
+            work(s, queued ? queue[at] : at, static_cast<int>(r));
+        }
+        if (queued) __syncthreads();
+    }
+}
+
 // ---- Two-stage items: R_tuv staged in shared memory
 // A ket pair of class Y carries NCD Cartesian columns (x contraction
 // groups), each one work item; R_tuv of a primitive quartet is the same for
@@ -897,6 +1030,20 @@ struct KetQueueR {
     int pq[KQ_CAP + 1];     // exclusive prefix of primitive quartets over the chunk's entries
     int sc[KQ_CAP];         // sub-chunk of each entry
     int n;
+};
+
+// The queue a kernel needs: of the two-stage items, or of the flat ones.
+template <bool TWO>
+struct QueueOf {
+    KetQueueR q;
+    __device__ KetQueueR* r() { return &q; }
+    __device__ int* flat() { return nullptr; }
+};
+template <>
+struct QueueOf<false> {
+    int q[LQ_CAP];
+    __device__ KetQueueR* r() { return nullptr; }
+    __device__ int* flat() { return q; }
 };
 
 // first index in [lo, hi) with a[i] >= key (a non-decreasing)

@@ -8,11 +8,27 @@
 //
 //   Gamma_{mnls} = deg [Dc_mn Dc_ls - k/2 sum_x (Dx_ml Dx_ns + Dx_ms Dx_nl)],
 //   deg = 1/2 x (2 if A != B) x (2 if C != D) x (2 if P1 != P2)
-// (aimd/qc/integrals.py:1298-1328). Centres A and B: shifted bra Hermite
-// expansions d/dA_x -> 2a E^{i+1,j} - i E^{i-1,j} with R up to L + 1 (the
-// reference's _grad_pass, :1049-1244). Centre C: the same identity on the
-// ket expansion, contracted with the bra-transformed Gamma. Centre D:
-// translational invariance, -(A + B + C), per column.
+// (aimd/qc/integrals.py:1298-1328).
+//
+// A primitive quartet's part of the energy is
+//   sum_{h,k} Y_h e_k (-1)^|k| R_{h+k}(P - Q),
+// with Y the bra's Hermite expansion contracted with Gamma and e the column's
+// ket expansion. The centres enter through P and Q, where d/dP_x raises h by
+// one (and d/dQ = -d/dP), and through the expansions, which depend on
+// X_AB = A - B and X_CD = C - D alone:
+//   G = sum Y_h e_k (-1)^|k| R_{h+k+1},  U, V = the same sum with dY/dX_AB, de/dX_CD
+//   dA = (a/p) G + U,  dB = (b/p) G - U,  dC = -(c/q) G + V,  dD = -(d/q) G - V
+// (D from translational invariance, -(A + B + C), per column). So one sum over
+// the column's box, X_h = sum_k e_k (-1)^|k| R_{h+k} to |h| = LAB + 1, gives
+// G = sum Y_h X_{h+1} and U = sum (dY)_h X_h, and Z_k = sum_h Y_h R_{h+k}, from
+// the same R values, gives V. The reference (and an earlier form of this file)
+// instead raises and lowers each Gaussian, 2a E^{i+1} - i E^{i-1}, with every
+// bra row's box widened by one in each direction (aimd/qc/integrals.py:
+// 1049-1244): for pp|pp some 900 multiply-adds a primitive quartet and column
+// in that step, against 180 here, and ten times the code: the kernels of a
+// small molecule are bound by fetching each instruction once. One B200, raised
+// form -> this one: methanol 6-31G** 16.4 -> 1.67 ms, (H2O)8 cc-pVDZ 73.1 ->
+// 10.2 ms, (H2O)32 1095 -> 178 ms.
 #pragma once
 #include "hf_eri.cuh"
 
@@ -43,7 +59,7 @@ template <int CX, int CY>
 constexpr bool grad_rsmem() { return QClass<CX, CY>::RSMEM; }
 
 // The other classes keep each thread's R_tuv (to L + 1) in a shared-memory
-// column while its passes run, where the columns of the CTA take at most
+// column while the box pass runs, where the columns of the CTA take at most
 // 96 KB (two CTAs per SM): R to L + 1 is the largest array of the
 // gradient body, and in registers it pushes the body into local memory.
 template <int CX, int CY, typename RT>
@@ -51,82 +67,54 @@ constexpr bool grad_rcol() {
     return !grad_rsmem<CX, CY>() && nherm(QClass<CX, CY>::L + 1) * sizeof(RT) * GRAD_THREADS <= 96 * 1024;
 }
 
-// Bra derivative coefficients of one primitive pair, per direction d:
-//   k = 0 (centre A): 2a E^{i+1,j}_t - i E^{i-1,j}_t
-//   k = 1 (centre B): 2b E^{i,j+1}_t - j E^{i,j-1}_t
-// for i <= LA, j <= LB, t <= LA + LB + 1, staged once per CTA so that the
-// per-column derivative pass reads one value instead of building it.
-template <int LA, int LB>
-struct BraD {
-    static constexpr int I = LA + 1, J = LB + 1, T = LA + LB + 2;
-    static constexpr int SIZE = 2 * 3 * I * J * T;
-    __device__ static int at(int k, int d, int i, int j, int t) { return (((k * 3 + d) * I + i) * J + j) * T + t; }
-};
-
+// E and dE/dX_AB of one bra pair's primitives, in the same layout (st.E, st.D).
 template <int LA, int LB, typename RT>
-__device__ __forceinline__ void stage_bra_d(const BraStageT<RT>& st) {
-    using BE = BraE<LA, LB, 1>;
-    using BD = BraD<LA, LB>;
-    for (int w = threadIdx.x; w < st.nbp * BD::SIZE; w += blockDim.x) {
-        const int ib = w / BD::SIZE, r = w % BD::SIZE;
-        const int t = r % BD::T, j = (r / BD::T) % BD::J, i = (r / (BD::T * BD::J)) % BD::I;
-        const int d = (r / (BD::T * BD::J * BD::I)) % 3, k = r / (BD::T * BD::J * BD::I * 3);
-        const RT* E = st.E + (size_t)ib * BE::SIZE;
-        const RT* sb = st.SB + (size_t)ib * SBW;
-        RT v;
-        if (k == 0) v = RT(2) * sb[5] * E[BE::at(d, i + 1, j, t)] - (i > 0 ? i * E[BE::at(d, i - 1, j, t)] : RT(0));
-        else v = RT(2) * sb[6] * E[BE::at(d, i, j + 1, t)] - (j > 0 ? j * E[BE::at(d, i, j - 1, t)] : RT(0));
-        st.D[(size_t)ib * BD::SIZE + r] = v;
-    }
-}
-
-// For runtime (i, j): row[t] = E^{ij}_t and drow[t] = 2c E^{i+1,j}_t - i E^{i-1,j}_t
-// (the d/dC_x expansion), selected by predicated copies.
-template <int LC, int LD, typename RT>
-__device__ __forceinline__ void ket_deriv_rows(const RT (&e)[LC + 2][LD + 1][LC + LD + 2], int i, int j, RT c,
-                                               RT (&row)[LC + LD + 2], RT (&drow)[LC + LD + 2]) {
+__device__ __forceinline__ void stage_bra_de(const BraStageT<RT>& st) {
+    using BE = BraE<LA, LB, 0>;
+    for (int w = threadIdx.x; w < st.nbp * 3; w += blockDim.x) {
+        const int ib = w / 3, d = w % 3;
+        const double* b = st.rec + (size_t)ib * PPW;
+        const double ip = 1.0 / (b[0] + b[1]), pa = b[6 + d], pb = b[9 + d];
+        double e[LA + 1][LB + 1][LA + LB + 1], de[LA + 1][LB + 1][LA + LB + 1];
+        hermite_e<LA, LB>(pa, pb, 0.5 * ip, d == 0 ? b[2] : 1.0, e);
+        hermite_de<LA, LB>(pa, pb, 0.5 * ip, b[1] * ip, b[0] * ip, 2.0 * b[0] * b[1] * ip * (pb - pa), e, de);
+        // exp(-mu |A - B|^2) is in the x table; the y and z tables carry their
+        // own derivative of it through de[0][0][0]
+        RT* out = st.E + (size_t)ib * BE::SIZE;
+        RT* dout = st.D + (size_t)ib * BE::SIZE;
 #pragma unroll
-    for (int t = 0; t <= LC + LD + 1; ++t) row[t] = drow[t] = RT(0);
+        for (int i = 0; i <= LA; ++i)
 #pragma unroll
-    for (int ii = 0; ii <= LC; ++ii)
+            for (int j = 0; j <= LB; ++j)
 #pragma unroll
-        for (int jj = 0; jj <= LD; ++jj)
-            if (ii == i && jj == j)
-#pragma unroll
-                for (int t = 0; t <= LC + LD + 1; ++t) {
-                    row[t] = t <= LC + LD ? e[ii][jj][t] : RT(0);
-                    drow[t] = RT(2) * c * e[ii + 1][jj][t] - (ii > 0 ? ii * e[ii > 0 ? ii - 1 : 0][jj][t] : RT(0));
+                for (int t = 0; t <= LA + LB; ++t) {
+                    out[BE::at(d, i, j, t)] = static_cast<RT>(e[i][j][t]);
+                    dout[BE::at(d, i, j, t)] = static_cast<RT>(de[i][j][t]);
                 }
+    }
+    stage_bra_scalars(st);
 }
 
-// Primitive loops of one gradient column with the bra-side work hoisted out
-// of the ket primitives: bra primitives outer; per bra primitive the
-// C-pass weights Y[kk]_h = sum_ab f_ab C_ab Gamma[ab][kk] E^{ab}_h (bra
-// only) are formed once, the ket primitives inner accumulate the ket step
-// Xs[kk]_h = sum_ik c_ik[kk] pref sum_box(cd) (-1)^|k| E^{cd}_k R_{h+k}
-// (h to LAB + 1) and the C pass, and the bra pass for centres A and B runs
-// once per bra primitive on Xs (it is linear in the ket step). Same sums as
-// the per-primitive-quartet order, regrouped.
+// Primitive loops of one gradient column (bra primitives [ib0, ib1)): bra
+// primitives outer, so that Y (the bra's E contracted with the Gamma column)
+// and the U sum, linear in X, are formed once per bra primitive.
 template <int CX, int CY, typename RT, bool RS>
-__device__ __forceinline__ void grad_prims_hoisted(const BraStageT<RT>& st, const RT (&Gr)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                   const double* __restrict__ rk, int nkp, int ic, int id, int kg,
-                                                   RT (&dA)[3], RT (&dB)[3], RT (&dC)[3], const RT* __restrict__ Rs,
-                                                   RT* Rcol, int ib0, int ib1) {
+__device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&Gr)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
+                                           const double* __restrict__ rk, int nkp, int ic, int id, int kg,
+                                           RT (&dA)[3], RT (&dB)[3], RT (&dC)[3], const RT* __restrict__ Rs,
+                                           RT* Rcol, int ib0, int ib1) {
     using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 1>;
-    using BD = BraD<Q::LA, Q::LB>;
+    using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L + 1;
-    constexpr int NH1 = nherm(LAB + 1);
+    constexpr int NHB = Q::NHB, NH1 = nherm(LAB + 1);
     constexpr int KG = Q::KG;
-    constexpr int UH = L >= 4 ? 1 : 16;     // rolled Hermite loops: smaller code (instruction fetch)
-    constexpr int UW = L >= 5 ? 1 : 16;
     const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
     const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
     const RT fcd = cart_norm(cx, cy, cz) * cart_norm(dx, dy, dz);
     for (int ib = ib0; ib < ib1; ++ib) {
         const RT* sb = st.SB + ib * SBW;
         const RT* E = st.E + (size_t)ib * BE::SIZE;
-        const RT* Db = st.D + (size_t)ib * BD::SIZE;
+        const RT* DE = st.D + (size_t)ib * BE::SIZE;
         // Gamma of row ab contracted with this bra primitive's coefficients and f_ab
         auto gq = [&](int ia, int jb, int kk) {
             const RT fab = cart_norm(cart_x(LA, ia), cart_y(LA, ia), cart_z(LA, ia)) *
@@ -136,127 +124,142 @@ __device__ __forceinline__ void grad_prims_hoisted(const BraStageT<RT>& st, cons
             for (int kab = 0; kab < Q::KAB; ++kab) s += sb[8 + kab] * Gr[kab * Q::NAB + ia * Q::NB + jb][kk];
             return s * fab;
         };
-        RT Y[KG][Q::NHB];
+        RT Y[KG][NHB], Xs[KG][NHB];
 #pragma unroll
         for (int kk = 0; kk < KG; ++kk)
 #pragma unroll
-            for (int h = 0; h < Q::NHB; ++h) Y[kk][h] = RT(0);
-#pragma unroll UH
-        for (int ia = 0; ia < Q::NA; ++ia) {
-            const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
+            for (int h = 0; h < NHB; ++h) Y[kk][h] = Xs[kk][h] = RT(0);
+        // one direction at a time, as bra_rows: per (az, bz) the x and y
+        // factors into W, then the z factor
 #pragma unroll
-            for (int jb = 0; jb < Q::NB; ++jb) {
-                const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                RT g[KG];
+        for (int az = 0; az <= LA; ++az)
 #pragma unroll
-                for (int kk = 0; kk < KG; ++kk) g[kk] = gq(ia, jb, kk);
+            for (int bz = 0; bz <= LB; ++bz) {
+                RT W[KG][ncart(LAB)];
 #pragma unroll
-                for (int t = 0; t <= ax + bx; ++t)
+                for (int kk = 0; kk < KG; ++kk)
 #pragma unroll
-                    for (int u = 0; u <= ay + by; ++u) {
-                        const RT e01 = E[BE::at(0, ax, bx, t)] * E[BE::at(1, ay, by, u)];
+                    for (int i = 0; i < ncart(LAB); ++i) W[kk][i] = RT(0);
 #pragma unroll
-                        for (int w = 0; w <= az + bz; ++w) {
-                            const RT e = e01 * E[BE::at(2, az, bz, w)];
+                for (int ay = 0; ay <= LA - az; ++ay)
 #pragma unroll
-                            for (int kk = 0; kk < KG; ++kk) Y[kk][hidx(t, u, w)] += g[kk] * e;
+                    for (int by = 0; by <= LB - bz; ++by) {
+                        const int ax = LA - az - ay, bx = LB - bz - by;
+#pragma unroll
+                        for (int kk = 0; kk < KG; ++kk) {
+                            const RT g = gq(cart_index(ay, az), cart_index(by, bz), kk);
+#pragma unroll
+                            for (int t = 0; t <= ax + bx; ++t) {
+                                const RT ge = g * E[BE::at(0, ax, bx, t)];
+#pragma unroll
+                                for (int u = 0; u <= ay + by; ++u)
+                                    W[kk][cart_index(t, u)] += ge * E[BE::at(1, ay, by, u)];
+                            }
                         }
                     }
+#pragma unroll
+                for (int t = 0; t <= LAB - az - bz; ++t)
+#pragma unroll
+                    for (int u = 0; u <= LAB - az - bz - t; ++u)
+#pragma unroll
+                        for (int w = 0; w <= az + bz; ++w)
+#pragma unroll
+                            for (int kk = 0; kk < KG; ++kk)
+                                Y[kk][hidx(t, u, w)] += E[BE::at(2, az, bz, w)] * W[kk][cart_index(t, u)];
             }
-        }
-        RT Xs[KG][NH1];
-#pragma unroll
-        for (int kk = 0; kk < KG; ++kk)
-#pragma unroll
-            for (int h = 0; h < NH1; ++h) Xs[kk][h] = RT(0);
+        RT gG[3] = {RT(0), RT(0), RT(0)};       // G summed over the ket primitives
         for (int ik = 0; ik < nkp; ++ik) {
             const KetRecT<RT> k = load_ket<RT>(rk + (size_t)ik * PPW);
-            const RT ec = k.a, q = ec + k.b, oo2q = RT(0.5) / q;
-            RT ex[LCD + 2], ey[LCD + 2], ez[LCD + 2], gx[LCD + 2], gy[LCD + 2], gz[LCD + 2];
+            const RT q = k.a + k.b, iq = RT(1) / q, oo2q = RT(0.5) * iq, cq = k.a * iq, dq = k.b * iq;
+            RT ex[LCD + 1], ey[LCD + 1], ez[LCD + 1], fx[LCD + 1], fy[LCD + 1], fz[LCD + 1];
             {
-                RT e[LC + 2][LD + 1][LCD + 2];
-                hermite_e<LC + 1, LD>(k.QAx, k.QBx, oo2q, k.K, e);
-                ket_deriv_rows<LC, LD>(e, cx, dx, ec, ex, gx);
-                hermite_e<LC + 1, LD>(k.QAy, k.QBy, oo2q, RT(1), e);
-                ket_deriv_rows<LC, LD>(e, cy, dy, ec, ey, gy);
-                hermite_e<LC + 1, LD>(k.QAz, k.QBz, oo2q, RT(1), e);
-                ket_deriv_rows<LC, LD>(e, cz, dz, ec, ez, gz);
-            }
-            RT ck[KG];
-#pragma unroll
-            for (int i = 0; i < KG; ++i) {
-                RT c = k.c[0];
-#pragma unroll
-                for (int j = 1; j < Q::KCD; ++j)
-                    if (j == kg * KG + i) c = k.c[j];
-                ck[i] = c * fcd;
+                RT e[LC + 1][LD + 1][LCD + 1], de[LC + 1][LD + 1][LCD + 1];
+                const RT m2 = RT(2) * k.a * dq;
+                hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, k.K, e);
+                hermite_de<LC, LD>(k.QAx, k.QBx, oo2q, dq, cq, m2 * (k.QBx - k.QAx), e, de);
+                select_row<LC, LD, LCD>(e, cx, dx, ex);
+                select_row<LC, LD, LCD>(de, cx, dx, fx);
+                hermite_e<LC, LD>(k.QAy, k.QBy, oo2q, RT(1), e);
+                hermite_de<LC, LD>(k.QAy, k.QBy, oo2q, dq, cq, m2 * (k.QBy - k.QAy), e, de);
+                select_row<LC, LD, LCD>(e, cy, dy, ey);
+                select_row<LC, LD, LCD>(de, cy, dy, fy);
+                hermite_e<LC, LD>(k.QAz, k.QBz, oo2q, RT(1), e);
+                hermite_de<LC, LD>(k.QAz, k.QBz, oo2q, dq, cq, m2 * (k.QBz - k.QAz), e, de);
+                select_row<LC, LD, LCD>(e, cz, dz, ez);
+                select_row<LC, LD, LCD>(de, cz, dz, fz);
             }
             auto body = [&](const auto& R, RT scale) {
-                RT sc[KG];
+                RT sc[KG], Yc[NHB];
 #pragma unroll
-                for (int kk = 0; kk < KG; ++kk) sc[kk] = scale * ck[kk];
-                // ket step for the bra pass, accumulated over the ket primitives
-#pragma unroll UH
-                for (int t = 0; t <= LAB + 1; ++t)
-#pragma unroll UH
-                    for (int u = 0; u <= LAB + 1 - t; ++u)
-#pragma unroll UW
-                        for (int w = 0; w <= LAB + 1 - t - u; ++w) {
-                            RT s = RT(0);
+                for (int i = 0; i < KG; ++i) {
+                    RT c = k.c[0];
 #pragma unroll
-                            for (int t2 = 0; t2 <= LCD; ++t2) {
-                                if (t2 > cx + dx) continue;
+                    for (int j = 1; j < Q::KCD; ++j)
+                        if (j == kg * KG + i) c = k.c[j];
+                    sc[i] = c * fcd * scale;
+                }
 #pragma unroll
-                                for (int u2 = 0; u2 <= LCD; ++u2) {
-                                    if (u2 > cy + dy) continue;
-                                    const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
+                for (int h = 0; h < NHB; ++h) {
+                    RT s = RT(0);
 #pragma unroll
-                                    for (int v2 = 0; v2 <= LCD; ++v2) {
-                                        if (v2 > cz + dz) continue;
-                                        s += ((v2 & 1) ? -exy * ez[v2] : exy * ez[v2]) * R[hidx(t + t2, u + u2, w + v2)];
-                                    }
-                                }
-                            }
+                    for (int kk = 0; kk < KG; ++kk) s += sc[kk] * Y[kk][h];
+                    Yc[h] = s;
+                }
+                // one pass over the box: X_h and Z_k from the same R values
+                RT X[NH1], vx = RT(0), vy = RT(0), vz = RT(0);
 #pragma unroll
-                            for (int kk = 0; kk < KG; ++kk) Xs[kk][hidx(t, u, w)] += sc[kk] * s;
-                        }
-                // C pass: dC_d += sum_k dE^{cd}_{d,k} Z_k with Z_k = (-1)^|k| sum_h Y_h R_{h+k},
-                // k over the ket box widened by one in at most one direction
-                // (the rows are zero beyond their box): Z is shared by the
-                // three directions
+                for (int h = 0; h < NH1; ++h) X[h] = RT(0);
 #pragma unroll
-                for (int t2 = 0; t2 <= LCD + 1; ++t2) {
-                    if (t2 > cx + dx + 1) continue;
+                for (int t2 = 0; t2 <= LCD; ++t2) {
+                    if (t2 > cx + dx) continue;
 #pragma unroll
-                    for (int u2 = 0; u2 <= LCD + 1; ++u2) {
-                        if (u2 > cy + dy + 1) continue;
+                    for (int u2 = 0; u2 <= LCD - t2; ++u2) {
+                        if (u2 > cy + dy) continue;
+                        const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
+                        const RT fxy = ((t2 + u2) & 1) ? -fx[t2] * ey[u2] : fx[t2] * ey[u2];
+                        const RT exf = ((t2 + u2) & 1) ? -ex[t2] * fy[u2] : ex[t2] * fy[u2];
 #pragma unroll
-                        for (int v2 = 0; v2 <= LCD + 1; ++v2) {
-                            if (v2 > cz + dz + 1) continue;
-                            if ((t2 > cx + dx) + (u2 > cy + dy) + (v2 > cz + dz) > 1) continue;
-                            RT z[KG];
+                        for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
+                            if (v2 > cz + dz) continue;
+                            const RT s = (v2 & 1) ? -ez[v2] : ez[v2];
+                            const RT e = exy * s;
+                            RT z = RT(0);
 #pragma unroll
-                            for (int kk = 0; kk < KG; ++kk) z[kk] = RT(0);
-#pragma unroll UH
-                            for (int t = 0; t <= LAB; ++t)
-#pragma unroll UH
-                                for (int u = 0; u <= LAB - t; ++u)
-#pragma unroll UW
-                                    for (int w = 0; w <= LAB - t - u; ++w) {
+                            for (int t = 0; t <= LAB + 1; ++t)
+#pragma unroll
+                                for (int u = 0; u <= LAB + 1 - t; ++u)
+#pragma unroll
+                                    for (int w = 0; w <= LAB + 1 - t - u; ++w) {
                                         const RT r = R[hidx(t + t2, u + u2, w + v2)];
-#pragma unroll
-                                        for (int kk = 0; kk < KG; ++kk) z[kk] += Y[kk][hidx(t, u, w)] * r;
+                                        X[hidx(t, u, w)] += e * r;
+                                        if (t + u + w <= LAB) z += Yc[hidx(t, u, w)] * r;
                                     }
-                            RT zs = RT(0);
-#pragma unroll
-                            for (int kk = 0; kk < KG; ++kk) zs += sc[kk] * z[kk];
-                            if ((t2 + u2 + v2) & 1) zs = -zs;
-                            dC[0] += gx[t2] * ey[u2] * ez[v2] * zs;
-                            dC[1] += ex[t2] * gy[u2] * ez[v2] * zs;
-                            dC[2] += ex[t2] * ey[u2] * gz[v2] * zs;
+                            vx += fxy * s * z;
+                            vy += exf * s * z;
+                            vz += ((v2 & 1) ? -exy : exy) * fz[v2] * z;
                         }
                     }
                 }
+                RT gx = RT(0), gy = RT(0), gz = RT(0);
+#pragma unroll
+                for (int t = 0; t <= LAB; ++t)
+#pragma unroll
+                    for (int u = 0; u <= LAB - t; ++u)
+#pragma unroll
+                        for (int w = 0; w <= LAB - t - u; ++w) {
+                            const RT y = Yc[hidx(t, u, w)];
+                            gx += y * X[hidx(t + 1, u, w)];
+                            gy += y * X[hidx(t, u + 1, w)];
+                            gz += y * X[hidx(t, u, w + 1)];
+#pragma unroll
+                            for (int kk = 0; kk < KG; ++kk) Xs[kk][hidx(t, u, w)] += sc[kk] * X[hidx(t, u, w)];
+                        }
+                gG[0] += gx;
+                gG[1] += gy;
+                gG[2] += gz;
+                dC[0] += vx - cq * gx;
+                dC[1] += vy - cq * gy;
+                dC[2] += vz - cq * gz;
             };
             if constexpr (RS) {
                 body(Rs + (size_t)(ik * st.nbp + ib) * nherm(L), RT(1));
@@ -264,216 +267,83 @@ __device__ __forceinline__ void grad_prims_hoisted(const BraStageT<RT>& st, cons
                 const RT p = sb[0];
                 const RT rs = rsqrt_t(p + q);
                 const RT alpha = p * q * rs * rs;
-                const RT pref = RT(TWO_PI_2_5) * sb[1] * (RT(2) * oo2q) * rs;
+                const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
                 RT R[nherm(L)];
+                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
                 if constexpr (grad_rcol<CX, CY, RT>()) {
-                    hermite_r_scaled<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, pref, R);
 #pragma unroll
                     for (int i = 0; i < nherm(L); ++i) Rcol[i * GRAD_THREADS] = R[i];
-                    body(RColumn<RT, GRAD_THREADS>{Rcol}, RT(1));
+                    body(RColumn<RT, GRAD_THREADS>{Rcol}, pref);
                 } else {
-                    hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
                     body(R, pref);
                 }
             }
         }
-        // bra pass (A, B) on the summed ket step, once per bra primitive
-#pragma unroll UH
-        for (int ia = 0; ia < Q::NA; ++ia) {
-            const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
+        // U on the summed X, once per bra primitive
+        RT ux = RT(0), uy = RT(0), uz = RT(0);
 #pragma unroll
-            for (int jb = 0; jb < Q::NB; ++jb) {
-                const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                RT g[KG];
+        for (int az = 0; az <= LA; ++az)
 #pragma unroll
-                for (int kk = 0; kk < KG; ++kk) g[kk] = gq(ia, jb, kk);
+            for (int bz = 0; bz <= LB; ++bz) {
+                RT W[KG][ncart(LAB)], Wz[KG][ncart(LAB)];       // E_z and dE_z applied
 #pragma unroll
-                for (int t = 0; t <= ax + bx + 1; ++t)
+                for (int t = 0; t <= LAB - az - bz; ++t)
 #pragma unroll
-                    for (int u = 0; u <= ay + by + 1; ++u)
+                    for (int u = 0; u <= LAB - az - bz - t; ++u)
 #pragma unroll
-                        for (int w = 0; w <= az + bz + 1; ++w) {
-                            const int over = (t > ax + bx) + (u > ay + by) + (w > az + bz);
-                            if (over > 1) continue;
-                            RT yv = RT(0);
+                        for (int kk = 0; kk < KG; ++kk) {
+                            RT s = RT(0), sz = RT(0);
 #pragma unroll
-                            for (int kk = 0; kk < KG; ++kk) yv += g[kk] * Xs[kk][hidx(t, u, w)];
-                            const RT e0 = E[BE::at(0, ax, bx, t)], e1 = E[BE::at(1, ay, by, u)],
-                                     e2 = E[BE::at(2, az, bz, w)];
-                            const RT y12 = yv * e1 * e2, y02 = yv * e0 * e2, y01 = yv * e0 * e1;
-                            dA[0] += y12 * Db[BD::at(0, 0, ax, bx, t)];
-                            dA[1] += y02 * Db[BD::at(0, 1, ay, by, u)];
-                            dA[2] += y01 * Db[BD::at(0, 2, az, bz, w)];
-                            dB[0] += y12 * Db[BD::at(1, 0, ax, bx, t)];
-                            dB[1] += y02 * Db[BD::at(1, 1, ay, by, u)];
-                            dB[2] += y01 * Db[BD::at(1, 2, az, bz, w)];
+                            for (int w = 0; w <= az + bz; ++w) {
+                                s += E[BE::at(2, az, bz, w)] * Xs[kk][hidx(t, u, w)];
+                                sz += DE[BE::at(2, az, bz, w)] * Xs[kk][hidx(t, u, w)];
+                            }
+                            W[kk][cart_index(t, u)] = s;
+                            Wz[kk][cart_index(t, u)] = sz;
                         }
+#pragma unroll
+                for (int ay = 0; ay <= LA - az; ++ay)
+#pragma unroll
+                    for (int by = 0; by <= LB - bz; ++by) {
+                        const int ax = LA - az - ay, bx = LB - bz - by;
+#pragma unroll
+                        for (int kk = 0; kk < KG; ++kk) {
+                            const RT g = gq(cart_index(ay, az), cart_index(by, bz), kk);
+#pragma unroll
+                            for (int t = 0; t <= ax + bx; ++t) {
+                                RT s = RT(0), sy = RT(0), sz = RT(0);
+#pragma unroll
+                                for (int u = 0; u <= ay + by; ++u) {
+                                    s += E[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
+                                    sy += DE[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
+                                    sz += E[BE::at(1, ay, by, u)] * Wz[kk][cart_index(t, u)];
+                                }
+                                const RT ge = g * E[BE::at(0, ax, bx, t)];
+                                ux += g * DE[BE::at(0, ax, bx, t)] * s;
+                                uy += ge * sy;
+                                uz += ge * sz;
+                            }
+                        }
+                    }
             }
-        }
+        const RT ap = sb[5] * sb[1], bp = sb[6] * sb[1];
+        dA[0] += ap * gG[0] + ux;
+        dA[1] += ap * gG[1] + uy;
+        dA[2] += ap * gG[2] + uz;
+        dB[0] += bp * gG[0] - ux;
+        dB[1] += bp * gG[1] - uy;
+        dB[2] += bp * gG[2] - uz;
     }
 }
 
-// The hoisted order for the d-shell bra classes, where its register
-// footprint (Gamma column, Y and the summed ket step per contraction group)
-// fits (up to the 127 doubles of the dd bras, whose pairs have one bra
-// primitive, so the bra pass runs once per column instead of once per ket
-// primitive); the per-primitive-quartet order for the others (measured:
-// hoisting the s/p bras, whose pairs have many primitives, was no faster).
-template <int CX, int CY, typename RT>
-constexpr bool grad_hoist() {
-    using Q = QClass<CX, CY>;
-    // d-shell bras only (few bra primitives; see eri_column)
-    return CX >= 3 && sizeof(RT) * (Q::NROW * Q::KG + Q::KG * (Q::NHB + nherm(Q::LAB + 1))) <= 1100;
-}
-
-// One primitive quartet (bra primitive sb/E/Db, ket primitive through its
-// column rows ex.. and derivative rows gx..) of one gradient column:
-// adds the A, B and C derivative parts. Everything is linear in pref * R.
-template <int CX, int CY, typename RT, typename RArr>
-__device__ __forceinline__ void grad_pq(const RT* sb, const RT* E, const RT* Db,
-                                        const RT (&Gr)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                        const RT (&ck)[QClass<CX, CY>::KG], int cx, int cy, int cz, int dx, int dy,
-                                        int dz, const RT (&ex)[QClass<CX, CY>::LCD + 2],
-                                        const RT (&ey)[QClass<CX, CY>::LCD + 2],
-                                        const RT (&ez)[QClass<CX, CY>::LCD + 2],
-                                        const RT (&gx)[QClass<CX, CY>::LCD + 2],
-                                        const RT (&gy)[QClass<CX, CY>::LCD + 2],
-                                        const RT (&gz)[QClass<CX, CY>::LCD + 2], const RArr& R, RT pref,
-                                        RT (&dA)[3], RT (&dB)[3], RT (&dC)[3]) {
-    using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 1>;
-    using BD = BraD<Q::LA, Q::LB>;
-    constexpr int LA = Q::LA, LB = Q::LB, LAB = Q::LAB, LCD = Q::LCD, L = Q::L + 1;
-    constexpr int NH1 = nherm(LAB + 1);
-    constexpr int UH = L >= 5 ? 1 : 16;      // rolled outer Hermite loops for large classes
-    constexpr int UW = L >= 7 ? 1 : 16;      // and the inner one for the largest (compile time)
-
-            // Gamma contracted with this bra primitive's coefficients and f_ab,
-            // then summed over the ket contractions: gq[ab] = sum_kk gb[ab][kk] ck[kk]
-            RT gq[Q::NAB];
-#pragma unroll
-            for (int ia = 0; ia < Q::NA; ++ia)
-#pragma unroll
-                for (int jb = 0; jb < Q::NB; ++jb) {
-                    const RT fab = cart_norm(cart_x(LA, ia), cart_y(LA, ia), cart_z(LA, ia)) *
-                                       cart_norm(cart_x(LB, jb), cart_y(LB, jb), cart_z(LB, jb));
-                    const int ab = ia * Q::NB + jb;
-                    RT s = 0.0;
-#pragma unroll
-                    for (int kab = 0; kab < Q::KAB; ++kab)
-#pragma unroll
-                        for (int kk = 0; kk < Q::KG; ++kk) s += sb[8 + kab] * Gr[kab * Q::NAB + ab][kk] * ck[kk];
-                    gq[ab] = s * fab * pref;
-                }
-            // bra pass (A, B): sum_ab gq[ab] sum_{h in dbox(ab)} dE_h Xb_h,
-            // Xb_h = sum_{k in box(cd)} (-1)^|k| E^{cd}_k R_{h+k}
-            RT Xb[NH1];
-#pragma unroll UH
-            for (int t = 0; t <= LAB + 1; ++t)
-#pragma unroll UH
-                for (int u = 0; u <= LAB + 1 - t; ++u)
-#pragma unroll UW
-                    for (int w = 0; w <= LAB + 1 - t - u; ++w) {
-                        RT s = 0.0;
-#pragma unroll
-                        for (int t2 = 0; t2 <= LCD; ++t2) {
-                            if (t2 > cx + dx) continue;
-#pragma unroll
-                            for (int u2 = 0; u2 <= LCD; ++u2) {
-                                if (u2 > cy + dy) continue;
-                                const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
-#pragma unroll
-                                for (int v2 = 0; v2 <= LCD; ++v2) {
-                                    if (v2 > cz + dz) continue;
-                                    s += ((v2 & 1) ? -exy * ez[v2] : exy * ez[v2]) * R[hidx(t + t2, u + u2, w + v2)];
-                                }
-                            }
-                        }
-                        Xb[hidx(t, u, w)] = s;
-                    }
-            // C pass: Y_h = sum_ab gq[ab] E^{ab}_h (h <= LAB), then
-            // dC_d += sum_h Y_h sum_k (-1)^|k| dE^{cd}_{d,k} R_{h+k} (in this
-            // order the per-direction form spills less than the Z form of
-            // the hoisted order)
-            RT Y[Q::NHB];
-#pragma unroll
-            for (int h = 0; h < Q::NHB; ++h) Y[h] = 0.0;
-#pragma unroll UH
-            for (int ia = 0; ia < Q::NA; ++ia) {
-                const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
-#pragma unroll
-                for (int jb = 0; jb < Q::NB; ++jb) {
-                    const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                    const RT g = gq[ia * Q::NB + jb];
-#pragma unroll
-                    for (int t = 0; t <= ax + bx + 1; ++t)
-#pragma unroll
-                        for (int u = 0; u <= ay + by + 1; ++u)
-#pragma unroll
-                            for (int w = 0; w <= az + bz + 1; ++w) {
-                                const int over = (t > ax + bx) + (u > ay + by) + (w > az + bz);
-                                if (over > 1) continue;
-                                const RT yv = g * Xb[hidx(t, u, w)];
-                                const RT e0 = E[BE::at(0, ax, bx, t)], e1 = E[BE::at(1, ay, by, u)],
-                                             e2 = E[BE::at(2, az, bz, w)];
-                                const RT e12 = e1 * e2, e02 = e0 * e2, e01 = e0 * e1;
-                                if (over == 0) Y[hidx(t, u, w)] += g * e01 * e2;
-                                const RT y12 = yv * e12, y02 = yv * e02, y01 = yv * e01;
-                                dA[0] += y12 * Db[BD::at(0, 0, ax, bx, t)];
-                                dA[1] += y02 * Db[BD::at(0, 1, ay, by, u)];
-                                dA[2] += y01 * Db[BD::at(0, 2, az, bz, w)];
-                                dB[0] += y12 * Db[BD::at(1, 0, ax, bx, t)];
-                                dB[1] += y02 * Db[BD::at(1, 1, ay, by, u)];
-                                dB[2] += y01 * Db[BD::at(1, 2, az, bz, w)];
-                            }
-                }
-            }
-#pragma unroll UH
-            for (int t = 0; t <= LAB; ++t)
-#pragma unroll UH
-                for (int u = 0; u <= LAB - t; ++u)
-#pragma unroll UW
-                    for (int w = 0; w <= LAB - t - u; ++w) {
-                        const RT yv = Y[hidx(t, u, w)];
-                        // one direction d at a time (one accumulator live)
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) {
-                            RT sd = 0.0;
-#pragma unroll
-                            for (int t2 = 0; t2 <= LCD + 1; ++t2) {
-                                if (t2 > cx + dx + (d == 0)) continue;
-#pragma unroll
-                                for (int u2 = 0; u2 <= LCD + 1; ++u2) {
-                                    if (u2 > cy + dy + (d == 1)) continue;
-                                    const RT fxy = (d == 0 ? gx[t2] : ex[t2]) * (d == 1 ? gy[u2] : ey[u2]);
-#pragma unroll
-                                    for (int v2 = 0; v2 <= LCD + 1; ++v2) {
-                                        if (v2 > cz + dz + (d == 2)) continue;
-                                        const RT r = ((t2 + u2 + v2) & 1) ? -R[hidx(t + t2, u + u2, w + v2)]
-                                                                              : R[hidx(t + t2, u + u2, w + v2)];
-                                        sd += fxy * (d == 2 ? gz[v2] : ez[v2]) * r;
-                                    }
-                                }
-                            }
-                            dC[d] += yv * sd;
-                        }
-                    }
-}
-
 // Gradient contribution of one column; adds A, B parts to gab and C, D
-// parts to the shared accumulator gsh[natm][3]. RS: pref * R_tuv (to L + 1)
+// parts to the shared accumulator gsh (low words [natm][3], then the high words). RS: pref * R_tuv (to L + 1)
 // of the ket pair's primitive quartets staged in Rs ([ik][ib][NH(L + 1)]).
 template <int CX, int CY, typename RT, bool RS = false>
 __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<RT>& st, int P2, double QQ, int ic,
-                                            int id, int kg, double (&gab)[6], facc* gsh,
+                                            int id, int kg, double (&gab)[6], unsigned* gsh,
                                             const RT* __restrict__ Rs, RT* Rcol, int ib0, int ib1) {
     using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 1>;
-    using BD = BraD<Q::LA, Q::LB>;
-    constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L + 1;
-    constexpr int NH1 = nherm(LAB + 1);
-    constexpr int UH = L >= 5 ? 1 : 16;      // rolled outer Hermite loops for large classes
-    constexpr int UW = L >= 7 ? 1 : 16;      // and the inner one for the largest (compile time)
     const BlockView& bv = a.q.bv;
     const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
     const int aC = bv.atom[C], aD = bv.atom[Dd];
@@ -517,75 +387,15 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
 #pragma unroll
         for (int kk = 0; kk < Q::KG; ++kk) Gr[r][kk] = static_cast<RT>(G[r][kk]);
     RT dA[3] = {0.0, 0.0, 0.0}, dB[3] = {0.0, 0.0, 0.0}, dC[3] = {0.0, 0.0, 0.0};
-    if constexpr (grad_hoist<CX, CY, RT>()) {
-        grad_prims_hoisted<CX, CY, RT, RS>(st, Gr, a.q.pv.rec + a.q.pv.slot[P2] * PPW, a.q.pv.npp[P2], ic, id, kg,
-                                           dA, dB, dC, Rs, Rcol, ib0, ib1);
-    } else {
-    const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
-    const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
-    const RT fcd = cart_norm(cx, cy, cz) * cart_norm(dx, dy, dz);
-    const double* rk = a.q.pv.rec + a.q.pv.slot[P2] * PPW;
-    const int nkp = a.q.pv.npp[P2];
-    for (int ik = 0; ik < nkp; ++ik) {
-        const KetRecT<RT> k = load_ket<RT>(rk + (size_t)ik * PPW);
-        const RT ec = k.a, q = ec + k.b, oo2q = RT(0.5) / q, iq = RT(2) * oo2q;
-        // ket E for this column, and d/dC_d of it (one extra in direction d)
-        RT ex[LCD + 2], ey[LCD + 2], ez[LCD + 2], gx[LCD + 2], gy[LCD + 2], gz[LCD + 2];
-        {
-            RT e[LC + 2][LD + 1][LCD + 2];
-            hermite_e<LC + 1, LD>(k.QAx, k.QBx, oo2q, k.K, e);
-            ket_deriv_rows<LC, LD>(e, cx, dx, ec, ex, gx);
-            hermite_e<LC + 1, LD>(k.QAy, k.QBy, oo2q, RT(1), e);
-            ket_deriv_rows<LC, LD>(e, cy, dy, ec, ey, gy);
-            hermite_e<LC + 1, LD>(k.QAz, k.QBz, oo2q, RT(1), e);
-            ket_deriv_rows<LC, LD>(e, cz, dz, ec, ez, gz);
-        }
-        RT ck[Q::KG];
-#pragma unroll
-        for (int i = 0; i < Q::KG; ++i) {
-            RT c = k.c[0];
-#pragma unroll
-            for (int j = 1; j < Q::KCD; ++j)
-                if (j == kg * Q::KG + i) c = k.c[j];
-            ck[i] = c * fcd;
-        }
-        for (int ib = ib0; ib < ib1; ++ib) {
-            const RT* sb = st.SB + ib * SBW;
-            const RT* E = st.E + (size_t)ib * BE::SIZE;
-            const RT* Db = st.D + (size_t)ib * BD::SIZE;
-            // everything below is linear in pref * R_tuv (R up to L + 1)
-            auto body = [&](const auto& R, RT pref) {
-                grad_pq<CX, CY, RT>(sb, E, Db, Gr, ck, cx, cy, cz, dx, dy, dz, ex, ey, ez, gx, gy, gz, R, pref, dA, dB,
-                                    dC);
-            };
-            if constexpr (RS) {
-                body(Rs + (size_t)(ik * st.nbp + ib) * nherm(L), RT(1));
-            } else {
-                const RT p = sb[0];
-                const RT rs = rsqrt_t(p + q);
-                const RT alpha = p * q * rs * rs;
-                const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
-                RT R[nherm(L)];
-                if constexpr (grad_rcol<CX, CY, RT>()) {
-                    hermite_r_scaled<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, pref, R);
-#pragma unroll
-                    for (int i = 0; i < nherm(L); ++i) Rcol[i * GRAD_THREADS] = R[i];
-                    body(RColumn<RT, GRAD_THREADS>{Rcol}, RT(1));
-                } else {
-                    hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
-                    body(R, pref);
-                }
-            }
-        }
-    }
-    }
+    grad_prims<CX, CY, RT, RS>(st, Gr, a.q.pv.rec + a.q.pv.slot[P2] * PPW, a.q.pv.npp[P2], ic, id, kg, dA, dB, dC, Rs,
+                               Rcol, ib0, ib1);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double da = dA[d], db = dB[d], dc = dC[d];
         gab[d] += da;
         gab[3 + d] += db;
-        fadd(gsh + 3 * aC + d, dc, FIX_G);
-        fadd(gsh + 3 * aD + d, -(da + db + dc), FIX_G);
+        sadd(gsh + 3 * aC + d, gsh + 3 * (a.natm + aC) + d, dc, FIX_G);
+        sadd(gsh + 3 * aD + d, gsh + 3 * (a.natm + aD) + d, -(da + db + dc), FIX_G);
     }
 }
 
@@ -596,51 +406,39 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
 
 template <int CX, int CY, typename RT>
 __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStageT<RT>& st, int spos, double (&gab)[6],
-                                               facc* gsh, KetQueueR& kq, int& rot, RT* Rbuf, int64_t w0,
-                                               int64_t w1) {
+                                               unsigned* gsh, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf) {
     using Q = QClass<CX, CY>;
     constexpr bool RS = grad_rsmem<CX, CY>();
     const double q1 = a.q.sortedQ[spos];
     const int nb = a.nblock;
     const double xf = 0.5 * fabs(a.kfac) * a.nx;
-    int64_t acc = 0;
-    for (int sub = 0; sub < NSUB; ++sub) {
-        const int seg = CY * NSUB + sub;
-        int64_t kb, ke;
-        ket_range<RT>(a.q, seg, spos, kb, ke);
-        if (ke <= kb) continue;
-        const int64_t wk = ket_work<CX, CY>(sub) * st.nbp;
-        int64_t k0, k1;
-        window_kets(w0, w1, acc, wk, ke - kb, k0, k1);
-        acc += (ke - kb) * wk;
-        if (k1 <= k0) continue;
-        auto keep = [&](int pos) {
-            const int P2 = a.q.sorted[pos];
-            const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-            const int aC = a.q.bv.atom[C], aD = a.q.bv.atom[Dd];
-            if (st.aA == st.aB && st.aB == aC && aC == aD) return false;
-            double gb = a.bmc[st.A * nb + st.B] * a.bmc[C * nb + Dd];
-            if (a.nx > 0)
-                gb += xf * (a.bmx[st.A * nb + C] * a.bmx[st.B * nb + Dd] + a.bmx[st.A * nb + Dd] * a.bmx[st.B * nb + C]);
-            const double deg = 0.5 * (st.A != st.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.P1 != P2 ? 2.0 : 1.0);
-            return q1 * a.q.sortedQ[pos] * deg * gb >= a.thr;
-        };
-        const int nkg = seg_groups<Q::KG, Q::NKG>(sub);
-        // item r = (contraction group, bra-primitive split, column)
-        const int nsp = bra_splits(st.nbp, sub, a.item_pq);
-        auto work = [&](int pos, int r, const RT* Rs) {
-            const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
-            grad_column<CX, CY, RT, RS>(a, st, a.q.sorted[pos], q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg,
-                                        gab, gsh, Rs, Rbuf + threadIdx.x, st.nbp * sp / nsp,
-                                        st.nbp * (sp + 1) / nsp);
-        };
-        const int j0 = a.q.seg_start[seg] + static_cast<int>(kb + k0);
-        if constexpr (RS) {
-            ket_items_r<Q::L + 1>(Q::NCD * nkg * nsp, j0, k1 - k0, kq, rot, st, a.q, Rbuf, keep, work);
-        } else {
-            ket_items(Q::NCD * nkg * nsp, j0, k1 - k0, kq, rot, keep,
-                      [&](int pos, int r) { work(pos, r, static_cast<const RT*>(nullptr)); });
-        }
+    auto keep = [&](int pos) {
+        const int P2 = a.q.sorted[pos];
+        const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
+        const int aC = a.q.bv.atom[C], aD = a.q.bv.atom[Dd];
+        if (st.aA == st.aB && st.aB == aC && aC == aD) return false;
+        double gb = a.bmc[st.A * nb + st.B] * a.bmc[C * nb + Dd];
+        if (a.nx > 0)
+            gb += xf * (a.bmx[st.A * nb + C] * a.bmx[st.B * nb + Dd] + a.bmx[st.A * nb + Dd] * a.bmx[st.B * nb + C]);
+        const double deg = 0.5 * (st.A != st.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.P1 != P2 ? 2.0 : 1.0);
+        return q1 * a.q.sortedQ[pos] * deg * gb >= a.thr;
+    };
+    // item r = (contraction group, bra-primitive split, column)
+    auto work = [&](int sub, int pos, int r, const RT* Rs) {
+        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.nbp, sub, a.item_pq);
+        const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
+        grad_column<CX, CY, RT, RS>(a, st, a.q.sorted[pos], q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
+                                    gsh, Rs, Rbuf + threadIdx.x, st.nbp * sp / nsp, st.nbp * (sp + 1) / nsp);
+    };
+    if constexpr (RS) {
+        int rot = 0;
+        for (int sub = 0; sub < NSUB; ++sub)
+            if (f.kcnt[sub] > 0)
+                ket_items_r<Q::L + 1>(f.nper[sub], f.kj0[sub], f.kcnt[sub], *kq, rot, st, a.q, Rbuf, keep,
+                                      [&](int pos, int r, const RT* Rs) { work(sub, pos, r, Rs); });
+    } else {
+        flat_items(f, true, queue, keep,
+                   [&](int sub, int pos, int r) { work(sub, pos, r, static_cast<const RT*>(nullptr)); });
     }
 }
 
@@ -657,45 +455,49 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
 template <int CX, int CY, typename RT>
 __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kernel(GradArgs a) {
     using Q0 = QClass<CX, 0>;
+    using Q = QClass<CX, CY>;
     extern __shared__ double smem[];
-    facc* gsh = reinterpret_cast<facc*>(smem);
+    unsigned* gsh = reinterpret_cast<unsigned*>(smem);      // low words [natm][3], then the high words
     RT* Rbuf = reinterpret_cast<RT*>(smem + 3 * a.natm);
     RT* Esm = Rbuf + a.rbuf;
     __shared__ BraStageT<RT> st;
-    __shared__ KetQueueR kq;
+    __shared__ FlatItems f;
+    __shared__ QueueOf<grad_rsmem<CX, CY>()> kq;
     __shared__ int sh[2];
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
-    for (int i = threadIdx.x; i < 3 * a.natm; i += blockDim.x) gsh[i] = 0;
+    for (int i = threadIdx.x; i < 6 * a.natm; i += blockDim.x) gsh[i] = 0u;
+    auto gadd = [&](int i, double v) { sadd(gsh + i, gsh + 3 * a.natm + i, v, FIX_G); };
     for (;;) {
         int c, b;
         next_chunk(a.plan, nbra, sh, c, b);                     // (its barrier also orders the zeroing)
         if (c >= total) break;                                  // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
-        const int nch = a.plan.off[b + 1] - a.plan.off[b], j = c - a.plan.off[b];
-        const int64_t W = bra_work<CX, CY, RT>(a.q, spos);
         if (threadIdx.x == 0) {
             load_stage(a.q, a.q.sorted[spos], st, Esm);
-            st.D = st.E + (size_t)st.nbp * BraE<Q0::LA, Q0::LB, 1>::SIZE;
+            st.D = st.E + (size_t)st.nbp * BraE<Q0::LA, Q0::LB, 0>::SIZE;
         }
         __syncthreads();
-        stage_bra_e<Q0::LA, Q0::LB, 1>(st);
-        __syncthreads();
-        stage_bra_d<Q0::LA, Q0::LB>(st);
+        if (threadIdx.x < 32) {
+            const int sub = threadIdx.x < NSUB ? threadIdx.x : 0;
+            plan_window<CX, CY, RT>(a.q, spos, st.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], Q::NCD,
+                                    seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.nbp, sub, a.item_pq), f);
+        }
+        stage_bra_de<Q0::LA, Q0::LB>(st);
         __syncthreads();
         double gab[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        int rot = 0;
-        grad_ket_class<CX, CY, RT>(a, st, spos, gab, gsh, kq, rot, Rbuf, chunk_edge(W, j, nch),
-                                   chunk_edge(W, j + 1, nch));
+        grad_ket_class<CX, CY, RT>(a, st, spos, gab, gsh, f, kq.r(), kq.flat(), Rbuf);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            if (gab[d] != 0.0) fadd(gsh + 3 * st.aA + d, gab[d], FIX_G);
-            if (gab[3 + d] != 0.0) fadd(gsh + 3 * st.aB + d, gab[3 + d], FIX_G);
+            if (gab[d] != 0.0) gadd(3 * st.aA + d, gab[d]);
+            if (gab[3 + d] != 0.0) gadd(3 * st.aB + d, gab[3 + d]);
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < 3 * a.natm; i += blockDim.x)
-        if (gsh[i] != 0) atomicAdd(a.grad + i, gsh[i]);
+    for (int i = threadIdx.x; i < 3 * a.natm; i += blockDim.x) {
+        const facc v = join_planes(gsh[i], gsh[3 * a.natm + i]);
+        if (v != 0) atomicAdd(a.grad + i, v);
+    }
 }
 
 // Elements of the staged-R buffer of the (CX, CY) gradient kernel (the
@@ -712,8 +514,7 @@ template <int CX, typename RT>
 size_t grad_smem_bytes(int natm, int max_bra_prims, size_t rbuf_elems) {
     using Q0 = QClass<CX, 0>;
     return sizeof(double) * 3 * (size_t)natm +
-           sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (BraE<Q0::LA, Q0::LB, 1>::SIZE +
-                                                              BraD<Q0::LA, Q0::LB>::SIZE + SBW));
+           sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (2 * BraE<Q0::LA, Q0::LB, 0>::SIZE + SBW));
 }
 
 }  // namespace hf

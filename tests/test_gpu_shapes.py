@@ -1,0 +1,54 @@
+"""
+The integral kernels at the edges of their work split, against the oracle:
+molecules of 1 to 33 atoms (fewer and more nuclei than the lanes of a warp),
+every basis set's classes and contraction counts, ket lists shorter than a
+warp and longer than one queue.
+
+Tolerances: 1e-10 per unit of the result's largest element (at least 1) for
+FP64 sums of up to 1e5 terms whose own rounding is 1e-16 and whose
+fixed-point step is 6e-14.
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MOLECULES = [("atom", "cc-pvdz"), ("water", "sto-3g"), ("water", "cc-pvdz"), ("tree7", "6-31g"), ("tree2", "6-31g*"),
+             ("cluster11", "6-31g**")]
+
+
+def _case(name, basis_name):
+    from aimd_b200 import geometry as G
+    from aimd_b200.basis import build_basis
+    if name == "atom":
+        sym, x = ["O"], np.array([[0.1, -0.2, 0.3]])
+    elif name == "water":
+        sym, x = G.water()
+    elif name.startswith("tree"):
+        sym, x = G.random_molecule(int(name[4:]))
+    else:
+        sym, x = G.water_cluster(int(name[7:]), seed=2)
+    basis = build_basis(sym, x, basis_name)
+    rng = np.random.default_rng(7)
+    r = np.linalg.norm(x[:, None] - x[None], axis=2)[np.ix_(basis.ao_atom, basis.ao_atom)]
+    D = rng.normal(size=(2, basis.nao, basis.nao)) * np.exp(-0.3 * r)
+    return basis, 0.5 * (D + D.transpose(0, 2, 1))
+
+
+def _close(got, ref, what):
+    tol = 1e-10 * max(1.0, float(np.abs(ref).max()))
+    assert np.abs(np.asarray(got) - ref).max() <= tol, what
+
+
+@pytest.mark.parametrize("name,basis_name", MOLECULES)
+def test_two_electron_gradient(name, basis_name):
+    from aimd_b200 import integrals as I
+    from oracle import hf_oracle as O
+    b, D = _case(name, basis_name)
+    _close(I.two_electron_gradient(b, D[0], [D[0]], 0.5), O.two_electron_gradient(b, D[0], [D[0]], 0.5), "RHF")
+    _close(I.two_electron_gradient(b, D[0] + D[1], list(D), 1.0),
+           O.two_electron_gradient(b, D[0] + D[1], list(D), 1.0), "UHF")
+    _close(I.two_electron_gradient(b, D[0], [], 0.0), O.two_electron_gradient(b, D[0], [], 0.0), "no exchange")
