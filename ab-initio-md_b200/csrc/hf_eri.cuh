@@ -1,21 +1,29 @@
 // Contracted block-quartet ERIs and their integral-direct J/K digestion.
 //
-// Work decomposition (one launch per bra pair class X):
-//   * one CTA per bra block pair P1 (class X, in Schwarz-sorted order);
-//   * the ket block pairs P2 of every class Y <= X that pass Q1 Q2 >= thr are
-//     a prefix of class Y's Q-sorted list (cut at P1's own position for
+// Work decomposition (one launch per bra class X and ket class Y <= X):
+//   * a chunk = (bra block pair P1, window of its ket list), taken by a CTA;
+//   * the ket block pairs P2 of class Y that pass Q1 Q2 >= thr are, in each
+//     segment, a prefix of its Q-sorted list (cut at P1's own position for
 //     Y == X, so each unordered pair of pairs is visited once);
 //   * one thread item = (ket pair P2, ket Cartesian component pair cd): it
 //     computes the column (ab|cd) for every bra row ab and every contraction
 //     combination, by McMurchie-Davidson: per primitive quartet R_tuv up to
 //     L = l_a+l_b+l_c+l_d, the ket Hermite->Cartesian step for its own cd,
-//     and after the ket primitive loop the bra step (the reference's
-//     _eri_block, aimd/qc/integrals.py:777-842, reorganised by column).
-// The bra pair's primitive E tables are staged once per CTA in shared
+//     and the bra step (the reference's _eri_block,
+//     aimd/qc/integrals.py:777-842, reorganised by column).
+// The bra pair's primitive E tables are staged once per chunk in shared
 // memory. Digestion: every exchange image of the 8-fold symmetry lands in a
 // row of the bra pair's functions, so K rows are accumulated in shared
-// memory and flushed once per CTA; J_ab accumulates in registers; only
-// J_cd goes straight to global memory.
+// memory and flushed once per chunk; J_ab accumulates in per-thread shared
+// slots; only J_cd goes straight to global memory.
+//
+// What bounds these kernels is instruction issue (FP64 chains at 8 warps per
+// SM) and, for small molecules, fetching the unrolled code of each kernel
+// once; DRAM traffic is negligible. Hence one pass over a column's box with
+// its conditions tested per box entry, no code for the entries that no column
+// reaches (t + u + v > LCD), and the bra step one direction at a time. With
+// those and the flat item lists, one B200: water 6-31G* 2.67 -> 0.37 ms,
+// (H2O)8 difference build 11.5 -> 4.4 ms, (H2O)32 cc-pVDZ 266 -> 118 ms.
 #pragma once
 #include "hf_device.cuh"
 
@@ -160,6 +168,56 @@ __device__ __forceinline__ void select_j(const RT (&e)[IM + 1][JM + 1][T + 1], i
         }
 }
 
+// Bra Hermite -> Cartesian step of one bra primitive, one direction at a time:
+// row(ia, jb, s) receives s[kk] = f_ab sum_{tuw} E^{ab}_tuw X[kk]_tuw for every
+// component pair (ia, jb). For each (az, bz) the sum over w is taken once for
+// all (t, u) (W), then the sums over u and t of its (ay, by): some 440
+// multiply-adds for dd, against three products for each of the 400 entries of
+// the rows' boxes.
+template <int LA, int LB, int KG, typename RT, typename Row>
+__device__ __forceinline__ void bra_rows(const RT* E, const RT (&X)[KG][nherm(LA + LB)], Row row) {
+    using BE = BraE<LA, LB, 0>;
+#pragma unroll
+    for (int az = 0; az <= LA; ++az)
+#pragma unroll
+        for (int bz = 0; bz <= LB; ++bz) {
+            RT W[KG][ncart(LA + LB)];
+#pragma unroll
+            for (int t = 0; t <= LA + LB - az - bz; ++t)
+#pragma unroll
+                for (int u = 0; u <= LA + LB - az - bz - t; ++u)
+#pragma unroll
+                    for (int kk = 0; kk < KG; ++kk) {
+                        RT s = E[BE::at(2, az, bz, 0)] * X[kk][hidx(t, u, 0)];
+#pragma unroll
+                        for (int w = 1; w <= az + bz; ++w) s += E[BE::at(2, az, bz, w)] * X[kk][hidx(t, u, w)];
+                        W[kk][cart_index(t, u)] = s;
+                    }
+#pragma unroll
+            for (int ay = 0; ay <= LA - az; ++ay)
+#pragma unroll
+                for (int by = 0; by <= LB - bz; ++by) {
+                    const int ax = LA - az - ay, bx = LB - bz - by;
+                    const RT fab = static_cast<RT>(cart_norm(ax, ay, az) * cart_norm(bx, by, bz));
+                    RT s[KG];
+#pragma unroll
+                    for (int kk = 0; kk < KG; ++kk) s[kk] = RT(0);
+#pragma unroll
+                    for (int t = 0; t <= ax + bx; ++t) {
+                        const RT e = fab * E[BE::at(0, ax, bx, t)];
+#pragma unroll
+                        for (int kk = 0; kk < KG; ++kk) {
+                            RT y = RT(0);
+#pragma unroll
+                            for (int u = 0; u <= ay + by; ++u) y += E[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
+                            s[kk] += e * y;
+                        }
+                    }
+                    row(cart_index(ay, az), cart_index(by, bz), s);
+                }
+        }
+}
+
 // v[r][kk] = (row r | cd, contraction kk) of the quartet (staged bra pair,
 // ket pair records rk with nkp primitive pairs); r = (ka*nB + kb)*NAB +
 // ia*NB + jb, kk = kc*nD + kd - kg*KG (compact contraction indices over the
@@ -181,8 +239,6 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
-    // classes with L >= 6 keep their outer Hermite loops rolled (compile time)
-    constexpr int UH = L >= 6 ? 1 : 16;
     const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
     const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
     const RT fcd = static_cast<RT>(cart_norm(cx, cy, cz) * cart_norm(dx, dy, dz));
@@ -220,36 +276,40 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
                     if (j == kg * Q::KG + i) c = k.c[j];
                 ck[i] = c * fcd;
             }
-            // ket step: Xs[kk]_tuv += ck[kk] pref sum_{box(cd)} (-1)^|k| E^{cd}_k R_{tuv+k}
+            // ket step: Xs[kk]_h += ck[kk] pref sum_{k in box(cd)} (-1)^|k| E^{cd}_k R_{h+k},
+            // box entries outer, so that a column's box conditions are tested
+            // once per entry and not once per (entry, h)
             auto ket_step = [&](const auto& R, RT scale) {
                 RT sc[Q::KG];
 #pragma unroll
                 for (int kk = 0; kk < Q::KG; ++kk) sc[kk] = scale * ck[kk];
-#pragma unroll UH
-                for (int t = 0; t <= LAB; ++t)
-#pragma unroll UH
-                    for (int u = 0; u <= LAB - t; ++u)
 #pragma unroll
-                        for (int w = 0; w <= LAB - t - u; ++w) {
-                            RT s = RT(0);
+                for (int t2 = 0; t2 <= LCD; ++t2) {
+                    if (t2 > cx + dx) continue;
 #pragma unroll
-                            for (int t2 = 0; t2 <= LCD; ++t2) {
-                                if (t2 > cx + dx) continue;
+                    for (int u2 = 0; u2 <= LCD - t2; ++u2) {
+                        if (u2 > cy + dy) continue;
+                        const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
 #pragma unroll
-                                for (int u2 = 0; u2 <= LCD; ++u2) {
-                                    if (u2 > cy + dy) continue;
-                                    const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
+                        for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
+                            if (v2 > cz + dz) continue;
+                            const RT e = (v2 & 1) ? -exy * ez[v2] : exy * ez[v2];
+                            RT es[Q::KG];
 #pragma unroll
-                                    for (int v2 = 0; v2 <= LCD; ++v2) {
-                                        if (v2 > cz + dz) continue;
-                                        const RT e = (v2 & 1) ? -exy * ez[v2] : exy * ez[v2];
-                                        s += e * R[hidx(t + t2, u + u2, w + v2)];
+                            for (int kk = 0; kk < Q::KG; ++kk) es[kk] = sc[kk] * e;
+#pragma unroll
+                            for (int t = 0; t <= LAB; ++t)
+#pragma unroll
+                                for (int u = 0; u <= LAB - t; ++u)
+#pragma unroll
+                                    for (int w = 0; w <= LAB - t - u; ++w) {
+                                        const RT r = R[hidx(t + t2, u + u2, w + v2)];
+#pragma unroll
+                                        for (int kk = 0; kk < Q::KG; ++kk) Xs[kk][hidx(t, u, w)] += es[kk] * r;
                                     }
-                                }
-                            }
-#pragma unroll
-                            for (int kk = 0; kk < Q::KG; ++kk) Xs[kk][hidx(t, u, w)] += sc[kk] * s;
                         }
+                    }
+                }
             };
             if constexpr (RS) {
                 ket_step(Rs + (size_t)(ik * st.nbp + ib) * nherm(L), RT(1));
@@ -265,37 +325,12 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
         }
         // bra step, once per bra primitive:
         // v[(ka,kb),ab][kk] += C[ka,kb] f_ab sum_box E^{ab}_tuv Xs[kk]_tuv
-        const RT* E = st.E + (size_t)ib * BE::SIZE;
-#pragma unroll UH
-        for (int ia = 0; ia < Q::NA; ++ia) {
-            const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
+        bra_rows<LA, LB, Q::KG>(st.E + (size_t)ib * BE::SIZE, Xs, [&](int ia, int jb, const RT (&s)[Q::KG]) {
 #pragma unroll
-            for (int jb = 0; jb < Q::NB; ++jb) {
-                const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                const RT fab = static_cast<RT>(cart_norm(ax, ay, az) * cart_norm(bx, by, bz));
-                RT s[Q::KG];
+            for (int kab = 0; kab < Q::KAB; ++kab)
 #pragma unroll
-                for (int kk = 0; kk < Q::KG; ++kk) s[kk] = RT(0);
-#pragma unroll
-                for (int t = 0; t <= ax + bx; ++t)
-#pragma unroll
-                    for (int u = 0; u <= ay + by; ++u) {
-                        const RT exy = E[BE::at(0, ax, bx, t)] * E[BE::at(1, ay, by, u)];
-#pragma unroll
-                        for (int w = 0; w <= az + bz; ++w) {
-                            const RT e = exy * E[BE::at(2, az, bz, w)];
-#pragma unroll
-                            for (int kk = 0; kk < Q::KG; ++kk) s[kk] += e * Xs[kk][hidx(t, u, w)];
-                        }
-                    }
-#pragma unroll
-                for (int kab = 0; kab < Q::KAB; ++kab) {
-                    const RT c = sb[8 + kab] * fab;
-#pragma unroll
-                    for (int kk = 0; kk < Q::KG; ++kk) v[kab * Q::NAB + ia * Q::NB + jb][kk] += c * s[kk];
-                }
-            }
-        }
+                for (int kk = 0; kk < Q::KG; ++kk) v[kab * Q::NAB + ia * Q::NB + jb][kk] += sb[8 + kab] * s[kk];
+        });
     }
 }
 
@@ -310,8 +345,6 @@ __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, co
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
-    // classes with L >= 6 keep their outer Hermite loops rolled (compile time)
-    constexpr int UH = L >= 6 ? 1 : 16;
     const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
     const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
     const RT fcd = static_cast<RT>(cart_norm(cx, cy, cz) * cart_norm(dx, dy, dz));
@@ -350,58 +383,39 @@ __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, co
             const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
             RT R[nherm(L)];
             hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
-            RT X[Q::NHB];
-#pragma unroll UH
-            for (int t = 0; t <= LAB; ++t)
-#pragma unroll UH
-                for (int u = 0; u <= LAB - t; ++u)
+            RT X[1][Q::NHB];
 #pragma unroll
-                    for (int w = 0; w <= LAB - t - u; ++w) {
-                        RT s = RT(0);
+            for (int h = 0; h < Q::NHB; ++h) X[0][h] = RT(0);
 #pragma unroll
-                        for (int t2 = 0; t2 <= LCD; ++t2) {
-                            if (t2 > cx + dx) continue;
+            for (int t2 = 0; t2 <= LCD; ++t2) {
+                if (t2 > cx + dx) continue;
 #pragma unroll
-                            for (int u2 = 0; u2 <= LCD; ++u2) {
-                                if (u2 > cy + dy) continue;
-                                const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
+                for (int u2 = 0; u2 <= LCD - t2; ++u2) {
+                    if (u2 > cy + dy) continue;
+                    const RT exy = pref * (((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2]);
 #pragma unroll
-                                for (int v2 = 0; v2 <= LCD; ++v2) {
-                                    if (v2 > cz + dz) continue;
-                                    const RT e = (v2 & 1) ? -exy * ez[v2] : exy * ez[v2];
-                                    s += e * R[hidx(t + t2, u + u2, w + v2)];
-                                }
-                            }
-                        }
-                        X[hidx(t, u, w)] = pref * s;
-                    }
-            // bra step: v[(ka,kb),ab][kk] += C[ka,kb] f_ab sum_box E^{ab}_tuv X[tuv] ck[kk]
-            const RT* E = st.E + (size_t)ib * BE::SIZE;
-#pragma unroll UH
-            for (int ia = 0; ia < Q::NA; ++ia) {
-                const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
+                    for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
+                        if (v2 > cz + dz) continue;
+                        const RT e = (v2 & 1) ? -exy * ez[v2] : exy * ez[v2];
 #pragma unroll
-                for (int jb = 0; jb < Q::NB; ++jb) {
-                    const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                    const RT fab = static_cast<RT>(cart_norm(ax, ay, az) * cart_norm(bx, by, bz));
-                    RT s = RT(0);
+                        for (int t = 0; t <= LAB; ++t)
 #pragma unroll
-                    for (int t = 0; t <= ax + bx; ++t)
+                            for (int u = 0; u <= LAB - t; ++u)
 #pragma unroll
-                        for (int u = 0; u <= ay + by; ++u) {
-                            const RT exy = E[BE::at(0, ax, bx, t)] * E[BE::at(1, ay, by, u)];
-#pragma unroll
-                            for (int w = 0; w <= az + bz; ++w) s += exy * E[BE::at(2, az, bz, w)] * X[hidx(t, u, w)];
-                        }
-                    s *= fab;
-#pragma unroll
-                    for (int kab = 0; kab < Q::KAB; ++kab) {
-                        const RT c = sb[8 + kab] * s;
-#pragma unroll
-                        for (int kk = 0; kk < Q::KG; ++kk) v[kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
+                                for (int w = 0; w <= LAB - t - u; ++w)
+                                    X[0][hidx(t, u, w)] += e * R[hidx(t + t2, u + u2, w + v2)];
                     }
                 }
             }
+            // bra step: v[(ka,kb),ab][kk] += C[ka,kb] f_ab sum_box E^{ab}_tuv X[tuv] ck[kk]
+            bra_rows<LA, LB, 1>(st.E + (size_t)ib * BE::SIZE, X, [&](int ia, int jb, const RT (&s)[1]) {
+#pragma unroll
+                for (int kab = 0; kab < Q::KAB; ++kab) {
+                    const RT c = sb[8 + kab] * s[0];
+#pragma unroll
+                    for (int kk = 0; kk < Q::KG; ++kk) v[kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
+                }
+            });
         }
     }
 }
@@ -462,57 +476,40 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
             for (int ic = 0; ic < Q::NC; ++ic) {
                 const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
                 const RT fc = static_cast<RT>(cart_norm(cx, cy, cz));
-                RT X[Q::NHB];
+                RT X[1][Q::NHB];
 #pragma unroll
-                for (int t = 0; t <= LAB; ++t)
+                for (int h = 0; h < Q::NHB; ++h) X[0][h] = RT(0);
+                const RT pf = pref * fc;
 #pragma unroll
-                    for (int u = 0; u <= LAB - t; ++u)
+                for (int t2 = 0; t2 <= LCD; ++t2) {
+                    if (t2 > cx + dx) continue;
 #pragma unroll
-                        for (int w = 0; w <= LAB - t - u; ++w) {
-                            RT s = RT(0);
+                    for (int u2 = 0; u2 <= LCD - t2; ++u2) {
+                        if (u2 > cy + dy) continue;
+                        const RT exy = pf * (((t2 + u2) & 1) ? -ex[cx][t2] * ey[cy][u2] : ex[cx][t2] * ey[cy][u2]);
 #pragma unroll
-                            for (int t2 = 0; t2 <= LCD; ++t2) {
-                                if (t2 > cx + dx) continue;
+                        for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
+                            if (v2 > cz + dz) continue;
+                            const RT e = (v2 & 1) ? -exy * ez[cz][v2] : exy * ez[cz][v2];
 #pragma unroll
-                                for (int u2 = 0; u2 <= LCD; ++u2) {
-                                    if (u2 > cy + dy) continue;
-                                    const RT exy = ((t2 + u2) & 1) ? -ex[cx][t2] * ey[cy][u2] : ex[cx][t2] * ey[cy][u2];
+                            for (int t = 0; t <= LAB; ++t)
 #pragma unroll
-                                    for (int v2 = 0; v2 <= LCD; ++v2) {
-                                        if (v2 > cz + dz) continue;
-                                        const RT e = (v2 & 1) ? -exy * ez[cz][v2] : exy * ez[cz][v2];
-                                        s += e * R[hidx(t + t2, u + u2, w + v2)];
-                                    }
-                                }
-                            }
-                            X[hidx(t, u, w)] = pref * fc * s;
-                        }
-                // bra step of column ic
+                                for (int u = 0; u <= LAB - t; ++u)
 #pragma unroll
-                for (int ia = 0; ia < Q::NA; ++ia) {
-                    const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
-#pragma unroll
-                    for (int jb = 0; jb < Q::NB; ++jb) {
-                        const int bx = cart_x(LB, jb), by = cart_y(LB, jb), bz = cart_z(LB, jb);
-                        const RT fab = static_cast<RT>(cart_norm(ax, ay, az) * cart_norm(bx, by, bz));
-                        RT s = RT(0);
-#pragma unroll
-                        for (int t = 0; t <= ax + bx; ++t)
-#pragma unroll
-                            for (int u = 0; u <= ay + by; ++u) {
-                                const RT exy = E[BE::at(0, ax, bx, t)] * E[BE::at(1, ay, by, u)];
-#pragma unroll
-                                for (int w = 0; w <= az + bz; ++w) s += exy * E[BE::at(2, az, bz, w)] * X[hidx(t, u, w)];
-                            }
-                        s *= fab;
-#pragma unroll
-                        for (int kab = 0; kab < Q::KAB; ++kab) {
-                            const RT c = sb[8 + kab] * s;
-#pragma unroll
-                            for (int kk = 0; kk < Q::KG; ++kk) v[ic][kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
+                                    for (int w = 0; w <= LAB - t - u; ++w)
+                                        X[0][hidx(t, u, w)] += e * R[hidx(t + t2, u + u2, w + v2)];
                         }
                     }
                 }
+                // bra step of column ic
+                bra_rows<LA, LB, 1>(E, X, [&](int ia, int jb, const RT (&s)[1]) {
+#pragma unroll
+                    for (int kab = 0; kab < Q::KAB; ++kab) {
+                        const RT c = sb[8 + kab] * s[0];
+#pragma unroll
+                        for (int kk = 0; kk < Q::KG; ++kk) v[ic][kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
+                    }
+                });
             }
         }
     }
@@ -694,7 +691,7 @@ template <int CX, int CY, int NS, bool KGLOBAL, typename ST>
 __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, int P2, int C, int Dd, int ic,
                                                  int id, int kg,
                                                  const double (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                 double* Jt, facc* Ksm) {
+                                                 double* Jt, unsigned* Ksm) {
     using Q = QClass<CX, CY>;
     const BlockView& bv = a.q.bv;
     const int nC = bv.ncon[C], nD = bv.ncon[Dd], oC = bv.ao[C], oD = bv.ao[Dd];
@@ -710,8 +707,18 @@ __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, 
         // K rows of the bra functions: shared accumulator, or the global K
         // itself (KGLOBAL, for bra classes whose rows would not fit)
         const bool kgl = KGLOBAL || a.kglobal;
-        facc* Ks = kgl ? nullptr : Ksm + (size_t)s * NF * n;
+        unsigned* Ks = KGLOBAL ? nullptr : Ksm + (size_t)s * NF * n;
+        const size_t hi = (size_t)NS * NF * n;          // the rows' high words
         facc* Kg = a.K + s * nn;
+        // row f of the shared rows is row g of K
+        auto kadd = [&](int f, int g, int col, double val) {
+            if (kgl) {
+                fadd(Kg + (size_t)g * n + col, val, fx);
+            } else {
+                unsigned* p = Ks + (size_t)f * n + col;
+                sadd(p, p + hi, val, fx);
+            }
+        };
 #pragma unroll
         for (int kk = 0; kk < Q::KG; ++kk) {
                 const int kq = kg * Q::KG + kk;
@@ -753,10 +760,8 @@ __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, 
                                 s1 += v[r][kk] * __ldg(D + nb_ * n + sg);
                                 s2 += v[r][kk] * __ldg(D + nb_ * n + l);
                             }
-                        facc* row = kgl ? Kg + (size_t)(st.oA + ka * Q::NA + ia) * n
-                                              : Ks + (size_t)(ka * Q::NA + ia) * n;
-                        fadd(row + l, g * s1, fx);
-                        fadd(row + sg, g * s2, fx);
+                        kadd(ka * Q::NA + ia, st.oA + ka * Q::NA + ia, l, g * s1);
+                        kadd(ka * Q::NA + ia, st.oA + ka * Q::NA + ia, sg, g * s2);
                     }
                 // K[n, l] and K[n, sg]: rows of B's functions
 #pragma unroll
@@ -775,22 +780,14 @@ __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, 
                                 s1 += v[r][kk] * __ldg(D + m * n + sg);
                                 s2 += v[r][kk] * __ldg(D + m * n + l);
                             }
-                        facc* row = kgl ? Kg + (size_t)(st.oB + kb * Q::NB + jb) * n
-                                              : Ks + (size_t)(NFA + kb * Q::NB + jb) * n;
-                        fadd(row + l, g * s1, fx);
-                        fadd(row + sg, g * s2, fx);
+                        kadd(NFA + kb * Q::NB + jb, st.oB + kb * Q::NB + jb, l, g * s1);
+                        kadd(NFA + kb * Q::NB + jb, st.oB + kb * Q::NB + jb, sg, g * s2);
                     }
             }
     }
 }
 
-// Items of ket class CY for the staged bra pair.
-// Work queue of one CTA: the ket pairs of a segment that pass a per-pair
-// test are compacted into shared memory in chunks of KQ_CAP (warp ballots,
-// warps in index order), then dealt to the threads as NPER items each,
-// so that lanes only receive live work. Dealing starts where the previous
-// chunk ended (rot), so ragged tails do not pile up on the low threads.
-// Every thread of the CTA must call this with the same j0 and cnt.
+// Queue chunk of the two-stage items (ket_items_r below).
 constexpr int KQ_CAP = 256;
 
 // Ket contraction groups of KG combinations that a segment's pairs need: its
@@ -821,12 +818,6 @@ __device__ __forceinline__ int bra_splits(int nbp, int sub, int item_pq) {
     return s < 1 ? 1 : (s > nbp ? nbp : s);
 }
 
-struct KetQueue {
-    int pos[KQ_CAP];
-    int wcnt[32];           // per-warp counts of one compaction step
-    int n;
-};
-
 // Compact the positions p0 .. p0+m-1 that pass keep() into q.pos[0 .. q.n)
 // in position order (per-warp ballots, warps in index order), so that the
 // queue, the item dealing and every per-thread partial sum are the same on
@@ -853,23 +844,6 @@ __device__ __forceinline__ void compact(Queue& q, int p0, int m, Keep keep, Stor
     }
     if (threadIdx.x == 0) q.n = n;
     __syncthreads();
-}
-
-template <typename Queue, typename Keep, typename Work>
-__device__ __forceinline__ void ket_items(int nper, int j0, int64_t cnt, Queue& q, int& rot, Keep keep, Work work) {
-    for (int64_t base = 0; base < cnt; base += KQ_CAP) {
-        const int m = static_cast<int>(cnt - base < KQ_CAP ? cnt - base : KQ_CAP);
-        compact(q, j0 + static_cast<int>(base), m, keep, [&](int slot, int pos) { q.pos[slot] = pos; });
-        const int items = q.n * nper;
-        int it = static_cast<int>(threadIdx.x) - rot;
-        if (it < 0) it += blockDim.x;
-        // column-major: neighbouring lanes take the same ket column of
-        // different ket pairs, so the column's box conditions are warp-uniform
-        const int nq = q.n;
-        for (; it < items; it += blockDim.x) work(q.pos[it % nq], it / nq);
-        rot = (rot + items) % static_cast<int>(blockDim.x);
-        __syncthreads();
-    }
 }
 
 // ---- Flat items
@@ -1155,80 +1129,66 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
     }
 }
 
-// The ket pairs of class CY for bra position spos whose work falls in the
-// chunk's window [w0, w1).
+// The items of the staged bra pair (position spos) in the window that f holds.
 template <int CX, int CY, int NS, bool KGLOBAL, typename RT>
 __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT>& st, int spos, double* Jt,
-                                             facc* Ksm, KetQueueR& kq, int& rot, RT* Rbuf, int64_t w0,
-                                             int64_t w1) {
+                                             unsigned* Ksm, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf) {
     using Q = QClass<CX, CY>;
     const double q1 = a.q.sortedQ[spos];
     const double* bm = a.bmax;
     const int nb = a.nblock;
-    int64_t acc = 0;
-    for (int sub = 0; sub < NSUB; ++sub) {
-        const int seg = CY * NSUB + sub;
-        int64_t kb, ke;
-        ket_range<RT>(a.q, seg, spos, kb, ke);
-        if (ke <= kb) continue;
-        const int64_t wk = ket_work<CX, CY>(sub) * st.nbp;
-        int64_t k0, k1;
-        window_kets(w0, w1, acc, wk, ke - kb, k0, k1);
-        acc += (ke - kb) * wk;
-        if (k1 <= k0) continue;
-        // difference densities: density-weighted test on the six block pairs
-        auto keep = [&](int pos) {
-            if (!bm) return true;
-            const int P2 = a.q.sorted[pos];
-            const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-            const double dm = fmax(fmax(bm[st.A * nb + st.B], bm[C * nb + Dd]),
-                                   fmax(fmax(bm[st.A * nb + C], bm[st.A * nb + Dd]),
-                                        fmax(bm[st.B * nb + C], bm[st.B * nb + Dd])));
-            return q1 * a.q.sortedQ[pos] * dm >= a.dthr;
-        };
-        // contraction groups that the segment's ket pairs actually carry
-        const int nkg = seg_groups<Q::KG, Q::NKG>(sub);
-        auto digest = [&](int P2, int C, int Dd, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
-            if constexpr (sizeof(RT) == sizeof(double)) {
-                jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, v, Jt, Ksm);
-            } else {
-                // FP32 quartets: digested (accumulated) in FP64
-                double vd[Q::NROW][Q::KG];
-#pragma unroll
-                for (int r = 0; r < Q::NROW; ++r)
-#pragma unroll
-                    for (int k = 0; k < Q::KG; ++k) vd[r][k] = static_cast<double>(v[r][k]);
-                jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, vd, Jt, Ksm);
-            }
-        };
-        // item r = (contraction group, bra-primitive split, column block)
-        const int nsp = bra_splits(st.nbp, sub, a.item_pq);
-        auto work = [&](int pos, int r, const RT* Rs) {
-            const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
-            const int ib0 = st.nbp * sp / nsp, ib1 = st.nbp * (sp + 1) / nsp;
-            const int P2 = a.q.sorted[pos];
-            const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-            const double* rk = a.q.pv.rec + a.q.pv.slot[P2] * PPW;
-            if constexpr (Q::CBLK) {
-                // item = the NC columns of one id
-                RT v[Q::NC][Q::NROW][Q::KG];
-                eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1);
-#pragma unroll
-                for (int ic = 0; ic < Q::NC; ++ic) digest(P2, C, Dd, ic, cd, kg, v[ic]);
-            } else {
-                RT v[Q::NROW][Q::KG];
-                eri_column<CX, CY, RT, Q::RSMEM>(st, rk, a.q.pv.npp[P2], cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0,
-                                                 ib1);
-                digest(P2, C, Dd, cd / Q::ND, cd % Q::ND, kg, v);
-            }
-        };
-        const int j0 = a.q.seg_start[seg] + static_cast<int>(kb + k0);
-        if constexpr (Q::RSMEM) {
-            ket_items_r<Q::L>(Q::NITEM * nkg * nsp, j0, k1 - k0, kq, rot, st, a.q, Rbuf, keep, work);
+    // difference densities: density-weighted test on the six block pairs
+    auto keep = [&](int pos) {
+        if (!bm) return true;
+        const int P2 = a.q.sorted[pos];
+        const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
+        const double dm = fmax(fmax(bm[st.A * nb + st.B], bm[C * nb + Dd]),
+                               fmax(fmax(bm[st.A * nb + C], bm[st.A * nb + Dd]),
+                                    fmax(bm[st.B * nb + C], bm[st.B * nb + Dd])));
+        return q1 * a.q.sortedQ[pos] * dm >= a.dthr;
+    };
+    auto digest = [&](int P2, int C, int Dd, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
+        if constexpr (sizeof(RT) == sizeof(double)) {
+            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, v, Jt, Ksm);
         } else {
-            ket_items(Q::NITEM * nkg * nsp, j0, k1 - k0, kq, rot, keep,
-                      [&](int pos, int r) { work(pos, r, static_cast<const RT*>(nullptr)); });
+            // FP32 quartets: digested (accumulated) in FP64
+            double vd[Q::NROW][Q::KG];
+#pragma unroll
+            for (int r = 0; r < Q::NROW; ++r)
+#pragma unroll
+                for (int k = 0; k < Q::KG; ++k) vd[r][k] = static_cast<double>(v[r][k]);
+            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, vd, Jt, Ksm);
         }
+    };
+    // item r = (contraction group that the segment's pairs carry, bra-primitive split, column block)
+    auto work = [&](int sub, int pos, int r, const RT* Rs) {
+        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.nbp, sub, a.item_pq);
+        const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
+        const int ib0 = st.nbp * sp / nsp, ib1 = st.nbp * (sp + 1) / nsp;
+        const int P2 = a.q.sorted[pos];
+        const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
+        const double* rk = a.q.pv.rec + a.q.pv.slot[P2] * PPW;
+        if constexpr (Q::CBLK) {
+            // item = the NC columns of one id
+            RT v[Q::NC][Q::NROW][Q::KG];
+            eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1);
+#pragma unroll
+            for (int ic = 0; ic < Q::NC; ++ic) digest(P2, C, Dd, ic, cd, kg, v[ic]);
+        } else {
+            RT v[Q::NROW][Q::KG];
+            eri_column<CX, CY, RT, Q::RSMEM>(st, rk, a.q.pv.npp[P2], cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1);
+            digest(P2, C, Dd, cd / Q::ND, cd % Q::ND, kg, v);
+        }
+    };
+    if constexpr (Q::RSMEM) {
+        int rot = 0;
+        for (int sub = 0; sub < NSUB; ++sub)
+            if (f.kcnt[sub] > 0)
+                ket_items_r<Q::L>(f.nper[sub], f.kj0[sub], f.kcnt[sub], *kq, rot, st, a.q, Rbuf, keep,
+                                  [&](int pos, int r, const RT* Rs) { work(sub, pos, r, Rs); });
+    } else {
+        flat_items(f, bm != nullptr, queue, keep,
+                   [&](int sub, int pos, int r) { work(sub, pos, r, static_cast<const RT*>(nullptr)); });
     }
 }
 
@@ -1268,12 +1228,14 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
     const int krows = a.kglobal ? 0 : KK::KROWS;
-    facc* Ksm = reinterpret_cast<facc*>(smem);
+    unsigned* Ksm = reinterpret_cast<unsigned*>(smem);     // low words of the K rows, then the high words
     double* Jt = smem + (size_t)krows * n;
     RT* Rbuf = reinterpret_cast<RT*>(Jt + NS * KK::NROW * JK_THREADS);
     RT* Esm = Rbuf + a.rbuf;
+    using QY = QClass<CX, Y>;
     __shared__ BraStageT<RT> st;
-    __shared__ KetQueueR kq;
+    __shared__ FlatItems f;
+    __shared__ QueueOf<QY::RSMEM> kq;
     __shared__ int sh[2];
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
@@ -1282,16 +1244,17 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
         next_chunk(a.plan, nbra, sh, c, b);
         if (c >= total) break;                                  // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
-        const int nch = a.plan.off[b + 1] - a.plan.off[b], j = c - a.plan.off[b];
-        const int64_t W = bra_work<CX, Y, RT>(a.q, spos);
         if (threadIdx.x == 0) load_stage(a.q, a.q.sorted[spos], st, Esm);
         for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * JK_THREADS; i += blockDim.x) smem[i] = 0.0;
         __syncthreads();
+        if (threadIdx.x < 32) {
+            const int sub = threadIdx.x < NSUB ? threadIdx.x : 0;
+            plan_window<CX, Y, RT>(a.q, spos, st.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], QY::NITEM,
+                                   seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.nbp, sub, a.item_pq), f);
+        }
         stage_bra_e<Q0::LA, Q0::LB, 0>(st);
         __syncthreads();
-        int rot = 0;
-        jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, kq, rot, Rbuf, chunk_edge(W, j, nch),
-                                                 chunk_edge(W, j + 1, nch));
+        jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf);
         __syncthreads();
         // flush J_ab: one thread per (set, row) sums the per-thread slots
         for (int i = threadIdx.x; i < NS * KK::NROW; i += blockDim.x) {
@@ -1308,7 +1271,7 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
         if (krows > 0) {
             constexpr int NFA = Q0::KA * Q0::NA;
             for (int i = threadIdx.x; i < krows * n; i += blockDim.x) {
-                const facc val = Ksm[i];
+                const facc val = join_planes(Ksm[i], Ksm[krows * n + i]);
                 if (val == 0) continue;
                 const int col = i % n, f = (i / n) % KK::NF, s = i / (n * KK::NF);
                 const int row = f < NFA ? st.oA + f : st.oB + (f - NFA);
@@ -1340,12 +1303,17 @@ size_t jk_smem_bytes(int nao, int max_bra_prims, size_t rbuf_elems, bool kglobal
 // ---------------------------------------------------------- Schwarz
 
 // Q[P] = max_ab |(ab|ab)|^(1/2) (the reference's _schwarz_kernel,
-// aimd/qc/integrals.py:864-883): one CTA per pair, one thread per column.
+// aimd/qc/integrals.py:864-883): one CTA per pair, its threads over (column,
+// range of the bra primitives). With one thread a column, a pair of
+// contracted s blocks (64 primitive pairs, one column) ran its 4096 primitive
+// quartets in one thread.
+constexpr int SCHWARZ_THREADS = 64;
 template <int CX>
-__global__ void __launch_bounds__(64) schwarz_kernel(QuartetArgs a, const int* pairs_of_class, double* Qout) {
+__global__ void __launch_bounds__(SCHWARZ_THREADS) schwarz_kernel(QuartetArgs a, const int* pairs_of_class, double* Qout) {
     using Q = QClass<CX, CX>;
     extern __shared__ double smem[];
     __shared__ BraStage st;
+    __shared__ double diag[Q::KAB][SCHWARZ_THREADS];    // partial (ab|ab) of each contraction combination
     __shared__ unsigned long long qmax;
     const int P = pairs_of_class[blockIdx.x];
     if (threadIdx.x == 0) {
@@ -1355,23 +1323,34 @@ __global__ void __launch_bounds__(64) schwarz_kernel(QuartetArgs a, const int* p
     __syncthreads();
     stage_bra_e<Q::LA, Q::LB, 0>(st);
     __syncthreads();
-    for (int cd = threadIdx.x; cd < Q::NCD; cd += blockDim.x) {
-        static_assert(Q::KG == Q::KCD, "diagonal quartets keep all contraction combinations in one item");
-        double v[Q::NROW][Q::KCD];
-        eri_column<CX, CX>(st, st.rec, st.nbp, cd / Q::ND, cd % Q::ND, 0, v, static_cast<const double*>(nullptr), 0,
-                           st.nbp);
-        double m = 0.0;
+    static_assert(Q::KG == Q::KCD, "diagonal quartets keep all contraction combinations in one item");
+    constexpr int NSP = SCHWARZ_THREADS / Q::NCD;       // ranges of the bra primitives
+    const int cd = threadIdx.x % Q::NCD, sp = threadIdx.x / Q::NCD;
+    const int ib0 = st.nbp * sp / NSP, ib1 = st.nbp * (sp + 1) / NSP;
+    if (sp < NSP) {
+        double m[Q::KAB];
 #pragma unroll
-        for (int ka = 0; ka < Q::KA; ++ka)
+        for (int kk = 0; kk < Q::KAB; ++kk) m[kk] = 0.0;
+        if (ib1 > ib0) {
+            double v[Q::NROW][Q::KCD];
+            eri_column<CX, CX>(st, st.rec, st.nbp, cd / Q::ND, cd % Q::ND, 0, v, static_cast<const double*>(nullptr),
+                               ib0, ib1);
 #pragma unroll
-            for (int kb = 0; kb < Q::KB; ++kb) {
-                if (ka >= st.nA || kb >= st.nB) continue;
-                const int kk = ka * st.nB + kb;
+            for (int kk = 0; kk < Q::KAB; ++kk)
 #pragma unroll
                 for (int r = 0; r < Q::NROW; ++r)
-                    if (r == kk * Q::NAB + cd) m = fmax(m, fabs(v[r][kk]));
-            }
-        atomicMax(&qmax, (unsigned long long)__double_as_longlong(m));   // m >= 0: bit order = value order
+                    if (r == kk * Q::NAB + cd) m[kk] = v[r][kk];
+        }
+#pragma unroll
+        for (int kk = 0; kk < Q::KAB; ++kk) diag[kk][threadIdx.x] = m[kk];
+    }
+    __syncthreads();
+    // one thread per (combination, column) sums its ranges in order
+    for (int i = threadIdx.x; i < st.nA * st.nB * Q::NCD; i += SCHWARZ_THREADS) {
+        const int kk = i / Q::NCD, c = i % Q::NCD;
+        double m = 0.0;
+        for (int s = 0; s < NSP; ++s) m += diag[kk][s * Q::NCD + c];
+        atomicMax(&qmax, (unsigned long long)__double_as_longlong(fabs(m)));   // bit order = value order
     }
     __syncthreads();
     if (threadIdx.x == 0) Qout[P] = sqrt(__longlong_as_double((long long)qmax));

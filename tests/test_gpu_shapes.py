@@ -52,3 +52,32 @@ def test_two_electron_gradient(name, basis_name):
     _close(I.two_electron_gradient(b, D[0] + D[1], list(D), 1.0),
            O.two_electron_gradient(b, D[0] + D[1], list(D), 1.0), "UHF")
     _close(I.two_electron_gradient(b, D[0], [], 0.0), O.two_electron_gradient(b, D[0], [], 0.0), "no exchange")
+
+
+@pytest.mark.parametrize("name,basis_name", MOLECULES)
+def test_jk_and_difference_build(name, basis_name):
+    """Full builds, and difference builds (queued ket pairs) whose threshold drops at most 1e-15 a quartet."""
+    import torch
+    from aimd_b200 import integrals as I
+    from aimd_b200.engine import engine_for
+    from oracle import hf_oracle as O
+    b, D = _case(name, basis_name)
+    J, K = I.jk(b, D)
+    Jr, Kr = O.jk_direct(b, D)
+    _close(J, Jr, "J")
+    _close(K, Kr, "K")
+    Dt = torch.as_tensor(D, device="cuda")
+    for scale in (1.0, 1e-4):
+        Ja, Ka = engine_for(b).jk_delta_acc(scale * Dt, 1e-12, 1e-15 * scale)
+        _close((Ja + Ja.transpose(1, 2)).cpu().numpy() / scale, Jr, "difference J")
+        _close((Ka + Ka.transpose(1, 2)).cpu().numpy() / scale, Kr, "difference K")
+
+
+@pytest.mark.parametrize("name,basis_name", MOLECULES)
+def test_schwarz_bounds(name, basis_name):
+    from aimd_b200 import integrals as I
+    from oracle import hf_oracle as O
+    b, _ = _case(name, basis_name)
+    Q = O.schwarz_bounds(b)
+    # Q^2 = max (ab|ab) is what is computed: rounding is relative to the largest integral
+    assert np.abs(I.schwarz_bounds(b) ** 2 - Q ** 2).max() <= 1e-12 * max(1.0, Q.max() ** 2)
