@@ -644,17 +644,6 @@ int class_status(aimd_ctx* c, cudaError_t r, const char* what, int cl, int nlaun
     return AIMD_ERR_CUDA;
 }
 
-#define AIMD_EACH_CLASS(CALL, WHAT)                                         \
-    do {                                                                    \
-        int r_;                                                             \
-        if ((r_ = class_status(c, CALL(0), WHAT, 0, cls_size(c, 0) > 0))) return r_;  \
-        if ((r_ = class_status(c, CALL(1), WHAT, 1, cls_size(c, 1) > 0))) return r_;  \
-        if ((r_ = class_status(c, CALL(2), WHAT, 2, cls_size(c, 2) > 0))) return r_;  \
-        if ((r_ = class_status(c, CALL(3), WHAT, 3, cls_size(c, 3) > 0))) return r_;  \
-        if ((r_ = class_status(c, CALL(4), WHAT, 4, cls_size(c, 4) > 0))) return r_;  \
-        if ((r_ = class_status(c, CALL(5), WHAT, 5, cls_size(c, 5) > 0))) return r_;  \
-    } while (0)
-
 // The six class launches of one call run concurrently on the context's
 // class streams, forked from and joined back into the caller's stream, so
 // the long-running d-shell classes overlap the others.
@@ -734,8 +723,10 @@ extern "C" int aimd_set_geometry(aimd_ctx* c, const double* pos, void* stream) {
     {
         const LaunchEnv e = launch_env(c);
         const QuartetArgs q = quartet_args(c, c->counts_jk);
-#define AIMD_SCHWARZ(X) launch_schwarz_c##X(e, q, st)
-        AIMD_EACH_CLASS(AIMD_SCHWARZ, "aimd_set_geometry/schwarz");
+#define AIMD_SCHWARZ(X, S) launch_schwarz_c##X(e, q, S)
+#define AIMD_NL(X) (cls_size(c, X) > 0 ? 1 : 0)
+        AIMD_EACH_CLASS_CONCURRENT(AIMD_SCHWARZ, "aimd_set_geometry/schwarz", AIMD_NL);
+#undef AIMD_NL
 #undef AIMD_SCHWARZ
     }
     // order: Q descending, then (stable) by segment; segment starts on the device
@@ -1086,31 +1077,33 @@ ShellView shell_view(aimd_ctx* c) {
 extern "C" int aimd_onee(aimd_ctx* c, const double* origin, double* S, double* T, double* M, double* V,
                          void* stream) {
     if (!c || !S || !T || !M || !V || !c->have_geometry) return AIMD_ERR_ARG;
-    int n = 0;
-    cudaError_t r = launch_onee(launch_env(c), shell_view(c), c->sp_cls_start, origin, S, T, M, V,
-                                static_cast<cudaStream_t>(stream), &n);
-    c->launches += n;
-    CK(r);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const LaunchEnv e = launch_env(c);
+    const ShellView sv = shell_view(c);
+#define AIMD_ONEE(X, S_) launch_onee(e, sv, X, c->sp_cls_start, origin, S, T, M, V, S_)
+#define AIMD_NL(X) (c->sp_cls_start[X + 1] > c->sp_cls_start[X] ? 1 : 0)
+    AIMD_EACH_CLASS_CONCURRENT(AIMD_ONEE, "aimd_onee", AIMD_NL);
+#undef AIMD_ONEE
     return AIMD_OK;
 }
 
 extern "C" int aimd_onee_grad(aimd_ctx* c, const double* W, const double* D, double* grad, void* stream) {
     if (!c || !W || !D || !grad || !c->have_geometry) return AIMD_ERR_ARG;
-    int n = 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CK(cudaMemsetAsync(c->gacc, 0, sizeof(facc) * 3 * c->natm, st));
-    cudaError_t r = launch_onee_grad(launch_env(c), shell_view(c), c->sp_cls_start, W, D, c->gacc, st, &n);
-    if (r == cudaSuccess) {
-        from_fixed(st, 3 * (size_t)c->natm, c->gacc, nullptr, FIX_G, grad, 1);
-        ++n;
-        r = cudaGetLastError();
-    }
-    c->launches += n;
-    if (r == cudaErrorInvalidConfiguration) {
+    if (sizeof(facc) * 3 * c->natm > 48 * 1024) {
         snprintf(g_err, sizeof g_err, "aimd_onee_grad: too many atoms for the shared accumulator");
         return AIMD_ERR_UNSUPPORTED;
     }
-    CK(r);
+    CK(cudaMemsetAsync(c->gacc, 0, sizeof(facc) * 3 * c->natm, st));
+    const LaunchEnv e = launch_env(c);
+    const ShellView sv = shell_view(c);
+#define AIMD_ONEE_G(X, S_) launch_onee_grad(e, sv, X, c->sp_cls_start, W, D, c->gacc, S_)
+    AIMD_EACH_CLASS_CONCURRENT(AIMD_ONEE_G, "aimd_onee_grad", AIMD_NL);
+#undef AIMD_ONEE_G
+#undef AIMD_NL
+    from_fixed(st, 3 * (size_t)c->natm, c->gacc, nullptr, FIX_G, grad, 1);
+    ++c->launches;
+    CK(cudaGetLastError());
     return AIMD_OK;
 }
 

@@ -63,10 +63,11 @@ AIMD_DECLARE_CLASS(5)
 #undef AIMD_DECLARE_CLASS
 #undef AIMD_DECLARE_TYPED
 
-cudaError_t launch_onee(const LaunchEnv& e, const ShellView& sv, const int* sp_cls_start, const double* origin,
-                        double* S, double* T, double* M, double* V, cudaStream_t st, int* nlaunch);
-cudaError_t launch_onee_grad(const LaunchEnv& e, const ShellView& sv, const int* sp_cls_start, const double* W,
-                             const double* D, facc* grad, cudaStream_t st, int* nlaunch);
+// one-electron kernels of shell-pair class cl
+cudaError_t launch_onee(const LaunchEnv& e, const ShellView& sv, int cl, const int* sp_cls_start, const double* origin,
+                        double* S, double* T, double* M, double* V, cudaStream_t st);
+cudaError_t launch_onee_grad(const LaunchEnv& e, const ShellView& sv, int cl, const int* sp_cls_start, const double* W,
+                             const double* D, facc* grad, cudaStream_t st);
 
 constexpr size_t kSmemLimit = 227 * 1024;     // dynamic shared memory per CTA (sm_100a)
 

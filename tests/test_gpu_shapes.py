@@ -81,3 +81,15 @@ def test_schwarz_bounds(name, basis_name):
     Q = O.schwarz_bounds(b)
     # Q^2 = max (ab|ab) is what is computed: rounding is relative to the largest integral
     assert np.abs(I.schwarz_bounds(b) ** 2 - Q ** 2).max() <= 1e-12 * max(1.0, Q.max() ** 2)
+
+
+@pytest.mark.parametrize("name,basis_name", MOLECULES)
+def test_one_electron(name, basis_name):
+    from aimd_b200 import integrals as I
+    from oracle import hf_oracle as O
+    b, D = _case(name, basis_name)
+    S, T, V = I.one_electron_matrices(b)
+    for got, ref, what in zip((S, T, V), O.one_electron_matrices(b), "STV"):
+        _close(got, ref, what)
+    _close(I.dipole_integrals(b), O.dipole_integrals(b), "dipole")
+    _close(I.one_electron_gradient(b, D[0], D[1]), O.one_electron_gradient(b, D[0], D[1]), "gradient")
