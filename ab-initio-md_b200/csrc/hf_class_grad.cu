@@ -34,7 +34,7 @@ cudaError_t AIMD_GRAD_NAME(const LaunchEnv& e, const GradArgs& a0, cudaStream_t 
     if (cnt == 0 || e.cls_count[CY] == 0) return cudaSuccess;
     GradArgs a = a0;
     a.rbuf = grad_rbuf_elems<CX, CY, RT>(e.maxbp[CX], e.maxbp[CY]);
-    const size_t smem = grad_smem_bytes<CX, RT>(e.natm, e.maxbp[CX], a.rbuf);
+    const size_t smem = grad_smem_bytes<CX, CY, RT>(e.natm, e.maxbp[CX], a.rbuf);
     const void* kernel = (const void*)grad2e_bra_kernel<CX, CY, RT>;
     cudaError_t r = set_smem_limit(kernel, smem);
     if (r != cudaSuccess) return r;

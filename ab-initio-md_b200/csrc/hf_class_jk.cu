@@ -44,10 +44,10 @@ cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0, cudaStream_t st) {
     a.rbuf = jk_rbuf_elems<CX, YK, RT>(e.maxbp[CX], YK >= 0 ? e.maxbp[YK] : 1);
     // K rows in shared memory unless they would not fit (large bases) or
     // the context asks for global rows
-    size_t smem = jk_smem_bytes<CX, 1, RT>(e.nao, e.maxbp[CX], a.rbuf, a.kglobal != 0);
+    size_t smem = jk_smem_bytes<CX, 1, (YK < 0 ? 0 : YK), RT>(e.nao, e.maxbp[CX], a.rbuf, a.kglobal != 0);
     if (!a.kglobal && smem + static_smem((const void*)jk_bra_kernel<CX, 1, RT, YK>) > kSmemLimit) {
         a.kglobal = 1;
-        smem = jk_smem_bytes<CX, 1, RT>(e.nao, e.maxbp[CX], a.rbuf, true);
+        smem = jk_smem_bytes<CX, 1, (YK < 0 ? 0 : YK), RT>(e.nao, e.maxbp[CX], a.rbuf, true);
     }
     const void* kernel = (const void*)jk_bra_kernel<CX, 1, RT, YK>;
     cudaError_t r = set_smem_limit(kernel, smem);

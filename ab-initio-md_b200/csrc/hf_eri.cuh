@@ -25,6 +25,8 @@
 // those and the flat item lists, one B200: water 6-31G* 2.67 -> 0.37 ms,
 // (H2O)8 difference build 11.5 -> 4.4 ms, (H2O)32 cc-pVDZ 266 -> 118 ms.
 #pragma once
+#include <type_traits>
+
 #include "hf_device.cuh"
 
 namespace hf {
@@ -71,21 +73,26 @@ struct BraE {
 // (double, or float for the mixed-precision quartets); they are computed in
 // FP64 either way.
 constexpr int SBW = 12;     // per bra primitive: p, 1/p, Px, Py, Pz, a, b, -, c0..c3
-template <typename RT>
-struct BraStageT {
+struct BraInfo {
     int P1, A, B, nbp, aA, aB;
     int nA, nB, oA, oB;
     const double* rec;      // bra primitive records (global)
-    RT* E;                  // [nbp][BraE::SIZE] (shared)
-    RT* SB;                 // [nbp][SBW] (shared)
-    RT* D;                  // gradients: [nbp][BraD::SIZE] derivative coefficients (shared)
 };
-using BraStage = BraStageT<double>;
+// Each thread's view: the pair's integers in shared memory, and pointers
+// derived from the kernel's shared array (held in registers, not in shared
+// memory, so that the compiler knows their address space).
+template <typename RT>
+struct BraStageT {
+    const BraInfo& i;
+    RT* SB;                 // [nbp][SBW] (shared)
+    RT* E;                  // [nbp][BraE::SIZE] (shared)
+    RT* D;                  // gradients: dE/dX_AB in the same layout (shared)
+};
 
 template <typename RT>
 __device__ __forceinline__ void stage_bra_scalars(const BraStageT<RT>& st) {
-    for (int ib = threadIdx.x; ib < st.nbp; ib += blockDim.x) {
-        const double* b = st.rec + (size_t)ib * PPW;
+    for (int ib = threadIdx.x; ib < st.i.nbp; ib += blockDim.x) {
+        const double* b = st.i.rec + (size_t)ib * PPW;
         RT* o = st.SB + (size_t)ib * SBW;
         const double p = b[0] + b[1];
         const double vals[SBW] = {p, 1.0 / p, b[3], b[4], b[5], b[0], b[1], 0.0, b[12], b[13], b[14], b[15]};
@@ -98,9 +105,9 @@ __device__ __forceinline__ void stage_bra_scalars(const BraStageT<RT>& st) {
 template <int LA, int LB, int G, typename RT>
 __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
     using BE = BraE<LA, LB, G>;
-    for (int w = threadIdx.x; w < st.nbp * 3; w += blockDim.x) {
+    for (int w = threadIdx.x; w < st.i.nbp * 3; w += blockDim.x) {
         const int ib = w / 3, d = w % 3;
-        const double* b = st.rec + (size_t)ib * PPW;
+        const double* b = st.i.rec + (size_t)ib * PPW;
         const double p = b[0] + b[1];
         double e[LA + 1 + G][LB + 1 + G][LA + LB + 1 + 2 * G];
         hermite_e<LA + G, LB + G>(b[6 + d], b[9 + d], 0.5 / p, d == 0 ? b[2] : 1.0, e);
@@ -232,10 +239,10 @@ __device__ __forceinline__ void bra_rows(const RT* E, const RT (&X)[KG][nherm(LA
 // RS = false: R_tuv of each primitive quartet is computed here; RS = true:
 // it is read from Rs, [ik][ib][NH(L)] pref * R_tuv staged by the CTA
 // (stage_r below) once for all the columns of the ket pair.
-template <int CX, int CY, typename RT, bool RS = false>
+template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp, int ic,
                                            int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                           const RT* __restrict__ Rs, int ib0, int ib1) {
+                                           const RT* __restrict__ Rs, int ib0, int ib1, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
@@ -312,14 +319,14 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
                 }
             };
             if constexpr (RS) {
-                ket_step(Rs + (size_t)(ik * st.nbp + ib) * nherm(L), RT(1));
+                ket_step(Rs + (size_t)(ik * st.i.nbp + ib) * nherm(L), RT(1));
             } else {
                 const RT p = sb[0];
                 const RT rs = rsqrt_t(p + q);
                 const RT alpha = p * q * rs * rs;
                 const RT pref = RT(TWO_PI_2_5) * sb[1] * (RT(2) * oo2q) * rs;
                 RT R[nherm(L)];
-                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
+                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
                 ket_step(R, pref);
             }
         }
@@ -338,10 +345,10 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
 // primitive quartet: the order for bra pairs with many primitives (ss, ps,
 // pp), where repeating the ket setup per bra primitive would cost more than
 // the bra steps it saves.
-template <int CX, int CY, typename RT>
+template <int CX, int CY, typename RT, typename Boys>
 __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp,
                                                      int ic, int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                     int ib0, int ib1) {
+                                                     int ib0, int ib1, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
@@ -382,7 +389,7 @@ __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, co
             const RT alpha = p * q * rs * rs;
             const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
             RT R[nherm(L)];
-            hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
+            hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
             RT X[1][Q::NHB];
 #pragma unroll
             for (int h = 0; h < Q::NHB; ++h) X[0][h] = RT(0);
@@ -424,11 +431,11 @@ __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, co
 // id (column-blocked items): the ket-outer order with R_tuv of each
 // primitive quartet computed once and applied to every column; the ket E
 // rows of a column come from the per-primitive table at compile-time ic.
-template <int CX, int CY, typename RT>
+template <int CX, int CY, typename RT, typename Boys>
 __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp,
                                                    int id, int kg,
                                                    RT (&v)[QClass<CX, CY>::NC][QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                   int ib0, int ib1) {
+                                                   int ib0, int ib1, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
@@ -470,7 +477,7 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
             const RT alpha = p * q * rs * rs;
             const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
             RT R[nherm(L)];
-            hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
+            hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
             const RT* E = st.E + (size_t)ib * BE::SIZE;
 #pragma unroll
             for (int ic = 0; ic < Q::NC; ++ic) {
@@ -518,12 +525,12 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
 // (row r | cd) of a quartet column: bra-outer order (the bra step once per
 // bra primitive) for the d-shell bra classes, whose pairs have few
 // primitives, and the ket-outer order for the others.
-template <int CX, int CY, typename RT, bool RS = false>
+template <int CX, int CY, typename RT, bool RS = false, typename Boys = BoysSeries>
 __device__ __forceinline__ void eri_column(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp, int ic,
                                            int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                           const RT* __restrict__ Rs, int ib0, int ib1) {
-    if constexpr (RS || CX >= 3) eri_column_bra_outer<CX, CY, RT, RS>(st, rk, nkp, ic, id, kg, v, Rs, ib0, ib1);
-    else eri_column_ket_outer<CX, CY, RT>(st, rk, nkp, ic, id, kg, v, ib0, ib1);
+                                           const RT* __restrict__ Rs, int ib0, int ib1, Boys boys = Boys()) {
+    if constexpr (RS || CX >= 3) eri_column_bra_outer<CX, CY, RT, RS>(st, rk, nkp, ic, id, kg, v, Rs, ib0, ib1, boys);
+    else eri_column_ket_outer<CX, CY, RT>(st, rk, nkp, ic, id, kg, v, ib0, ib1, boys);
 }
 
 // Everything the quartet kernels share.
@@ -538,6 +545,7 @@ struct QuartetArgs {
     // nullptr: everything in FP64.
     const int64_t* counts_hi;
     const int* seg_start;       // [NSEG + 1] sorted position of each segment (device)
+    const double* boys;         // Boys tables of all orders (device)
     int npair;
     int cls_start[NCLS + 1];    // sorted positions of each angular class (geometry independent)
     int nao;
@@ -642,8 +650,7 @@ __device__ __forceinline__ void next_chunk(const WorkPlan& plan, int nbra, int* 
     b = sh[1];
 }
 
-template <typename RT>
-__device__ __forceinline__ void load_stage(const QuartetArgs& a, int P1, BraStageT<RT>& st, RT* E) {
+__device__ __forceinline__ void load_info(const QuartetArgs& a, int P1, BraInfo& st) {
     st.P1 = P1;
     st.A = a.pv.pa_blk[P1];
     st.B = a.pv.pb_blk[P1];
@@ -655,9 +662,33 @@ __device__ __forceinline__ void load_stage(const QuartetArgs& a, int P1, BraStag
     st.nB = a.bv.ncon[st.B];
     st.oA = a.bv.ao[st.A];
     st.oB = a.bv.ao[st.B];
-    st.SB = E;                                   // [nbp][SBW] scalars, then the E tables
-    st.E = E + (size_t)st.nbp * SBW;
 }
+// The stage in the shared array E: [nbp][SBW] scalars, then the E tables of
+// `size` elements a primitive, then (gradients) the dE/dX_AB tables.
+template <typename RT>
+__device__ __forceinline__ BraStageT<RT> stage_view(const BraInfo& info, RT* E, int size) {
+    RT* e = E + info.nbp * SBW;
+    return BraStageT<RT>{info, E, e, e + info.nbp * size};
+}
+
+// How the quartets of one kernel evaluate the Boys function of order L: from
+// the shared table (copied by the CTA before its first chunk) or by series.
+template <int L, typename RT, bool TABLE>
+struct BoysOf {
+    static constexpr bool table = TABLE && sizeof(RT) == sizeof(double);
+    using type = std::conditional_t<table, BoysShared, BoysSeries>;
+    static constexpr int elems = table ? BOYS_COLS * boys_rows(L) : 0;      // doubles of shared memory
+    __device__ static type get(const double* shared) {
+        if constexpr (table) return type{shared};
+        else return type{};
+    }
+    __device__ static void stage(const double* tables, double* shared) {
+        if constexpr (table) {
+            const double2* src = reinterpret_cast<const double2*>(tables + boys_offset(L));
+            for (int i = threadIdx.x; i < elems / 2; i += blockDim.x) reinterpret_cast<double2*>(shared)[i] = __ldg(src + i);
+        }
+    }
+};
 
 struct JKArgs {
     QuartetArgs q;
@@ -695,7 +726,7 @@ __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, 
     using Q = QClass<CX, CY>;
     const BlockView& bv = a.q.bv;
     const int nC = bv.ncon[C], nD = bv.ncon[Dd], oC = bv.ao[C], oD = bv.ao[Dd];
-    const double g = 1.0 / ((st.A == st.B ? 2.0 : 1.0) * (C == Dd ? 2.0 : 1.0) * (st.P1 == P2 ? 2.0 : 1.0));
+    const double g = 1.0 / ((st.i.A == st.i.B ? 2.0 : 1.0) * (C == Dd ? 2.0 : 1.0) * (st.i.P1 == P2 ? 2.0 : 1.0));
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
     const double fx = __ldg(a.fix);
@@ -731,13 +762,13 @@ __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, 
                 for (int ka = 0; ka < Q::KA; ++ka)
 #pragma unroll
                     for (int kb = 0; kb < Q::KB; ++kb) {
-                        if (ka >= st.nA || kb >= st.nB) continue;
+                        if (ka >= st.i.nA || kb >= st.i.nB) continue;
 #pragma unroll
                         for (int ia = 0; ia < Q::NA; ++ia)
 #pragma unroll
                             for (int jb = 0; jb < Q::NB; ++jb) {
-                                const int r = (ka * st.nB + kb) * Q::NAB + ia * Q::NB + jb;
-                                const int m = st.oA + ka * Q::NA + ia, nb_ = st.oB + kb * Q::NB + jb;
+                                const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
+                                const int m = st.i.oA + ka * Q::NA + ia, nb_ = st.i.oB + kb * Q::NB + jb;
                                 jcd += v[r][kk] * __ldg(D + (size_t)m * n + nb_);
                                 Jt[(s * Q::NROW + r) * blockDim.x + threadIdx.x] += 2.0 * g * v[r][kk] * dls;
                             }
@@ -748,40 +779,40 @@ __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, 
                 for (int ka = 0; ka < Q::KA; ++ka)
 #pragma unroll
                     for (int ia = 0; ia < Q::NA; ++ia) {
-                        if (ka >= st.nA) continue;
+                        if (ka >= st.i.nA) continue;
                         double s1 = 0.0, s2 = 0.0;
 #pragma unroll
                         for (int kb = 0; kb < Q::KB; ++kb)
 #pragma unroll
                             for (int jb = 0; jb < Q::NB; ++jb) {
-                                if (kb >= st.nB) continue;
-                                const int r = (ka * st.nB + kb) * Q::NAB + ia * Q::NB + jb;
-                                const size_t nb_ = st.oB + kb * Q::NB + jb;
+                                if (kb >= st.i.nB) continue;
+                                const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
+                                const size_t nb_ = st.i.oB + kb * Q::NB + jb;
                                 s1 += v[r][kk] * __ldg(D + nb_ * n + sg);
                                 s2 += v[r][kk] * __ldg(D + nb_ * n + l);
                             }
-                        kadd(ka * Q::NA + ia, st.oA + ka * Q::NA + ia, l, g * s1);
-                        kadd(ka * Q::NA + ia, st.oA + ka * Q::NA + ia, sg, g * s2);
+                        kadd(ka * Q::NA + ia, st.i.oA + ka * Q::NA + ia, l, g * s1);
+                        kadd(ka * Q::NA + ia, st.i.oA + ka * Q::NA + ia, sg, g * s2);
                     }
                 // K[n, l] and K[n, sg]: rows of B's functions
 #pragma unroll
                 for (int kb = 0; kb < Q::KB; ++kb)
 #pragma unroll
                     for (int jb = 0; jb < Q::NB; ++jb) {
-                        if (kb >= st.nB) continue;
+                        if (kb >= st.i.nB) continue;
                         double s1 = 0.0, s2 = 0.0;
 #pragma unroll
                         for (int ka = 0; ka < Q::KA; ++ka)
 #pragma unroll
                             for (int ia = 0; ia < Q::NA; ++ia) {
-                                if (ka >= st.nA) continue;
-                                const int r = (ka * st.nB + kb) * Q::NAB + ia * Q::NB + jb;
-                                const size_t m = st.oA + ka * Q::NA + ia;
+                                if (ka >= st.i.nA) continue;
+                                const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
+                                const size_t m = st.i.oA + ka * Q::NA + ia;
                                 s1 += v[r][kk] * __ldg(D + m * n + sg);
                                 s2 += v[r][kk] * __ldg(D + m * n + l);
                             }
-                        kadd(NFA + kb * Q::NB + jb, st.oB + kb * Q::NB + jb, l, g * s1);
-                        kadd(NFA + kb * Q::NB + jb, st.oB + kb * Q::NB + jb, sg, g * s2);
+                        kadd(NFA + kb * Q::NB + jb, st.i.oB + kb * Q::NB + jb, l, g * s1);
+                        kadd(NFA + kb * Q::NB + jb, st.i.oB + kb * Q::NB + jb, sg, g * s2);
                     }
             }
     }
@@ -919,7 +950,7 @@ __device__ __forceinline__ void plan_window(const QuartetArgs& q, int spos, int 
 template <typename Keep, typename Work>
 __device__ __forceinline__ void flat_items(FlatItems& f, bool queued, int* queue, Keep keep, Work work) {
     constexpr int PER = LQ_CAP / 128;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int total = f.kpre[NSUB];
     for (int base = 0; base < total; base += queued ? LQ_CAP : total) {
         if (queued) {
@@ -1060,7 +1091,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
     constexpr int NH = nherm(L);
     constexpr int B = RSmem<L, RT>::RB_PQ;
     const int lane = threadIdx.x & 31;
-    const int nbp = st.nbp;
+    const int nbp = st.i.nbp;
     for (int64_t base = 0; base < cnt; base += KQ_CAP) {
         const int m = static_cast<int>(cnt - base < KQ_CAP ? cnt - base : KQ_CAP);
         compact(q, j0 + static_cast<int>(base), m, keep, [&](int slot, int pos) {
@@ -1130,9 +1161,10 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
 }
 
 // The items of the staged bra pair (position spos) in the window that f holds.
-template <int CX, int CY, int NS, bool KGLOBAL, typename RT>
+template <int CX, int CY, int NS, bool KGLOBAL, typename RT, typename Boys>
 __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT>& st, int spos, double* Jt,
-                                             unsigned* Ksm, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf) {
+                                             unsigned* Ksm, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf,
+                                             Boys boys) {
     using Q = QClass<CX, CY>;
     const double q1 = a.q.sortedQ[spos];
     const double* bm = a.bmax;
@@ -1142,9 +1174,9 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
         if (!bm) return true;
         const int P2 = a.q.sorted[pos];
         const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-        const double dm = fmax(fmax(bm[st.A * nb + st.B], bm[C * nb + Dd]),
-                               fmax(fmax(bm[st.A * nb + C], bm[st.A * nb + Dd]),
-                                    fmax(bm[st.B * nb + C], bm[st.B * nb + Dd])));
+        const double dm = fmax(fmax(bm[st.i.A * nb + st.i.B], bm[C * nb + Dd]),
+                               fmax(fmax(bm[st.i.A * nb + C], bm[st.i.A * nb + Dd]),
+                                    fmax(bm[st.i.B * nb + C], bm[st.i.B * nb + Dd])));
         return q1 * a.q.sortedQ[pos] * dm >= a.dthr;
     };
     auto digest = [&](int P2, int C, int Dd, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
@@ -1162,21 +1194,22 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
     };
     // item r = (contraction group that the segment's pairs carry, bra-primitive split, column block)
     auto work = [&](int sub, int pos, int r, const RT* Rs) {
-        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.nbp, sub, a.item_pq);
+        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
-        const int ib0 = st.nbp * sp / nsp, ib1 = st.nbp * (sp + 1) / nsp;
+        const int ib0 = st.i.nbp * sp / nsp, ib1 = st.i.nbp * (sp + 1) / nsp;
         const int P2 = a.q.sorted[pos];
         const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
         const double* rk = a.q.pv.rec + a.q.pv.slot[P2] * PPW;
         if constexpr (Q::CBLK) {
             // item = the NC columns of one id
             RT v[Q::NC][Q::NROW][Q::KG];
-            eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1);
+            eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1, boys);
 #pragma unroll
             for (int ic = 0; ic < Q::NC; ++ic) digest(P2, C, Dd, ic, cd, kg, v[ic]);
         } else {
             RT v[Q::NROW][Q::KG];
-            eri_column<CX, CY, RT, Q::RSMEM>(st, rk, a.q.pv.npp[P2], cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1);
+            eri_column<CX, CY, RT, Q::RSMEM>(st, rk, a.q.pv.npp[P2], cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1,
+                                                 boys);
             digest(P2, C, Dd, cd / Q::ND, cd % Q::ND, kg, v);
         }
     };
@@ -1207,8 +1240,16 @@ struct JKKernel {
     static constexpr int KROWS = KGLOBAL ? 0 : NS * NF;
 };
 
-// Dynamic shared memory: K rows [NS][NF][nao] (unless KGLOBAL), per-thread
-// J_ab slots [NS][NROW][blockDim], bra stage.
+// The Boys function of the (CX, Y) J/K kernel: from the table up to the ds
+// bras. The dp bras hold the most K rows (58 KB at 800 AOs); with the table
+// beside them the L1 cache shrinks by as much and their kernels were 3 to 15 %
+// slower at (H2O)32; for dd it made no difference.
+template <int CX, int Y, typename RT>
+using JKBoys = BoysOf<QClass<CX, Y>::L, RT, (CX <= 3)>;
+
+// Dynamic shared memory: Boys table, per-thread J_ab slots
+// [NS][NROW][blockDim], K rows [NS][NF][nao] (unless KGLOBAL), staged R, bra
+// stage.
 constexpr int JK_THREADS = 128;
 
 // RT = double: the FP64 quartets; RT = float: the FP32 quartets of the
@@ -1224,37 +1265,46 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
     using Q0 = QClass<CX, 0>;
     constexpr int Y = YK < 0 ? 0 : YK;      // the unsplit kernel (CX = 0) has one ket class too
     static_assert(YK >= 0 || CX == 0, "bra classes above ss are split by ket class");
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
     const int krows = a.kglobal ? 0 : KK::KROWS;
-    unsigned* Ksm = reinterpret_cast<unsigned*>(smem);     // low words of the K rows, then the high words
-    double* Jt = smem + (size_t)krows * n;
-    RT* Rbuf = reinterpret_cast<RT*>(Jt + NS * KK::NROW * JK_THREADS);
-    RT* Esm = Rbuf + a.rbuf;
     using QY = QClass<CX, Y>;
-    __shared__ BraStageT<RT> st;
+    using Boys = JKBoys<CX, Y, RT>;
+    double* btab = smem;                                    // Boys table
+    double* Jt = btab + Boys::elems;                        // per-thread J_ab slots
+    unsigned* Ksm = reinterpret_cast<unsigned*>(Jt + NS * KK::NROW * JK_THREADS);   // low words of the K rows, then the high words
+    RT* Rbuf = reinterpret_cast<RT*>(Jt + NS * KK::NROW * JK_THREADS + (size_t)krows * n);
+    RT* Esm = Rbuf + a.rbuf;
+    __shared__ BraInfo info;
     __shared__ FlatItems f;
     __shared__ QueueOf<QY::RSMEM> kq;
     __shared__ int sh[2];
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
+    bool staged = false;        // the Boys table is in shared memory
     for (;;) {
         int c, b;
         next_chunk(a.plan, nbra, sh, c, b);
         if (c >= total) break;                                  // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
-        if (threadIdx.x == 0) load_stage(a.q, a.q.sorted[spos], st, Esm);
-        for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * JK_THREADS; i += blockDim.x) smem[i] = 0.0;
+        if (threadIdx.x == 0) load_info(a.q, a.q.sorted[spos], info);
+        if (!staged) {
+            Boys::stage(a.q.boys, btab);
+            staged = true;
+        }
+        for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * JK_THREADS; i += blockDim.x) Jt[i] = 0.0;
         __syncthreads();
+        const BraStageT<RT> st = stage_view(info, Esm, KK::ESIZE);
         if (threadIdx.x < 32) {
             const int sub = threadIdx.x < NSUB ? threadIdx.x : 0;
-            plan_window<CX, Y, RT>(a.q, spos, st.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], QY::NITEM,
-                                   seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.nbp, sub, a.item_pq), f);
+            plan_window<CX, Y, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], QY::NITEM,
+                                   seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
         }
         stage_bra_e<Q0::LA, Q0::LB, 0>(st);
         __syncthreads();
-        jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf);
+        jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf,
+                                                 Boys::get(btab));
         __syncthreads();
         // flush J_ab: one thread per (set, row) sums the per-thread slots
         for (int i = threadIdx.x; i < NS * KK::NROW; i += blockDim.x) {
@@ -1263,8 +1313,8 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
             if (val == 0.0) continue;
             const int s = i / KK::NROW, r = i % KK::NROW;
             const int kab = r / Q0::NAB, ab = r % Q0::NAB;
-            const int ka = kab / st.nB, kb = kab % st.nB;
-            const int m = st.oA + ka * Q0::NA + ab / Q0::NB, nb_ = st.oB + kb * Q0::NB + ab % Q0::NB;
+            const int ka = kab / st.i.nB, kb = kab % st.i.nB;
+            const int m = st.i.oA + ka * Q0::NA + ab / Q0::NB, nb_ = st.i.oB + kb * Q0::NB + ab % Q0::NB;
             fadd(a.J + s * nn + (size_t)m * n + nb_, val, __ldg(a.fix));
         }
         // flush K rows
@@ -1274,7 +1324,7 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
                 const facc val = join_planes(Ksm[i], Ksm[krows * n + i]);
                 if (val == 0) continue;
                 const int col = i % n, f = (i / n) % KK::NF, s = i / (n * KK::NF);
-                const int row = f < NFA ? st.oA + f : st.oB + (f - NFA);
+                const int row = f < NFA ? st.i.oA + f : st.i.oB + (f - NFA);
                 atomicAdd(a.K + s * nn + (size_t)row * n + col, val);     // integer: order-independent
             }
         }
@@ -1292,11 +1342,11 @@ size_t jk_rbuf_elems(int max_bra_prims, int max_ket_prims) {
     return 0;
 }
 
-template <int CX, int NS, typename RT>
+template <int CX, int NS, int Y, typename RT>
 size_t jk_smem_bytes(int nao, int max_bra_prims, size_t rbuf_elems, bool kglobal) {
     using KK = JKKernel<CX, NS>;
     const size_t krows = kglobal ? 0 : KK::KROWS;
-    return sizeof(double) * (krows * nao + (size_t)NS * KK::NROW * JK_THREADS) +
+    return sizeof(double) * (krows * nao + (size_t)NS * KK::NROW * JK_THREADS + JKBoys<CX, Y, RT>::elems) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (KK::ESIZE + SBW));
 }
 
@@ -1311,29 +1361,30 @@ constexpr int SCHWARZ_THREADS = 64;
 template <int CX>
 __global__ void __launch_bounds__(SCHWARZ_THREADS) schwarz_kernel(QuartetArgs a, const int* pairs_of_class, double* Qout) {
     using Q = QClass<CX, CX>;
-    extern __shared__ double smem[];
-    __shared__ BraStage st;
+    extern __shared__ __align__(16) double smem[];
+    __shared__ BraInfo info;
     __shared__ double diag[Q::KAB][SCHWARZ_THREADS];    // partial (ab|ab) of each contraction combination
     __shared__ unsigned long long qmax;
     const int P = pairs_of_class[blockIdx.x];
     if (threadIdx.x == 0) {
-        load_stage(a, P, st, smem);
+        load_info(a, P, info);
         qmax = 0ull;
     }
     __syncthreads();
+    const BraStageT<double> st = stage_view(info, smem, BraE<Q::LA, Q::LB, 0>::SIZE);
     stage_bra_e<Q::LA, Q::LB, 0>(st);
     __syncthreads();
     static_assert(Q::KG == Q::KCD, "diagonal quartets keep all contraction combinations in one item");
     constexpr int NSP = SCHWARZ_THREADS / Q::NCD;       // ranges of the bra primitives
     const int cd = threadIdx.x % Q::NCD, sp = threadIdx.x / Q::NCD;
-    const int ib0 = st.nbp * sp / NSP, ib1 = st.nbp * (sp + 1) / NSP;
+    const int ib0 = st.i.nbp * sp / NSP, ib1 = st.i.nbp * (sp + 1) / NSP;
     if (sp < NSP) {
         double m[Q::KAB];
 #pragma unroll
         for (int kk = 0; kk < Q::KAB; ++kk) m[kk] = 0.0;
         if (ib1 > ib0) {
             double v[Q::NROW][Q::KCD];
-            eri_column<CX, CX>(st, st.rec, st.nbp, cd / Q::ND, cd % Q::ND, 0, v, static_cast<const double*>(nullptr),
+            eri_column<CX, CX>(st, st.i.rec, st.i.nbp, cd / Q::ND, cd % Q::ND, 0, v, static_cast<const double*>(nullptr),
                                ib0, ib1);
 #pragma unroll
             for (int kk = 0; kk < Q::KAB; ++kk)
@@ -1346,7 +1397,7 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS) schwarz_kernel(QuartetArgs a,
     }
     __syncthreads();
     // one thread per (combination, column) sums its ranges in order
-    for (int i = threadIdx.x; i < st.nA * st.nB * Q::NCD; i += SCHWARZ_THREADS) {
+    for (int i = threadIdx.x; i < st.i.nA * st.i.nB * Q::NCD; i += SCHWARZ_THREADS) {
         const int kk = i / Q::NCD, c = i % Q::NCD;
         double m = 0.0;
         for (int s = 0; s < NSP; ++s) m += diag[kk][s * Q::NCD + c];

@@ -71,9 +71,9 @@ constexpr bool grad_rcol() {
 template <int LA, int LB, typename RT>
 __device__ __forceinline__ void stage_bra_de(const BraStageT<RT>& st) {
     using BE = BraE<LA, LB, 0>;
-    for (int w = threadIdx.x; w < st.nbp * 3; w += blockDim.x) {
+    for (int w = threadIdx.x; w < st.i.nbp * 3; w += blockDim.x) {
         const int ib = w / 3, d = w % 3;
-        const double* b = st.rec + (size_t)ib * PPW;
+        const double* b = st.i.rec + (size_t)ib * PPW;
         const double ip = 1.0 / (b[0] + b[1]), pa = b[6 + d], pb = b[9 + d];
         double e[LA + 1][LB + 1][LA + LB + 1], de[LA + 1][LB + 1][LA + LB + 1];
         hermite_e<LA, LB>(pa, pb, 0.5 * ip, d == 0 ? b[2] : 1.0, e);
@@ -98,11 +98,11 @@ __device__ __forceinline__ void stage_bra_de(const BraStageT<RT>& st) {
 // Primitive loops of one gradient column (bra primitives [ib0, ib1)): bra
 // primitives outer, so that Y (the bra's E contracted with the Gamma column)
 // and the U sum, linear in X, are formed once per bra primitive.
-template <int CX, int CY, typename RT, bool RS>
+template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&Gr)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
                                            const double* __restrict__ rk, int nkp, int ic, int id, int kg,
                                            RT (&dA)[3], RT (&dB)[3], RT (&dC)[3], const RT* __restrict__ Rs,
-                                           RT* Rcol, int ib0, int ib1) {
+                                           RT* Rcol, int ib0, int ib1, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L + 1;
@@ -262,14 +262,14 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                 dC[2] += vz - cq * gz;
             };
             if constexpr (RS) {
-                body(Rs + (size_t)(ik * st.nbp + ib) * nherm(L), RT(1));
+                body(Rs + (size_t)(ik * st.i.nbp + ib) * nherm(L), RT(1));
             } else {
                 const RT p = sb[0];
                 const RT rs = rsqrt_t(p + q);
                 const RT alpha = p * q * rs * rs;
                 const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
                 RT R[nherm(L)];
-                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R);
+                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
                 if constexpr (grad_rcol<CX, CY, RT>()) {
 #pragma unroll
                     for (int i = 0; i < nherm(L); ++i) Rcol[i * GRAD_THREADS] = R[i];
@@ -339,19 +339,20 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
 // Gradient contribution of one column; adds A, B parts to gab and C, D
 // parts to the shared accumulator gsh (low words [natm][3], then the high words). RS: pref * R_tuv (to L + 1)
 // of the ket pair's primitive quartets staged in Rs ([ik][ib][NH(L + 1)]).
-template <int CX, int CY, typename RT, bool RS = false>
+template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<RT>& st, int P2, double QQ, int ic,
                                             int id, int kg, double (&gab)[6], unsigned* gsh,
-                                            const RT* __restrict__ Rs, RT* Rcol, int ib0, int ib1) {
+                                            const RT* __restrict__ Rs, RT* Rcol, int ib0, int ib1,
+                                            Boys boys) {
     using Q = QClass<CX, CY>;
     const BlockView& bv = a.q.bv;
     const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
     const int aC = bv.atom[C], aD = bv.atom[Dd];
-    if (st.aA == st.aB && st.aB == aC && aC == aD) return;          // one-centre: invariant
+    if (st.i.aA == st.i.aB && st.i.aB == aC && aC == aD) return;          // one-centre: invariant
     const int nC = bv.ncon[C], nD = bv.ncon[Dd], oC = bv.ao[C], oD = bv.ao[Dd];
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
-    const double deg = 0.5 * (st.A != st.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.P1 != P2 ? 2.0 : 1.0);
+    const double deg = 0.5 * (st.i.A != st.i.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.i.P1 != P2 ? 2.0 : 1.0);
     // Gamma column
     double G[Q::NROW][Q::KG];
     double gmax = 0.0;
@@ -363,10 +364,10 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
         const size_t l = oC + kc * Q::NC + ic, sg = oD + kd * Q::ND + id;
 #pragma unroll
         for (int r = 0; r < Q::NROW; ++r) {
-            const int kab = r / Q::NAB, ab = r % Q::NAB, ka = kab / st.nB, kb = kab % st.nB;
+            const int kab = r / Q::NAB, ab = r % Q::NAB, ka = kab / st.i.nB, kb = kab % st.i.nB;
             double val = 0.0;
-            if (cv && kab < st.nA * st.nB) {
-                const size_t m = st.oA + ka * Q::NA + ab / Q::NB, nb_ = st.oB + kb * Q::NB + ab % Q::NB;
+            if (cv && kab < st.i.nA * st.i.nB) {
+                const size_t m = st.i.oA + ka * Q::NA + ab / Q::NB, nb_ = st.i.oB + kb * Q::NB + ab % Q::NB;
                 val = __ldg(a.Dc + m * n + nb_) * __ldg(a.Dc + l * n + sg);
                 for (int x = 0; x < a.nx; ++x) {
                     const double* X = a.Dx + x * nn;
@@ -388,7 +389,7 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
         for (int kk = 0; kk < Q::KG; ++kk) Gr[r][kk] = static_cast<RT>(G[r][kk]);
     RT dA[3] = {0.0, 0.0, 0.0}, dB[3] = {0.0, 0.0, 0.0}, dC[3] = {0.0, 0.0, 0.0};
     grad_prims<CX, CY, RT, RS>(st, Gr, a.q.pv.rec + a.q.pv.slot[P2] * PPW, a.q.pv.npp[P2], ic, id, kg, dA, dB, dC, Rs,
-                               Rcol, ib0, ib1);
+                               Rcol, ib0, ib1, boys);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double da = dA[d], db = dB[d], dc = dC[d];
@@ -404,9 +405,10 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
 // |Dx|_AD |Dx|_BC)] >= max|Gamma|, can reach the threshold and the quartet
 // is not one-centre; the exact per-column test follows in grad_column.
 
-template <int CX, int CY, typename RT>
+template <int CX, int CY, typename RT, typename Boys>
 __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStageT<RT>& st, int spos, double (&gab)[6],
-                                               unsigned* gsh, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf) {
+                                               unsigned* gsh, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf,
+                                               Boys boys) {
     using Q = QClass<CX, CY>;
     constexpr bool RS = grad_rsmem<CX, CY>();
     const double q1 = a.q.sortedQ[spos];
@@ -416,19 +418,19 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
         const int P2 = a.q.sorted[pos];
         const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
         const int aC = a.q.bv.atom[C], aD = a.q.bv.atom[Dd];
-        if (st.aA == st.aB && st.aB == aC && aC == aD) return false;
-        double gb = a.bmc[st.A * nb + st.B] * a.bmc[C * nb + Dd];
+        if (st.i.aA == st.i.aB && st.i.aB == aC && aC == aD) return false;
+        double gb = a.bmc[st.i.A * nb + st.i.B] * a.bmc[C * nb + Dd];
         if (a.nx > 0)
-            gb += xf * (a.bmx[st.A * nb + C] * a.bmx[st.B * nb + Dd] + a.bmx[st.A * nb + Dd] * a.bmx[st.B * nb + C]);
-        const double deg = 0.5 * (st.A != st.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.P1 != P2 ? 2.0 : 1.0);
+            gb += xf * (a.bmx[st.i.A * nb + C] * a.bmx[st.i.B * nb + Dd] + a.bmx[st.i.A * nb + Dd] * a.bmx[st.i.B * nb + C]);
+        const double deg = 0.5 * (st.i.A != st.i.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.i.P1 != P2 ? 2.0 : 1.0);
         return q1 * a.q.sortedQ[pos] * deg * gb >= a.thr;
     };
     // item r = (contraction group, bra-primitive split, column)
     auto work = [&](int sub, int pos, int r, const RT* Rs) {
-        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.nbp, sub, a.item_pq);
+        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         grad_column<CX, CY, RT, RS>(a, st, a.q.sorted[pos], q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
-                                    gsh, Rs, Rbuf + threadIdx.x, st.nbp * sp / nsp, st.nbp * (sp + 1) / nsp);
+                                    gsh, Rs, Rbuf + threadIdx.x, st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp, boys);
     };
     if constexpr (RS) {
         int rot = 0;
@@ -442,10 +444,16 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
     }
 }
 
+// The Boys function of the (CX, CY) gradient kernel: from the table up to
+// order L + 1 = 5, where the table and the R columns leave room for two CTAs
+// an SM (58 + 29 KB); by series above.
+template <int CX, int CY, typename RT>
+using GradBoys = BoysOf<QClass<CX, CY>::L + 1, RT, (QClass<CX, CY>::L + 1 <= 5)>;
+
 // One kernel per (bra class, ket class), persistent: a CTA runs chunks
 // (bra pair of class CX, window of its ket pairs of class CY) of the
 // launch's work plan until it is used up. Dynamic shared memory: gradient
-// accumulator [natm][3] (one per CTA, flushed at the end), staged R, bra E
+// accumulator [natm][3] (one per CTA, flushed at the end), Boys table, staged R, bra E
 // tables (+1).
 // RT = double: the FP64 quartets; RT = float: the FP32 quartets of the
 // mixed-precision path (accumulated in FP64).
@@ -456,41 +464,46 @@ template <int CX, int CY, typename RT>
 __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kernel(GradArgs a) {
     using Q0 = QClass<CX, 0>;
     using Q = QClass<CX, CY>;
-    extern __shared__ double smem[];
-    unsigned* gsh = reinterpret_cast<unsigned*>(smem);      // low words [natm][3], then the high words
-    RT* Rbuf = reinterpret_cast<RT*>(smem + 3 * a.natm);
+    using Boys = GradBoys<CX, CY, RT>;
+    extern __shared__ __align__(16) double smem[];
+    double* btab = smem;                                                // Boys table
+    unsigned* gsh = reinterpret_cast<unsigned*>(btab + Boys::elems);    // low words [natm][3], then the high words
+    RT* Rbuf = reinterpret_cast<RT*>(btab + Boys::elems + 3 * a.natm);
     RT* Esm = Rbuf + a.rbuf;
-    __shared__ BraStageT<RT> st;
+    __shared__ BraInfo info;
     __shared__ FlatItems f;
     __shared__ QueueOf<grad_rsmem<CX, CY>()> kq;
     __shared__ int sh[2];
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
     for (int i = threadIdx.x; i < 6 * a.natm; i += blockDim.x) gsh[i] = 0u;
+    bool staged = false;        // the Boys table is in shared memory
     auto gadd = [&](int i, double v) { sadd(gsh + i, gsh + 3 * a.natm + i, v, FIX_G); };
     for (;;) {
         int c, b;
         next_chunk(a.plan, nbra, sh, c, b);                     // (its barrier also orders the zeroing)
         if (c >= total) break;                                  // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
-        if (threadIdx.x == 0) {
-            load_stage(a.q, a.q.sorted[spos], st, Esm);
-            st.D = st.E + (size_t)st.nbp * BraE<Q0::LA, Q0::LB, 0>::SIZE;
+        if (threadIdx.x == 0) load_info(a.q, a.q.sorted[spos], info);
+        if (!staged) {
+            Boys::stage(a.q.boys, btab);
+            staged = true;
         }
         __syncthreads();
+        const BraStageT<RT> st = stage_view(info, Esm, BraE<Q0::LA, Q0::LB, 0>::SIZE);
         if (threadIdx.x < 32) {
             const int sub = threadIdx.x < NSUB ? threadIdx.x : 0;
-            plan_window<CX, CY, RT>(a.q, spos, st.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], Q::NCD,
-                                    seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.nbp, sub, a.item_pq), f);
+            plan_window<CX, CY, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], Q::NCD,
+                                    seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
         }
         stage_bra_de<Q0::LA, Q0::LB>(st);
         __syncthreads();
         double gab[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        grad_ket_class<CX, CY, RT>(a, st, spos, gab, gsh, f, kq.r(), kq.flat(), Rbuf);
+        grad_ket_class<CX, CY, RT>(a, st, spos, gab, gsh, f, kq.r(), kq.flat(), Rbuf, Boys::get(btab));
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            if (gab[d] != 0.0) gadd(3 * st.aA + d, gab[d]);
-            if (gab[3 + d] != 0.0) gadd(3 * st.aB + d, gab[3 + d]);
+            if (gab[d] != 0.0) gadd(3 * st.i.aA + d, gab[d]);
+            if (gab[3 + d] != 0.0) gadd(3 * st.i.aB + d, gab[3 + d]);
         }
         __syncthreads();
     }
@@ -510,10 +523,10 @@ size_t grad_rbuf_elems(int max_bra_prims, int max_ket_prims) {
     return 0;
 }
 
-template <int CX, typename RT>
+template <int CX, int CY, typename RT>
 size_t grad_smem_bytes(int natm, int max_bra_prims, size_t rbuf_elems) {
     using Q0 = QClass<CX, 0>;
-    return sizeof(double) * 3 * (size_t)natm +
+    return sizeof(double) * (3 * (size_t)natm + GradBoys<CX, CY, RT>::elems) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (2 * BraE<Q0::LA, Q0::LB, 0>::SIZE + SBW));
 }
 

@@ -93,3 +93,19 @@ def test_one_electron(name, basis_name):
         _close(got, ref, what)
     _close(I.dipole_integrals(b), O.dipole_integrals(b), "dipole")
     _close(I.one_electron_gradient(b, D[0], D[1]), O.one_electron_gradient(b, D[0], D[1]), "gradient")
+
+
+@pytest.mark.parametrize("distance", [0.3, 1.4, 2.9, 4.4, 5.1, 6.3, 9.0, 17.0])
+def test_boys_arguments(distance):
+    """An O-H pair from overlapping to far apart: Boys arguments 0 to some thousands, both sides of the table's end."""
+    from aimd_b200 import integrals as I
+    from aimd_b200.basis import build_basis
+    from oracle import hf_oracle as O
+    x = np.array([[0.0, 0.0, 0.0], distance * np.array([0.48, 0.60, 0.64])])
+    b = build_basis(["O", "H"], x, "cc-pvdz")
+    rng = np.random.default_rng(3)
+    D = rng.normal(size=(b.nao, b.nao))
+    D = D + D.T
+    for got, ref, what in zip(I.jk(b, D), O.jk_direct(b, D), "JK"):
+        _close(got, ref, what)
+    _close(I.two_electron_gradient(b, D, [D], 0.5), O.two_electron_gradient(b, D, [D], 0.5), "gradient")
