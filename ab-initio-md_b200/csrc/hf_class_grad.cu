@@ -29,17 +29,22 @@ using RT = float;
 #define AIMD_GRAD_NAME AIMD_CAT(AIMD_CAT(AIMD_CAT(launch_grad32_c, AIMD_CLASS), _), AIMD_KET)
 #endif
 
-cudaError_t AIMD_GRAD_NAME(const LaunchEnv& e, const GradArgs& a0, cudaStream_t st) {
+cudaError_t AIMD_GRAD_NAME(const LaunchEnv& e, const GradArgs& a0) {
     const int cnt = e.cls_count[CX];
     if (cnt == 0 || e.cls_count[CY] == 0) return cudaSuccess;
+    constexpr int rt = sizeof(RT) == sizeof(double) ? 0 : 1;
     GradArgs a = a0;
     a.rbuf = grad_rbuf_elems<CX, CY, RT>(e.maxbp[CX], e.maxbp[CY]);
     const size_t smem = grad_smem_bytes<CX, CY, RT>(e.natm, e.maxbp[CX], a.rbuf);
     const void* kernel = (const void*)grad2e_bra_kernel<CX, CY, RT>;
-    cudaError_t r = set_smem_limit(kernel, smem);
-    if (r != cudaSuccess) return r;
-    a.plan = e.plan_of(CX, CY, sizeof(RT) == sizeof(double) ? 0 : 1);
-    grad2e_bra_kernel<CX, CY, RT><<<persistent_grid(kernel, GRAD_THREADS, smem, e.nsm), GRAD_THREADS, smem, st>>>(a);
+    LaunchSlot& slot = e.slot(1, rt, CX, CY);
+    if (slot.grid == 0) {
+        cudaError_t r = set_smem_limit(kernel, smem);
+        if (r != cudaSuccess) return r;
+        slot.grid = persistent_grid(kernel, GRAD_THREADS, smem, e.nsm);
+    }
+    a.plan = e.plan_of(CX, CY, rt);
+    grad2e_bra_kernel<CX, CY, RT><<<slot.grid, GRAD_THREADS, smem, e.stream_of(CX, CY)>>>(a);
     return cudaGetLastError();
 }
 

@@ -39,40 +39,47 @@ using RT = float;
 // unit's copy for all of them.
 namespace {
 template <int YK>
-cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0, cudaStream_t st) {
+cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0) {
+    constexpr int Y = YK < 0 ? 0 : YK;
+    constexpr int rt = sizeof(RT) == sizeof(double) ? 0 : 1;
     JKArgs a = a0;
-    a.rbuf = jk_rbuf_elems<CX, YK, RT>(e.maxbp[CX], YK >= 0 ? e.maxbp[YK] : 1);
-    // K rows in shared memory unless they would not fit (large bases) or
-    // the context asks for global rows
-    size_t smem = jk_smem_bytes<CX, 1, (YK < 0 ? 0 : YK), RT>(e.nao, e.maxbp[CX], a.rbuf, a.kglobal != 0);
-    if (!a.kglobal && smem + static_smem((const void*)jk_bra_kernel<CX, 1, RT, YK>) > kSmemLimit) {
-        a.kglobal = 1;
-        smem = jk_smem_bytes<CX, 1, (YK < 0 ? 0 : YK), RT>(e.nao, e.maxbp[CX], a.rbuf, true);
-    }
+    a.rbuf = jk_rbuf_elems<CX, YK, RT>(e.maxbp[CX], e.maxbp[Y]);
     const void* kernel = (const void*)jk_bra_kernel<CX, 1, RT, YK>;
-    cudaError_t r = set_smem_limit(kernel, smem);
-    if (r != cudaSuccess) return r;
-    a.plan = e.plan_of(CX, YK < 0 ? 0 : YK, sizeof(RT) == sizeof(double) ? 0 : 1);
-    jk_bra_kernel<CX, 1, RT, YK><<<persistent_grid(kernel, JK_THREADS, smem, e.nsm), JK_THREADS, smem, st>>>(a);
+    LaunchSlot& slot = e.slot(0, rt, CX, Y);
+    if (slot.grid == 0) {
+        // K rows in shared memory unless they would not fit (large bases) or
+        // the context asks for global rows
+        slot.kglobal = a.kglobal;
+        if (!slot.kglobal && jk_smem_bytes<CX, 1, Y, RT>(e.nao, e.maxbp[CX], a.rbuf, false) + static_smem(kernel) > kSmemLimit)
+            slot.kglobal = 1;
+        const size_t smem = jk_smem_bytes<CX, 1, Y, RT>(e.nao, e.maxbp[CX], a.rbuf, slot.kglobal != 0);
+        cudaError_t r = set_smem_limit(kernel, smem);
+        if (r != cudaSuccess) return r;
+        slot.grid = persistent_grid(kernel, JK_THREADS, smem, e.nsm);
+    }
+    a.kglobal = slot.kglobal;
+    a.plan = e.plan_of(CX, Y, rt);
+    jk_bra_kernel<CX, 1, RT, YK><<<slot.grid, JK_THREADS, jk_smem_bytes<CX, 1, Y, RT>(e.nao, e.maxbp[CX], a.rbuf, a.kglobal != 0),
+                                   e.stream_of(CX, Y)>>>(a);
     return cudaGetLastError();
 }
 }  // namespace
 
-// split bra classes: one launch per non-empty ket class (largest first), in
-// order on st; the others: one launch over all ket classes
-cudaError_t AIMD_JK_NAME(const LaunchEnv& e, const JKArgs& a, cudaStream_t st) {
+// split bra classes: one launch per non-empty ket class (largest first); the
+// others: one launch over all ket classes
+cudaError_t AIMD_JK_NAME(const LaunchEnv& e, const JKArgs& a) {
     const int cnt = e.cls_count[CX];
     if (cnt == 0) return cudaSuccess;
     if constexpr (!JKKernel<CX, 1>::SPLIT) {
-        return launch_one<-1>(e, a, st);
+        return launch_one<-1>(e, a);
     } else {
         cudaError_t r = cudaSuccess;
-        if constexpr (CX >= 5) if (r == cudaSuccess && e.cls_count[5]) r = launch_one<5>(e, a, st);
-        if constexpr (CX >= 4) if (r == cudaSuccess && e.cls_count[4]) r = launch_one<4>(e, a, st);
-        if constexpr (CX >= 3) if (r == cudaSuccess && e.cls_count[3]) r = launch_one<3>(e, a, st);
-        if constexpr (CX >= 2) if (r == cudaSuccess && e.cls_count[2]) r = launch_one<2>(e, a, st);
-        if (r == cudaSuccess && e.cls_count[1]) r = launch_one<1>(e, a, st);
-        if (r == cudaSuccess && e.cls_count[0]) r = launch_one<0>(e, a, st);
+        if constexpr (CX >= 5) if (r == cudaSuccess && e.cls_count[5]) r = launch_one<5>(e, a);
+        if constexpr (CX >= 4) if (r == cudaSuccess && e.cls_count[4]) r = launch_one<4>(e, a);
+        if constexpr (CX >= 3) if (r == cudaSuccess && e.cls_count[3]) r = launch_one<3>(e, a);
+        if constexpr (CX >= 2) if (r == cudaSuccess && e.cls_count[2]) r = launch_one<2>(e, a);
+        if (r == cudaSuccess && e.cls_count[1]) r = launch_one<1>(e, a);
+        if (r == cudaSuccess && e.cls_count[0]) r = launch_one<0>(e, a);
         return r;
     }
 }

@@ -628,26 +628,24 @@ __device__ __forceinline__ int64_t chunk_edge(int64_t W, int j, int nch) {
     return q * j + (r * j) / nch;
 }
 
-// The next chunk of the launch for this CTA: thread 0 takes it from the
-// counter and finds its bra (last b with off[b] <= c); all threads return
-// the same (c, b) and c >= off[nbra] when the plan is used up.
-__device__ __forceinline__ void next_chunk(const WorkPlan& plan, int nbra, int* sh, int& c, int& b) {
-    if (threadIdx.x == 0) {
-        const int cc = atomicAdd(plan.next, 1);
-        int lo = 0, hi = nbra;                          // off[lo] <= cc < off[hi] while cc < total
-        if (cc < plan.off[nbra]) {
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (plan.off[mid] <= cc) lo = mid;
-                else hi = mid;
-            }
-        }
-        sh[0] = cc;
-        sh[1] = lo;
+// The next chunk of the launch for this CTA (warp 0 calls it): lane 0 takes
+// it from the counter, the lanes search its bra together, 32 entries a step
+// (last b with off[b] <= c; a lone thread's binary search was a chain of a
+// dozen loads that the CTA waited for, once a chunk). c >= off[nbra] when the
+// plan is used up.
+__device__ __forceinline__ void next_chunk(const WorkPlan& plan, int nbra, int total, int& c, int& b) {
+    const int lane = threadIdx.x & 31;
+    int cc = 0;
+    if (lane == 0) cc = atomicAdd(plan.next, 1);
+    c = __shfl_sync(0xffffffffu, cc, 0);
+    int lo = 0, hi = nbra;                              // off[lo] <= c < off[hi] while c < total
+    while (c < total && hi - lo > 1) {
+        const int step = (hi - lo + 31) / 32, at = lo + lane * step;
+        const unsigned le = __ballot_sync(0xffffffffu, at < hi && plan.off[at] <= c);
+        lo += (31 - __clz(le)) * step;                  // lane 0 always holds: le != 0
+        hi = lo + step < hi ? lo + step : hi;
     }
-    __syncthreads();
-    c = sh[0];
-    b = sh[1];
+    b = lo;
 }
 
 __device__ __forceinline__ void load_info(const QuartetArgs& a, int P1, BraInfo& st) {
@@ -1282,22 +1280,31 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
     __shared__ int sh[2];
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
-    bool staged = false;        // the Boys table is in shared memory
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double fx = __ldg(a.fix);
+    bool staged = false;        // the Boys table is in shared memory, and the accumulators are zero
     for (;;) {
-        int c, b;
-        next_chunk(a.plan, nbra, sh, c, b);
+        if (warp == 0) {
+            int c, b;
+            next_chunk(a.plan, nbra, total, c, b);
+            if (lane == 0) {
+                sh[0] = c;
+                sh[1] = b;
+                if (c < total) load_info(a.q, a.q.sorted[a.q.cls_start[CX] + b], info);
+            }
+        }
+        __syncthreads();
+        const int c = sh[0], b = sh[1];
         if (c >= total) break;                                  // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
-        if (threadIdx.x == 0) load_info(a.q, a.q.sorted[spos], info);
         if (!staged) {
             Boys::stage(a.q.boys, btab);
+            for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * JK_THREADS; i += blockDim.x) Jt[i] = 0.0;
             staged = true;
         }
-        for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * JK_THREADS; i += blockDim.x) Jt[i] = 0.0;
-        __syncthreads();
         const BraStageT<RT> st = stage_view(info, Esm, KK::ESIZE);
-        if (threadIdx.x < 32) {
-            const int sub = threadIdx.x < NSUB ? threadIdx.x : 0;
+        if (warp == 0) {
+            const int sub = lane < NSUB ? lane : 0;
             plan_window<CX, Y, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], QY::NITEM,
                                    seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
         }
@@ -1306,25 +1313,33 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
         jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf,
                                                  Boys::get(btab));
         __syncthreads();
-        // flush J_ab: one thread per (set, row) sums the per-thread slots
-        for (int i = threadIdx.x; i < NS * KK::NROW; i += blockDim.x) {
+        // flush J_ab: a warp a (set, row) sums the threads' slots (in a fixed
+        // order) and clears them
+        for (int i = warp; i < NS * KK::NROW; i += JK_THREADS / 32) {
             double val = 0.0;
-            for (int t = 0; t < JK_THREADS; ++t) val += Jt[i * JK_THREADS + t];
-            if (val == 0.0) continue;
+#pragma unroll
+            for (int t = 0; t < JK_THREADS; t += 32) {
+                val += Jt[i * JK_THREADS + t + lane];
+                Jt[i * JK_THREADS + t + lane] = 0.0;
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) val += __shfl_xor_sync(0xffffffffu, val, d);
+            if (lane != 0 || val == 0.0) continue;
             const int s = i / KK::NROW, r = i % KK::NROW;
             const int kab = r / Q0::NAB, ab = r % Q0::NAB;
             const int ka = kab / st.i.nB, kb = kab % st.i.nB;
             const int m = st.i.oA + ka * Q0::NA + ab / Q0::NB, nb_ = st.i.oB + kb * Q0::NB + ab % Q0::NB;
-            fadd(a.J + s * nn + (size_t)m * n + nb_, val, __ldg(a.fix));
+            fadd(a.J + s * nn + (size_t)m * n + nb_, val, fx);
         }
-        // flush K rows
+        // flush and clear the K rows
         if (krows > 0) {
             constexpr int NFA = Q0::KA * Q0::NA;
             for (int i = threadIdx.x; i < krows * n; i += blockDim.x) {
                 const facc val = join_planes(Ksm[i], Ksm[krows * n + i]);
                 if (val == 0) continue;
-                const int col = i % n, f = (i / n) % KK::NF, s = i / (n * KK::NF);
-                const int row = f < NFA ? st.i.oA + f : st.i.oB + (f - NFA);
+                Ksm[i] = Ksm[krows * n + i] = 0u;
+                const int col = i % n, f_ = (i / n) % KK::NF, s = i / (n * KK::NF);
+                const int row = f_ < NFA ? st.i.oA + f_ : st.i.oB + (f_ - NFA);
                 atomicAdd(a.K + s * nn + (size_t)row * n + col, val);     // integer: order-independent
             }
         }

@@ -477,22 +477,30 @@ __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kerne
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
     for (int i = threadIdx.x; i < 6 * a.natm; i += blockDim.x) gsh[i] = 0u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool staged = false;        // the Boys table is in shared memory
     auto gadd = [&](int i, double v) { sadd(gsh + i, gsh + 3 * a.natm + i, v, FIX_G); };
     for (;;) {
-        int c, b;
-        next_chunk(a.plan, nbra, sh, c, b);                     // (its barrier also orders the zeroing)
+        if (warp == 0) {
+            int c, b;
+            next_chunk(a.plan, nbra, total, c, b);
+            if (lane == 0) {
+                sh[0] = c;
+                sh[1] = b;
+                if (c < total) load_info(a.q, a.q.sorted[a.q.cls_start[CX] + b], info);
+            }
+        }
+        __syncthreads();                                        // (also orders the zeroing)
+        const int c = sh[0], b = sh[1];
         if (c >= total) break;                                  // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
-        if (threadIdx.x == 0) load_info(a.q, a.q.sorted[spos], info);
         if (!staged) {
             Boys::stage(a.q.boys, btab);
             staged = true;
         }
-        __syncthreads();
         const BraStageT<RT> st = stage_view(info, Esm, BraE<Q0::LA, Q0::LB, 0>::SIZE);
-        if (threadIdx.x < 32) {
-            const int sub = threadIdx.x < NSUB ? threadIdx.x : 0;
+        if (warp == 0) {
+            const int sub = lane < NSUB ? lane : 0;
             plan_window<CX, CY, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], Q::NCD,
                                     seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
         }

@@ -128,8 +128,9 @@ struct aimd_ctx {
     int item_pq = ITEM_PQ;
     double* bmc;            // gradient: [nblock][nblock] max |Dc| and max over x of |Dx|
     double* bmx;
-    cudaStream_t cls_stream[NCLS];
-    cudaEvent_t ev_fork, ev_join[NCLS];
+    cudaStream_t streams[NSTREAM] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[NSTREAM] = {};
+    LaunchSlot slots[2 * 2 * NCLS * NCLS];
     int maxbp[NCLS];        // largest primitive-pair count of a block pair, per class
     double thr_jk = -1.0, thr_g = -1.0;
     // mixed precision: quartets with Q1 Q2 < fp32_cutoff run in FP32
@@ -306,8 +307,8 @@ extern "C" int aimd_create(aimd_ctx** out, int natm, int nao, int nblock, const 
         c->cub_bytes = std::max(b1, b2);
         CK(cudaMalloc(&c->cub_tmp, c->cub_bytes));
     }
-    for (int i = 0; i < NCLS; ++i) {
-        CK(cudaStreamCreateWithFlags(&c->cls_stream[i], cudaStreamNonBlocking));
+    for (int i = 0; i < NSTREAM; ++i) {
+        CK(cudaStreamCreateWithFlags(&c->streams[i], cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&c->ev_join[i], cudaEventDisableTiming));
     }
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
@@ -323,8 +324,8 @@ extern "C" int aimd_destroy(aimd_ctx* c) {
                     c->tmp_idx, c->seg_id, c->seg_keys, c->seg_keys_out, c->seg_start, c->tmpQ, c->sortedQ,
                     c->sorted, c->counts_jk, c->counts_g, c->counts_d, c->bmax, c->dmax, c->jkfix, c->plan, c->plan_next, c->bmc, c->bmx, c->counts_hi, c->counts_hi_d, c->cub_tmp, c->pos, c->boys, c->jacc, c->kacc, c->gacc};
     for (void* p : ptrs) cudaFree(p);
-    for (int i = 0; i < NCLS; ++i) {
-        if (c->cls_stream[i]) cudaStreamDestroy(c->cls_stream[i]);
+    for (int i = 0; i < NSTREAM; ++i) {
+        if (c->streams[i]) cudaStreamDestroy(c->streams[i]);
         if (c->ev_join[i]) cudaEventDestroy(c->ev_join[i]);
     }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -547,6 +548,8 @@ LaunchEnv launch_env(aimd_ctx* c) {
     e.plan = c->plan;
     e.plan_next = c->plan_next;
     e.plan_stride = c->npair + NCLS;
+    e.slots = c->slots;
+    e.streams = c->streams;
     return e;
 }
 
@@ -643,83 +646,72 @@ void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, cudaStream_t s
     ++c->launches;
 }
 
-// all (CX, CY <= CX) gradient kernels of bra class CX, in order on one stream
-template <int CX>
-cudaError_t launch_grad_class(const LaunchEnv& e, const GradArgs& a, cudaStream_t st) {
+int cls_size(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
+
+// all (X, Y <= X) gradient kernels, the costly classes first
+cudaError_t launch_grads(const LaunchEnv& e, const GradArgs& a) {
     cudaError_t r = cudaSuccess;
     const bool mixed = a.q.counts_hi != nullptr;
-#define AIMD_G1(X, Y)                                                             \
-    if (r == cudaSuccess && CX == X) r = launch_grad_c##X##_##Y(e, a, st);       \
-    if (r == cudaSuccess && CX == X && mixed) r = launch_grad32_c##X##_##Y(e, a, st);
+#define AIMD_G1(X, Y)                                                     \
+    if (r == cudaSuccess) r = launch_grad_c##X##_##Y(e, a);              \
+    if (r == cudaSuccess && mixed) r = launch_grad32_c##X##_##Y(e, a);
+    AIMD_G1(5, 5) AIMD_G1(5, 4) AIMD_G1(5, 3) AIMD_G1(5, 2) AIMD_G1(5, 1) AIMD_G1(5, 0)
+    AIMD_G1(4, 4) AIMD_G1(4, 3) AIMD_G1(4, 2) AIMD_G1(4, 1) AIMD_G1(4, 0)
+    AIMD_G1(3, 3) AIMD_G1(3, 2) AIMD_G1(3, 1) AIMD_G1(3, 0)
+    AIMD_G1(2, 2) AIMD_G1(2, 1) AIMD_G1(2, 0)
+    AIMD_G1(1, 1) AIMD_G1(1, 0)
     AIMD_G1(0, 0)
-    AIMD_G1(1, 0) AIMD_G1(1, 1)
-    AIMD_G1(2, 0) AIMD_G1(2, 1) AIMD_G1(2, 2)
-    AIMD_G1(3, 0) AIMD_G1(3, 1) AIMD_G1(3, 2) AIMD_G1(3, 3)
-    AIMD_G1(4, 0) AIMD_G1(4, 1) AIMD_G1(4, 2) AIMD_G1(4, 3) AIMD_G1(4, 4)
-    AIMD_G1(5, 0) AIMD_G1(5, 1) AIMD_G1(5, 2) AIMD_G1(5, 3) AIMD_G1(5, 4) AIMD_G1(5, 5)
 #undef AIMD_G1
     return r;
 }
-
-// kernel launches of one class step: J/K one per type, the gradient one
-// per (bra class, non-empty ket class) and type
-int cls_size(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
-int jk_launches(aimd_ctx* c, int cl, bool mixed) {
-    if (cls_size(c, cl) == 0) return 0;
-    int n = 1;
-    if (cl >= 1) {          // split bra classes: one kernel per non-empty ket class
-        n = 0;
-        for (int y = 0; y <= cl; ++y) n += cls_size(c, y) > 0 ? 1 : 0;
-    }
-    return mixed ? 2 * n : n;
+cudaError_t launch_jks(const LaunchEnv& e, const JKArgs& a) {
+    cudaError_t r = cudaSuccess;
+    const bool mixed = a.q.counts_hi != nullptr;
+#define AIMD_J1(X)                                            \
+    if (r == cudaSuccess) r = launch_jk_c##X(e, a);          \
+    if (r == cudaSuccess && mixed) r = launch_jk32_c##X(e, a);
+    AIMD_J1(5) AIMD_J1(4) AIMD_J1(3) AIMD_J1(2) AIMD_J1(1) AIMD_J1(0)
+#undef AIMD_J1
+    return r;
 }
-int grad_launches(aimd_ctx* c, int cl, bool mixed) {
+// kernel launches of launch_jks and launch_grads: one per non-empty (bra
+// class, ket class) and type
+int class_pair_launches(aimd_ctx* c, bool mixed) {
     int n = 0;
-    for (int y = 0; y <= cl; ++y) n += (cls_size(c, cl) > 0 && cls_size(c, y) > 0) ? 1 : 0;
+    for (int x = 0; x < NCLS; ++x)
+        for (int y = 0; y <= x; ++y) n += (cls_size(c, x) > 0 && cls_size(c, y) > 0) ? 1 : 0;
     return mixed ? 2 * n : n;
 }
 
-inline cudaError_t first_error(cudaError_t a, cudaError_t b) { return a != cudaSuccess ? a : b; }
-
-int class_status(aimd_ctx* c, cudaError_t r, const char* what, int cl, int nlaunch) {
+int launch_status(aimd_ctx* c, cudaError_t r, const char* what, int nlaunch) {
     if (r == cudaSuccess) {
         c->launches += nlaunch;
         return AIMD_OK;
     }
     if (r == cudaErrorInvalidConfiguration) {
-        snprintf(g_err, sizeof g_err, "%s (pair class %d): shared memory beyond the 227 KB per-CTA limit",
-                 what, cl);
+        snprintf(g_err, sizeof g_err, "%s: shared memory beyond the 227 KB per-CTA limit", what);
         return AIMD_ERR_UNSUPPORTED;
     }
-    snprintf(g_err, sizeof g_err, "%s (pair class %d): %s", what, cl, cudaGetErrorString(r));
+    snprintf(g_err, sizeof g_err, "%s: %s", what, cudaGetErrorString(r));
     return AIMD_ERR_CUDA;
 }
 
-// The six class launches of one call run concurrently on the context's
-// class streams, forked from and joined back into the caller's stream, so
-// the long-running d-shell classes overlap the others.
-#define AIMD_EACH_CLASS_CONCURRENT(CALL, WHAT, NLAUNCH)                               \
-    do {                                                                              \
-        CK(cudaEventRecord(c->ev_fork, st));                                          \
-        int r_ = AIMD_OK;                                                             \
-        for (int x_ = NCLS - 1; x_ >= 0 && r_ == AIMD_OK; --x_) {                     \
-            CK(cudaStreamWaitEvent(c->cls_stream[x_], c->ev_fork, 0));                \
-            cudaStream_t cs_ = c->cls_stream[x_];                                     \
-            cudaError_t e_ = cudaSuccess;                                             \
-            switch (x_) {                                                             \
-                case 0: e_ = CALL(0, cs_); break;                                     \
-                case 1: e_ = CALL(1, cs_); break;                                     \
-                case 2: e_ = CALL(2, cs_); break;                                     \
-                case 3: e_ = CALL(3, cs_); break;                                     \
-                case 4: e_ = CALL(4, cs_); break;                                     \
-                default: e_ = CALL(5, cs_); break;                                    \
-            }                                                                         \
-            r_ = class_status(c, e_, WHAT, x_, NLAUNCH(x_));                          \
-            CK(cudaEventRecord(c->ev_join[x_], cs_));                                 \
-            CK(cudaStreamWaitEvent(st, c->ev_join[x_], 0));                           \
-        }                                                                             \
-        if (r_) return r_;                                                            \
-    } while (0)
+// The class launches of one call run concurrently on the context's streams,
+// forked from and joined back into the caller's stream: a class pair's kernel
+// of a small molecule leaves most of the device idle, and at any size the tail
+// of one kernel overlaps the next. The streams are joined even where a launch
+// failed, so that the caller's stream covers what did start.
+template <typename Launch>
+int run_concurrent(aimd_ctx* c, cudaStream_t st, int nstream, const char* what, int nlaunch, Launch launch) {
+    CK(cudaEventRecord(c->ev_fork, st));
+    for (int i = 0; i < nstream; ++i) CK(cudaStreamWaitEvent(c->streams[i], c->ev_fork, 0));
+    const int status = launch_status(c, launch(), what, nlaunch);
+    for (int i = 0; i < nstream; ++i) {
+        CK(cudaEventRecord(c->ev_join[i], c->streams[i]));
+        CK(cudaStreamWaitEvent(st, c->ev_join[i], 0));
+    }
+    return status;
+}
 
 // The FP64-prefix table of the mixed-precision path (nullptr when off).
 int hi_counts(aimd_ctx* c, cudaStream_t st, const int64_t** out) {
@@ -774,11 +766,18 @@ extern "C" int aimd_set_geometry(aimd_ctx* c, const double* pos, void* stream) {
     {
         const LaunchEnv e = launch_env(c);
         const QuartetArgs q = quartet_args(c, c->counts_jk);
-#define AIMD_SCHWARZ(X, S) launch_schwarz_c##X(e, q, S)
-#define AIMD_NL(X) (cls_size(c, X) > 0 ? 1 : 0)
-        AIMD_EACH_CLASS_CONCURRENT(AIMD_SCHWARZ, "aimd_set_geometry/schwarz", AIMD_NL);
-#undef AIMD_NL
-#undef AIMD_SCHWARZ
+        int n = 0;
+        for (int cl = 0; cl < NCLS; ++cl) n += cls_size(c, cl) > 0;
+        const int r = run_concurrent(c, st, NCLS, "aimd_set_geometry/schwarz", n, [&] {
+            cudaError_t x = launch_schwarz_c5(e, q, c->streams[5]);
+            if (x == cudaSuccess) x = launch_schwarz_c4(e, q, c->streams[4]);
+            if (x == cudaSuccess) x = launch_schwarz_c3(e, q, c->streams[3]);
+            if (x == cudaSuccess) x = launch_schwarz_c2(e, q, c->streams[2]);
+            if (x == cudaSuccess) x = launch_schwarz_c1(e, q, c->streams[1]);
+            if (x == cudaSuccess) x = launch_schwarz_c0(e, q, c->streams[0]);
+            return x;
+        });
+        if (r) return r;
     }
     // order: Q descending, then (stable) by segment; segment starts on the device
     const int nbk = (np + 127) / 128;
@@ -844,11 +843,8 @@ extern "C" int aimd_jk(aimd_ctx* c, int nset, const double* D, double* J, double
         a.kglobal = c->jk_global_rows;
         a.item_pq = c->item_pq;
         plan_launches(c, a.q, mixed, st);
-#define AIMD_JK(X, S) first_error(launch_jk_c##X(e, a, S), mixed ? launch_jk32_c##X(e, a, S) : cudaSuccess)
-#define AIMD_NL(X) jk_launches(c, X, mixed)
-        AIMD_EACH_CLASS_CONCURRENT(AIMD_JK, "aimd_jk", AIMD_NL);
-#undef AIMD_NL
-#undef AIMD_JK
+        if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
+            return r;
         from_fixed(st, nn, c->jacc, c->jkfix, 0.0, J + s0 * nn, 0);
         from_fixed(st, nn, c->kacc, c->jkfix, 0.0, K + s0 * nn, 0);
         c->launches += 2;
@@ -921,11 +917,8 @@ extern "C" int aimd_jk_delta(aimd_ctx* c, int nset, const double* D, double* J, 
         a.kglobal = c->jk_global_rows;
         a.item_pq = c->item_pq;
         plan_launches(c, a.q, mixed, st);
-#define AIMD_JK(X, S) first_error(launch_jk_c##X(e, a, S), mixed ? launch_jk32_c##X(e, a, S) : cudaSuccess)
-#define AIMD_NL(X) jk_launches(c, X, mixed)
-        AIMD_EACH_CLASS_CONCURRENT(AIMD_JK, "aimd_jk_delta", AIMD_NL);
-#undef AIMD_NL
-#undef AIMD_JK
+        if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk_delta", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
+            return r;
         from_fixed(st, nn, c->jacc, c->jkfix, 0.0, J + s0 * nn, 0);
         from_fixed(st, nn, c->kacc, c->jkfix, 0.0, K + s0 * nn, 0);
         c->launches += 2;
@@ -1093,11 +1086,8 @@ extern "C" int aimd_grad2e(aimd_ctx* c, const double* Dc, int nx, const double* 
     a.item_pq = c->item_pq;
     plan_launches(c, a.q, mixed, st);
     const LaunchEnv e = launch_env(c);
-#define AIMD_GRAD(X, S) launch_grad_class<X>(e, a, S)
-#define AIMD_NL(X) grad_launches(c, X, mixed)
-    AIMD_EACH_CLASS_CONCURRENT(AIMD_GRAD, "aimd_grad2e", AIMD_NL);
-#undef AIMD_NL
-#undef AIMD_GRAD
+    if (int r = run_concurrent(c, st, NSTREAM, "aimd_grad2e", class_pair_launches(c, mixed), [&] { return launch_grads(e, a); }))
+        return r;
     from_fixed(st, 3 * (size_t)c->natm, c->gacc, nullptr, FIX_G, grad, 0);
     ++c->launches;
     CK(cudaGetLastError());
@@ -1123,6 +1113,11 @@ ShellView shell_view(aimd_ctx* c) {
     s.pair_j = c->sp_j;
     return s;
 }
+int shell_classes(aimd_ctx* c) {        // non-empty shell-pair classes
+    int n = 0;
+    for (int cl = 0; cl < NCLS; ++cl) n += c->sp_cls_start[cl + 1] > c->sp_cls_start[cl];
+    return n;
+}
 }  // namespace
 
 extern "C" int aimd_onee(aimd_ctx* c, const double* origin, double* S, double* T, double* M, double* V,
@@ -1131,10 +1126,13 @@ extern "C" int aimd_onee(aimd_ctx* c, const double* origin, double* S, double* T
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const LaunchEnv e = launch_env(c);
     const ShellView sv = shell_view(c);
-#define AIMD_ONEE(X, S_) launch_onee(e, sv, X, c->sp_cls_start, origin, S, T, M, V, S_)
-#define AIMD_NL(X) (c->sp_cls_start[X + 1] > c->sp_cls_start[X] ? 1 : 0)
-    AIMD_EACH_CLASS_CONCURRENT(AIMD_ONEE, "aimd_onee", AIMD_NL);
-#undef AIMD_ONEE
+    if (int r = run_concurrent(c, st, NCLS, "aimd_onee", shell_classes(c), [&] {
+            cudaError_t x = cudaSuccess;
+            for (int cl = NCLS - 1; cl >= 0 && x == cudaSuccess; --cl)
+                x = launch_onee(e, sv, cl, c->sp_cls_start, origin, S, T, M, V, c->streams[cl]);
+            return x;
+        }))
+        return r;
     return AIMD_OK;
 }
 
@@ -1148,10 +1146,13 @@ extern "C" int aimd_onee_grad(aimd_ctx* c, const double* W, const double* D, dou
     CK(cudaMemsetAsync(c->gacc, 0, sizeof(facc) * 3 * c->natm, st));
     const LaunchEnv e = launch_env(c);
     const ShellView sv = shell_view(c);
-#define AIMD_ONEE_G(X, S_) launch_onee_grad(e, sv, X, c->sp_cls_start, W, D, c->gacc, S_)
-    AIMD_EACH_CLASS_CONCURRENT(AIMD_ONEE_G, "aimd_onee_grad", AIMD_NL);
-#undef AIMD_ONEE_G
-#undef AIMD_NL
+    if (int r = run_concurrent(c, st, NCLS, "aimd_onee_grad", shell_classes(c), [&] {
+            cudaError_t x = cudaSuccess;
+            for (int cl = NCLS - 1; cl >= 0 && x == cudaSuccess; --cl)
+                x = launch_onee_grad(e, sv, cl, c->sp_cls_start, W, D, c->gacc, c->streams[cl]);
+            return x;
+        }))
+        return r;
     from_fixed(st, 3 * (size_t)c->natm, c->gacc, nullptr, FIX_G, grad, 1);
     ++c->launches;
     CK(cudaGetLastError());

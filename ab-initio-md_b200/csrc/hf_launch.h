@@ -13,6 +13,15 @@
 
 namespace hf {
 
+// Launch parameters of a class kernel on one context, found at its first
+// launch: the attribute and occupancy queries cost as much host time as the
+// launch, and a small molecule's build is some twenty launches long.
+struct LaunchSlot {
+    int grid = 0;       // CTAs (0: not yet known)
+    int kglobal = 0;    // J/K: K rows in global memory
+};
+constexpr int NSTREAM = 12;     // streams that the class kernels of one call are spread over
+
 struct LaunchEnv {
     int cls_count[NCLS];     // block pairs per class
     int cls_start[NCLS + 1]; // start of each class in the class-grouped order
@@ -27,6 +36,10 @@ struct LaunchEnv {
     int* plan;
     int* plan_next;
     int plan_stride;
+    LaunchSlot* slots;       // [2 kinds: J/K, gradient][2 types][NCLS][NCLS]
+    LaunchSlot& slot(int kind, int rt, int cx, int cy) const { return slots[((kind * 2 + rt) * NCLS + cx) * NCLS + cy]; }
+    const cudaStream_t* streams;    // [NSTREAM], forked from the call's stream
+    cudaStream_t stream_of(int cx, int cy) const { return streams[(cx * (cx + 1) / 2 + cy) % NSTREAM]; }
     WorkPlan plan_of(int cx, int cy, int rt) const {
         return WorkPlan{plan + (size_t)(rt * NCLS + cy) * plan_stride + cls_start[cx] + cx,
                         plan_next + (rt * NCLS + cx) * NCLS + cy};
@@ -40,16 +53,17 @@ inline int persistent_grid(const void* kernel, int threads, size_t smem, int nsm
     return per * nsm;
 }
 
+// The J/K and gradient launchers use the streams of the environment.
 // Status: cudaSuccess, a CUDA error, or cudaErrorInvalidConfiguration when
 // the shared-memory request exceeds the per-CTA limit.
 #define AIMD_DECLARE_TYPED(X, S)                                                                       \
-    cudaError_t launch_jk##S##_c##X(const LaunchEnv& e, const JKArgs& a, cudaStream_t st);              \
-    cudaError_t launch_grad##S##_c##X##_0(const LaunchEnv& e, const GradArgs& a, cudaStream_t st);     \
-    cudaError_t launch_grad##S##_c##X##_1(const LaunchEnv& e, const GradArgs& a, cudaStream_t st);     \
-    cudaError_t launch_grad##S##_c##X##_2(const LaunchEnv& e, const GradArgs& a, cudaStream_t st);     \
-    cudaError_t launch_grad##S##_c##X##_3(const LaunchEnv& e, const GradArgs& a, cudaStream_t st);     \
-    cudaError_t launch_grad##S##_c##X##_4(const LaunchEnv& e, const GradArgs& a, cudaStream_t st);     \
-    cudaError_t launch_grad##S##_c##X##_5(const LaunchEnv& e, const GradArgs& a, cudaStream_t st);
+    cudaError_t launch_jk##S##_c##X(const LaunchEnv& e, const JKArgs& a);              \
+    cudaError_t launch_grad##S##_c##X##_0(const LaunchEnv& e, const GradArgs& a);     \
+    cudaError_t launch_grad##S##_c##X##_1(const LaunchEnv& e, const GradArgs& a);     \
+    cudaError_t launch_grad##S##_c##X##_2(const LaunchEnv& e, const GradArgs& a);     \
+    cudaError_t launch_grad##S##_c##X##_3(const LaunchEnv& e, const GradArgs& a);     \
+    cudaError_t launch_grad##S##_c##X##_4(const LaunchEnv& e, const GradArgs& a);     \
+    cudaError_t launch_grad##S##_c##X##_5(const LaunchEnv& e, const GradArgs& a);
 #define AIMD_DECLARE_CLASS(X)                                                                          \
     cudaError_t launch_schwarz_c##X(const LaunchEnv& e, const QuartetArgs& q, cudaStream_t st);         \
     AIMD_DECLARE_TYPED(X, )                                                                            \
