@@ -34,36 +34,35 @@ using RT = float;
 #define AIMD_JK_NAME AIMD_CAT(launch_jk32_c, AIMD_CLASS)
 #endif
 
-// Internal linkage: every class unit instantiates launch_one<YK> for its own
-// (class, type), and identical external names would let the linker keep one
-// unit's copy for all of them.
-namespace {
-template <int YK>
+// One (class, ket class, type) launch. Every class unit instantiates it for its
+// own class, so class and type are template arguments: an internal name alone
+// does not keep the units' copies apart (the compiler makes it from a hash of
+// the unit, which two units of one source compiled at once can share).
+template <int X, int YK, typename T>
 cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0) {
     constexpr int Y = YK < 0 ? 0 : YK;
-    constexpr int rt = sizeof(RT) == sizeof(double) ? 0 : 1;
+    constexpr int rt = sizeof(T) == sizeof(double) ? 0 : 1;
     JKArgs a = a0;
-    a.rbuf = jk_rbuf_elems<CX, YK, RT>(e.maxbp[CX], e.maxbp[Y]);
-    const void* kernel = (const void*)jk_bra_kernel<CX, 1, RT, YK>;
-    LaunchSlot& slot = e.slot(0, rt, CX, Y);
+    a.rbuf = jk_rbuf_elems<X, YK, T>(e.maxbp[X], e.maxbp[Y]);
+    const void* kernel = (const void*)jk_bra_kernel<X, 1, T, YK>;
+    LaunchSlot& slot = e.slot(0, rt, X, Y);
     if (slot.grid == 0) {
         // K rows in shared memory unless they would not fit (large bases) or
         // the context asks for global rows
         slot.kglobal = a.kglobal;
-        if (!slot.kglobal && jk_smem_bytes<CX, 1, Y, RT>(e.nao, e.maxbp[CX], a.rbuf, false) + static_smem(kernel) > kSmemLimit)
+        if (!slot.kglobal && jk_smem_bytes<X, 1, Y, T>(e.nao, e.maxbp[X], a.rbuf, false) + static_smem(kernel) > kSmemLimit)
             slot.kglobal = 1;
-        const size_t smem = jk_smem_bytes<CX, 1, Y, RT>(e.nao, e.maxbp[CX], a.rbuf, slot.kglobal != 0);
+        const size_t smem = jk_smem_bytes<X, 1, Y, T>(e.nao, e.maxbp[X], a.rbuf, slot.kglobal != 0);
         cudaError_t r = set_smem_limit(kernel, smem);
         if (r != cudaSuccess) return r;
         slot.grid = persistent_grid(kernel, JK_THREADS, smem, e.nsm);
     }
     a.kglobal = slot.kglobal;
-    a.plan = e.plan_of(CX, Y, rt);
-    jk_bra_kernel<CX, 1, RT, YK><<<slot.grid, JK_THREADS, jk_smem_bytes<CX, 1, Y, RT>(e.nao, e.maxbp[CX], a.rbuf, a.kglobal != 0),
-                                   e.stream_of(CX, Y)>>>(a);
+    a.plan = e.plan_of(X, Y, rt);
+    jk_bra_kernel<X, 1, T, YK><<<slot.grid, JK_THREADS, jk_smem_bytes<X, 1, Y, T>(e.nao, e.maxbp[X], a.rbuf, a.kglobal != 0),
+                                   e.stream_of(X, Y)>>>(a);
     return cudaGetLastError();
 }
-}  // namespace
 
 // split bra classes: one launch per non-empty ket class (largest first); the
 // others: one launch over all ket classes
@@ -71,15 +70,15 @@ cudaError_t AIMD_JK_NAME(const LaunchEnv& e, const JKArgs& a) {
     const int cnt = e.cls_count[CX];
     if (cnt == 0) return cudaSuccess;
     if constexpr (!JKKernel<CX, 1>::SPLIT) {
-        return launch_one<-1>(e, a);
+        return launch_one<CX, -1, RT>(e, a);
     } else {
         cudaError_t r = cudaSuccess;
-        if constexpr (CX >= 5) if (r == cudaSuccess && e.cls_count[5]) r = launch_one<5>(e, a);
-        if constexpr (CX >= 4) if (r == cudaSuccess && e.cls_count[4]) r = launch_one<4>(e, a);
-        if constexpr (CX >= 3) if (r == cudaSuccess && e.cls_count[3]) r = launch_one<3>(e, a);
-        if constexpr (CX >= 2) if (r == cudaSuccess && e.cls_count[2]) r = launch_one<2>(e, a);
-        if (r == cudaSuccess && e.cls_count[1]) r = launch_one<1>(e, a);
-        if (r == cudaSuccess && e.cls_count[0]) r = launch_one<0>(e, a);
+        if constexpr (CX >= 5) if (r == cudaSuccess && e.cls_count[5]) r = launch_one<CX, 5, RT>(e, a);
+        if constexpr (CX >= 4) if (r == cudaSuccess && e.cls_count[4]) r = launch_one<CX, 4, RT>(e, a);
+        if constexpr (CX >= 3) if (r == cudaSuccess && e.cls_count[3]) r = launch_one<CX, 3, RT>(e, a);
+        if constexpr (CX >= 2) if (r == cudaSuccess && e.cls_count[2]) r = launch_one<CX, 2, RT>(e, a);
+        if (r == cudaSuccess && e.cls_count[1]) r = launch_one<CX, 1, RT>(e, a);
+        if (r == cudaSuccess && e.cls_count[0]) r = launch_one<CX, 0, RT>(e, a);
         return r;
     }
 }
