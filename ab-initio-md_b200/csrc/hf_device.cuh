@@ -249,36 +249,40 @@ __host__ __device__ constexpr int boys_offset(int N) {      // first element of 
     return o;
 }
 
-// How hermite_r gets g[n] = (-2 alpha)^n F_n(T): evaluated, or (FP64) from the
+// How hermite_r gets g[n] = scale (-2 alpha)^n F_n(T): evaluated, or (FP64) from the
 // shared table of order N.
 struct BoysSeries {
     template <int L, typename RT>
-    __device__ __forceinline__ void operator()(RT alpha, RT T, RT (&g)[L + 1]) const {
+    __device__ __forceinline__ void operator()(RT alpha, RT T, RT scale, RT (&g)[L + 1]) const {
         boys_scaled<L>(alpha, T, g);
+#pragma unroll
+        for (int n = 0; n <= L; ++n) g[n] *= scale;
     }
 };
 struct BoysShared {
     const double* t;
     template <int L>
-    __device__ __forceinline__ void operator()(double alpha, double T, double (&g)[L + 1]) const {
+    __device__ __forceinline__ void operator()(double alpha, double T, double scale, double (&g)[L + 1]) const {
         constexpr int NR = boys_rows(L);
         if (!(T < 36 + 3 * L)) {        // (NaN too)
             const double r = rsqrt(T);
             double s = r * r;
             s = fma(s, fma(-T, s, 1.0), s) * -alpha;        // 1 / T to rounding
-            g[0] = 0.88622692545275801365 * r;
+            g[0] = 0.88622692545275801365 * r * scale;
 #pragma unroll
             for (int n = 1; n <= L; ++n) g[n] = g[n - 1] * ((2 * n - 1) * s);
             return;
         }
-        const int i = static_cast<int>(T * 8.0);
-        const double d = T - (i + 0.5) * 0.125;
-        const double* c = t + i;
+        // row floor(8 T), as the integer nearest to 8 T - 1/2: adding 1.5 2^52
+        // leaves it in the low word (no conversion instructions)
+        const double m = fma(T, 8.0, -0.5) + 6755399441055744.0;
+        const double d = fma(-0.125, m - 6755399441055744.0, T - 0.0625);
+        const double* c = t + __double2loint(m);
         double f = c[7 * NR];
 #pragma unroll
         for (int j = 6; j >= 0; --j) f = fma(f, d, c[j * NR]);
         if constexpr (L == 0) {
-            g[0] = f;
+            g[0] = f * scale;
         } else {
             double e = 1.0 / 40320;
             e = fma(e, d, -1.0 / 5040);
@@ -291,7 +295,7 @@ struct BoysShared {
             const double e0 = c[8 * NR], ex = fma(e * d, e0, e0);
             const double m2a = -2.0 * alpha, T2 = 2.0 * T;
             double pw[L + 1];
-            pw[0] = 1.0;
+            pw[0] = scale;
 #pragma unroll
             for (int n = 1; n <= L; ++n) pw[n] = pw[n - 1] * m2a;
             g[L] = pw[L] * f;
@@ -314,9 +318,7 @@ template <int L, typename RT, typename Arr, typename Boys = BoysSeries>
 __device__ __forceinline__ void hermite_r_scaled(RT alpha, RT X, RT Y, RT Z, RT scale, Arr&& R, Boys boys = Boys()) {
     const RT T = alpha * (X * X + Y * Y + Z * Z);
     RT g[L + 1];
-    boys.template operator()<L>(alpha, T, g);
-#pragma unroll
-    for (int n = 0; n <= L; ++n) g[n] *= scale;
+    boys.template operator()<L>(alpha, T, scale, g);
     R[0] = g[L];
 #pragma unroll
     for (int n = L - 1; n >= 0; --n) {

@@ -72,7 +72,9 @@ struct BraE {
 // scalars are held in the arithmetic type RT of the kernel that reads them
 // (double, or float for the mixed-precision quartets); they are computed in
 // FP64 either way.
-constexpr int SBW = 12;     // per bra primitive: p, 1/p, Px, Py, Pz, a, b, -, c0..c3
+// per bra primitive: p, Px, Py, Pz, a/p, b/p, -, -, then c0..c3, the contraction
+// products times 2 pi^(5/2) K / p (K = exp(-mu |A - B|^2)); 16-byte aligned
+constexpr int SBW = 12;
 struct BraInfo {
     int P1, A, B, nbp, aA, aB;
     int nA, nB, oA, oB;
@@ -94,8 +96,9 @@ __device__ __forceinline__ void stage_bra_scalars(const BraStageT<RT>& st) {
     for (int ib = threadIdx.x; ib < st.i.nbp; ib += blockDim.x) {
         const double* b = st.i.rec + (size_t)ib * PPW;
         RT* o = st.SB + (size_t)ib * SBW;
-        const double p = b[0] + b[1];
-        const double vals[SBW] = {p, 1.0 / p, b[3], b[4], b[5], b[0], b[1], 0.0, b[12], b[13], b[14], b[15]};
+        const double p = b[0] + b[1], ip = 1.0 / p, f = TWO_PI_2_5 * b[2] * ip;
+        const double vals[SBW] = {p, b[3], b[4], b[5], b[0] * ip, b[1] * ip, 0.0, 0.0,
+                                  f * b[12], f * b[13], f * b[14], f * b[15]};
 #pragma unroll
         for (int i = 0; i < SBW; ++i) o[i] = static_cast<RT>(vals[i]);
     }
@@ -110,7 +113,7 @@ __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
         const double* b = st.i.rec + (size_t)ib * PPW;
         const double p = b[0] + b[1];
         double e[LA + 1 + G][LB + 1 + G][LA + LB + 1 + 2 * G];
-        hermite_e<LA + G, LB + G>(b[6 + d], b[9 + d], 0.5 / p, d == 0 ? b[2] : 1.0, e);
+        hermite_e<LA + G, LB + G>(b[6 + d], b[9 + d], 0.5 / p, 1.0, e);      // K is in the scalars
         RT* out = st.E + (size_t)ib * BE::SIZE;
 #pragma unroll
         for (int i = 0; i < LA + 1 + G; ++i)
@@ -120,6 +123,20 @@ __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
                 for (int t = 0; t < LA + LB + 1 + 2 * G; ++t) out[BE::at(d, i, j, t)] = static_cast<RT>(e[i][j][t]);
     }
     stage_bra_scalars(st);
+}
+
+// The bra primitive's exponent sum and centre, in vector loads.
+template <typename RT>
+struct BraPrim {
+    RT p, X, Y, Z;
+};
+__device__ __forceinline__ BraPrim<double> load_bra(const double* sb) {
+    const double2 u = *reinterpret_cast<const double2*>(sb), v = *reinterpret_cast<const double2*>(sb + 2);
+    return BraPrim<double>{u.x, u.y, v.x, v.y};
+}
+__device__ __forceinline__ BraPrim<float> load_bra(const float* sb) {
+    const float4 u = *reinterpret_cast<const float4*>(sb);
+    return BraPrim<float>{u.x, u.y, u.z, u.w};
 }
 
 // One primitive-pair record of a ket pair (16 doubles, 128-byte aligned),
@@ -195,9 +212,12 @@ __device__ __forceinline__ void bra_rows(const RT* E, const RT (&X)[KG][nherm(LA
                 for (int u = 0; u <= LA + LB - az - bz - t; ++u)
 #pragma unroll
                     for (int kk = 0; kk < KG; ++kk) {
-                        RT s = E[BE::at(2, az, bz, 0)] * X[kk][hidx(t, u, 0)];
+                        RT s = X[kk][hidx(t, u, 0)];                // (E^{00}_0 = 1)
+                        if (az + bz > 0) {
+                            s *= E[BE::at(2, az, bz, 0)];
 #pragma unroll
-                        for (int w = 1; w <= az + bz; ++w) s += E[BE::at(2, az, bz, w)] * X[kk][hidx(t, u, w)];
+                            for (int w = 1; w <= az + bz; ++w) s += E[BE::at(2, az, bz, w)] * X[kk][hidx(t, u, w)];
+                        }
                         W[kk][cart_index(t, u)] = s;
                     }
 #pragma unroll
@@ -208,17 +228,19 @@ __device__ __forceinline__ void bra_rows(const RT* E, const RT (&X)[KG][nherm(LA
                     const RT fab = static_cast<RT>(cart_norm(ax, ay, az) * cart_norm(bx, by, bz));
                     RT s[KG];
 #pragma unroll
-                    for (int kk = 0; kk < KG; ++kk) s[kk] = RT(0);
+                    for (int kk = 0; kk < KG; ++kk) {
+                        s[kk] = RT(0);
 #pragma unroll
-                    for (int t = 0; t <= ax + bx; ++t) {
-                        const RT e = fab * E[BE::at(0, ax, bx, t)];
+                        for (int t = 0; t <= ax + bx; ++t) {
+                            RT y = W[kk][cart_index(t, 0)];
+                            if (ay + by > 0) {
+                                y *= E[BE::at(1, ay, by, 0)];
 #pragma unroll
-                        for (int kk = 0; kk < KG; ++kk) {
-                            RT y = RT(0);
-#pragma unroll
-                            for (int u = 0; u <= ay + by; ++u) y += E[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
-                            s[kk] += e * y;
+                                for (int u = 1; u <= ay + by; ++u) y += E[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
+                            }
+                            s[kk] += ax + bx > 0 ? E[BE::at(0, ax, bx, t)] * y : y;
                         }
+                        s[kk] *= fab;
                     }
                     row(cart_index(ay, az), cart_index(by, bz), s);
                 }
@@ -237,12 +259,12 @@ __device__ __forceinline__ void bra_rows(const RT* E, const RT (&X)[KG][nherm(LA
 // primitive quartet (the reference applies it per primitive quartet,
 // aimd/qc/integrals.py:777-842).
 // RS = false: R_tuv of each primitive quartet is computed here; RS = true:
-// it is read from Rs, [ik][ib][NH(L)] pref * R_tuv staged by the CTA
+// it is read from Rs, [ik][ib][NH(L)] R_tuv / sqrt(p + q) staged by the CTA
 // (stage_r below) once for all the columns of the ket pair.
 template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp, int ic,
                                            int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                           const RT* __restrict__ Rs, int ib0, int ib1, Boys boys) {
+                                           const RT* __restrict__ Rs, int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
@@ -267,7 +289,7 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
             RT ex[LCD + 1], ey[LCD + 1], ez[LCD + 1];
             {
                 RT e[LC + 1][LD + 1][LCD + 1];
-                hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, k.K, e);
+                hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, RT(1), e);
                 select_row<LC, LD, LCD>(e, cx, dx, ex);
                 hermite_e<LC, LD>(k.QAy, k.QBy, oo2q, RT(1), e);
                 select_row<LC, LD, LCD>(e, cy, dy, ey);
@@ -281,53 +303,58 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
 #pragma unroll
                 for (int j = 1; j < Q::KCD; ++j)
                     if (j == kg * Q::KG + i) c = k.c[j];
-                ck[i] = c * fcd;
+                ck[i] = c * (fcd * k.K * (RT(2) * oo2q));
             }
-            // ket step: Xs[kk]_h += ck[kk] pref sum_{k in box(cd)} (-1)^|k| E^{cd}_k R_{h+k},
+            // ket step: Xs[kk]_h += ck[kk] sum_{k in box(cd)} (-1)^|k| E^{cd}_k R_{h+k},
             // box entries outer, so that a column's box conditions are tested
-            // once per entry and not once per (entry, h)
-            auto ket_step = [&](const auto& R, RT scale) {
-                RT sc[Q::KG];
+            // once per entry and not once per (entry, h); with several
+            // contraction combinations the sum is formed once and then scaled
+            auto ket_step = [&](const auto& R) {
+                RT X[Q::NHB];
 #pragma unroll
-                for (int kk = 0; kk < Q::KG; ++kk) sc[kk] = scale * ck[kk];
+                for (int h = 0; h < Q::NHB; ++h) X[h] = Q::KG > 1 ? RT(0) : Xs[0][h];
+                const RT sc = Q::KG > 1 ? RT(1) : ck[0];
 #pragma unroll
                 for (int t2 = 0; t2 <= LCD; ++t2) {
                     if (t2 > cx + dx) continue;
 #pragma unroll
                     for (int u2 = 0; u2 <= LCD - t2; ++u2) {
                         if (u2 > cy + dy) continue;
-                        const RT exy = ((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2];
+                        const RT exy = sc * (((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2]);
 #pragma unroll
                         for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
                             if (v2 > cz + dz) continue;
                             const RT e = (v2 & 1) ? -exy * ez[v2] : exy * ez[v2];
-                            RT es[Q::KG];
-#pragma unroll
-                            for (int kk = 0; kk < Q::KG; ++kk) es[kk] = sc[kk] * e;
 #pragma unroll
                             for (int t = 0; t <= LAB; ++t)
 #pragma unroll
                                 for (int u = 0; u <= LAB - t; ++u)
 #pragma unroll
-                                    for (int w = 0; w <= LAB - t - u; ++w) {
-                                        const RT r = R[hidx(t + t2, u + u2, w + v2)];
-#pragma unroll
-                                        for (int kk = 0; kk < Q::KG; ++kk) Xs[kk][hidx(t, u, w)] += es[kk] * r;
-                                    }
+                                    for (int w = 0; w <= LAB - t - u; ++w)
+                                        X[hidx(t, u, w)] += e * R[hidx(t + t2, u + u2, w + v2)];
                         }
                     }
                 }
+#pragma unroll
+                for (int h = 0; h < Q::NHB; ++h) {
+                    if constexpr (Q::KG > 1) Xs[0][h] += ck[0] * X[h];
+                    else Xs[0][h] = X[h];
+                }
+#pragma unroll
+                for (int kk = 1; kk < Q::KG; ++kk) {
+                    if (kk >= nk) continue;
+#pragma unroll
+                    for (int h = 0; h < Q::NHB; ++h) Xs[kk][h] += ck[kk] * X[h];
+                }
             };
             if constexpr (RS) {
-                ket_step(Rs + (size_t)(ik * st.i.nbp + ib) * nherm(L), RT(1));
+                ket_step(Rs + (size_t)(ik * st.i.nbp + ib) * nherm(L));
             } else {
-                const RT p = sb[0];
-                const RT rs = rsqrt_t(p + q);
-                const RT alpha = p * q * rs * rs;
-                const RT pref = RT(TWO_PI_2_5) * sb[1] * (RT(2) * oo2q) * rs;
+                const BraPrim<RT> b = load_bra(sb);
+                const RT rs = rsqrt_t(b.p + q);
                 RT R[nherm(L)];
-                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
-                ket_step(R, pref);
+                hermite_r_scaled<L>(b.p * q * (rs * rs), b.X - k.Qx, b.Y - k.Qy, b.Z - k.Qz, rs, R, boys);
+                ket_step(R);
             }
         }
         // bra step, once per bra primitive:
@@ -341,88 +368,52 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
     }
 }
 
-// Ket primitives outermost, bra primitives inner, R_tuv and the bra step per
-// primitive quartet: the order for bra pairs with many primitives (ss, ps,
-// pp), where repeating the ket setup per bra primitive would cost more than
-// the bra steps it saves.
+// Ket ss: one column, R_tuv is the ket step itself. Ket primitives outermost,
+// bra primitives inner, the bra step per primitive quartet: the order for bra
+// pairs with many primitives (ss, ps, pp). The bra-contracted rows A of one
+// ket primitive meet its nk contraction combinations once.
 template <int CX, int CY, typename RT, typename Boys>
 __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp,
-                                                     int ic, int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                     int ib0, int ib1, Boys boys) {
+                                                     int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
+                                                     int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
-    constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
-    const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
-    const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
-    const RT fcd = static_cast<RT>(cart_norm(cx, cy, cz) * cart_norm(dx, dy, dz));
+    constexpr int LA = Q::LA, LB = Q::LB, L = Q::L;
+    static_assert(Q::LCD == 0, "ket ss");
+    const int nab = st.i.nA * st.i.nB;
 #pragma unroll
     for (int r = 0; r < Q::NROW; ++r)
 #pragma unroll
         for (int k = 0; k < Q::KG; ++k) v[r][k] = RT(0);
     for (int ik = 0; ik < nkp; ++ik) {
         const KetRecT<RT> k = load_ket<RT>(rk + (size_t)ik * PPW);
-        const RT q = k.a + k.b, oo2q = RT(0.5) / q, iq = RT(2) * oo2q;
-        // ket E coefficients of this column only (box t2 <= cx+dx, ...)
-        RT ex[LCD + 1], ey[LCD + 1], ez[LCD + 1];
-        {
-            RT e[LC + 1][LD + 1][LCD + 1];
-            hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, k.K, e);
-            select_row<LC, LD, LCD>(e, cx, dx, ex);
-            hermite_e<LC, LD>(k.QAy, k.QBy, oo2q, RT(1), e);
-            select_row<LC, LD, LCD>(e, cy, dy, ey);
-            hermite_e<LC, LD>(k.QAz, k.QBz, oo2q, RT(1), e);
-            select_row<LC, LD, LCD>(e, cz, dz, ez);
-        }
-        RT ck[Q::KG];
+        const RT q = k.a + k.b;
+        RT A[Q::NROW];
 #pragma unroll
-        for (int i = 0; i < Q::KG; ++i) {
+        for (int r = 0; r < Q::NROW; ++r) A[r] = RT(0);
+        for (int ib = ib0; ib < ib1; ++ib) {
+            const RT* sb = st.SB + ib * SBW;
+            const BraPrim<RT> b = load_bra(sb);
+            const RT rs = rsqrt_t(b.p + q);
+            RT R[1][nherm(L)];
+            hermite_r_scaled<L>(b.p * q * (rs * rs), b.X - k.Qx, b.Y - k.Qy, b.Z - k.Qz, rs, R[0], boys);
+            bra_rows<LA, LB, 1>(st.E + (size_t)ib * BE::SIZE, R, [&](int ia, int jb, const RT (&s)[1]) {
+#pragma unroll
+                for (int kab = 0; kab < Q::KAB; ++kab)
+                    if (kab == 0 || kab < nab) A[kab * Q::NAB + ia * Q::NB + jb] += sb[8 + kab] * s[0];
+            });
+        }
+        const RT ck0 = k.K / q;
+#pragma unroll
+        for (int kk = 0; kk < Q::KG; ++kk) {
+            if (kk > 0 && kk >= nk) continue;
             RT c = k.c[0];
 #pragma unroll
             for (int j = 1; j < Q::KCD; ++j)
-                if (j == kg * Q::KG + i) c = k.c[j];
-            ck[i] = c * fcd;
-        }
-        for (int ib = ib0; ib < ib1; ++ib) {
-            const RT* sb = st.SB + ib * SBW;
-            const RT p = sb[0];
-            const RT rs = rsqrt_t(p + q);
-            const RT alpha = p * q * rs * rs;
-            const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
-            RT R[nherm(L)];
-            hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
-            RT X[1][Q::NHB];
+                if (j == kg * Q::KG + kk) c = k.c[j];
+            c *= ck0;
 #pragma unroll
-            for (int h = 0; h < Q::NHB; ++h) X[0][h] = RT(0);
-#pragma unroll
-            for (int t2 = 0; t2 <= LCD; ++t2) {
-                if (t2 > cx + dx) continue;
-#pragma unroll
-                for (int u2 = 0; u2 <= LCD - t2; ++u2) {
-                    if (u2 > cy + dy) continue;
-                    const RT exy = pref * (((t2 + u2) & 1) ? -ex[t2] * ey[u2] : ex[t2] * ey[u2]);
-#pragma unroll
-                    for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
-                        if (v2 > cz + dz) continue;
-                        const RT e = (v2 & 1) ? -exy * ez[v2] : exy * ez[v2];
-#pragma unroll
-                        for (int t = 0; t <= LAB; ++t)
-#pragma unroll
-                            for (int u = 0; u <= LAB - t; ++u)
-#pragma unroll
-                                for (int w = 0; w <= LAB - t - u; ++w)
-                                    X[0][hidx(t, u, w)] += e * R[hidx(t + t2, u + u2, w + v2)];
-                    }
-                }
-            }
-            // bra step: v[(ka,kb),ab][kk] += C[ka,kb] f_ab sum_box E^{ab}_tuv X[tuv] ck[kk]
-            bra_rows<LA, LB, 1>(st.E + (size_t)ib * BE::SIZE, X, [&](int ia, int jb, const RT (&s)[1]) {
-#pragma unroll
-                for (int kab = 0; kab < Q::KAB; ++kab) {
-                    const RT c = sb[8 + kab] * s[0];
-#pragma unroll
-                    for (int kk = 0; kk < Q::KG; ++kk) v[kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
-                }
-            });
+            for (int r = 0; r < Q::NROW; ++r) v[r][kk] += A[r] * c;
         }
     }
 }
@@ -435,12 +426,13 @@ template <int CX, int CY, typename RT, typename Boys>
 __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp,
                                                    int id, int kg,
                                                    RT (&v)[QClass<CX, CY>::NC][QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                   int ib0, int ib1, Boys boys) {
+                                                   int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
-    const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
+    const int dx = LD ? cart_x(LD, id) : 0, dy = LD ? cart_y(LD, id) : 0, dz = LD ? cart_z(LD, id) : 0;
     const RT fd = static_cast<RT>(cart_norm(dx, dy, dz));
+    const int nab = st.i.nA * st.i.nB;
 #pragma unroll
     for (int c = 0; c < Q::NC; ++c)
 #pragma unroll
@@ -449,12 +441,12 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
             for (int k = 0; k < Q::KG; ++k) v[c][r][k] = RT(0);
     for (int ik = 0; ik < nkp; ++ik) {
         const KetRecT<RT> k = load_ket<RT>(rk + (size_t)ik * PPW);
-        const RT q = k.a + k.b, oo2q = RT(0.5) / q, iq = RT(2) * oo2q;
+        const RT q = k.a + k.b, oo2q = RT(0.5) / q;
         // ket E of this id: ex[i][t] = E^{i, dx}_t for every i <= LC
         RT ex[LC + 1][LCD + 1], ey[LC + 1][LCD + 1], ez[LC + 1][LCD + 1];
         {
             RT e[LC + 1][LD + 1][LCD + 1];
-            hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, k.K, e);
+            hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, RT(1), e);
             select_j<LC, LD, LCD>(e, dx, ex);
             hermite_e<LC, LD>(k.QAy, k.QBy, oo2q, RT(1), e);
             select_j<LC, LD, LCD>(e, dy, ey);
@@ -468,16 +460,14 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
 #pragma unroll
             for (int j = 1; j < Q::KCD; ++j)
                 if (j == kg * Q::KG + i) c = k.c[j];
-            ck[i] = c * fd;
+            ck[i] = c * (fd * k.K * (RT(2) * oo2q));
         }
         for (int ib = ib0; ib < ib1; ++ib) {
             const RT* sb = st.SB + ib * SBW;
-            const RT p = sb[0];
-            const RT rs = rsqrt_t(p + q);
-            const RT alpha = p * q * rs * rs;
-            const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
+            const BraPrim<RT> b = load_bra(sb);
+            const RT rs = rsqrt_t(b.p + q);
             RT R[nherm(L)];
-            hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
+            hermite_r_scaled<L>(b.p * q * (rs * rs), b.X - k.Qx, b.Y - k.Qy, b.Z - k.Qz, rs, R, boys);
             const RT* E = st.E + (size_t)ib * BE::SIZE;
 #pragma unroll
             for (int ic = 0; ic < Q::NC; ++ic) {
@@ -486,14 +476,13 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
                 RT X[1][Q::NHB];
 #pragma unroll
                 for (int h = 0; h < Q::NHB; ++h) X[0][h] = RT(0);
-                const RT pf = pref * fc;
 #pragma unroll
                 for (int t2 = 0; t2 <= LCD; ++t2) {
                     if (t2 > cx + dx) continue;
 #pragma unroll
                     for (int u2 = 0; u2 <= LCD - t2; ++u2) {
                         if (u2 > cy + dy) continue;
-                        const RT exy = pf * (((t2 + u2) & 1) ? -ex[cx][t2] * ey[cy][u2] : ex[cx][t2] * ey[cy][u2]);
+                        const RT exy = fc * (((t2 + u2) & 1) ? -ex[cx][t2] * ey[cy][u2] : ex[cx][t2] * ey[cy][u2]);
 #pragma unroll
                         for (int v2 = 0; v2 <= LCD - t2 - u2; ++v2) {
                             if (v2 > cz + dz) continue;
@@ -512,9 +501,11 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
                 bra_rows<LA, LB, 1>(E, X, [&](int ia, int jb, const RT (&s)[1]) {
 #pragma unroll
                     for (int kab = 0; kab < Q::KAB; ++kab) {
+                        if (kab > 0 && kab >= nab) continue;
                         const RT c = sb[8 + kab] * s[0];
 #pragma unroll
-                        for (int kk = 0; kk < Q::KG; ++kk) v[ic][kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
+                        for (int kk = 0; kk < Q::KG; ++kk)
+                            if (kk == 0 || kk < nk) v[ic][kab * Q::NAB + ia * Q::NB + jb][kk] += c * ck[kk];
                     }
                 });
             }
@@ -522,15 +513,19 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
     }
 }
 
-// (row r | cd) of a quartet column: bra-outer order (the bra step once per
-// bra primitive) for the d-shell bra classes, whose pairs have few
-// primitives, and the ket-outer order for the others.
+// (row r | cd) of a quartet column, nk contraction combinations of the ket:
+// bra-outer order (the bra step once per bra primitive) for the d-shell bra
+// classes, whose pairs have few primitives; ket-outer order for ss, ps and pp
+// bras against ss kets (against p kets: column blocks, and here the diagonal
+// quartets of the Schwarz bounds).
 template <int CX, int CY, typename RT, bool RS = false, typename Boys = BoysSeries>
 __device__ __forceinline__ void eri_column(const BraStageT<RT>& st, const double* __restrict__ rk, int nkp, int ic,
                                            int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                           const RT* __restrict__ Rs, int ib0, int ib1, Boys boys = Boys()) {
-    if constexpr (RS || CX >= 3) eri_column_bra_outer<CX, CY, RT, RS>(st, rk, nkp, ic, id, kg, v, Rs, ib0, ib1, boys);
-    else eri_column_ket_outer<CX, CY, RT>(st, rk, nkp, ic, id, kg, v, ib0, ib1, boys);
+                                           const RT* __restrict__ Rs, int ib0, int ib1, int nk, Boys boys = Boys()) {
+    if constexpr (RS || CX >= 3 || CY > 0)
+        eri_column_bra_outer<CX, CY, RT, RS>(st, rk, nkp, ic, id, kg, v, Rs, ib0, ib1, nk, boys);
+    else
+        eri_column_ket_outer<CX, CY, RT>(st, rk, nkp, kg, v, ib0, ib1, nk, boys);
 }
 
 // Everything the quartet kernels share.
@@ -668,6 +663,11 @@ __device__ __forceinline__ BraStageT<RT> stage_view(const BraInfo& info, RT* E, 
     RT* e = E + info.nbp * SBW;
     return BraStageT<RT>{info, E, e, e + info.nbp * size};
 }
+
+// The bra stage holds vectors of 16 bytes: what lies before it in shared memory
+// is rounded up to a multiple of four elements (of either type).
+__host__ __device__ constexpr size_t even(size_t n) { return (n + 1) & ~(size_t)1; }
+__host__ __device__ constexpr size_t fours(size_t n) { return (n + 3) & ~(size_t)3; }
 
 // How the quartets of one kernel evaluate the Boys function of order L: from
 // the shared table (copied by the CTA before its first chunk) or by series.
@@ -828,6 +828,12 @@ __device__ __forceinline__ int seg_groups(int sub) {
     const int ncs = cb == 0 ? 1 : (cb == 1 ? 2 : 4);
     const int g = (ncs + KG - 1) / KG;
     return g < NKG ? g : NKG;
+}
+// contraction combinations of a segment's pairs in their group kg
+template <int KG>
+__device__ __forceinline__ int group_combos(int sub, int kg) {
+    const int cb = sub % NCONB, n = (cb == 0 ? 1 : (cb == 1 ? 2 : 4)) - kg * KG;
+    return n < KG ? n : KG;
 }
 template <int CX, int CY>
 __device__ __forceinline__ int64_t ket_work(int sub) {
@@ -1011,7 +1017,7 @@ __device__ __forceinline__ void flat_items(FlatItems& f, bool queued, int* queue
 // fit RB_PQ slots of a shared buffer (plus the largest single ket pair),
 // and per sub-chunk:
 //   stage 1: one thread per primitive quartet (ket pair i, ket primitive ik,
-//            bra primitive ib) writes pref * R_tuv into the buffer;
+//            bra primitive ib) writes R_tuv / sqrt(p + q) into the buffer;
 //   stage 2: the column items of the sub-chunk's ket pairs read it.
 template <int L, typename RT>
 struct RSmem {
@@ -1058,23 +1064,21 @@ __device__ __forceinline__ int lower_bound_i(const int* a, int lo, int hi, int k
     return lo;
 }
 
-// pref * R_tuv of primitive quartet (bra primitive ib of the stage, ket
+// R_tuv / sqrt(p + q) of primitive quartet (bra primitive ib of the stage, ket
 // primitive record kr) into out[NH(L)] (shared memory).
 template <int L, typename RT>
 __device__ __forceinline__ void stage_r(const BraStageT<RT>& st, int ib, const double* __restrict__ kr, RT* out) {
     const double2* r2 = reinterpret_cast<const double2*>(kr);
     const double2 ab = __ldg(r2 + 0), kq = __ldg(r2 + 1), qyz = __ldg(r2 + 2);
-    const RT* sb = st.SB + ib * SBW;
-    const RT p = sb[0], q = static_cast<RT>(ab.x) + static_cast<RT>(ab.y);
-    const RT rs = rsqrt_t(p + q);
-    const RT alpha = p * q * rs * rs;
-    const RT pref = RT(TWO_PI_2_5) * sb[1] * (RT(1) / q) * rs;
-    const RT X = sb[2] - static_cast<RT>(kq.y), Y = sb[3] - static_cast<RT>(qyz.x), Z = sb[4] - static_cast<RT>(qyz.y);
+    const BraPrim<RT> b = load_bra(st.SB + ib * SBW);
+    const RT q = static_cast<RT>(ab.x) + static_cast<RT>(ab.y);
+    const RT rs = rsqrt_t(b.p + q), alpha = b.p * q * (rs * rs);
+    const RT X = b.X - static_cast<RT>(kq.y), Y = b.Y - static_cast<RT>(qyz.x), Z = b.Z - static_cast<RT>(qyz.y);
     if constexpr (RSmem<L, RT>::INPLACE) {
-        hermite_r_scaled<L>(alpha, X, Y, Z, pref, out);
+        hermite_r_scaled<L>(alpha, X, Y, Z, rs, out);
     } else {
         RT R[nherm(L)];
-        hermite_r_scaled<L>(alpha, X, Y, Z, pref, R);
+        hermite_r_scaled<L>(alpha, X, Y, Z, rs, R);
 #pragma unroll
         for (int h = 0; h < nherm(L); ++h) out[h] = R[h];
     }
@@ -1195,19 +1199,20 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
         const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         const int ib0 = st.i.nbp * sp / nsp, ib1 = st.i.nbp * (sp + 1) / nsp;
+        const int nk = group_combos<Q::KG>(sub, kg);
         const int P2 = a.q.sorted[pos];
         const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
         const double* rk = a.q.pv.rec + a.q.pv.slot[P2] * PPW;
         if constexpr (Q::CBLK) {
             // item = the NC columns of one id
             RT v[Q::NC][Q::NROW][Q::KG];
-            eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1, boys);
+            eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1, nk, boys);
 #pragma unroll
             for (int ic = 0; ic < Q::NC; ++ic) digest(P2, C, Dd, ic, cd, kg, v[ic]);
         } else {
             RT v[Q::NROW][Q::KG];
             eri_column<CX, CY, RT, Q::RSMEM>(st, rk, a.q.pv.npp[P2], cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1,
-                                                 boys);
+                                                 nk, boys);
             digest(P2, C, Dd, cd / Q::ND, cd % Q::ND, kg, v);
         }
     };
@@ -1272,7 +1277,7 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
     double* btab = smem;                                    // Boys table
     double* Jt = btab + Boys::elems;                        // per-thread J_ab slots
     unsigned* Ksm = reinterpret_cast<unsigned*>(Jt + NS * KK::NROW * JK_THREADS);   // low words of the K rows, then the high words
-    RT* Rbuf = reinterpret_cast<RT*>(Jt + NS * KK::NROW * JK_THREADS + (size_t)krows * n);
+    RT* Rbuf = reinterpret_cast<RT*>(Jt + NS * KK::NROW * JK_THREADS + even((size_t)krows * n));
     RT* Esm = Rbuf + a.rbuf;
     __shared__ BraInfo info;
     __shared__ FlatItems f;
@@ -1352,7 +1357,7 @@ template <int CX, int YK, typename RT>
 size_t jk_rbuf_elems(int max_bra_prims, int max_ket_prims) {
     if constexpr (YK >= 0) {
         using Q = QClass<CX, YK>;
-        if constexpr (Q::RSMEM) return rsmem_bytes<Q::L, RT>(max_bra_prims, max_ket_prims) / sizeof(RT);
+        if constexpr (Q::RSMEM) return fours(rsmem_bytes<Q::L, RT>(max_bra_prims, max_ket_prims) / sizeof(RT));
     }
     return 0;
 }
@@ -1361,7 +1366,7 @@ template <int CX, int NS, int Y, typename RT>
 size_t jk_smem_bytes(int nao, int max_bra_prims, size_t rbuf_elems, bool kglobal) {
     using KK = JKKernel<CX, NS>;
     const size_t krows = kglobal ? 0 : KK::KROWS;
-    return sizeof(double) * (krows * nao + (size_t)NS * KK::NROW * JK_THREADS + JKBoys<CX, Y, RT>::elems) +
+    return sizeof(double) * (even(krows * nao) + (size_t)NS * KK::NROW * JK_THREADS + JKBoys<CX, Y, RT>::elems) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (KK::ESIZE + SBW));
 }
 
@@ -1400,7 +1405,7 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS) schwarz_kernel(QuartetArgs a,
         if (ib1 > ib0) {
             double v[Q::NROW][Q::KCD];
             eri_column<CX, CX>(st, st.i.rec, st.i.nbp, cd / Q::ND, cd % Q::ND, 0, v, static_cast<const double*>(nullptr),
-                               ib0, ib1);
+                               ib0, ib1, Q::KCD);
 #pragma unroll
             for (int kk = 0; kk < Q::KAB; ++kk)
 #pragma unroll

@@ -76,10 +76,10 @@ __device__ __forceinline__ void stage_bra_de(const BraStageT<RT>& st) {
         const double* b = st.i.rec + (size_t)ib * PPW;
         const double ip = 1.0 / (b[0] + b[1]), pa = b[6 + d], pb = b[9 + d];
         double e[LA + 1][LB + 1][LA + LB + 1], de[LA + 1][LB + 1][LA + LB + 1];
-        hermite_e<LA, LB>(pa, pb, 0.5 * ip, d == 0 ? b[2] : 1.0, e);
+        hermite_e<LA, LB>(pa, pb, 0.5 * ip, 1.0, e);        // K is in the scalars
         hermite_de<LA, LB>(pa, pb, 0.5 * ip, b[1] * ip, b[0] * ip, 2.0 * b[0] * b[1] * ip * (pb - pa), e, de);
-        // exp(-mu |A - B|^2) is in the x table; the y and z tables carry their
-        // own derivative of it through de[0][0][0]
+        // exp(-mu |A - B|^2) is in the scalars; each direction's table carries
+        // its derivative through de[0][0][0]
         RT* out = st.E + (size_t)ib * BE::SIZE;
         RT* dout = st.D + (size_t)ib * BE::SIZE;
 #pragma unroll
@@ -102,7 +102,7 @@ template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&Gr)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
                                            const double* __restrict__ rk, int nkp, int ic, int id, int kg,
                                            RT (&dA)[3], RT (&dB)[3], RT (&dC)[3], const RT* __restrict__ Rs,
-                                           RT* Rcol, int ib0, int ib1, Boys boys) {
+                                           RT* Rcol, int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
     using BE = BraE<Q::LA, Q::LB, 0>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L + 1;
@@ -111,6 +111,7 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
     const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
     const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
     const RT fcd = cart_norm(cx, cy, cz) * cart_norm(dx, dy, dz);
+    const int nab = st.i.nA * st.i.nB;
     for (int ib = ib0; ib < ib1; ++ib) {
         const RT* sb = st.SB + ib * SBW;
         const RT* E = st.E + (size_t)ib * BE::SIZE;
@@ -121,7 +122,8 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                            cart_norm(cart_x(LB, jb), cart_y(LB, jb), cart_z(LB, jb));
             RT s = RT(0);
 #pragma unroll
-            for (int kab = 0; kab < Q::KAB; ++kab) s += sb[8 + kab] * Gr[kab * Q::NAB + ia * Q::NB + jb][kk];
+            for (int kab = 0; kab < Q::KAB; ++kab)
+                if (kab == 0 || kab < nab) s += sb[8 + kab] * Gr[kab * Q::NAB + ia * Q::NB + jb][kk];
             return s * fab;
         };
         RT Y[KG][NHB], Xs[KG][NHB];
@@ -147,25 +149,29 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                         const int ax = LA - az - ay, bx = LB - bz - by;
 #pragma unroll
                         for (int kk = 0; kk < KG; ++kk) {
+                            if (kk > 0 && kk >= nk) continue;
                             const RT g = gq(cart_index(ay, az), cart_index(by, bz), kk);
 #pragma unroll
                             for (int t = 0; t <= ax + bx; ++t) {
-                                const RT ge = g * E[BE::at(0, ax, bx, t)];
+                                const RT ge = ax + bx > 0 ? g * E[BE::at(0, ax, bx, t)] : g;
 #pragma unroll
                                 for (int u = 0; u <= ay + by; ++u)
-                                    W[kk][cart_index(t, u)] += ge * E[BE::at(1, ay, by, u)];
+                                    W[kk][cart_index(t, u)] += ay + by > 0 ? ge * E[BE::at(1, ay, by, u)] : ge;
                             }
                         }
                     }
 #pragma unroll
-                for (int t = 0; t <= LAB - az - bz; ++t)
+                for (int kk = 0; kk < KG; ++kk) {
+                    if (kk > 0 && kk >= nk) continue;
 #pragma unroll
-                    for (int u = 0; u <= LAB - az - bz - t; ++u)
+                    for (int t = 0; t <= LAB - az - bz; ++t)
 #pragma unroll
-                        for (int w = 0; w <= az + bz; ++w)
+                        for (int u = 0; u <= LAB - az - bz - t; ++u)
 #pragma unroll
-                            for (int kk = 0; kk < KG; ++kk)
-                                Y[kk][hidx(t, u, w)] += E[BE::at(2, az, bz, w)] * W[kk][cart_index(t, u)];
+                            for (int w = 0; w <= az + bz; ++w)
+                                Y[kk][hidx(t, u, w)] += az + bz > 0 ? E[BE::at(2, az, bz, w)] * W[kk][cart_index(t, u)]
+                                                                    : W[kk][cart_index(t, u)];
+                }
             }
         RT gG[3] = {RT(0), RT(0), RT(0)};       // G summed over the ket primitives
         for (int ik = 0; ik < nkp; ++ik) {
@@ -175,7 +181,7 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
             {
                 RT e[LC + 1][LD + 1][LCD + 1], de[LC + 1][LD + 1][LCD + 1];
                 const RT m2 = RT(2) * k.a * dq;
-                hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, k.K, e);
+                hermite_e<LC, LD>(k.QAx, k.QBx, oo2q, RT(1), e);
                 hermite_de<LC, LD>(k.QAx, k.QBx, oo2q, dq, cq, m2 * (k.QBx - k.QAx), e, de);
                 select_row<LC, LD, LCD>(e, cx, dx, ex);
                 select_row<LC, LD, LCD>(de, cx, dx, fx);
@@ -188,22 +194,24 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                 select_row<LC, LD, LCD>(e, cz, dz, ez);
                 select_row<LC, LD, LCD>(de, cz, dz, fz);
             }
-            auto body = [&](const auto& R, RT scale) {
+            auto body = [&](const auto& R) {
                 RT sc[KG], Yc[NHB];
+                const RT fk = fcd * k.K * iq;
 #pragma unroll
                 for (int i = 0; i < KG; ++i) {
                     RT c = k.c[0];
 #pragma unroll
                     for (int j = 1; j < Q::KCD; ++j)
                         if (j == kg * KG + i) c = k.c[j];
-                    sc[i] = c * fcd * scale;
+                    sc[i] = c * fk;
                 }
 #pragma unroll
-                for (int h = 0; h < NHB; ++h) {
-                    RT s = RT(0);
+                for (int h = 0; h < NHB; ++h) Yc[h] = sc[0] * Y[0][h];
 #pragma unroll
-                    for (int kk = 0; kk < KG; ++kk) s += sc[kk] * Y[kk][h];
-                    Yc[h] = s;
+                for (int kk = 1; kk < KG; ++kk) {
+                    if (kk >= nk) continue;
+#pragma unroll
+                    for (int h = 0; h < NHB; ++h) Yc[h] += sc[kk] * Y[kk][h];
                 }
                 // one pass over the box: X_h and Z_k from the same R values
                 RT X[NH1], vx = RT(0), vy = RT(0), vz = RT(0);
@@ -251,9 +259,13 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                             gx += y * X[hidx(t + 1, u, w)];
                             gy += y * X[hidx(t, u + 1, w)];
                             gz += y * X[hidx(t, u, w + 1)];
-#pragma unroll
-                            for (int kk = 0; kk < KG; ++kk) Xs[kk][hidx(t, u, w)] += sc[kk] * X[hidx(t, u, w)];
                         }
+#pragma unroll
+                for (int kk = 0; kk < KG; ++kk) {
+                    if (kk > 0 && kk >= nk) continue;
+#pragma unroll
+                    for (int h = 0; h < NHB; ++h) Xs[kk][h] += sc[kk] * X[h];
+                }
                 gG[0] += gx;
                 gG[1] += gy;
                 gG[2] += gz;
@@ -262,20 +274,18 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                 dC[2] += vz - cq * gz;
             };
             if constexpr (RS) {
-                body(Rs + (size_t)(ik * st.i.nbp + ib) * nherm(L), RT(1));
+                body(Rs + (size_t)(ik * st.i.nbp + ib) * nherm(L));
             } else {
-                const RT p = sb[0];
-                const RT rs = rsqrt_t(p + q);
-                const RT alpha = p * q * rs * rs;
-                const RT pref = RT(TWO_PI_2_5) * sb[1] * iq * rs;
+                const BraPrim<RT> b = load_bra(sb);
+                const RT rs = rsqrt_t(b.p + q);
                 RT R[nherm(L)];
-                hermite_r<L>(alpha, sb[2] - k.Qx, sb[3] - k.Qy, sb[4] - k.Qz, R, boys);
+                hermite_r_scaled<L>(b.p * q * (rs * rs), b.X - k.Qx, b.Y - k.Qy, b.Z - k.Qz, rs, R, boys);
                 if constexpr (grad_rcol<CX, CY, RT>()) {
 #pragma unroll
                     for (int i = 0; i < nherm(L); ++i) Rcol[i * GRAD_THREADS] = R[i];
-                    body(RColumn<RT, GRAD_THREADS>{Rcol}, pref);
+                    body(RColumn<RT, GRAD_THREADS>{Rcol});
                 } else {
-                    body(R, pref);
+                    body(R);
                 }
             }
         }
@@ -285,48 +295,54 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
         for (int az = 0; az <= LA; ++az)
 #pragma unroll
             for (int bz = 0; bz <= LB; ++bz) {
-                RT W[KG][ncart(LAB)], Wz[KG][ncart(LAB)];       // E_z and dE_z applied
 #pragma unroll
-                for (int t = 0; t <= LAB - az - bz; ++t)
+                for (int kk = 0; kk < KG; ++kk) {
+                    if (kk > 0 && kk >= nk) continue;
+                    RT W[ncart(LAB)], Wz[ncart(LAB)];       // E_z and dE_z applied
 #pragma unroll
-                    for (int u = 0; u <= LAB - az - bz - t; ++u)
+                    for (int t = 0; t <= LAB - az - bz; ++t)
 #pragma unroll
-                        for (int kk = 0; kk < KG; ++kk) {
-                            RT s = RT(0), sz = RT(0);
+                        for (int u = 0; u <= LAB - az - bz - t; ++u) {
+                            RT s = Xs[kk][hidx(t, u, 0)], sz = RT(0);
+                            if (az + bz > 0) {
+                                s *= E[BE::at(2, az, bz, 0)];
 #pragma unroll
-                            for (int w = 0; w <= az + bz; ++w) {
-                                s += E[BE::at(2, az, bz, w)] * Xs[kk][hidx(t, u, w)];
-                                sz += DE[BE::at(2, az, bz, w)] * Xs[kk][hidx(t, u, w)];
+                                for (int w = 1; w <= az + bz; ++w) s += E[BE::at(2, az, bz, w)] * Xs[kk][hidx(t, u, w)];
                             }
-                            W[kk][cart_index(t, u)] = s;
-                            Wz[kk][cart_index(t, u)] = sz;
+#pragma unroll
+                            for (int w = 0; w <= az + bz; ++w) sz += DE[BE::at(2, az, bz, w)] * Xs[kk][hidx(t, u, w)];
+                            W[cart_index(t, u)] = s;
+                            Wz[cart_index(t, u)] = sz;
                         }
 #pragma unroll
-                for (int ay = 0; ay <= LA - az; ++ay)
+                    for (int ay = 0; ay <= LA - az; ++ay)
 #pragma unroll
-                    for (int by = 0; by <= LB - bz; ++by) {
-                        const int ax = LA - az - ay, bx = LB - bz - by;
-#pragma unroll
-                        for (int kk = 0; kk < KG; ++kk) {
+                        for (int by = 0; by <= LB - bz; ++by) {
+                            const int ax = LA - az - ay, bx = LB - bz - by;
                             const RT g = gq(cart_index(ay, az), cart_index(by, bz), kk);
 #pragma unroll
                             for (int t = 0; t <= ax + bx; ++t) {
-                                RT s = RT(0), sy = RT(0), sz = RT(0);
+                                RT s = W[cart_index(t, 0)], sy = RT(0), sz = Wz[cart_index(t, 0)];
+                                if (ay + by > 0) {
+                                    s *= E[BE::at(1, ay, by, 0)];
+                                    sz *= E[BE::at(1, ay, by, 0)];
 #pragma unroll
-                                for (int u = 0; u <= ay + by; ++u) {
-                                    s += E[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
-                                    sy += DE[BE::at(1, ay, by, u)] * W[kk][cart_index(t, u)];
-                                    sz += E[BE::at(1, ay, by, u)] * Wz[kk][cart_index(t, u)];
+                                    for (int u = 1; u <= ay + by; ++u) {
+                                        s += E[BE::at(1, ay, by, u)] * W[cart_index(t, u)];
+                                        sz += E[BE::at(1, ay, by, u)] * Wz[cart_index(t, u)];
+                                    }
                                 }
-                                const RT ge = g * E[BE::at(0, ax, bx, t)];
+#pragma unroll
+                                for (int u = 0; u <= ay + by; ++u) sy += DE[BE::at(1, ay, by, u)] * W[cart_index(t, u)];
+                                const RT ge = ax + bx > 0 ? g * E[BE::at(0, ax, bx, t)] : g;
                                 ux += g * DE[BE::at(0, ax, bx, t)] * s;
                                 uy += ge * sy;
                                 uz += ge * sz;
                             }
                         }
-                    }
+                }
             }
-        const RT ap = sb[5] * sb[1], bp = sb[6] * sb[1];
+        const RT ap = sb[4], bp = sb[5];
         dA[0] += ap * gG[0] + ux;
         dA[1] += ap * gG[1] + uy;
         dA[2] += ap * gG[2] + uz;
@@ -337,13 +353,13 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
 }
 
 // Gradient contribution of one column; adds A, B parts to gab and C, D
-// parts to the shared accumulator gsh (low words [natm][3], then the high words). RS: pref * R_tuv (to L + 1)
+// parts to the shared accumulator gsh (low words [natm][3], then the high words). RS: R_tuv / sqrt(p + q) (to L + 1)
 // of the ket pair's primitive quartets staged in Rs ([ik][ib][NH(L + 1)]).
 template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<RT>& st, int P2, double QQ, int ic,
                                             int id, int kg, double (&gab)[6], unsigned* gsh,
                                             const RT* __restrict__ Rs, RT* Rcol, int ib0, int ib1,
-                                            Boys boys) {
+                                            int nk, Boys boys) {
     using Q = QClass<CX, CY>;
     const BlockView& bv = a.q.bv;
     const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
@@ -389,7 +405,7 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
         for (int kk = 0; kk < Q::KG; ++kk) Gr[r][kk] = static_cast<RT>(G[r][kk]);
     RT dA[3] = {0.0, 0.0, 0.0}, dB[3] = {0.0, 0.0, 0.0}, dC[3] = {0.0, 0.0, 0.0};
     grad_prims<CX, CY, RT, RS>(st, Gr, a.q.pv.rec + a.q.pv.slot[P2] * PPW, a.q.pv.npp[P2], ic, id, kg, dA, dB, dC, Rs,
-                               Rcol, ib0, ib1, boys);
+                               Rcol, ib0, ib1, nk, boys);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double da = dA[d], db = dB[d], dc = dC[d];
@@ -430,7 +446,8 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
         const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         grad_column<CX, CY, RT, RS>(a, st, a.q.sorted[pos], q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
-                                    gsh, Rs, Rbuf + threadIdx.x, st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp, boys);
+                                    gsh, Rs, Rbuf + threadIdx.x, st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp,
+                                    group_combos<Q::KG>(sub, kg), boys);
     };
     if constexpr (RS) {
         int rot = 0;
@@ -468,7 +485,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kerne
     extern __shared__ __align__(16) double smem[];
     double* btab = smem;                                                // Boys table
     unsigned* gsh = reinterpret_cast<unsigned*>(btab + Boys::elems);    // low words [natm][3], then the high words
-    RT* Rbuf = reinterpret_cast<RT*>(btab + Boys::elems + 3 * a.natm);
+    RT* Rbuf = reinterpret_cast<RT*>(btab + Boys::elems + even(3 * a.natm));
     RT* Esm = Rbuf + a.rbuf;
     __shared__ BraInfo info;
     __shared__ FlatItems f;
@@ -526,7 +543,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kerne
 template <int CX, int CY, typename RT>
 size_t grad_rbuf_elems(int max_bra_prims, int max_ket_prims) {
     if constexpr (grad_rsmem<CX, CY>())
-        return rsmem_bytes<QClass<CX, CY>::L + 1, RT>(max_bra_prims, max_ket_prims) / sizeof(RT);
+        return fours(rsmem_bytes<QClass<CX, CY>::L + 1, RT>(max_bra_prims, max_ket_prims) / sizeof(RT));
     if constexpr (grad_rcol<CX, CY, RT>()) return (size_t)nherm(QClass<CX, CY>::L + 1) * GRAD_THREADS;
     return 0;
 }
@@ -534,7 +551,7 @@ size_t grad_rbuf_elems(int max_bra_prims, int max_ket_prims) {
 template <int CX, int CY, typename RT>
 size_t grad_smem_bytes(int natm, int max_bra_prims, size_t rbuf_elems) {
     using Q0 = QClass<CX, 0>;
-    return sizeof(double) * (3 * (size_t)natm + GradBoys<CX, CY, RT>::elems) +
+    return sizeof(double) * (even(3 * (size_t)natm) + GradBoys<CX, CY, RT>::elems) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (2 * BraE<Q0::LA, Q0::LB, 0>::SIZE + SBW));
 }
 
