@@ -594,17 +594,21 @@ __host__ __device__ constexpr int ket_prims2(int ppb) {
 template <int CX, int CY>
 __device__ __forceinline__ int64_t ket_work(int sub);
 
-// Work units of bra position spos against ket class CY in the ket ranges
-// that the kernels of type RT evaluate.
-template <int CX, int CY, typename RT>
-__device__ int64_t bra_work(const QuartetArgs& q, int spos) {
-    int64_t w = 0;
+// Work units of bra position spos against ket class CY in the FP64 (w[0]) and
+// FP32 (w[1]) ket ranges.
+template <int CX, int CY>
+__device__ void bra_work(const QuartetArgs& q, int spos, int64_t (&w)[2]) {
+    w[0] = w[1] = 0;
     for (int sub = 0; sub < NSUB; ++sub) {
-        int64_t kb, ke;
-        ket_range<RT>(q, CY * NSUB + sub, spos, kb, ke);
-        if (ke > kb) w += (ke - kb) * ket_work<CX, CY>(sub);
+        const size_t i = (size_t)(CY * NSUB + sub) * (q.npair + 1) + spos;
+        const int64_t cnt = q.counts[i], hi = q.counts_hi && q.counts_hi[i] < cnt ? q.counts_hi[i] : cnt;
+        const int64_t unit = ket_work<CX, CY>(sub);
+        w[0] += hi * unit;
+        w[1] += (cnt - hi) * unit;
     }
-    return w * q.pv.npp[q.sorted[spos]];
+    const int npp = q.pv.npp[q.sorted[spos]];
+    w[0] *= npp;
+    w[1] *= npp;
 }
 
 // Kets [k0, k1) of a segment of len kets, each of weight wk, whose work
@@ -691,9 +695,9 @@ struct BoysOf {
 struct JKArgs {
     QuartetArgs q;
     const double* D;    // [nset][nao][nao], symmetric
-    facc* J;            // un-symmetrised accumulators, same shape (fixed point, scale *fix)
+    facc* J;            // un-symmetrised accumulators, same shape (fixed point)
     facc* K;
-    const double* fix;  // device scalar: the fixed-point scale of J and K (jk_fix_for(max |D|))
+    const double* dmax; // device scalar max |D|: the fixed-point scale of J and K is jk_fix_for(*dmax)
     // density-weighted screening (difference densities): skip a quartet when
     // Q1 Q2 max|D| over its six density blocks < dthr; bmax = nullptr: off
     const double* bmax; // [nblock][nblock] max |D| per block pair (all sets)
@@ -720,14 +724,13 @@ template <int CX, int CY, int NS, bool KGLOBAL, typename ST>
 __device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, int P2, int C, int Dd, int ic,
                                                  int id, int kg,
                                                  const double (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                 double* Jt, unsigned* Ksm) {
+                                                 double* Jt, unsigned* Ksm, double fx) {
     using Q = QClass<CX, CY>;
     const BlockView& bv = a.q.bv;
     const int nC = bv.ncon[C], nD = bv.ncon[Dd], oC = bv.ao[C], oD = bv.ao[Dd];
     const double g = 1.0 / ((st.i.A == st.i.B ? 2.0 : 1.0) * (C == Dd ? 2.0 : 1.0) * (st.i.P1 == P2 ? 2.0 : 1.0));
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
-    const double fx = __ldg(a.fix);
     constexpr int NFA = Q::KA * Q::NA;      // A slots, then B slots
     constexpr int NF = NFA + Q::KB * Q::NB;
 #pragma unroll
@@ -1166,7 +1169,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
 template <int CX, int CY, int NS, bool KGLOBAL, typename RT, typename Boys>
 __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT>& st, int spos, double* Jt,
                                              unsigned* Ksm, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf,
-                                             Boys boys) {
+                                             Boys boys, double fx) {
     using Q = QClass<CX, CY>;
     const double q1 = a.q.sortedQ[spos];
     const double* bm = a.bmax;
@@ -1183,7 +1186,7 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
     };
     auto digest = [&](int P2, int C, int Dd, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
         if constexpr (sizeof(RT) == sizeof(double)) {
-            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, v, Jt, Ksm);
+            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, v, Jt, Ksm, fx);
         } else {
             // FP32 quartets: digested (accumulated) in FP64
             double vd[Q::NROW][Q::KG];
@@ -1191,7 +1194,7 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
             for (int r = 0; r < Q::NROW; ++r)
 #pragma unroll
                 for (int k = 0; k < Q::KG; ++k) vd[r][k] = static_cast<double>(v[r][k]);
-            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, vd, Jt, Ksm);
+            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, vd, Jt, Ksm, fx);
         }
     };
     // item r = (contraction group that the segment's pairs carry, bra-primitive split, column block)
@@ -1286,7 +1289,7 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
     const int nbra = a.q.cls_start[CX + 1] - a.q.cls_start[CX];
     const int total = a.plan.off[nbra];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double fx = __ldg(a.fix);
+    const double fx = jk_fix_for(__ldg(a.dmax));
     bool staged = false;        // the Boys table is in shared memory, and the accumulators are zero
     for (;;) {
         if (warp == 0) {
@@ -1316,7 +1319,7 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
         stage_bra_e<Q0::LA, Q0::LB, 0>(st);
         __syncthreads();
         jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf,
-                                                 Boys::get(btab));
+                                                 Boys::get(btab), fx);
         __syncthreads();
         // flush J_ab: a warp a (set, row) sums the threads' slots (in a fixed
         // order) and clears them

@@ -118,10 +118,10 @@ struct aimd_ctx {
     int64_t* counts_g;
     int64_t* counts_d;      // difference-density builds (threshold changes every call)
     double* bmax;           // [nblock][nblock] max |D| per block pair
-    double* dmax;           // [1] max over bmax
-    double* jkfix;          // [1] fixed-point scale of the J/K accumulators
+    double* dmax;           // [1] max over bmax, behind the J/K accumulators (cleared with them)
     int* plan;              // work plans of the class kernels (LaunchEnv::plan_of)
     int* plan_next;         // their chunk counters
+    int64_t* bra_work;      // [2 types][NCLS][npair] work units of each bra (bra_work_kernel)
     // launch shape (aimd_set_launch_shape): work-plan chunks per resident
     // CTA, primitive quartets per split column item
     int plan_chunks = 8;
@@ -216,8 +216,9 @@ extern "C" int aimd_create(aimd_ctx** out, int natm, int nao, int nblock, const 
     c->charges_host.assign(charges, charges + natm);
     CK(dalloc(&c->pos, 3 * (size_t)natm));
     CK(up_d(&c->boys, boys_tables().data(), boys_tables().size()));
-    CK(dalloc(&c->jacc, (size_t)nao * nao));
-    CK(dalloc(&c->kacc, (size_t)nao * nao));
+    CK(dalloc(&c->jacc, 2 * (size_t)nao * nao + 1));
+    c->kacc = c->jacc + (size_t)nao * nao;
+    c->dmax = reinterpret_cast<double*>(c->jacc + 2 * (size_t)nao * nao);
     CK(dalloc(&c->gacc, 3 * (size_t)natm));
     // shell pairs (si >= sj) grouped by class (l_i >= l_j after orientation)
     {
@@ -292,10 +293,9 @@ extern "C" int aimd_create(aimd_ctx** out, int natm, int nao, int nblock, const 
         CK(dalloc(&c->counts_hi_d, (size_t)NSEG * (np + 1)));
         CK(dalloc(&c->counts_hi, (size_t)NSEG * (np + 1)));
         CK(dalloc(&c->bmax, (size_t)nblock * nblock));
-        CK(dalloc(&c->dmax, 1));
-        CK(dalloc(&c->jkfix, 1));
         CK(dalloc(&c->plan, (size_t)2 * NCLS * (np + NCLS)));
         CK(dalloc(&c->plan_next, (size_t)2 * NCLS * NCLS));
+        CK(dalloc(&c->bra_work, (size_t)2 * NCLS * np));
         CK(dalloc(&c->bmc, (size_t)nblock * nblock));
         CK(dalloc(&c->bmx, (size_t)nblock * nblock));
         for (int cl = 0; cl < NCLS; ++cl) c->maxbp[cl] = 1;
@@ -322,7 +322,7 @@ extern "C" int aimd_destroy(aimd_ctx* c) {
                     c->sh_atom, c->sh_l, c->sh_ao, c->sh_p0, c->sh_np, c->sp_i, c->sp_j, c->sh_exp, c->sh_coef,
                     c->charges, c->pa, c->pb, c->npp, c->slot, c->rec, c->Q, c->by_class, c->idx_in,
                     c->tmp_idx, c->seg_id, c->seg_keys, c->seg_keys_out, c->seg_start, c->tmpQ, c->sortedQ,
-                    c->sorted, c->counts_jk, c->counts_g, c->counts_d, c->bmax, c->dmax, c->jkfix, c->plan, c->plan_next, c->bmc, c->bmx, c->counts_hi, c->counts_hi_d, c->cub_tmp, c->pos, c->boys, c->jacc, c->kacc, c->gacc};
+                    c->sorted, c->counts_jk, c->counts_g, c->counts_d, c->bmax, c->plan, c->plan_next, c->bra_work, c->bmc, c->bmx, c->counts_hi, c->counts_hi_d, c->cub_tmp, c->pos, c->boys, c->jacc, c->gacc};
     for (void* p : ptrs) cudaFree(p);
     for (int i = 0; i < NSTREAM; ++i) {
         if (c->streams[i]) cudaStreamDestroy(c->streams[i]);
@@ -454,50 +454,47 @@ __global__ void quartet_count_kernel(int npair, ClsStart cs, const int* seg_star
     }
 }
 
-// bmax[I][J] = max over the functions of blocks I, J and the sets of |D|
-__global__ void block_dmax_kernel(int nblock, int nao, int nset, const int* blk_l, const int* blk_ncon,
-                                  const int* blk_ao, const double* D, double* bmax) {
+// bmax[I][J] = max over the functions of blocks I, J and the sets of |D|;
+// dmax (optional, zero before) = max over all of them, as the bits of a double
+// >= 0, whose order is that of the values (a NaN element of D is passed over by
+// fmax, as in the maximum itself)
+__global__ void __launch_bounds__(128) block_dmax_kernel(int nblock, int nao, int nset, const int* blk_l,
+                                                         const int* blk_ncon, const int* blk_ao, const double* D,
+                                                         double* bmax, unsigned long long* dmax) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nblock * nblock) return;
-    const int I = i / nblock, J = i % nblock;
-    const int nI = blk_ncon[I] * ncart(blk_l[I]), nJ = blk_ncon[J] * ncart(blk_l[J]);
-    const size_t nn = (size_t)nao * nao;
     double m = 0.0;
-    for (int s = 0; s < nset; ++s)
-        for (int a = 0; a < nI; ++a)
-            for (int b = 0; b < nJ; ++b) m = fmax(m, fabs(D[s * nn + (size_t)(blk_ao[I] + a) * nao + blk_ao[J] + b]));
-    bmax[i] = m;
+    if (i < nblock * nblock) {
+        const int I = i / nblock, J = i % nblock;
+        const int nI = blk_ncon[I] * ncart(blk_l[I]), nJ = blk_ncon[J] * ncart(blk_l[J]);
+        const size_t nn = (size_t)nao * nao;
+        for (int s = 0; s < nset; ++s)
+            for (int a = 0; a < nI; ++a)
+                for (int b = 0; b < nJ; ++b) m = fmax(m, fabs(D[s * nn + (size_t)(blk_ao[I] + a) * nao + blk_ao[J] + b]));
+        bmax[i] = m;
+    }
+    if (!dmax) return;
+    for (int d = 16; d > 0; d >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(dmax, (unsigned long long)__double_as_longlong(m));
 }
 
-// out = acc / scale (add = 0) or out += acc / scale (add = 1); the scale is
-// *scale_p when that is given (a device scalar), else scale
-__global__ void from_fixed_kernel(size_t n, const facc* acc, const double* scale_p, double scale, double* out,
-                                  int add) {
+// out = acc / scale (add = 0) or out += acc / scale (add = 1)
+__global__ void from_fixed_kernel(size_t n, const facc* acc, double scale, double* out, int add) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double v = from_fixed(acc[i], scale_p ? *scale_p : scale);
+    const double v = from_fixed(acc[i], scale);
     out[i] = add ? out[i] + v : v;
 }
-void from_fixed(cudaStream_t st, size_t n, const facc* acc, const double* scale_p, double scale, double* out,
-                int add) {
-    from_fixed_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, acc, scale_p, scale, out, add);
+// J and K at once, at the scale of the largest density element *dmax
+__global__ void jk_from_fixed_kernel(size_t n, const facc* jacc, const facc* kacc, const double* dmax, double* J,
+                                     double* K) {
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double scale = jk_fix_for(*dmax);
+    J[i] = from_fixed(jacc[i], scale);
+    K[i] = from_fixed(kacc[i], scale);
 }
-
-// *out = max of x[0 .. n); fix (optional) = jk_fix_for(*out)
-__global__ void max_reduce_kernel(int n, const double* x, double* out, double* fix) {
-    __shared__ double sm[256];
-    double m = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, x[i]);
-    sm[threadIdx.x] = m;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (threadIdx.x < w) sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + w]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        *out = sm[0];
-        if (fix) *fix = jk_fix_for(sm[0]);
-    }
+void from_fixed(cudaStream_t st, size_t n, const facc* acc, double scale, double* out, int add) {
+    from_fixed_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, acc, scale, out, add);
 }
 
 PairView pair_view(aimd_ctx* c) { return PairView{c->pa, c->pb, c->slot, c->npp, c->rec}; }
@@ -553,7 +550,31 @@ LaunchEnv launch_env(aimd_ctx* c) {
     return e;
 }
 
-// Work plan of the (CX, CY, RT) launch (one CTA of PLAN_THREADS): per bra
+// Work of every (bra position, ket class, type), one thread each:
+// work[(rt NCLS + cy) npair + s], read by the planner below. (Summing a bra's
+// 18 segments inside the planner, which has one CTA a class pair, took most of
+// its 0.4 ms at (H2O)32.)
+__global__ void __launch_bounds__(128) bra_work_kernel(QuartetArgs q, int64_t* work) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x, cy = blockIdx.y;
+    if (s >= q.npair) return;
+    int cx = 0;
+    while (s >= q.cls_start[cx + 1]) ++cx;
+    if (cy > cx) return;
+    int64_t w[2];
+#define AIMD_WORK(X, Y) \
+    if (cx == X && cy == Y) bra_work<X, Y>(q, s, w);
+    AIMD_WORK(0, 0)
+    AIMD_WORK(1, 0) AIMD_WORK(1, 1)
+    AIMD_WORK(2, 0) AIMD_WORK(2, 1) AIMD_WORK(2, 2)
+    AIMD_WORK(3, 0) AIMD_WORK(3, 1) AIMD_WORK(3, 2) AIMD_WORK(3, 3)
+    AIMD_WORK(4, 0) AIMD_WORK(4, 1) AIMD_WORK(4, 2) AIMD_WORK(4, 3) AIMD_WORK(4, 4)
+    AIMD_WORK(5, 0) AIMD_WORK(5, 1) AIMD_WORK(5, 2) AIMD_WORK(5, 3) AIMD_WORK(5, 4) AIMD_WORK(5, 5)
+#undef AIMD_WORK
+    work[(size_t)cy * q.npair + s] = w[0];
+    if (q.counts_hi) work[(size_t)(NCLS + cy) * q.npair + s] = w[1];
+}
+
+// Work plan of the (CX, CY, type) launch (one CTA of PLAN_THREADS): per bra
 // of class CX its chunk count ceil(W / target), target = max(total W /
 // parts, PLAN_MIN_WORK) with parts = chunks per resident CTA x resident
 // CTAs, as an exclusive prefix in off[0 .. nbra]; the launch's chunk
@@ -573,77 +594,58 @@ __device__ T block_sum(T v, T* red) {
     return t;
 }
 
-template <int CX, int CY, typename RT>
-__device__ void plan_launch(const QuartetArgs& q, int* off, int* next, int parts) {
-    __shared__ int64_t red[PLAN_THREADS / 32];
-    __shared__ int ired[PLAN_THREADS / 32];
-    const int nbra = q.cls_start[CX + 1] - q.cls_start[CX];
-    const int per = (nbra + PLAN_THREADS - 1) / PLAN_THREADS;
-    const int b0 = min(nbra, (int)threadIdx.x * per), b1 = min(nbra, b0 + per);
-    int64_t w = 0;
-    for (int b = b0; b < b1; ++b) w += bra_work<CX, CY, RT>(q, q.cls_start[CX] + b);
-    const int64_t W = block_sum(w, red);
-    int64_t target = W / parts;
-    if (target < PLAN_MIN_WORK) target = PLAN_MIN_WORK;
-    int cnt = 0;
-    for (int b = b0; b < b1; ++b) {
-        const int64_t wb = bra_work<CX, CY, RT>(q, q.cls_start[CX] + b);
-        off[b] = (int)((wb + target - 1) / target);
-        cnt += off[b];
-    }
-    // exclusive scan of the per-thread counts (threads in index order)
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = cnt;
-    for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
-    }
-    if (lane == 31) ired[warp] = incl;
-    __syncthreads();
-    int base = incl - cnt;
-    for (int w2 = 0; w2 < warp; ++w2) base += ired[w2];
-    for (int b = b0; b < b1; ++b) {
-        const int k = off[b];
-        off[b] = base;
-        base += k;
-    }
-    if (threadIdx.x == PLAN_THREADS - 1) {
-        off[nbra] = base;                               // the last thread ends at the total
-        *next = 0;
-    }
-}
-
 // one CTA per (bra class, ket class <= bra class, type): blockIdx.x = pair
 // index CX (CX + 1) / 2 + CY, blockIdx.y = type (0: FP64 ranges, 1: FP32)
-__global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, int* plan, int* plan_next, int stride,
-                                                            int parts) {
+__global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, const int64_t* work, int* plan,
+                                                            int* plan_next, int stride, int parts) {
+    __shared__ int64_t red[PLAN_THREADS / 32];
+    __shared__ int ired[PLAN_THREADS / 32];
     int cx = 0;
     while ((cx + 1) * (cx + 2) / 2 <= (int)blockIdx.x) ++cx;
     const int cy = blockIdx.x - cx * (cx + 1) / 2, rt = blockIdx.y;
     int* off = plan + (size_t)(rt * NCLS + cy) * stride + q.cls_start[cx] + cx;
-    int* next = plan_next + (rt * NCLS + cx) * NCLS + cy;
-#define AIMD_PLAN(X, Y)                                                         \
-    if (cx == X && cy == Y) {                                                   \
-        if (rt == 0) plan_launch<X, Y, double>(q, off, next, parts);           \
-        else plan_launch<X, Y, float>(q, off, next, parts);                    \
+    const int64_t* w = work + (size_t)(rt * NCLS + cy) * q.npair + q.cls_start[cx];
+    const int nbra = q.cls_start[cx + 1] - q.cls_start[cx];
+    int64_t mine = 0;
+    for (int b = threadIdx.x; b < nbra; b += PLAN_THREADS) mine += w[b];
+    const int64_t W = block_sum(mine, red);
+    int64_t target = W / parts;
+    if (target < PLAN_MIN_WORK) target = PLAN_MIN_WORK;
+    // exclusive scan over the bras, PLAN_THREADS at a time
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int b0 = 0; b0 < nbra; b0 += PLAN_THREADS) {
+        const int b = b0 + threadIdx.x;
+        const int cnt = b < nbra ? static_cast<int>((w[b] + target - 1) / target) : 0;
+        int incl = cnt;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        __syncthreads();                                // the sums of the step before are read
+        if (lane == 31) ired[warp] = incl;
+        __syncthreads();
+        int before = base, total = 0;
+        for (int v = 0; v < PLAN_THREADS / 32; ++v) {
+            if (v < warp) before += ired[v];
+            total += ired[v];
+        }
+        if (b < nbra) off[b] = before + incl - cnt;
+        base += total;
     }
-    AIMD_PLAN(0, 0)
-    AIMD_PLAN(1, 0) AIMD_PLAN(1, 1)
-    AIMD_PLAN(2, 0) AIMD_PLAN(2, 1) AIMD_PLAN(2, 2)
-    AIMD_PLAN(3, 0) AIMD_PLAN(3, 1) AIMD_PLAN(3, 2) AIMD_PLAN(3, 3)
-    AIMD_PLAN(4, 0) AIMD_PLAN(4, 1) AIMD_PLAN(4, 2) AIMD_PLAN(4, 3) AIMD_PLAN(4, 4)
-    AIMD_PLAN(5, 0) AIMD_PLAN(5, 1) AIMD_PLAN(5, 2) AIMD_PLAN(5, 3) AIMD_PLAN(5, 4) AIMD_PLAN(5, 5)
-#undef AIMD_PLAN
+    if (threadIdx.x == 0) {
+        off[nbra] = base;
+        plan_next[(rt * NCLS + cx) * NCLS + cy] = 0;
+    }
 }
 
 // Plans of every class launch of one call (mixed: the FP32 ones too), on st
 // before the class streams fork.
 void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, cudaStream_t st) {
-    plan_kernel<<<dim3(NCLS * (NCLS + 1) / 2, mixed ? 2 : 1), PLAN_THREADS, 0, st>>>(q, c->plan, c->plan_next,
-                                                                                   c->npair + NCLS,
-                                                                                   c->plan_chunks * 2 * c->nsm);
-    ++c->launches;
+    bra_work_kernel<<<dim3((c->npair + 127) / 128, NCLS), 128, 0, st>>>(q, c->bra_work);
+    plan_kernel<<<dim3(NCLS * (NCLS + 1) / 2, mixed ? 2 : 1), PLAN_THREADS, 0, st>>>(
+        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, c->plan_chunks * 2 * c->nsm);
+    c->launches += 2;
 }
 
 int cls_size(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
@@ -819,10 +821,10 @@ extern "C" int aimd_jk(aimd_ctx* c, int nset, const double* D, double* J, double
     const size_t nn = (size_t)c->nao * c->nao;
     // fixed-point scale of the accumulators from max |D| over the sets
     const int nb2 = c->nblock * c->nblock;
+    CK(cudaMemsetAsync(c->jacc, 0, sizeof(facc) * (2 * nn + 1), st));
     block_dmax_kernel<<<(nb2 + 127) / 128, 128, 0, st>>>(c->nblock, c->nao, nset, c->blk_l, c->blk_ncon, c->blk_ao, D,
-                                                         c->bmax);
-    max_reduce_kernel<<<1, 256, 0, st>>>(nb2, c->bmax, c->dmax, c->jkfix);
-    c->launches += 2;
+                                                         c->bmax, reinterpret_cast<unsigned long long*>(c->dmax));
+    ++c->launches;
 
     // one pass per density (UHF: alpha and beta)
     const LaunchEnv e = launch_env(c);
@@ -833,9 +835,8 @@ extern "C" int aimd_jk(aimd_ctx* c, int nset, const double* D, double* J, double
         a.D = D + s0 * nn;
         a.J = c->jacc;
         a.K = c->kacc;
-        a.fix = c->jkfix;
-        CK(cudaMemsetAsync(c->jacc, 0, sizeof(facc) * nn, st));
-        CK(cudaMemsetAsync(c->kacc, 0, sizeof(facc) * nn, st));
+        a.dmax = c->dmax;
+        if (s0 > 0) CK(cudaMemsetAsync(c->jacc, 0, sizeof(facc) * 2 * nn, st));
         a.bmax = nullptr;
         a.nblock = c->nblock;
         a.dthr = 0.0;
@@ -845,9 +846,9 @@ extern "C" int aimd_jk(aimd_ctx* c, int nset, const double* D, double* J, double
         plan_launches(c, a.q, mixed, st);
         if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
             return r;
-        from_fixed(st, nn, c->jacc, c->jkfix, 0.0, J + s0 * nn, 0);
-        from_fixed(st, nn, c->kacc, c->jkfix, 0.0, K + s0 * nn, 0);
-        c->launches += 2;
+        jk_from_fixed_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(nn, c->jacc, c->kacc, c->dmax, J + s0 * nn,
+                                                                           K + s0 * nn);
+        ++c->launches;
         CK(cudaGetLastError());
     }
     return AIMD_OK;
@@ -881,10 +882,10 @@ extern "C" int aimd_jk_delta(aimd_ctx* c, int nset, const double* D, double* J, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t nn = (size_t)c->nao * c->nao;
     const int nb2 = c->nblock * c->nblock;
+    CK(cudaMemsetAsync(c->jacc, 0, sizeof(facc) * (2 * nn + 1), st));
     block_dmax_kernel<<<(nb2 + 127) / 128, 128, 0, st>>>(c->nblock, c->nao, nset, c->blk_l, c->blk_ncon, c->blk_ao, D,
-                                                         c->bmax);
-    max_reduce_kernel<<<1, 256, 0, st>>>(nb2, c->bmax, c->dmax, c->jkfix);
-    c->launches += 2;
+                                                         c->bmax, reinterpret_cast<unsigned long long*>(c->dmax));
+    ++c->launches;
     CK(cudaGetLastError());
     // enumerate at max(thr, dthr / max|D|): the integral screen still holds,
     // and no quartet that the density-weighted test keeps is missed
@@ -907,9 +908,8 @@ extern "C" int aimd_jk_delta(aimd_ctx* c, int nset, const double* D, double* J, 
         a.D = D + s0 * nn;
         a.J = c->jacc;
         a.K = c->kacc;
-        a.fix = c->jkfix;
-        CK(cudaMemsetAsync(c->jacc, 0, sizeof(facc) * nn, st));
-        CK(cudaMemsetAsync(c->kacc, 0, sizeof(facc) * nn, st));
+        a.dmax = c->dmax;
+        if (s0 > 0) CK(cudaMemsetAsync(c->jacc, 0, sizeof(facc) * 2 * nn, st));
         a.bmax = c->bmax;
         a.nblock = c->nblock;
         a.dthr = dthr;
@@ -919,9 +919,9 @@ extern "C" int aimd_jk_delta(aimd_ctx* c, int nset, const double* D, double* J, 
         plan_launches(c, a.q, mixed, st);
         if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk_delta", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
             return r;
-        from_fixed(st, nn, c->jacc, c->jkfix, 0.0, J + s0 * nn, 0);
-        from_fixed(st, nn, c->kacc, c->jkfix, 0.0, K + s0 * nn, 0);
-        c->launches += 2;
+        jk_from_fixed_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(nn, c->jacc, c->kacc, c->dmax, J + s0 * nn,
+                                                                           K + s0 * nn);
+        ++c->launches;
         CK(cudaGetLastError());
     }
     return AIMD_OK;
@@ -1058,11 +1058,11 @@ extern "C" int aimd_grad2e(aimd_ctx* c, const double* Dc, int nx, const double* 
     CK(cudaMemsetAsync(c->gacc, 0, sizeof(facc) * 3 * c->natm, st));
     const int nb2 = c->nblock * c->nblock;
     block_dmax_kernel<<<(nb2 + 127) / 128, 128, 0, st>>>(c->nblock, c->nao, 1, c->blk_l, c->blk_ncon, c->blk_ao, Dc,
-                                                         c->bmc);
+                                                         c->bmc, nullptr);
     ++c->launches;
     if (nx > 0) {
         block_dmax_kernel<<<(nb2 + 127) / 128, 128, 0, st>>>(c->nblock, c->nao, nx, c->blk_l, c->blk_ncon, c->blk_ao,
-                                                             Dx, c->bmx);
+                                                             Dx, c->bmx, nullptr);
         ++c->launches;
     }
     CK(cudaGetLastError());
@@ -1088,7 +1088,7 @@ extern "C" int aimd_grad2e(aimd_ctx* c, const double* Dc, int nx, const double* 
     const LaunchEnv e = launch_env(c);
     if (int r = run_concurrent(c, st, NSTREAM, "aimd_grad2e", class_pair_launches(c, mixed), [&] { return launch_grads(e, a); }))
         return r;
-    from_fixed(st, 3 * (size_t)c->natm, c->gacc, nullptr, FIX_G, grad, 0);
+    from_fixed(st, 3 * (size_t)c->natm, c->gacc, FIX_G, grad, 0);
     ++c->launches;
     CK(cudaGetLastError());
     return AIMD_OK;
@@ -1153,7 +1153,7 @@ extern "C" int aimd_onee_grad(aimd_ctx* c, const double* W, const double* D, dou
             return x;
         }))
         return r;
-    from_fixed(st, 3 * (size_t)c->natm, c->gacc, nullptr, FIX_G, grad, 1);
+    from_fixed(st, 3 * (size_t)c->natm, c->gacc, FIX_G, grad, 1);
     ++c->launches;
     CK(cudaGetLastError());
     return AIMD_OK;
