@@ -540,11 +540,25 @@ struct QuartetArgs {
     // nullptr: everything in FP64.
     const int64_t* counts_hi;
     const int* seg_start;       // [NSEG + 1] sorted position of each segment (device)
+    const int4* meta;           // [3][npair] what an item needs of the pair at a sorted position (PairMeta)
     const double* boys;         // Boys tables of all orders (device)
     int npair;
     int cls_start[NCLS + 1];    // sorted positions of each angular class (geometry independent)
     int nao;
 };
+
+// One pair by its sorted position: three 16-byte loads, neighbouring positions
+// side by side, where pair index -> blocks -> contractions, AOs and atoms was a
+// chain of three dependent loads at the start of every item.
+struct PairMeta {
+    int P, npp, nA, nB, oA, oB, aA, aB, A, B;
+    const double* rec;      // primitive records
+};
+__device__ __forceinline__ PairMeta load_meta(const QuartetArgs& a, int pos) {
+    const int4 u = __ldg(a.meta + pos), v = __ldg(a.meta + a.npair + pos), w = __ldg(a.meta + 2 * a.npair + pos);
+    const int64_t slot = static_cast<int64_t>((static_cast<uint64_t>(static_cast<unsigned>(w.w)) << 32) | static_cast<unsigned>(w.z));
+    return PairMeta{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w, w.x, w.y, a.pv.rec + slot * PPW};
+}
 
 // Ket range [b, e) of segment seg for bra position spos that the kernels of
 // arithmetic type RT evaluate: the FP64 prefix, or the FP32 tail.
@@ -606,7 +620,7 @@ __device__ void bra_work(const QuartetArgs& q, int spos, int64_t (&w)[2]) {
         w[0] += hi * unit;
         w[1] += (cnt - hi) * unit;
     }
-    const int npp = q.pv.npp[q.sorted[spos]];
+    const int npp = load_meta(q, spos).npp;
     w[0] *= npp;
     w[1] *= npp;
 }
@@ -630,15 +644,17 @@ __device__ __forceinline__ int64_t chunk_edge(int64_t W, int j, int nch) {
 // The next chunk of the launch for this CTA (warp 0 calls it): lane 0 takes
 // it from the counter, the lanes search its bra together, 32 entries a step
 // (last b with off[b] <= c; a lone thread's binary search was a chain of a
-// dozen loads that the CTA waited for, once a chunk). c >= off[nbra] when the
-// plan is used up.
+// dozen loads that the CTA waited for, once a chunk). c = -1 when the plan is
+// used up. Chunks are taken from the last on: bras of many primitives come
+// last in the order, and the long chunks should not be the launch's tail.
 __device__ __forceinline__ void next_chunk(const WorkPlan& plan, int nbra, int total, int& c, int& b) {
     const int lane = threadIdx.x & 31;
     int cc = 0;
     if (lane == 0) cc = atomicAdd(plan.next, 1);
-    c = __shfl_sync(0xffffffffu, cc, 0);
-    int lo = 0, hi = nbra;                              // off[lo] <= c < off[hi] while c < total
-    while (c < total && hi - lo > 1) {
+    cc = __shfl_sync(0xffffffffu, cc, 0);
+    c = cc < total ? total - 1 - cc : -1;
+    int lo = 0, hi = nbra;                              // off[lo] <= c < off[hi]
+    while (c >= 0 && hi - lo > 1) {
         const int step = (hi - lo + 31) / 32, at = lo + lane * step;
         const unsigned le = __ballot_sync(0xffffffffu, at < hi && plan.off[at] <= c);
         lo += (31 - __clz(le)) * step;                  // lane 0 always holds: le != 0
@@ -647,6 +663,20 @@ __device__ __forceinline__ void next_chunk(const WorkPlan& plan, int nbra, int t
     b = lo;
 }
 
+__device__ __forceinline__ void load_info(const QuartetArgs& a, const PairMeta& m, BraInfo& st) {
+    st.P1 = m.P;
+    st.A = m.A;
+    st.B = m.B;
+    st.nbp = m.npp;
+    st.rec = m.rec;
+    st.aA = m.aA;
+    st.aB = m.aB;
+    st.nA = m.nA;
+    st.nB = m.nB;
+    st.oA = m.oA;
+    st.oB = m.oB;
+}
+// by pair index (the Schwarz bounds, before the pairs are sorted)
 __device__ __forceinline__ void load_info(const QuartetArgs& a, int P1, BraInfo& st) {
     st.P1 = P1;
     st.A = a.pv.pa_blk[P1];
@@ -721,14 +751,13 @@ struct JKArgs {
 // K rows m, n belong to the bra pair: Ksm[set][slot][col], slot < KA*NA for
 // A's functions, then B's.
 template <int CX, int CY, int NS, bool KGLOBAL, typename ST>
-__device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, int P2, int C, int Dd, int ic,
+__device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, const PairMeta& ket, int ic,
                                                  int id, int kg,
                                                  const double (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
                                                  double* Jt, unsigned* Ksm, double fx) {
     using Q = QClass<CX, CY>;
-    const BlockView& bv = a.q.bv;
-    const int nC = bv.ncon[C], nD = bv.ncon[Dd], oC = bv.ao[C], oD = bv.ao[Dd];
-    const double g = 1.0 / ((st.i.A == st.i.B ? 2.0 : 1.0) * (C == Dd ? 2.0 : 1.0) * (st.i.P1 == P2 ? 2.0 : 1.0));
+    const int nC = ket.nA, nD = ket.nB, oC = ket.oA, oD = ket.oB;
+    const double g = (st.i.A == st.i.B ? 0.5 : 1.0) * (ket.A == ket.B ? 0.5 : 1.0) * (st.i.P1 == ket.P ? 0.5 : 1.0);
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
     constexpr int NFA = Q::KA * Q::NA;      // A slots, then B slots
@@ -999,10 +1028,11 @@ __device__ __forceinline__ void flat_items(FlatItems& f, bool queued, int* queue
             }
             __syncthreads();
         }
-        const int64_t items = f.pre[NSUB];
-        int s = 0;
-        for (int64_t it = threadIdx.x; it < items; it += blockDim.x) {
-            while (it >= f.pre[s + 1]) ++s;
+        // from the last segment (pairs of the most primitives) to the first, so
+        // that the threads part at short items
+        int s = NSUB - 1;
+        for (int64_t it = f.pre[NSUB] - 1 - threadIdx.x; it >= 0; it -= blockDim.x) {
+            while (it < f.pre[s]) --s;
             const unsigned loc = static_cast<unsigned>(it - f.pre[s]), nq = f.cnt[s];
             const unsigned r = loc / nq;
             const int at = f.j0[s] + static_cast<int>(loc - r * nq);
@@ -1101,7 +1131,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
         const int m = static_cast<int>(cnt - base < KQ_CAP ? cnt - base : KQ_CAP);
         compact(q, j0 + static_cast<int>(base), m, keep, [&](int slot, int pos) {
             q.pos[slot] = pos;
-            q.pq[slot] = qa.pv.npp[qa.sorted[pos]] * nbp;          // primitive quartets of the entry
+            q.pq[slot] = load_meta(qa, pos).npp * nbp;              // primitive quartets of the entry
         });
         const int ne = q.n;
         if (ne == 0) continue;                                      // uniform: q.n is shared
@@ -1146,8 +1176,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
                 const int i = lower_bound_i(q.pq, f, l + 1, pq0 + w + 1) - 1;   // last entry with pq <= pq0 + w
                 const int rem = pq0 + w - q.pq[i];
                 const int ik = rem / nbp, ib = rem - ik * nbp;
-                const int P2 = qa.sorted[q.pos[i]];
-                stage_r<L>(st, ib, qa.pv.rec + (qa.pv.slot[P2] + ik) * PPW, Rbuf + (size_t)w * NH);
+                stage_r<L>(st, ib, load_meta(qa, q.pos[i]).rec + (size_t)ik * PPW, Rbuf + (size_t)w * NH);
             }
             __syncthreads();
             // stage 2: the column items of the sub-chunk, column-major as in ket_items
@@ -1177,16 +1206,16 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
     // difference densities: density-weighted test on the six block pairs
     auto keep = [&](int pos) {
         if (!bm) return true;
-        const int P2 = a.q.sorted[pos];
-        const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
+        const PairMeta k = load_meta(a.q, pos);
+        const int C = k.A, Dd = k.B;
         const double dm = fmax(fmax(bm[st.i.A * nb + st.i.B], bm[C * nb + Dd]),
                                fmax(fmax(bm[st.i.A * nb + C], bm[st.i.A * nb + Dd]),
                                     fmax(bm[st.i.B * nb + C], bm[st.i.B * nb + Dd])));
         return q1 * a.q.sortedQ[pos] * dm >= a.dthr;
     };
-    auto digest = [&](int P2, int C, int Dd, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
+    auto digest = [&](const PairMeta& k, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
         if constexpr (sizeof(RT) == sizeof(double)) {
-            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, v, Jt, Ksm, fx);
+            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, k, ic, id, kg, v, Jt, Ksm, fx);
         } else {
             // FP32 quartets: digested (accumulated) in FP64
             double vd[Q::NROW][Q::KG];
@@ -1194,7 +1223,7 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
             for (int r = 0; r < Q::NROW; ++r)
 #pragma unroll
                 for (int k = 0; k < Q::KG; ++k) vd[r][k] = static_cast<double>(v[r][k]);
-            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, P2, C, Dd, ic, id, kg, vd, Jt, Ksm, fx);
+            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, k, ic, id, kg, vd, Jt, Ksm, fx);
         }
     };
     // item r = (contraction group that the segment's pairs carry, bra-primitive split, column block)
@@ -1203,20 +1232,18 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         const int ib0 = st.i.nbp * sp / nsp, ib1 = st.i.nbp * (sp + 1) / nsp;
         const int nk = group_combos<Q::KG>(sub, kg);
-        const int P2 = a.q.sorted[pos];
-        const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-        const double* rk = a.q.pv.rec + a.q.pv.slot[P2] * PPW;
+        const PairMeta k = load_meta(a.q, pos);
         if constexpr (Q::CBLK) {
             // item = the NC columns of one id
             RT v[Q::NC][Q::NROW][Q::KG];
-            eri_cols_ket_outer<CX, CY, RT>(st, rk, a.q.pv.npp[P2], cd, kg, v, ib0, ib1, nk, boys);
+            eri_cols_ket_outer<CX, CY, RT>(st, k.rec, k.npp, cd, kg, v, ib0, ib1, nk, boys);
 #pragma unroll
-            for (int ic = 0; ic < Q::NC; ++ic) digest(P2, C, Dd, ic, cd, kg, v[ic]);
+            for (int ic = 0; ic < Q::NC; ++ic) digest(k, ic, cd, kg, v[ic]);
         } else {
             RT v[Q::NROW][Q::KG];
-            eri_column<CX, CY, RT, Q::RSMEM>(st, rk, a.q.pv.npp[P2], cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1,
+            eri_column<CX, CY, RT, Q::RSMEM>(st, k.rec, k.npp, cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1,
                                                  nk, boys);
-            digest(P2, C, Dd, cd / Q::ND, cd % Q::ND, kg, v);
+            digest(k, cd / Q::ND, cd % Q::ND, kg, v);
         }
     };
     if constexpr (Q::RSMEM) {
@@ -1298,12 +1325,12 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
             if (lane == 0) {
                 sh[0] = c;
                 sh[1] = b;
-                if (c < total) load_info(a.q, a.q.sorted[a.q.cls_start[CX] + b], info);
+                if (c >= 0) load_info(a.q, load_meta(a.q, a.q.cls_start[CX] + b), info);
             }
         }
         __syncthreads();
         const int c = sh[0], b = sh[1];
-        if (c >= total) break;                                  // uniform: c is shared
+        if (c < 0) break;                                       // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
         if (!staged) {
             Boys::stage(a.q.boys, btab);

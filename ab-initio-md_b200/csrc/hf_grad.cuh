@@ -356,19 +356,17 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
 // parts to the shared accumulator gsh (low words [natm][3], then the high words). RS: R_tuv / sqrt(p + q) (to L + 1)
 // of the ket pair's primitive quartets staged in Rs ([ik][ib][NH(L + 1)]).
 template <int CX, int CY, typename RT, bool RS, typename Boys>
-__device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<RT>& st, int P2, double QQ, int ic,
+__device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<RT>& st, const PairMeta& ket, double QQ, int ic,
                                             int id, int kg, double (&gab)[6], unsigned* gsh,
                                             const RT* __restrict__ Rs, RT* Rcol, int ib0, int ib1,
                                             int nk, Boys boys) {
     using Q = QClass<CX, CY>;
-    const BlockView& bv = a.q.bv;
-    const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-    const int aC = bv.atom[C], aD = bv.atom[Dd];
+    const int aC = ket.aA, aD = ket.aB;
     if (st.i.aA == st.i.aB && st.i.aB == aC && aC == aD) return;          // one-centre: invariant
-    const int nC = bv.ncon[C], nD = bv.ncon[Dd], oC = bv.ao[C], oD = bv.ao[Dd];
+    const int nC = ket.nA, nD = ket.nB, oC = ket.oA, oD = ket.oB;
     const int n = a.q.nao;
     const size_t nn = (size_t)n * n;
-    const double deg = 0.5 * (st.i.A != st.i.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.i.P1 != P2 ? 2.0 : 1.0);
+    const double deg = 0.5 * (st.i.A != st.i.B ? 2.0 : 1.0) * (ket.A != ket.B ? 2.0 : 1.0) * (st.i.P1 != ket.P ? 2.0 : 1.0);
     // Gamma column
     double G[Q::NROW][Q::KG];
     double gmax = 0.0;
@@ -404,7 +402,7 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
 #pragma unroll
         for (int kk = 0; kk < Q::KG; ++kk) Gr[r][kk] = static_cast<RT>(G[r][kk]);
     RT dA[3] = {0.0, 0.0, 0.0}, dB[3] = {0.0, 0.0, 0.0}, dC[3] = {0.0, 0.0, 0.0};
-    grad_prims<CX, CY, RT, RS>(st, Gr, a.q.pv.rec + a.q.pv.slot[P2] * PPW, a.q.pv.npp[P2], ic, id, kg, dA, dB, dC, Rs,
+    grad_prims<CX, CY, RT, RS>(st, Gr, ket.rec, ket.npp, ic, id, kg, dA, dB, dC, Rs,
                                Rcol, ib0, ib1, nk, boys);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -431,21 +429,20 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
     const int nb = a.nblock;
     const double xf = 0.5 * fabs(a.kfac) * a.nx;
     auto keep = [&](int pos) {
-        const int P2 = a.q.sorted[pos];
-        const int C = a.q.pv.pa_blk[P2], Dd = a.q.pv.pb_blk[P2];
-        const int aC = a.q.bv.atom[C], aD = a.q.bv.atom[Dd];
+        const PairMeta k = load_meta(a.q, pos);
+        const int C = k.A, Dd = k.B, aC = k.aA, aD = k.aB;
         if (st.i.aA == st.i.aB && st.i.aB == aC && aC == aD) return false;
         double gb = a.bmc[st.i.A * nb + st.i.B] * a.bmc[C * nb + Dd];
         if (a.nx > 0)
             gb += xf * (a.bmx[st.i.A * nb + C] * a.bmx[st.i.B * nb + Dd] + a.bmx[st.i.A * nb + Dd] * a.bmx[st.i.B * nb + C]);
-        const double deg = 0.5 * (st.i.A != st.i.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.i.P1 != P2 ? 2.0 : 1.0);
+        const double deg = 0.5 * (st.i.A != st.i.B ? 2.0 : 1.0) * (C != Dd ? 2.0 : 1.0) * (st.i.P1 != k.P ? 2.0 : 1.0);
         return q1 * a.q.sortedQ[pos] * deg * gb >= a.thr;
     };
     // item r = (contraction group, bra-primitive split, column)
     auto work = [&](int sub, int pos, int r, const RT* Rs) {
         const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
-        grad_column<CX, CY, RT, RS>(a, st, a.q.sorted[pos], q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
+        grad_column<CX, CY, RT, RS>(a, st, load_meta(a.q, pos), q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
                                     gsh, Rs, Rbuf + threadIdx.x, st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp,
                                     group_combos<Q::KG>(sub, kg), boys);
     };
@@ -504,12 +501,12 @@ __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kerne
             if (lane == 0) {
                 sh[0] = c;
                 sh[1] = b;
-                if (c < total) load_info(a.q, a.q.sorted[a.q.cls_start[CX] + b], info);
+                if (c >= 0) load_info(a.q, load_meta(a.q, a.q.cls_start[CX] + b), info);
             }
         }
         __syncthreads();                                        // (also orders the zeroing)
         const int c = sh[0], b = sh[1];
-        if (c >= total) break;                                  // uniform: c is shared
+        if (c < 0) break;                                       // uniform: c is shared
         const int spos = a.q.cls_start[CX] + b;
         if (!staged) {
             Boys::stage(a.q.boys, btab);

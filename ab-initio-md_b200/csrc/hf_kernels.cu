@@ -114,6 +114,7 @@ struct aimd_ctx {
     double* tmpQ;
     double* sortedQ;
     int* sorted;
+    int4* meta;             // [3][npair] pairs by sorted position (PairMeta)
     int64_t* counts_jk;     // [NSEG][npair + 1] kept ket prefix per (ket segment, bra position)
     int64_t* counts_g;
     int64_t* counts_d;      // difference-density builds (threshold changes every call)
@@ -287,6 +288,7 @@ extern "C" int aimd_create(aimd_ctx** out, int natm, int nao, int nblock, const 
         CK(dalloc(&c->Q, np));
         CK(dalloc(&c->sortedQ, np));
         CK(dalloc(&c->sorted, np));
+        CK(dalloc(&c->meta, 3 * (size_t)np));
         CK(dalloc(&c->counts_jk, (size_t)NSEG * (np + 1)));
         CK(dalloc(&c->counts_g, (size_t)NSEG * (np + 1)));
         CK(dalloc(&c->counts_d, (size_t)NSEG * (np + 1)));
@@ -322,7 +324,7 @@ extern "C" int aimd_destroy(aimd_ctx* c) {
                     c->sh_atom, c->sh_l, c->sh_ao, c->sh_p0, c->sh_np, c->sp_i, c->sp_j, c->sh_exp, c->sh_coef,
                     c->charges, c->pa, c->pb, c->npp, c->slot, c->rec, c->Q, c->by_class, c->idx_in,
                     c->tmp_idx, c->seg_id, c->seg_keys, c->seg_keys_out, c->seg_start, c->tmpQ, c->sortedQ,
-                    c->sorted, c->counts_jk, c->counts_g, c->counts_d, c->bmax, c->plan, c->plan_next, c->bra_work, c->bmc, c->bmx, c->counts_hi, c->counts_hi_d, c->cub_tmp, c->pos, c->boys, c->jacc, c->gacc};
+                    c->sorted, c->meta, c->counts_jk, c->counts_g, c->counts_d, c->bmax, c->plan, c->plan_next, c->bra_work, c->bmc, c->bmx, c->counts_hi, c->counts_hi_d, c->cub_tmp, c->pos, c->boys, c->jacc, c->gacc};
     for (void* p : ptrs) cudaFree(p);
     for (int i = 0; i < NSTREAM; ++i) {
         if (c->streams[i]) cudaStreamDestroy(c->streams[i]);
@@ -398,9 +400,17 @@ __global__ void gather_seg_kernel(int n, const int* order, const int* seg_id, in
     if (i < n) keys[i] = seg_id[order[i]];
 }
 
-__global__ void gather_q_kernel(int n, const int* order, const double* Q, double* out) {
+// Q and PairMeta of the pair at each sorted position
+__global__ void gather_pairs_kernel(int n, const int* order, const double* Q, PairView pv, BlockView bv, double* outQ,
+                                    int4* meta) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = Q[order[i]];
+    if (i >= n) return;
+    const int P = order[i], A = pv.pa_blk[P], B = pv.pb_blk[P];
+    const uint64_t slot = static_cast<uint64_t>(pv.slot[P]);
+    outQ[i] = Q[P];
+    meta[i] = make_int4(P, pv.npp[P], bv.ncon[A], bv.ncon[B]);
+    meta[n + i] = make_int4(bv.ao[A], bv.ao[B], bv.atom[A], bv.atom[B]);
+    meta[2 * n + i] = make_int4(A, B, static_cast<int>(slot & 0xffffffffu), static_cast<int>(slot >> 32));
 }
 
 // seg_start[y] = first sorted position with segment >= y (keys sorted ascending).
@@ -510,6 +520,7 @@ QuartetArgs quartet_args(aimd_ctx* c, const int64_t* counts) {
     q.counts_hi = nullptr;
     q.seg_start = c->seg_start;
     q.boys = c->boys;
+    q.meta = c->meta;
     q.npair = c->npair;
     for (int i = 0; i <= NCLS; ++i) q.cls_start[i] = c->cls_start[i];
     q.nao = c->nao;
@@ -791,7 +802,7 @@ extern "C" int aimd_set_geometry(aimd_ctx* c, const double* pos, void* stream) {
     bytes = c->cub_bytes;
     CK(cub::DeviceRadixSort::SortPairs(c->cub_tmp, bytes, c->seg_keys, c->seg_keys_out, c->tmp_idx, c->sorted, np, 0,
                                        sizeof(int) * 8, st));
-    gather_q_kernel<<<nbk, 128, 0, st>>>(np, c->sorted, c->Q, c->sortedQ);
+    gather_pairs_kernel<<<nbk, 128, 0, st>>>(np, c->sorted, c->Q, pair_view(c), block_view(c), c->sortedQ, c->meta);
     seg_start_kernel<<<1, NSEG + 1, 0, st>>>(np, c->seg_keys_out, c->seg_start);
     c->launches += 6;
     CK(cudaGetLastError());
