@@ -29,22 +29,31 @@ using RT = float;
 #define AIMD_GRAD_NAME AIMD_CAT(AIMD_CAT(AIMD_CAT(launch_grad32_c, AIMD_CLASS), _), AIMD_KET)
 #endif
 
+template <int X, int Y, typename T>
+size_t grad_bytes(const LaunchEnv& e, const LaunchSlot& s) {
+    return grad_smem_bytes<X, Y, T>(e.natm, s.nx, e.nao, e.maxbp[X],
+                                    grad_rbuf_elems<X, Y, T>(s.threads, e.maxbp[X], e.maxbp[Y]), s.dglobal != 0);
+}
+
 cudaError_t AIMD_GRAD_NAME(const LaunchEnv& e, const GradArgs& a0) {
     const int cnt = e.cls_count[CX];
     if (cnt == 0 || e.cls_count[CY] == 0) return cudaSuccess;
     constexpr int rt = sizeof(RT) == sizeof(double) ? 0 : 1;
     GradArgs a = a0;
-    a.rbuf = grad_rbuf_elems<CX, CY, RT>(e.maxbp[CX], e.maxbp[CY]);
-    const size_t smem = grad_smem_bytes<CX, CY, RT>(e.natm, e.maxbp[CX], a.rbuf);
     const void* kernel = (const void*)grad2e_bra_kernel<CX, CY, RT>;
     LaunchSlot& slot = e.slot(1, rt, CX, CY);
-    if (slot.grid == 0) {
-        cudaError_t r = set_smem_limit(kernel, smem);
-        if (r != cudaSuccess) return r;
-        slot.grid = persistent_grid(kernel, GRAD_THREADS, smem, e.nsm);
+    if (slot.grid == 0 || slot.nx != a.nx) {
+        slot.nx = a.nx;
+        const cudaError_t r = class_shape(kernel, e, 1, CX, slot, grad_bytes<CX, CY, RT>);
+        if (r != cudaSuccess) {
+            slot.grid = 0;
+            return r;
+        }
     }
+    a.rbuf = grad_rbuf_elems<CX, CY, RT>(slot.threads, e.maxbp[CX], e.maxbp[CY]);
+    a.dglobal = slot.dglobal;
     a.plan = e.plan_of(CX, CY, rt);
-    grad2e_bra_kernel<CX, CY, RT><<<slot.grid, GRAD_THREADS, smem, e.stream_of(CX, CY)>>>(a);
+    grad2e_bra_kernel<CX, CY, RT><<<slot.grid, slot.threads, slot.smem, e.stream_of(CX, CY)>>>(a);
     return cudaGetLastError();
 }
 

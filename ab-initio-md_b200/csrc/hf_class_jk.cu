@@ -39,6 +39,12 @@ using RT = float;
 // does not keep the units' copies apart (the compiler makes it from a hash of
 // the unit, which two units of one source compiled at once can share).
 template <int X, int YK, typename T>
+size_t jk_bytes(const LaunchEnv& e, const LaunchSlot& s) {
+    constexpr int Y = YK < 0 ? 0 : YK;
+    return jk_smem_bytes<X, 1, Y, T>(s.threads, e.nao, e.maxbp[X], jk_rbuf_elems<X, YK, T>(e.maxbp[X], e.maxbp[Y]),
+                                     s.kglobal != 0, s.dglobal != 0);
+}
+template <int X, int YK, typename T>
 cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0) {
     constexpr int Y = YK < 0 ? 0 : YK;
     constexpr int rt = sizeof(T) == sizeof(double) ? 0 : 1;
@@ -47,20 +53,14 @@ cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0) {
     const void* kernel = (const void*)jk_bra_kernel<X, 1, T, YK>;
     LaunchSlot& slot = e.slot(0, rt, X, Y);
     if (slot.grid == 0) {
-        // K rows in shared memory unless they would not fit (large bases) or
-        // the context asks for global rows
         slot.kglobal = a.kglobal;
-        if (!slot.kglobal && jk_smem_bytes<X, 1, Y, T>(e.nao, e.maxbp[X], a.rbuf, false) + static_smem(kernel) > kSmemLimit)
-            slot.kglobal = 1;
-        const size_t smem = jk_smem_bytes<X, 1, Y, T>(e.nao, e.maxbp[X], a.rbuf, slot.kglobal != 0);
-        cudaError_t r = set_smem_limit(kernel, smem);
+        const cudaError_t r = class_shape(kernel, e, 0, X, slot, jk_bytes<X, YK, T>);
         if (r != cudaSuccess) return r;
-        slot.grid = persistent_grid(kernel, JK_THREADS, smem, e.nsm);
     }
     a.kglobal = slot.kglobal;
+    a.dglobal = slot.dglobal;
     a.plan = e.plan_of(X, Y, rt);
-    jk_bra_kernel<X, 1, T, YK><<<slot.grid, JK_THREADS, jk_smem_bytes<X, 1, Y, T>(e.nao, e.maxbp[X], a.rbuf, a.kglobal != 0),
-                                   e.stream_of(X, Y)>>>(a);
+    jk_bra_kernel<X, 1, T, YK><<<slot.grid, slot.threads, slot.smem, e.stream_of(X, Y)>>>(a);
     return cudaGetLastError();
 }
 

@@ -24,6 +24,11 @@
 // reaches (t + u + v > LCD), and the bra step one direction at a time. With
 // those and the flat item lists, one B200: water 6-31G* 2.67 -> 0.37 ms,
 // (H2O)8 difference build 11.5 -> 4.4 ms, (H2O)32 cc-pVDZ 266 -> 118 ms.
+// Digestion took as long as the integrals (dp|ps 4.9 of 6.8 ms, pp|ps 6.5 of
+// 9.4, ps|ss 5.3 of 16.3): the bra functions' rows of D, read at the scattered
+// columns of a warp's ket pairs, were a cache line a lane and load. With the
+// rows in shared memory and the columns of an item digested together:
+// (H2O)32 93 -> 70 ms, (H2O)8 difference build 3.25 -> 1.95 ms.
 #pragma once
 #include <type_traits>
 
@@ -577,16 +582,6 @@ __device__ __forceinline__ void ket_range(const QuartetArgs& a, int seg, int spo
     }
 }
 
-// A thread's R_tuv in shared memory: element i at p[i * NT] (NT = threads
-// of the CTA, p = base + threadIdx.x), so that a warp's accesses to one
-// element fall in distinct banks. Frees the registers (or the local
-// memory) that a large R array takes through the contraction passes.
-template <typename RT, int NT>
-struct RColumn {
-    RT* p;
-    __device__ __forceinline__ RT& operator[](int i) const { return p[i * NT]; }
-};
-
 // ---------------------------------------------------------------- work plan
 // The class kernels are persistent: their CTAs take chunks of (bra pair,
 // ket window) from a device counter until the launch's plan is used up, so
@@ -722,6 +717,14 @@ struct BoysOf {
     }
 };
 
+// CTA sizes. The class kernels hold up to 255 registers a thread, so that an
+// SM runs eight of their warps: as two CTAs of four or one of eight
+// (class_shape picks per context). Small CTAs wait less for one
+// another and for the start and end of a chunk; large ones share one copy of
+// the K rows, the D rows and the Boys table, which together pass half of an
+// SM's shared memory at 800 AOs.
+constexpr int CLASS_THREADS = 256;      // the largest
+
 struct JKArgs {
     QuartetArgs q;
     const double* D;    // [nset][nao][nao], symmetric
@@ -737,113 +740,139 @@ struct JKArgs {
     // 1: the K rows of the bra functions accumulate in global memory (set per
     // launch when the per-CTA shared rows, NF x nao doubles, would not fit)
     int kglobal;
+    // 1: the bra functions' rows of D are read from D itself (set per launch
+    // when they would not fit beside the K rows), 0: staged in shared memory
+    int dglobal;
     WorkPlan plan;      // chunks of the launch (set per launch)
     int item_pq;        // primitive quartets per split column item (launch shape)
 };
 
-// Digest one column (fixed ket component pair cd, all ket contractions kk)
-// of a quartet for NS densities. Each tensor element the block reaches is
-// visited n_gen = (A==B ? 2:1)(C==D ? 2:1)(P1==P2 ? 2:1) times under the 8
-// index maps, so each image carries g = 1/n_gen:
+// Digest the NCB columns (ic0 + c, id) of a quartet (all ket contractions kk)
+// for NS densities. Each tensor element the block reaches is visited
+// n_gen = (A==B ? 2:1)(C==D ? 2:1)(P1==P2 ? 2:1) times under the 8 index maps,
+// so each image carries g = 1/n_gen:
 //   J[m,n] += 2g v D[l,s],  J[l,s] += 2g v D[m,n]
 //   K[m,l] += g v D[n,s],   K[n,l] += g v D[m,s],  K[m,s] += g v D[n,l],  K[n,s] += g v D[m,l]
 // (m in A, n in B, l in C, s in D); the host forms J + J^T and K + K^T.
 // K rows m, n belong to the bra pair: Ksm[set][slot][col], slot < KA*NA for
-// A's functions, then B's.
-template <int CX, int CY, int NS, bool KGLOBAL, typename ST>
-__device__ __forceinline__ void jk_digest_column(const JKArgs& a, const ST& st, const PairMeta& ket, int ic,
-                                                 int id, int kg,
-                                                 const double (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
-                                                 double* Jt, unsigned* Ksm, double fx) {
+// A's functions, then B's; so do the rows of D that K needs, which DA and DB
+// point to (staged in shared memory, or D itself where they do not fit). The
+// columns of one block of an item share their s: their parts of K[., s] and
+// J_ab are summed first.
+template <int CX, int CY, int NS, bool KGLOBAL, int NCB, typename ST, typename RT>
+__device__ __forceinline__ void jk_digest(const JKArgs& a, const ST& st, const PairMeta& ket, int ic0, int id, int kg,
+                                          const RT (&v)[NCB][QClass<CX, CY>::NROW][QClass<CX, CY>::KG], double* Jt,
+                                          unsigned* Ksm, const double* DA, const double* DB, double fx) {
     using Q = QClass<CX, CY>;
+    static_assert(NS == 1, "one density a pass");
     const int nC = ket.nA, nD = ket.nB, oC = ket.oA, oD = ket.oB;
     const double g = (st.i.A == st.i.B ? 0.5 : 1.0) * (ket.A == ket.B ? 0.5 : 1.0) * (st.i.P1 == ket.P ? 0.5 : 1.0);
+    const double gf = g * fx;               // scaled to fixed point (a power of two: exact)
     const int n = a.q.nao;
-    const size_t nn = (size_t)n * n;
     constexpr int NFA = Q::KA * Q::NA;      // A slots, then B slots
     constexpr int NF = NFA + Q::KB * Q::NB;
+    const double* __restrict__ D = a.D;
+    // K rows of the bra functions: shared accumulator, or the global K
+    // itself (KGLOBAL, for bra classes whose rows would not fit)
+    const bool kgl = KGLOBAL || a.kglobal;
+    auto kadd = [&](int f, int row, int col, double val) {      // row f of the shared rows is that row of K
+        if (kgl) {
+            fadd(a.K + (size_t)row * n + col, val, 1.0);
+        } else {
+            unsigned* p = Ksm + (size_t)f * n + col;
+            sadd(p, p + (size_t)NF * n, val, 1.0);
+        }
+    };
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        const double* __restrict__ D = a.D + s * nn;
-        // K rows of the bra functions: shared accumulator, or the global K
-        // itself (KGLOBAL, for bra classes whose rows would not fit)
-        const bool kgl = KGLOBAL || a.kglobal;
-        unsigned* Ks = KGLOBAL ? nullptr : Ksm + (size_t)s * NF * n;
-        const size_t hi = (size_t)NS * NF * n;          // the rows' high words
-        facc* Kg = a.K + s * nn;
-        // row f of the shared rows is row g of K
-        auto kadd = [&](int f, int g, int col, double val) {
-            if (kgl) {
-                fadd(Kg + (size_t)g * n + col, val, fx);
-            } else {
-                unsigned* p = Ks + (size_t)f * n + col;
-                sadd(p, p + hi, val, fx);
+    for (int kk = 0; kk < Q::KG; ++kk) {
+        const int kq = kg * Q::KG + kk;
+        if (kq >= nC * nD) continue;
+        const int kc = kq / nD, kd = kq % nD;
+        const int l = oC + kc * Q::NC + ic0, sg = oD + kd * Q::ND + id;     // columns l + c
+        double dls[NCB], jcd[NCB];
+#pragma unroll
+        for (int c = 0; c < NCB; ++c) {
+            dls[c] = 2.0 * g * __ldg(D + (size_t)(l + c) * n + sg);
+            jcd[c] = 0.0;
+        }
+#pragma unroll
+        for (int ka = 0; ka < Q::KA; ++ka)
+#pragma unroll
+            for (int kb = 0; kb < Q::KB; ++kb) {
+                if (ka >= st.i.nA || kb >= st.i.nB) continue;
+#pragma unroll
+                for (int ia = 0; ia < Q::NA; ++ia)
+#pragma unroll
+                    for (int jb = 0; jb < Q::NB; ++jb) {
+                        const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
+                        const int m = ka * Q::NA + ia, nb_ = st.i.oB + kb * Q::NB + jb;
+                        const double dmn = DA[(size_t)m * n + nb_];
+                        double jab = 0.0;
+#pragma unroll
+                        for (int c = 0; c < NCB; ++c) {
+                            jcd[c] += (double)v[c][r][kk] * dmn;
+                            jab += (double)v[c][r][kk] * dls[c];
+                        }
+                        Jt[r * blockDim.x + threadIdx.x] += jab;
+                    }
             }
-        };
 #pragma unroll
-        for (int kk = 0; kk < Q::KG; ++kk) {
-                const int kq = kg * Q::KG + kk;
-                if (kq >= nC * nD) continue;
-                const int kc = kq / nD, kd = kq % nD;
-                const int l = oC + kc * Q::NC + ic, sg = oD + kd * Q::ND + id;
-                const double dls = __ldg(D + (size_t)l * n + sg);
-                double jcd = 0.0;
+        for (int c = 0; c < NCB; ++c) fadd(a.J + (size_t)(l + c) * n + sg, 2.0 * gf * jcd[c], 1.0);
+        // K[m, l] and K[m, sg]: rows of A's functions
 #pragma unroll
-                for (int ka = 0; ka < Q::KA; ++ka)
+        for (int ka = 0; ka < Q::KA; ++ka)
 #pragma unroll
-                    for (int kb = 0; kb < Q::KB; ++kb) {
-                        if (ka >= st.i.nA || kb >= st.i.nB) continue;
+            for (int ia = 0; ia < Q::NA; ++ia) {
+                if (ka >= st.i.nA) continue;
+                double s1[NCB], s2 = 0.0;
 #pragma unroll
-                        for (int ia = 0; ia < Q::NA; ++ia)
-#pragma unroll
-                            for (int jb = 0; jb < Q::NB; ++jb) {
-                                const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
-                                const int m = st.i.oA + ka * Q::NA + ia, nb_ = st.i.oB + kb * Q::NB + jb;
-                                jcd += v[r][kk] * __ldg(D + (size_t)m * n + nb_);
-                                Jt[(s * Q::NROW + r) * blockDim.x + threadIdx.x] += 2.0 * g * v[r][kk] * dls;
-                            }
-                    }
-                fadd(a.J + s * nn + (size_t)l * n + sg, 2.0 * g * jcd, fx);
-                // K[m, l] and K[m, sg]: rows of A's functions
-#pragma unroll
-                for (int ka = 0; ka < Q::KA; ++ka)
-#pragma unroll
-                    for (int ia = 0; ia < Q::NA; ++ia) {
-                        if (ka >= st.i.nA) continue;
-                        double s1 = 0.0, s2 = 0.0;
-#pragma unroll
-                        for (int kb = 0; kb < Q::KB; ++kb)
-#pragma unroll
-                            for (int jb = 0; jb < Q::NB; ++jb) {
-                                if (kb >= st.i.nB) continue;
-                                const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
-                                const size_t nb_ = st.i.oB + kb * Q::NB + jb;
-                                s1 += v[r][kk] * __ldg(D + nb_ * n + sg);
-                                s2 += v[r][kk] * __ldg(D + nb_ * n + l);
-                            }
-                        kadd(ka * Q::NA + ia, st.i.oA + ka * Q::NA + ia, l, g * s1);
-                        kadd(ka * Q::NA + ia, st.i.oA + ka * Q::NA + ia, sg, g * s2);
-                    }
-                // K[n, l] and K[n, sg]: rows of B's functions
+                for (int c = 0; c < NCB; ++c) s1[c] = 0.0;
 #pragma unroll
                 for (int kb = 0; kb < Q::KB; ++kb)
 #pragma unroll
                     for (int jb = 0; jb < Q::NB; ++jb) {
                         if (kb >= st.i.nB) continue;
-                        double s1 = 0.0, s2 = 0.0;
+                        const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
+                        const double* row = DB + (size_t)(kb * Q::NB + jb) * n;
+                        const double ds = row[sg];
 #pragma unroll
-                        for (int ka = 0; ka < Q::KA; ++ka)
-#pragma unroll
-                            for (int ia = 0; ia < Q::NA; ++ia) {
-                                if (ka >= st.i.nA) continue;
-                                const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
-                                const size_t m = st.i.oA + ka * Q::NA + ia;
-                                s1 += v[r][kk] * __ldg(D + m * n + sg);
-                                s2 += v[r][kk] * __ldg(D + m * n + l);
-                            }
-                        kadd(NFA + kb * Q::NB + jb, st.i.oB + kb * Q::NB + jb, l, g * s1);
-                        kadd(NFA + kb * Q::NB + jb, st.i.oB + kb * Q::NB + jb, sg, g * s2);
+                        for (int c = 0; c < NCB; ++c) {
+                            s1[c] += (double)v[c][r][kk] * ds;
+                            s2 += (double)v[c][r][kk] * row[l + c];
+                        }
                     }
+                const int f = ka * Q::NA + ia;
+#pragma unroll
+                for (int c = 0; c < NCB; ++c) kadd(f, st.i.oA + f, l + c, gf * s1[c]);
+                kadd(f, st.i.oA + f, sg, gf * s2);
+            }
+        // K[n, l] and K[n, sg]: rows of B's functions
+#pragma unroll
+        for (int kb = 0; kb < Q::KB; ++kb)
+#pragma unroll
+            for (int jb = 0; jb < Q::NB; ++jb) {
+                if (kb >= st.i.nB) continue;
+                double s1[NCB], s2 = 0.0;
+#pragma unroll
+                for (int c = 0; c < NCB; ++c) s1[c] = 0.0;
+#pragma unroll
+                for (int ka = 0; ka < Q::KA; ++ka)
+#pragma unroll
+                    for (int ia = 0; ia < Q::NA; ++ia) {
+                        if (ka >= st.i.nA) continue;
+                        const int r = (ka * st.i.nB + kb) * Q::NAB + ia * Q::NB + jb;
+                        const double* row = DA + (size_t)(ka * Q::NA + ia) * n;
+                        const double ds = row[sg];
+#pragma unroll
+                        for (int c = 0; c < NCB; ++c) {
+                            s1[c] += (double)v[c][r][kk] * ds;
+                            s2 += (double)v[c][r][kk] * row[l + c];
+                        }
+                    }
+                const int f = kb * Q::NB + jb;
+#pragma unroll
+                for (int c = 0; c < NCB; ++c) kadd(NFA + f, st.i.oB + f, l + c, gf * s1[c]);
+                kadd(NFA + f, st.i.oB + f, sg, gf * s2);
             }
     }
 }
@@ -923,8 +952,8 @@ __device__ __forceinline__ void compact(Queue& q, int p0, int m, Keep keep, Stor
 // barrier after each, left threads idle: at (H2O)32 a bra pair has some 50 ket
 // pairs in a segment, and 128 threads share them.
 // Where ket pairs are tested (difference builds, gradients), the list runs
-// over the pairs that passed, queued LQ_CAP at a time.
-constexpr int LQ_CAP = 1024;
+// over the pairs that passed, queued eight a thread at a time.
+constexpr int LQ_CAP = 8 * 256;     // queue entries: eight a thread
 template <typename T>
 __device__ __forceinline__ T warp_incl(T v) {
     const int lane = threadIdx.x & 31;
@@ -985,10 +1014,11 @@ __device__ __forceinline__ void plan_window(const QuartetArgs& q, int spos, int 
 // every run); queue holds LQ_CAP ints. All threads of the CTA call this.
 template <typename Keep, typename Work>
 __device__ __forceinline__ void flat_items(FlatItems& f, bool queued, int* queue, Keep keep, Work work) {
-    constexpr int PER = LQ_CAP / 128;
+    constexpr int PER = 8;                              // pairs a thread tests at a time
+    const int cap = PER * static_cast<int>(blockDim.x);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int total = f.kpre[NSUB];
-    for (int base = 0; base < total; base += queued ? LQ_CAP : total) {
+    for (int base = 0; base < total; base += queued ? cap : total) {
         if (queued) {
             if (threadIdx.x < NSUB) f.cnt[threadIdx.x] = 0;
             // PER consecutive pairs a thread
@@ -1198,7 +1228,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
 template <int CX, int CY, int NS, bool KGLOBAL, typename RT, typename Boys>
 __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT>& st, int spos, double* Jt,
                                              unsigned* Ksm, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf,
-                                             Boys boys, double fx) {
+                                             Boys boys, const double* DA, const double* DB, double fx) {
     using Q = QClass<CX, CY>;
     const double q1 = a.q.sortedQ[spos];
     const double* bm = a.bmax;
@@ -1213,19 +1243,6 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
                                     fmax(bm[st.i.B * nb + C], bm[st.i.B * nb + Dd])));
         return q1 * a.q.sortedQ[pos] * dm >= a.dthr;
     };
-    auto digest = [&](const PairMeta& k, int ic, int id, int kg, const RT (&v)[Q::NROW][Q::KG]) {
-        if constexpr (sizeof(RT) == sizeof(double)) {
-            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, k, ic, id, kg, v, Jt, Ksm, fx);
-        } else {
-            // FP32 quartets: digested (accumulated) in FP64
-            double vd[Q::NROW][Q::KG];
-#pragma unroll
-            for (int r = 0; r < Q::NROW; ++r)
-#pragma unroll
-                for (int k = 0; k < Q::KG; ++k) vd[r][k] = static_cast<double>(v[r][k]);
-            jk_digest_column<CX, CY, NS, KGLOBAL>(a, st, k, ic, id, kg, vd, Jt, Ksm, fx);
-        }
-    };
     // item r = (contraction group that the segment's pairs carry, bra-primitive split, column block)
     auto work = [&](int sub, int pos, int r, const RT* Rs) {
         const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
@@ -1237,13 +1254,11 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
             // item = the NC columns of one id
             RT v[Q::NC][Q::NROW][Q::KG];
             eri_cols_ket_outer<CX, CY, RT>(st, k.rec, k.npp, cd, kg, v, ib0, ib1, nk, boys);
-#pragma unroll
-            for (int ic = 0; ic < Q::NC; ++ic) digest(k, ic, cd, kg, v[ic]);
+            jk_digest<CX, CY, NS, KGLOBAL, Q::NC>(a, st, k, 0, cd, kg, v, Jt, Ksm, DA, DB, fx);
         } else {
-            RT v[Q::NROW][Q::KG];
-            eri_column<CX, CY, RT, Q::RSMEM>(st, k.rec, k.npp, cd / Q::ND, cd % Q::ND, kg, v, Rs, ib0, ib1,
-                                                 nk, boys);
-            digest(k, cd / Q::ND, cd % Q::ND, kg, v);
+            RT v[1][Q::NROW][Q::KG];
+            eri_column<CX, CY, RT, Q::RSMEM>(st, k.rec, k.npp, cd / Q::ND, cd % Q::ND, kg, v[0], Rs, ib0, ib1, nk, boys);
+            jk_digest<CX, CY, NS, KGLOBAL, 1>(a, st, k, cd / Q::ND, cd % Q::ND, kg, v, Jt, Ksm, DA, DB, fx);
         }
     };
     if constexpr (Q::RSMEM) {
@@ -1273,27 +1288,21 @@ struct JKKernel {
     static constexpr int KROWS = KGLOBAL ? 0 : NS * NF;
 };
 
-// The Boys function of the (CX, Y) J/K kernel: from the table up to the ds
-// bras. The dp bras hold the most K rows (58 KB at 800 AOs); with the table
-// beside them the L1 cache shrinks by as much and their kernels were 3 to 15 %
-// slower at (H2O)32; for dd it made no difference.
+// The Boys function of the (CX, Y) J/K kernel: from the table, except for the
+// two-stage classes (a few per cent of a cc-pVDZ build, with R staged).
 template <int CX, int Y, typename RT>
-using JKBoys = BoysOf<QClass<CX, Y>::L, RT, (CX <= 3)>;
+using JKBoys = BoysOf<QClass<CX, Y>::L, RT, !QClass<CX, Y>::RSMEM>;
 
 // Dynamic shared memory: Boys table, per-thread J_ab slots
-// [NS][NROW][blockDim], K rows [NS][NF][nao] (unless KGLOBAL), staged R, bra
-// stage.
-constexpr int JK_THREADS = 128;
+// [NS][NROW][blockDim], K rows [NS][NF][nao] (unless KGLOBAL), D rows
+// [NF][nao] (unless dglobal), staged R, bra stage.
 
 // RT = double: the FP64 quartets; RT = float: the FP32 quartets of the
 // mixed-precision path (their J/K contributions still accumulate in FP64).
 // YK = ket class of this kernel (-1: the ss bras, whose only ket class is ss).
 // Persistent: a CTA runs chunks of the launch's work plan until it is used up.
-#ifndef AIMD_JK_MINB
-#define AIMD_JK_MINB 1
-#endif
 template <int CX, int NS, typename RT, int YK>
-__global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs a) {
+__global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
     using KK = JKKernel<CX, NS>;
     using Q0 = QClass<CX, 0>;
     constexpr int Y = YK < 0 ? 0 : YK;      // the unsplit kernel (CX = 0) has one ket class too
@@ -1304,10 +1313,12 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
     const int krows = a.kglobal ? 0 : KK::KROWS;
     using QY = QClass<CX, Y>;
     using Boys = JKBoys<CX, Y, RT>;
+    const int nt = blockDim.x;
     double* btab = smem;                                    // Boys table
     double* Jt = btab + Boys::elems;                        // per-thread J_ab slots
-    unsigned* Ksm = reinterpret_cast<unsigned*>(Jt + NS * KK::NROW * JK_THREADS);   // low words of the K rows, then the high words
-    RT* Rbuf = reinterpret_cast<RT*>(Jt + NS * KK::NROW * JK_THREADS + even((size_t)krows * n));
+    unsigned* Ksm = reinterpret_cast<unsigned*>(Jt + NS * KK::NROW * nt);   // low words of the K rows, then the high words
+    double* Dsm = Jt + NS * KK::NROW * nt + even((size_t)krows * n);       // the bra functions' rows of D
+    RT* Rbuf = reinterpret_cast<RT*>(Dsm + (a.dglobal ? 0 : even((size_t)KK::NF * n)));
     RT* Esm = Rbuf + a.rbuf;
     __shared__ BraInfo info;
     __shared__ FlatItems f;
@@ -1334,7 +1345,7 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
         const int spos = a.q.cls_start[CX] + b;
         if (!staged) {
             Boys::stage(a.q.boys, btab);
-            for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * JK_THREADS; i += blockDim.x) Jt[i] = 0.0;
+            for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * nt; i += blockDim.x) Jt[i] = 0.0;
             staged = true;
         }
         const BraStageT<RT> st = stage_view(info, Esm, KK::ESIZE);
@@ -1344,18 +1355,26 @@ __global__ void __launch_bounds__(JK_THREADS, AIMD_JK_MINB) jk_bra_kernel(JKArgs
                                    seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
         }
         stage_bra_e<Q0::LA, Q0::LB, 0>(st);
+        const double *DA = a.D + (size_t)info.oA * n, *DB = a.D + (size_t)info.oB * n;
+        if (!a.dglobal) {
+            constexpr int NFA = Q0::KA * Q0::NA;
+            const int na = info.nA * Q0::NA * n, nb = info.nB * Q0::NB * n;
+            for (int i = threadIdx.x; i < na; i += nt) Dsm[i] = __ldg(DA + i);
+            for (int i = threadIdx.x; i < nb; i += nt) Dsm[NFA * n + i] = __ldg(DB + i);
+            DA = Dsm;
+            DB = Dsm + NFA * n;
+        }
         __syncthreads();
         jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf,
-                                                 Boys::get(btab), fx);
+                                                 Boys::get(btab), DA, DB, fx);
         __syncthreads();
         // flush J_ab: a warp a (set, row) sums the threads' slots (in a fixed
         // order) and clears them
-        for (int i = warp; i < NS * KK::NROW; i += JK_THREADS / 32) {
+        for (int i = warp; i < NS * KK::NROW; i += nt / 32) {
             double val = 0.0;
-#pragma unroll
-            for (int t = 0; t < JK_THREADS; t += 32) {
-                val += Jt[i * JK_THREADS + t + lane];
-                Jt[i * JK_THREADS + t + lane] = 0.0;
+            for (int t = 0; t < nt; t += 32) {
+                val += Jt[i * nt + t + lane];
+                Jt[i * nt + t + lane] = 0.0;
             }
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) val += __shfl_xor_sync(0xffffffffu, val, d);
@@ -1393,10 +1412,11 @@ size_t jk_rbuf_elems(int max_bra_prims, int max_ket_prims) {
 }
 
 template <int CX, int NS, int Y, typename RT>
-size_t jk_smem_bytes(int nao, int max_bra_prims, size_t rbuf_elems, bool kglobal) {
+size_t jk_smem_bytes(int threads, int nao, int max_bra_prims, size_t rbuf_elems, bool kglobal, bool dglobal) {
     using KK = JKKernel<CX, NS>;
     const size_t krows = kglobal ? 0 : KK::KROWS;
-    return sizeof(double) * (even(krows * nao) + (size_t)NS * KK::NROW * JK_THREADS + JKBoys<CX, Y, RT>::elems) +
+    return sizeof(double) * (even(krows * nao) + (dglobal ? 0 : even((size_t)KK::NF * nao)) +
+                             (size_t)NS * KK::NROW * threads + JKBoys<CX, Y, RT>::elems) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (KK::ESIZE + SBW));
 }
 

@@ -47,25 +47,29 @@ struct GradArgs {
     const double* bmc;      // [nblock][nblock] max |Dc| per block pair
     const double* bmx;      // [nblock][nblock] max over x of |Dx| per block pair (nx > 0)
     int nblock;
+    int dglobal;            // 1: the bra functions' rows of Dx are read from Dx itself, 0: staged in shared memory (set per launch)
     WorkPlan plan;          // chunks of the launch (set per launch)
     int item_pq;            // primitive quartets per split column item (launch shape)
 };
 
-constexpr int GRAD_THREADS = 128;
 
 // Two-stage items (R_tuv to L + 1 staged per primitive quartet) for the
 // gradient of class pair (CX, CY): the same classes as the J/K build.
 template <int CX, int CY>
 constexpr bool grad_rsmem() { return QClass<CX, CY>::RSMEM; }
 
-// The other classes keep each thread's R_tuv (to L + 1) in a shared-memory
-// column while the box pass runs, where the columns of the CTA take at most
-// 96 KB (two CTAs per SM): R to L + 1 is the largest array of the
-// gradient body, and in registers it pushes the body into local memory.
+// Of the other classes, those with more than 20 R_tuv (to L + 1) keep each
+// thread's in shared memory while the box pass runs: R is the largest array of
+// the gradient body, and in registers it pushes the body into local memory.
+// Up to 84 values (L + 1 = 6, 172 KB for the eight warps of an SM); an odd
+// stride, so that a warp's accesses to one element spread over the banks.
 template <int CX, int CY, typename RT>
 constexpr bool grad_rcol() {
-    return !grad_rsmem<CX, CY>() && nherm(QClass<CX, CY>::L + 1) * sizeof(RT) * GRAD_THREADS <= 96 * 1024;
+    constexpr int NH = nherm(QClass<CX, CY>::L + 1);
+    return !grad_rsmem<CX, CY>() && NH > 20 && NH <= 84;
 }
+template <int CX, int CY>
+constexpr int grad_rstride() { return nherm(QClass<CX, CY>::L + 1) | 1; }
 
 // E and dE/dX_AB of one bra pair's primitives, in the same layout (st.E, st.D).
 template <int LA, int LB, typename RT>
@@ -282,8 +286,8 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                 hermite_r_scaled<L>(b.p * q * (rs * rs), b.X - k.Qx, b.Y - k.Qy, b.Z - k.Qz, rs, R, boys);
                 if constexpr (grad_rcol<CX, CY, RT>()) {
 #pragma unroll
-                    for (int i = 0; i < nherm(L); ++i) Rcol[i * GRAD_THREADS] = R[i];
-                    body(RColumn<RT, GRAD_THREADS>{Rcol});
+                    for (int i = 0; i < nherm(L); ++i) Rcol[i] = R[i];
+                    body(Rcol);
                 } else {
                     body(R);
                 }
@@ -359,7 +363,7 @@ template <int CX, int CY, typename RT, bool RS, typename Boys>
 __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<RT>& st, const PairMeta& ket, double QQ, int ic,
                                             int id, int kg, double (&gab)[6], unsigned* gsh,
                                             const RT* __restrict__ Rs, RT* Rcol, int ib0, int ib1,
-                                            int nk, Boys boys) {
+                                            int nk, Boys boys, const double* Dsm) {
     using Q = QClass<CX, CY>;
     const int aC = ket.aA, aD = ket.aB;
     if (st.i.aA == st.i.aB && st.i.aB == aC && aC == aD) return;          // one-centre: invariant
@@ -381,12 +385,13 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
             const int kab = r / Q::NAB, ab = r % Q::NAB, ka = kab / st.i.nB, kb = kab % st.i.nB;
             double val = 0.0;
             if (cv && kab < st.i.nA * st.i.nB) {
-                const size_t m = st.i.oA + ka * Q::NA + ab / Q::NB, nb_ = st.i.oB + kb * Q::NB + ab % Q::NB;
-                val = __ldg(a.Dc + m * n + nb_) * __ldg(a.Dc + l * n + sg);
+                const int m = ka * Q::NA + ab / Q::NB, nb_ = kb * Q::NB + ab % Q::NB;
+                val = __ldg(a.Dc + (size_t)(st.i.oA + m) * n + st.i.oB + nb_) * __ldg(a.Dc + l * n + sg);
                 for (int x = 0; x < a.nx; ++x) {
-                    const double* X = a.Dx + x * nn;
-                    val -= 0.5 * a.kfac * (__ldg(X + m * n + l) * __ldg(X + nb_ * n + sg) +
-                                           __ldg(X + m * n + sg) * __ldg(X + nb_ * n + l));
+                    constexpr int NFA = Q::KA * Q::NA, NF = NFA + Q::KB * Q::NB;
+                    const double* Xm = (a.dglobal ? a.Dx + x * nn + (size_t)st.i.oA * n : Dsm + (size_t)x * NF * n) + (size_t)m * n;
+                    const double* Xn = (a.dglobal ? a.Dx + x * nn + (size_t)st.i.oB * n : Dsm + (size_t)(x * NF + NFA) * n) + (size_t)nb_ * n;
+                    val -= 0.5 * a.kfac * (Xm[l] * Xn[sg] + Xm[sg] * Xn[l]);
                 }
                 val *= deg;
             }
@@ -422,7 +427,7 @@ __device__ __forceinline__ void grad_column(const GradArgs& a, const BraStageT<R
 template <int CX, int CY, typename RT, typename Boys>
 __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStageT<RT>& st, int spos, double (&gab)[6],
                                                unsigned* gsh, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf,
-                                               Boys boys) {
+                                               Boys boys, const double* Dsm) {
     using Q = QClass<CX, CY>;
     constexpr bool RS = grad_rsmem<CX, CY>();
     const double q1 = a.q.sortedQ[spos];
@@ -443,8 +448,8 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
         const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         grad_column<CX, CY, RT, RS>(a, st, load_meta(a.q, pos), q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
-                                    gsh, Rs, Rbuf + threadIdx.x, st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp,
-                                    group_combos<Q::KG>(sub, kg), boys);
+                                    gsh, Rs, Rbuf + threadIdx.x * grad_rstride<CX, CY>(), st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp,
+                                    group_combos<Q::KG>(sub, kg), boys, Dsm);
     };
     if constexpr (RS) {
         int rot = 0;
@@ -459,30 +464,29 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
 }
 
 // The Boys function of the (CX, CY) gradient kernel: from the table up to
-// order L + 1 = 5, where the table and the R columns leave room for two CTAs
-// an SM (58 + 29 KB); by series above.
+// order L + 1 = 5, by series above (whose R columns leave no room for it).
 template <int CX, int CY, typename RT>
 using GradBoys = BoysOf<QClass<CX, CY>::L + 1, RT, (QClass<CX, CY>::L + 1 <= 5)>;
 
 // One kernel per (bra class, ket class), persistent: a CTA runs chunks
 // (bra pair of class CX, window of its ket pairs of class CY) of the
 // launch's work plan until it is used up. Dynamic shared memory: gradient
-// accumulator [natm][3] (one per CTA, flushed at the end), Boys table, staged R, bra E
+// accumulator [natm][3] (one per CTA, flushed at the end), Boys table, D rows, staged R, bra E
 // tables (+1).
 // RT = double: the FP64 quartets; RT = float: the FP32 quartets of the
 // mixed-precision path (accumulated in FP64).
-#ifndef AIMD_GRAD_MINB
-#define AIMD_GRAD_MINB 1
-#endif
 template <int CX, int CY, typename RT>
-__global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kernel(GradArgs a) {
+__global__ void __launch_bounds__(CLASS_THREADS) grad2e_bra_kernel(GradArgs a) {
     using Q0 = QClass<CX, 0>;
     using Q = QClass<CX, CY>;
     using Boys = GradBoys<CX, CY, RT>;
     extern __shared__ __align__(16) double smem[];
     double* btab = smem;                                                // Boys table
     unsigned* gsh = reinterpret_cast<unsigned*>(btab + Boys::elems);    // low words [natm][3], then the high words
-    RT* Rbuf = reinterpret_cast<RT*>(btab + Boys::elems + even(3 * a.natm));
+    constexpr int NFA = Q::KA * Q::NA, NF = NFA + Q::KB * Q::NB;
+    const int n = a.q.nao;
+    double* Dsm = btab + Boys::elems + even(3 * a.natm);                // the bra functions' rows of Dx [nx][NF][nao]
+    RT* Rbuf = reinterpret_cast<RT*>(Dsm + (a.dglobal ? 0 : even((size_t)a.nx * NF * n)));
     RT* Esm = Rbuf + a.rbuf;
     __shared__ BraInfo info;
     __shared__ FlatItems f;
@@ -519,9 +523,17 @@ __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kerne
                                     seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
         }
         stage_bra_de<Q0::LA, Q0::LB>(st);
+        if (!a.dglobal) {
+            const int na = info.nA * Q::NA * n, nb = info.nB * Q::NB * n;
+            for (int x = 0; x < a.nx; ++x) {
+                const double* X = a.Dx + (size_t)x * n * n;
+                for (int i = threadIdx.x; i < na; i += blockDim.x) Dsm[(size_t)x * NF * n + i] = __ldg(X + (size_t)info.oA * n + i);
+                for (int i = threadIdx.x; i < nb; i += blockDim.x) Dsm[((size_t)x * NF + NFA) * n + i] = __ldg(X + (size_t)info.oB * n + i);
+            }
+        }
         __syncthreads();
         double gab[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        grad_ket_class<CX, CY, RT>(a, st, spos, gab, gsh, f, kq.r(), kq.flat(), Rbuf, Boys::get(btab));
+        grad_ket_class<CX, CY, RT>(a, st, spos, gab, gsh, f, kq.r(), kq.flat(), Rbuf, Boys::get(btab), Dsm);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             if (gab[d] != 0.0) gadd(3 * st.i.aA + d, gab[d]);
@@ -538,17 +550,18 @@ __global__ void __launch_bounds__(GRAD_THREADS, AIMD_GRAD_MINB) grad2e_bra_kerne
 // Elements of the staged-R buffer of the (CX, CY) gradient kernel (the
 // two-stage classes), or of its threads' R columns.
 template <int CX, int CY, typename RT>
-size_t grad_rbuf_elems(int max_bra_prims, int max_ket_prims) {
+size_t grad_rbuf_elems(int threads, int max_bra_prims, int max_ket_prims) {
     if constexpr (grad_rsmem<CX, CY>())
         return fours(rsmem_bytes<QClass<CX, CY>::L + 1, RT>(max_bra_prims, max_ket_prims) / sizeof(RT));
-    if constexpr (grad_rcol<CX, CY, RT>()) return (size_t)nherm(QClass<CX, CY>::L + 1) * GRAD_THREADS;
+    if constexpr (grad_rcol<CX, CY, RT>()) return fours((size_t)grad_rstride<CX, CY>() * threads);
     return 0;
 }
 
 template <int CX, int CY, typename RT>
-size_t grad_smem_bytes(int natm, int max_bra_prims, size_t rbuf_elems) {
+size_t grad_smem_bytes(int natm, int nx, int nao, int max_bra_prims, size_t rbuf_elems, bool dglobal) {
     using Q0 = QClass<CX, 0>;
-    return sizeof(double) * (even(3 * (size_t)natm) + GradBoys<CX, CY, RT>::elems) +
+    constexpr size_t NF = Q0::KA * Q0::NA + Q0::KB * Q0::NB;
+    return sizeof(double) * (even(3 * (size_t)natm) + GradBoys<CX, CY, RT>::elems + (dglobal ? 0 : even(nx * NF * nao))) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (2 * BraE<Q0::LA, Q0::LB, 0>::SIZE + SBW));
 }
 

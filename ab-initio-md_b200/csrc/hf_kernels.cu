@@ -87,6 +87,51 @@ const std::vector<double>& boys_tables() {
 
 }  // namespace
 
+// Which CTA size, and whether the D rows are staged. Eight warps an SM where
+// they fit, as two CTAs of four or one of eight; one of eight from the start
+// where the bras are few and their rows the largest (J/K: dd; gradient: dp and
+// dd). D rows are staged from the class on whose digestion or Gamma column
+// reads enough of them: J/K from pp, the gradient from ps. Measured at (H2O)32
+// (J/K / gradient; staging from the class given on): ps 71.2 / 155.1, pp 70.0 /
+// 157.3, ds 70.2 / -, dp 75.3 / 163.7, nowhere 80 / 168 ms; one CTA of eight
+// warps from dp on in J/K: (H2O)8 difference build 1.95 -> 2.05 ms. Where eight
+// warps do not fit with the D rows: six (156.4 against 161.2 ms), then without
+// them (they are read through the L1 cache), and K rows in global memory last.
+cudaError_t hf::class_shape(const void* kernel, const LaunchEnv& e, int kind, int cx, LaunchSlot& slot,
+                            size_t (*bytes)(const LaunchEnv&, const LaunchSlot&)) {
+    constexpr size_t kSmemSM = 228 * 1024, kReserved = 1024;    // of an SM; of each CTA
+    const size_t fixed = static_smem(kernel);
+    const bool stage = cx >= (kind == 0 ? 2 : 1);
+    const int tmin = cx >= (kind == 0 ? 5 : 4) ? 256 : 128;
+    const int kglobal = slot.kglobal;
+    auto fits = [&](int k, bool d, int t, int ctas) {
+        slot.kglobal = k;
+        slot.dglobal = d ? 0 : 1;
+        slot.threads = t;
+        const size_t b = bytes(e, slot) + fixed;
+        return b <= kSmemLimit && (b + kReserved) * ctas <= kSmemSM;
+    };
+    auto search = [&]() -> bool {
+        for (int k = kglobal; k < 2; ++k) {
+            if (stage) {
+                for (int t = tmin; t <= CLASS_THREADS; t *= 2)
+                    if (fits(k, true, t, CLASS_THREADS / t)) return true;
+                if (fits(k, true, 192, 1)) return true;
+            }
+            for (int t = 128; t <= CLASS_THREADS; t *= 2)
+                if (fits(k, false, t, CLASS_THREADS / t)) return true;
+            for (int t = 128; t >= 32; t /= 2)
+                if (fits(k, false, t, 1)) return true;
+        }
+        return false;
+    };
+    if (!search()) return cudaErrorInvalidConfiguration;
+    slot.smem = bytes(e, slot);
+    const cudaError_t r = set_smem_limit(kernel, slot.smem);
+    if (r == cudaSuccess) slot.grid = persistent_grid(kernel, slot.threads, slot.smem, e.nsm);
+    return r;
+}
+
 struct aimd_ctx {
     int natm, nao, nblock, nshell, npair, nspair;
     int nsm;
@@ -587,8 +632,8 @@ __global__ void __launch_bounds__(128) bra_work_kernel(QuartetArgs q, int64_t* w
 
 // Work plan of the (CX, CY, type) launch (one CTA of PLAN_THREADS): per bra
 // of class CX its chunk count ceil(W / target), target = max(total W /
-// parts, PLAN_MIN_WORK) with parts = chunks per resident CTA x resident
-// CTAs, as an exclusive prefix in off[0 .. nbra]; the launch's chunk
+// parts, PLAN_MIN_WORK), as an exclusive prefix in off[0 .. nbra] (a bra is at
+// least one chunk: only the bras of many quartets are cut); the launch's chunk
 // counter is zeroed.
 constexpr int PLAN_THREADS = 1024;
 constexpr int64_t PLAN_MIN_WORK = 4096;
@@ -651,11 +696,14 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, const
 }
 
 // Plans of every class launch of one call (mixed: the FP32 ones too), on st
-// before the class streams fork.
-void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, cudaStream_t st) {
+// before the class streams fork; per_sm chunks an SM at the default launch
+// shape (two for J/K, four for the gradient: with 16, as many as the bras of a
+// large molecule make anyway, (H2O)32 J/K took 79 against 73 ms and the (H2O)8
+// difference build 5.6 against 2.8, in one CTA an SM).
+void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, int per_sm, cudaStream_t st) {
     bra_work_kernel<<<dim3((c->npair + 127) / 128, NCLS), 128, 0, st>>>(q, c->bra_work);
     plan_kernel<<<dim3(NCLS * (NCLS + 1) / 2, mixed ? 2 : 1), PLAN_THREADS, 0, st>>>(
-        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, c->plan_chunks * 2 * c->nsm);
+        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, std::max(1, c->plan_chunks * per_sm * c->nsm / 8));
     c->launches += 2;
 }
 
@@ -853,8 +901,9 @@ extern "C" int aimd_jk(aimd_ctx* c, int nset, const double* D, double* J, double
         a.dthr = 0.0;
         a.rbuf = 0;
         a.kglobal = c->jk_global_rows;
+        a.dglobal = 0;
         a.item_pq = c->item_pq;
-        plan_launches(c, a.q, mixed, st);
+        plan_launches(c, a.q, mixed, 2, st);
         if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
             return r;
         jk_from_fixed_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(nn, c->jacc, c->kacc, c->dmax, J + s0 * nn,
@@ -926,8 +975,9 @@ extern "C" int aimd_jk_delta(aimd_ctx* c, int nset, const double* D, double* J, 
         a.dthr = dthr;
         a.rbuf = 0;
         a.kglobal = c->jk_global_rows;
+        a.dglobal = 0;
         a.item_pq = c->item_pq;
-        plan_launches(c, a.q, mixed, st);
+        plan_launches(c, a.q, mixed, 2, st);
         if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk_delta", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
             return r;
         jk_from_fixed_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(nn, c->jacc, c->kacc, c->dmax, J + s0 * nn,
@@ -1094,8 +1144,9 @@ extern "C" int aimd_grad2e(aimd_ctx* c, const double* Dc, int nx, const double* 
     a.bmc = c->bmc;
     a.bmx = c->bmx;
     a.nblock = c->nblock;
+    a.dglobal = 0;
     a.item_pq = c->item_pq;
-    plan_launches(c, a.q, mixed, st);
+    plan_launches(c, a.q, mixed, 4, st);
     const LaunchEnv e = launch_env(c);
     if (int r = run_concurrent(c, st, NSTREAM, "aimd_grad2e", class_pair_launches(c, mixed), [&] { return launch_grads(e, a); }))
         return r;

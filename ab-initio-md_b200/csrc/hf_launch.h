@@ -18,7 +18,11 @@ namespace hf {
 // launch, and a small molecule's build is some twenty launches long.
 struct LaunchSlot {
     int grid = 0;       // CTAs (0: not yet known)
+    int threads = 0;    // of a CTA
     int kglobal = 0;    // J/K: K rows in global memory
+    int dglobal = 0;    // the bra functions' density rows read from global memory
+    int nx = -1;        // gradient: exchange densities that the slot was made for
+    size_t smem = 0;    // dynamic shared memory
 };
 constexpr int NSTREAM = 12;     // streams that the class kernels of one call are spread over
 
@@ -110,5 +114,11 @@ inline size_t static_smem(const void* kernel) {
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kernel) == cudaSuccess ? fa.sharedSizeBytes : 0;
 }
+
+// CTA size and shared-memory layout of a class kernel of bra class cx (kind 0:
+// J/K, 1: gradient); bytes(e, slot) is its dynamic shared memory for
+// slot.threads, slot.kglobal, slot.dglobal and slot.nx. (hf_kernels.cu)
+cudaError_t class_shape(const void* kernel, const LaunchEnv& e, int kind, int cx, LaunchSlot& slot,
+                        size_t (*bytes)(const LaunchEnv&, const LaunchSlot&));
 
 }  // namespace hf

@@ -65,8 +65,9 @@ int aimd_set_fp32_cutoff(aimd_ctx *ctx, double cutoff);
 
 /* Launch shape of the context's J/K and gradient kernels (no counterpart
  * in the reference, whose numba loops have no launch geometry): the work of
- * each class launch is cut into about chunks_per_cta x (resident CTAs)
- * chunks that the persistent CTAs take in turn (1..64, default 8), and a
+ * each class launch is cut into chunks that the persistent CTAs take in
+ * turn, about chunks_per_cta / 4 an SM for J/K and chunks_per_cta / 2 for the
+ * gradient, and at least one a bra pair (1..64, default 8), and a
  * column item of a pair with many primitive quartets is split over bra
  * primitives into items of about item_pq quartets (4..4096, default 32).
  * Results change only by rounding; aimd_b200.engine.Engine.autotune picks

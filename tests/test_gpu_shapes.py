@@ -109,3 +109,52 @@ def test_boys_arguments(distance):
     for got, ref, what in zip(I.jk(b, D), O.jk_direct(b, D), "JK"):
         _close(got, ref, what)
     _close(I.two_electron_gradient(b, D, [D], 0.5), O.two_electron_gradient(b, D, [D], 0.5), "gradient")
+
+
+def _cluster(n):
+    from aimd_b200 import geometry as G
+    from aimd_b200.basis import build_basis
+    # n waters on a grid of 3.1 A: any n, no random placement
+    _, mono = G.water()
+    k = int(np.ceil(n ** (1.0 / 3.0)))
+    cells = [(i, j, m) for i in range(k) for j in range(k) for m in range(k)][:n]
+    x = np.concatenate([mono - mono[0] + 5.86 * np.array(c, dtype=float) for c in cells])
+    b = build_basis(["O", "H", "H"] * n, x, "cc-pvdz")
+    rng = np.random.default_rng(1)
+    r = np.linalg.norm(x[:, None] - x[None], axis=2)[np.ix_(b.ao_atom, b.ao_atom)]
+    D = rng.normal(size=r.shape) * np.exp(-0.5 * r)
+    return b, 0.5 * (D + D.T)
+
+
+@pytest.mark.parametrize("n", [1, 9, 44])
+def test_jk_row_layouts_agree(n, monkeypatch):
+    """
+    K rows in shared and in global memory, D rows staged or not: at 44 waters
+    (1100 AOs) the dp kernels no longer hold both sets of rows.
+    """
+    import torch
+    from aimd_b200.engine import Engine
+    b, D = _cluster(n)
+    Dt = torch.as_tensor(D[None], device="cuda")
+    out = []
+    for rows in ("0", "1"):
+        monkeypatch.setenv("AIMD_JK_GLOBAL_K_ROWS", rows)
+        eng = Engine(b)
+        eng.set_geometry(b.positions)
+        out.append([t.cpu().numpy() for t in eng.jk_acc(Dt, 1e-12)])
+    for x, y in zip(*out):
+        _close(x, y, "row layouts")
+
+
+@pytest.mark.parametrize("n", [1, 8, 27])
+def test_gradient_exchange_layouts_agree(n):
+    """One exchange density, and the same with a second one of zeros (twice the D rows, which at 27 waters do not fit)."""
+    import torch
+    from aimd_b200 import integrals as I
+    b, D = _cluster(n)
+    Dt = torch.as_tensor(D, device="cuda")
+    one = I.two_electron_gradient_device(b, Dt, Dt[None].contiguous(), 0.5).cpu().numpy()
+    two = I.two_electron_gradient_device(b, Dt, torch.stack([Dt, torch.zeros_like(Dt)]), 0.5).cpu().numpy()
+    none = I.two_electron_gradient_device(b, Dt, torch.empty((0, b.nao, b.nao), dtype=torch.float64, device="cuda"), 0.5)
+    _close(two, one, "exchange densities")
+    assert np.isfinite(none.cpu().numpy()).all()
