@@ -41,6 +41,7 @@ SIGNATURES = {
     "aimd_grad2e": (_i, [_vp, _vp, _i, _vp, _d, _d, _d, _vp, _vp]),
     "aimd_onee": (_i, [_vp, _f64p, _vp, _vp, _vp, _vp, _vp]),
     "aimd_onee_grad": (_i, [_vp, _vp, _vp, _vp, _vp]),
+    "aimd_eigh": (_i, [_i, _vp, _vp, _vp, _i, _vp]),
     "aimd_quartet_counts": (_i, [_vp, _i, _i64p]),
     "aimd_pair_data": (_i, [_vp, _i32p, _i32p, _i32p]),
     "aimd_launch_count": (ctypes.c_uint64, [_vp]),
@@ -49,6 +50,8 @@ SIGNATURES = {
     "aimd_last_error": (ctypes.c_char_p, []),
     "aimd_version": (_i, []),
 }
+
+EIGH_MAX = 64       # AIMD_EIGH_MAX
 
 _lib = None
 

@@ -52,6 +52,7 @@ def _units() -> list[tuple[str, str, list[str]]]:
     units.sort(key=lambda u: -cost(u))
     units.append((os.path.join(CSRC, "hf_onee.cu"), os.path.join(OBJ_DIR, "hf_onee.o"), []))
     units.append((os.path.join(CSRC, "hf_kernels.cu"), os.path.join(OBJ_DIR, "hf_kernels.o"), []))
+    units.append((os.path.join(CSRC, "hf_eigh.cu"), os.path.join(OBJ_DIR, "hf_eigh.o"), []))
     return units
 
 

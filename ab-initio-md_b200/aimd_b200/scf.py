@@ -225,6 +225,36 @@ class DIIS:
         return self.focks[-1].clone()
 
 
+class _Orbitals:
+    """
+    Eigenvectors (columns, ascending eigenvalues) of the Fock matrices of one
+    SCF loop. Up to ``EIGH_MAX`` orbitals by the one-CTA Jacobi kernel, started
+    from the iteration before (from scratch every tenth call, so that the
+    vectors' rounding does not add up); by torch.linalg.eigh above, and for
+    matrices that are not finite, which that refuses.
+    """
+
+    def __init__(self, nspin: int) -> None:
+        self.vectors: list[torch.Tensor | None] = [None] * nspin
+        self.calls = [0] * nspin
+
+    def __call__(self, spin: int, F: torch.Tensor, finite: bool = True) -> torch.Tensor:
+        from . import _lib
+        n = F.shape[0]
+        if n > _lib.EIGH_MAX or not finite:
+            return torch.linalg.eigh(F)[1]
+        F = F.contiguous()
+        V = self.vectors[spin]
+        warm = V is not None and self.calls[spin] % 10 != 0
+        if V is None:
+            V = self.vectors[spin] = torch.empty_like(F)
+        self.calls[spin] += 1
+        w = torch.empty(n, dtype=F.dtype, device=F.device)
+        _lib.check(_lib.load().aimd_eigh(n, F.data_ptr(), V.data_ptr(), w.data_ptr(), int(warm),
+                                         torch.cuda.current_stream().cuda_stream), "aimd_eigh")
+        return V
+
+
 @dataclass(frozen=True, eq=False)
 class SCFIntegrals:
     """S, h = T + V, X and E_nuc at one geometry (device tensors)."""
@@ -653,6 +683,7 @@ class SCFSolver:
         history: list[dict[str, float]] = []
         converged = False
         eye = torch.eye(Ik.nmo, dtype=torch.float64, device=Ds.device)
+        orbitals = _Orbitals(nspin)
         inc = {"D": None, "n": 0} if opt.incremental_fock else None
         def evaluate(F):
             e_t = 0.5 * g * torch.sum(Ds * (H[None] + F))
@@ -703,8 +734,7 @@ class SCFSolver:
                 Fo = Fo + opt.level_shift * (eye - Do)
             Dn = torch.empty_like(Ds)
             for s in range(nspin):
-                _, Cp = torch.linalg.eigh(Fo[s])
-                C = X @ Cp[:, :nocc[s]]
+                C = X @ orbitals(s, Fo[s], np.isfinite(err_norm))[:, :nocc[s]]
                 Dn[s] = C @ C.T
             if stabilize and opt.damping > 0.0:
                 Dn = (1.0 - opt.damping) * Dn + opt.damping * Ds

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/aimd_b200.h"
+#include "hf_eigh.h"
 #include "hf_launch.h"
 
 using namespace hf;
@@ -1218,6 +1219,16 @@ extern "C" int aimd_onee_grad(aimd_ctx* c, const double* W, const double* D, dou
     from_fixed(st, 3 * (size_t)c->natm, c->gacc, FIX_G, grad, 1);
     ++c->launches;
     CK(cudaGetLastError());
+    return AIMD_OK;
+}
+
+extern "C" int aimd_eigh(int n, const double* A, double* V, double* w, int warm, void* stream) {
+    if (n < 1 || !A || !V || !w) return AIMD_ERR_ARG;
+    if (n > AIMD_EIGH_MAX) {
+        snprintf(g_err, sizeof g_err, "aimd_eigh: n = %d exceeds %d", n, AIMD_EIGH_MAX);
+        return AIMD_ERR_UNSUPPORTED;
+    }
+    CK(launch_eigh(n, A, V, w, warm, static_cast<cudaStream_t>(stream)));
     return AIMD_OK;
 }
 

@@ -141,6 +141,15 @@ int aimd_onee_grad(aimd_ctx *ctx, const double *W, const double *D, double *grad
 int aimd_quartet_counts(aimd_ctx *ctx, int which, int64_t *out_host);
 int aimd_pair_data(aimd_ctx *ctx, int *npp_host, int *cls_host, int *sorted_host);
 
+/* Eigenvalues w[n] (ascending) and eigenvectors V[n][n] (in columns) of the
+ * symmetric matrix A[n][n] (its lower triangle is read), n <= AIMD_EIGH_MAX;
+ * device memory, asynchronous on stream. warm != 0: V holds orthonormal
+ * starting vectors, such as those of a nearby matrix (the SCF iteration
+ * before). aimd/qc/scf.py (numpy.linalg.eigh of the orthogonalised Fock
+ * matrix in SCFSolver._iterate, :863-923). AIMD_ERR_UNSUPPORTED above the size. */
+#define AIMD_EIGH_MAX 64
+int aimd_eigh(int n, const double *A, double *V, double *w, int warm, void *stream);
+
 /* Sizes of the context's basis: atoms and AOs. */
 int aimd_sizes(aimd_ctx *ctx, int *natm, int *nao);
 
