@@ -1174,6 +1174,7 @@ ShellView shell_view(aimd_ctx* c) {
     s.charges = c->charges;
     s.pair_i = c->sp_i;
     s.pair_j = c->sp_j;
+    s.boys = c->boys;
     return s;
 }
 int shell_classes(aimd_ctx* c) {        // non-empty shell-pair classes

@@ -14,16 +14,22 @@ template <int CL>
 cudaError_t onee_class(const LaunchEnv& e, const ShellView& sv, int b0, int b1, const double* o, double* S, double* T,
                        double* M, double* V, cudaStream_t st) {
     const auto kernel = onee_kernel<cls_la(CL), cls_lb(CL)>;
-    kernel<<<onee_grid((const void*)kernel, 0, e.nsm, b1 - b0), ONEE_THREADS, 0, st>>>(sv, b0, b1, o[0], o[1], o[2], S, T,
-                                                                                       M, V);
+    const size_t smem = sizeof(double) * BoysOf<cls_la(CL) + cls_lb(CL), double, true>::elems;
+    const cudaError_t r = set_smem_limit((const void*)kernel, smem);
+    if (r != cudaSuccess) return r;
+    kernel<<<onee_grid((const void*)kernel, smem, e.nsm, b1 - b0), ONEE_THREADS, smem, st>>>(sv, b0, b1, o[0], o[1], o[2], S,
+                                                                                             T, M, V);
     return cudaGetLastError();
 }
 template <int CL>
 cudaError_t onee_grad_class(const LaunchEnv& e, const ShellView& sv, int b0, int b1, const double* W, const double* D,
                             facc* grad, cudaStream_t st) {
-    const size_t smem = sizeof(facc) * 3 * e.natm;
-    if (smem > 48 * 1024) return cudaErrorInvalidConfiguration;
+    const size_t acc = sizeof(facc) * 3 * e.natm;
+    if (acc > 48 * 1024) return cudaErrorInvalidConfiguration;
     const auto kernel = onee_grad_kernel<cls_la(CL), cls_lb(CL)>;
+    const size_t smem = acc + sizeof(double) * BoysOf<cls_la(CL) + cls_lb(CL) + 1, double, true>::elems;
+    const cudaError_t r = set_smem_limit((const void*)kernel, smem);
+    if (r != cudaSuccess) return r;
     kernel<<<onee_grid((const void*)kernel, smem, e.nsm, b1 - b0), ONEE_THREADS, smem, st>>>(sv, b0, b1, W, D, grad);
     return cudaGetLastError();
 }

@@ -14,10 +14,10 @@
 // shells carries up to 64 primitive pairs times every nucleus, which one
 // thread a pair worked through alone while the device waited for it; and the
 // nuclei's forces went through compare-and-swap loops on one address a warp.
-// Bound by FP64 issue now. (H2O)32 cc-pVDZ on one B200, all six classes:
+// Bound by FP64 issue now; the Boys function comes from the shared table. (H2O)32 cc-pVDZ on one B200, all six classes:
 // integrals 5.0 -> 1.4 ms, gradient 23.5 -> 2.1 ms.
 #pragma once
-#include "hf_device.cuh"
+#include "hf_eri.cuh"
 
 namespace hf {
 
@@ -34,6 +34,7 @@ struct ShellView {
     const double* charges;
     const int* pair_i;  // shell pairs (si >= sj), grouped by class (li, lj) with li >= lj
     const int* pair_j;
+    const double* boys; // Boys tables of all orders
 };
 
 // -1/2 <i| d^2/dx^2 |j> from overlap factors e[i][j][0] (j up to J+2 present)
@@ -66,6 +67,11 @@ template <int LI, int LJ>
 __global__ void __launch_bounds__(ONEE_THREADS) onee_kernel(ShellView sv, int p_begin, int p_end, double ox, double oy,
                                                             double oz, double* S, double* T, double* M, double* V) {
     constexpr int NI = ncart(LI), NJ = ncart(LJ), L = LI + LJ;
+    using Boys = BoysOf<L, double, true>;
+    extern __shared__ __align__(16) double smem[];      // Boys table
+    Boys::stage(sv.boys, smem);
+    __syncthreads();
+    const auto boys = Boys::get(smem);
     const int lane = threadIdx.x & 31, nwarp = gridDim.x * (ONEE_THREADS / 32);
     const int al = atom_lanes(sv.natm), c0 = lane & (al - 1), k0 = lane / al, kl = 32 / al;
     const double sqpi = sqrt(PI);
@@ -114,7 +120,7 @@ __global__ void __launch_bounds__(ONEE_THREADS) onee_kernel(ShellView sv, int p_
             for (int c = c0; c < sv.natm; c += al) {
                 double R[nherm(L)];
                 hermite_r<L>(p, (Ax - sv.pos[3 * c]) - bp * ABx, (Ay - sv.pos[3 * c + 1]) - bp * ABy,
-                             (Az - sv.pos[3 * c + 2]) - bp * ABz, R);
+                             (Az - sv.pos[3 * c + 2]) - bp * ABz, R, boys);
                 const double w = -sv.charges[c] * 2.0 * PI * ip_;
 #pragma unroll
                 for (int h = 0; h < nherm(L); ++h) rsum[h] += w * R[h];
@@ -177,10 +183,14 @@ __global__ void __launch_bounds__(ONEE_THREADS) onee_kernel(ShellView sv, int p_
 template <int LI, int LJ>
 __global__ void __launch_bounds__(ONEE_THREADS) onee_grad_kernel(ShellView sv, int p_begin, int p_end,
                                                                  const double* W, const double* Dm, facc* grad) {
-    extern __shared__ unsigned gsh[];       // low words [natm][3], then the high words
+    using Boys = BoysOf<LI + LJ + 1, double, true>;
+    extern __shared__ __align__(16) double smem[];      // Boys table, then the accumulator
+    unsigned* gsh = reinterpret_cast<unsigned*>(smem + Boys::elems);    // low words [natm][3], then the high words
     const int n3 = 3 * sv.natm;
     for (int i = threadIdx.x; i < 2 * n3; i += blockDim.x) gsh[i] = 0u;
+    Boys::stage(sv.boys, smem);
     __syncthreads();
+    const auto boys = Boys::get(smem);
     auto gadd = [&](int i, double v) { sadd(gsh + i, gsh + n3 + i, v, FIX_G); };
     constexpr int NI = ncart(LI), NJ = ncart(LJ), L = LI + LJ, NH = nherm(L);
     const int lane = threadIdx.x & 31, nwarp = gridDim.x * (ONEE_THREADS / 32);
@@ -296,7 +306,7 @@ __global__ void __launch_bounds__(ONEE_THREADS) onee_grad_kernel(ShellView sv, i
             for (int c = c0; c < sv.natm; c += al) {
                 double R[nherm(L + 1)];
                 hermite_r<L + 1>(p, (Ax - sv.pos[3 * c]) - bp * ABx, (Ay - sv.pos[3 * c + 1]) - bp * ABy,
-                                 (Az - sv.pos[3 * c + 2]) - bp * ABz, R);
+                                 (Az - sv.pos[3 * c + 2]) - bp * ABz, R, boys);
                 const double w = -sv.charges[c] * 2.0 * PI * ip_;
                 double g[3] = {0.0, 0.0, 0.0};
 #pragma unroll
