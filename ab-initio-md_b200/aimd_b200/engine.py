@@ -135,12 +135,11 @@ class Engine:
             x = positions.detach().to(self.device, torch.float64).reshape(self.natm, 3)
             key = x.cpu().numpy().tobytes()
         else:
-            arr = np.array(positions, dtype=float).reshape(self.natm, 3)
-            key = arr.tobytes()
-            x = torch.from_numpy(arr).to(self.device)
-        if key == self._pos_key:
+            x = np.array(positions, dtype=float).reshape(self.natm, 3)
+            key = x.tobytes()
+        if key == self._pos_key:        # (before any copy: every Fock build comes by here)
             return
-        self.pos.copy_(x)
+        self.pos.copy_(x if isinstance(x, torch.Tensor) else torch.from_numpy(x))
         _lib.check(self.lib.aimd_set_geometry(self.handle, ctypes.c_void_p(self.pos.data_ptr()), _stream()),
                    "aimd_set_geometry")
         self._pos_key = key

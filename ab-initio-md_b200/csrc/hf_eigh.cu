@@ -19,7 +19,20 @@
 
 namespace {
 
-constexpr int EIGH_THREADS = 512;
+// Pair p of the m/2 disjoint pairs of a round (the circle method on m players,
+// m - 1 rounds): pair 0 is player m - 1 against the round's number, the others
+// move on by one each round, so that a thread needs no index arithmetic and no
+// shared table to follow its pair.
+struct Pair {
+    int i, j;
+    __device__ Pair(int p, int m) : i(p == 0 ? m - 1 : p), j(p == 0 ? 0 : m - 1 - p) {}
+    __device__ void advance(int m) {
+        if (i != m - 1) i = i + 1 == m - 1 ? 0 : i + 1;
+        j = j + 1 == m - 1 ? 0 : j + 1;
+    }
+};
+
+constexpr int EIGH_THREADS = 1024;     // one 2 x 2 block of rotations a thread at n = 64
 constexpr int EIGH_MAX_SWEEPS = 30;     // (a NaN matrix ends here)
 
 __device__ double block_sum(double v, double* red) {
@@ -37,9 +50,16 @@ __device__ double block_sum(double v, double* red) {
 __global__ void __launch_bounds__(EIGH_THREADS) jacobi_kernel(int n, const double* __restrict__ Ain, double* V, double* w,
                                                               int warm) {
     extern __shared__ double sm[];
-    __shared__ double red[EIGH_THREADS / 32], cs[AIMD_EIGH_MAX / 2], sn[AIMD_EIGH_MAX / 2];
-    __shared__ int pi[AIMD_EIGH_MAX / 2], pj[AIMD_EIGH_MAX / 2];
+    __shared__ double red[EIGH_THREADS / 32];
+    __shared__ double2 rot[AIMD_EIGH_MAX / 2];              // (cos, sin) of the round's rotations
     const int m = (n + 1) & ~1, ld = m + 1, h = m / 2;      // odd n: one idle row and column of zeros
+    static_assert(AIMD_EIGH_MAX * AIMD_EIGH_MAX / 2 <= 2 * EIGH_THREADS, "two rotations of the vectors a thread");
+    const int e0 = threadIdx.x, e1 = threadIdx.x + EIGH_THREADS;
+    auto rotate = [](double* u, const Pair& q, double2 g) {
+        const double u0 = u[q.i], u1 = u[q.j];
+        u[q.i] = g.x * u0 - g.y * u1;
+        u[q.j] = g.y * u0 + g.x * u1;
+    };
     double *A = sm, *U = sm + m * ld, *T = sm + 2 * m * ld;
     for (int e = threadIdx.x; e < m * m; e += EIGH_THREADS) {
         const int i = e / m, j = e % m;
@@ -79,48 +99,39 @@ __global__ void __launch_bounds__(EIGH_THREADS) jacobi_kernel(int n, const doubl
         // rounding (uniform: every thread sums alike)
         if (off <= n * 1e-31 * norm) break;
         const bool last = off <= 1e-26 * norm;
+        Pair rp(threadIdx.x < h ? threadIdx.x : 0, m), bp(e0 < h * h ? e0 / h : 0, m), bq(e0 % h, m), v0(e0 % h, m), v1(e1 % h, m);
         for (int r = 0; r < m - 1; ++r) {
             if (threadIdx.x < h) {
-                const int p = threadIdx.x;
-                int i = p == 0 ? m - 1 : (r + p) % (m - 1), j = p == 0 ? r : (r - p + m - 1) % (m - 1);
-                if (i > j) {
-                    const int t = i;
-                    i = j;
-                    j = t;
-                }
+                const int i = rp.i, j = rp.j;
                 double c = 1.0, s = 0.0;
                 const double aij = A[i * ld + j];
-                if (j < n && fabs(aij) > 1e-300) {
+                if (i < n && j < n && fabs(aij) > 1e-300) {
                     const double th = (A[j * ld + j] - A[i * ld + i]) / (2.0 * aij);
                     const double t = copysign(1.0 / (fabs(th) + sqrt(1.0 + th * th)), th);
                     c = 1.0 / sqrt(1.0 + t * t);
                     s = t * c;
                 }
-                cs[p] = c;
-                sn[p] = s;
-                pi[p] = i;
-                pj[p] = j;
+                rot[threadIdx.x] = make_double2(c, s);
             }
             __syncthreads();
             // one 2 x 2 block of A per pair of rotations, both sides at once
-            for (int e = threadIdx.x; e < h * h; e += EIGH_THREADS) {
-                const int p = e / h, q = e % h;
-                const int i = pi[p] * ld, j = pj[p] * ld, k = pi[q], l = pj[q];
-                const double c = cs[q], s = sn[q], a0 = A[i + k], a1 = A[i + l], b0 = A[j + k], b1 = A[j + l];
-                const double x0 = c * a0 - s * a1, x1 = s * a0 + c * a1, y0 = c * b0 - s * b1, y1 = s * b0 + c * b1;
-                const double d = cs[p], t = sn[p];
-                A[i + k] = d * x0 - t * y0;
-                A[i + l] = d * x1 - t * y1;
-                A[j + k] = t * x0 + d * y0;
-                A[j + l] = t * x1 + d * y1;
+            if (e0 < h * h) {
+                const int i = bp.i * ld, j = bp.j * ld, k = bq.i, l = bq.j;
+                const double2 q = rot[e0 % h], p = rot[e0 / h];
+                const double a0 = A[i + k], a1 = A[i + l], b0 = A[j + k], b1 = A[j + l];
+                const double x0 = q.x * a0 - q.y * a1, x1 = q.y * a0 + q.x * a1, y0 = q.x * b0 - q.y * b1, y1 = q.y * b0 + q.x * b1;
+                A[i + k] = p.x * x0 - p.y * y0;
+                A[i + l] = p.x * x1 - p.y * y1;
+                A[j + k] = p.y * x0 + p.x * y0;
+                A[j + l] = p.y * x1 + p.x * y1;
             }
-            for (int e = threadIdx.x; e < n * h; e += EIGH_THREADS) {
-                const int q = e % h;
-                double* u = U + e / h * ld;
-                const double c = cs[q], s = sn[q], u0 = u[pi[q]], u1 = u[pj[q]];
-                u[pi[q]] = c * u0 - s * u1;
-                u[pj[q]] = s * u0 + c * u1;
-            }
+            if (e0 < n * h) rotate(U + e0 / h * ld, v0, rot[e0 % h]);
+            if (e1 < n * h) rotate(U + e1 / h * ld, v1, rot[e1 % h]);
+            rp.advance(m);
+            bp.advance(m);
+            bq.advance(m);
+            v0.advance(m);
+            v1.advance(m);
             __syncthreads();
         }
         if (last) break;

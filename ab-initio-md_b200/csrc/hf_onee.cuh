@@ -15,7 +15,7 @@
 // thread a pair worked through alone while the device waited for it; and the
 // nuclei's forces went through compare-and-swap loops on one address a warp.
 // Bound by FP64 issue now; the Boys function comes from the shared table. (H2O)32 cc-pVDZ on one B200, all six classes:
-// integrals 5.0 -> 1.4 ms, gradient 23.5 -> 2.1 ms.
+// integrals 5.0 -> 1.0 ms, gradient 23.5 -> 1.6 ms.
 #pragma once
 #include "hf_eri.cuh"
 
