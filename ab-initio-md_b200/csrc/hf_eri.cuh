@@ -594,6 +594,7 @@ __device__ __forceinline__ void ket_range(const QuartetArgs& a, int seg, int spo
 struct WorkPlan {
     const int* off;     // [nbra + 1] chunk prefix over the bras of the class (off[nbra]: chunks)
     int* next;          // chunk counter of the launch (zeroed with the plan)
+    const int* pq;      // primitive quartets per split column item of the launch
 };
 
 __host__ __device__ constexpr int ket_prims2(int ppb) {
@@ -712,6 +713,7 @@ struct BoysOf {
     __device__ static void stage(const double* tables, double* shared) {
         if constexpr (table) {
             const double2* src = reinterpret_cast<const double2*>(tables + boys_offset(L));
+#pragma unroll 4
             for (int i = threadIdx.x; i < elems / 2; i += blockDim.x) reinterpret_cast<double2*>(shared)[i] = __ldg(src + i);
         }
     }
@@ -744,7 +746,6 @@ struct JKArgs {
     // when they would not fit beside the K rows), 0: staged in shared memory
     int dglobal;
     WorkPlan plan;      // chunks of the launch (set per launch)
-    int item_pq;        // primitive quartets per split column item (launch shape)
 };
 
 // Digest the NCB columns (ic0 + c, id) of a quartet (all ket contractions kk)
@@ -905,9 +906,10 @@ __device__ __forceinline__ int64_t ket_work(int sub) {
 // Bra-primitive splits of the column items of a ket segment: an item of a
 // pair of many primitive quartets would run them all in one thread while
 // the rest of the CTA waits at the next barrier, so such items are split
-// over ranges of the bra primitives (about item_pq quartets each, a launch
-// shape of the context, default ITEM_PQ; the partial columns are linear in
-// the quartets and are digested one by one).
+// over ranges of the bra primitives (about item_pq quartets each: at most the
+// launch shape of the context, default ITEM_PQ, and fewer where the launch
+// would not fill the device with items of that length; the partial columns are
+// linear in the quartets and are digested one by one).
 constexpr int ITEM_PQ = 32;
 __device__ __forceinline__ int bra_splits(int nbp, int sub, int item_pq) {
     const int s = nbp * ket_prims2(sub / NCONB) / (2 * item_pq);
@@ -972,6 +974,7 @@ struct FlatItems {
     int kpre[NSUB + 1];         // pairs before each segment
     int nper[NSUB];             // items per ket pair
     int wsum[32];
+    int item_pq;                // primitive quartets per split item of the launch
 };
 
 // The window of chunk j of nch of bra position spos (warp 0 calls it, one lane
@@ -1245,7 +1248,7 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
     };
     // item r = (contraction group that the segment's pairs carry, bra-primitive split, column block)
     auto work = [&](int sub, int pos, int r, const RT* Rs) {
-        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
+        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, f.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         const int ib0 = st.i.nbp * sp / nsp, ib1 = st.i.nbp * (sp + 1) / nsp;
         const int nk = group_combos<Q::KG>(sub, kg);
@@ -1328,6 +1331,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
     const int total = a.plan.off[nbra];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double fx = jk_fix_for(__ldg(a.dmax));
+    if (threadIdx.x == 0) f.item_pq = *a.plan.pq;               // (read after the first barrier)
     bool staged = false;        // the Boys table is in shared memory, and the accumulators are zero
     for (;;) {
         if (warp == 0) {
@@ -1352,14 +1356,16 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
         if (warp == 0) {
             const int sub = lane < NSUB ? lane : 0;
             plan_window<CX, Y, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], QY::NITEM,
-                                   seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
+                                   seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.i.nbp, sub, f.item_pq), f);
         }
         stage_bra_e<Q0::LA, Q0::LB, 0>(st);
         const double *DA = a.D + (size_t)info.oA * n, *DB = a.D + (size_t)info.oB * n;
         if (!a.dglobal) {
             constexpr int NFA = Q0::KA * Q0::NA;
             const int na = info.nA * Q0::NA * n, nb = info.nB * Q0::NB * n;
+#pragma unroll 4
             for (int i = threadIdx.x; i < na; i += nt) Dsm[i] = __ldg(DA + i);
+#pragma unroll 4
             for (int i = threadIdx.x; i < nb; i += nt) Dsm[NFA * n + i] = __ldg(DB + i);
             DA = Dsm;
             DB = Dsm + NFA * n;

@@ -49,7 +49,6 @@ struct GradArgs {
     int nblock;
     int dglobal;            // 1: the bra functions' rows of Dx are read from Dx itself, 0: staged in shared memory (set per launch)
     WorkPlan plan;          // chunks of the launch (set per launch)
-    int item_pq;            // primitive quartets per split column item (launch shape)
 };
 
 
@@ -445,7 +444,7 @@ __device__ __forceinline__ void grad_ket_class(const GradArgs& a, const BraStage
     };
     // item r = (contraction group, bra-primitive split, column)
     auto work = [&](int sub, int pos, int r, const RT* Rs) {
-        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, a.item_pq);
+        const int nkg = seg_groups<Q::KG, Q::NKG>(sub), nsp = bra_splits(st.i.nbp, sub, f.item_pq);
         const int kg = r % nkg, sp = (r / nkg) % nsp, cd = r / (nkg * nsp);
         grad_column<CX, CY, RT, RS>(a, st, load_meta(a.q, pos), q1 * a.q.sortedQ[pos], cd / Q::ND, cd % Q::ND, kg, gab,
                                     gsh, Rs, Rbuf + threadIdx.x * grad_rstride<CX, CY>(), st.i.nbp * sp / nsp, st.i.nbp * (sp + 1) / nsp,
@@ -496,6 +495,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) grad2e_bra_kernel(GradArgs a) {
     const int total = a.plan.off[nbra];
     for (int i = threadIdx.x; i < 6 * a.natm; i += blockDim.x) gsh[i] = 0u;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) f.item_pq = *a.plan.pq;           // (read after the first barrier)
     bool staged = false;        // the Boys table is in shared memory
     auto gadd = [&](int i, double v) { sadd(gsh + i, gsh + 3 * a.natm + i, v, FIX_G); };
     for (;;) {
@@ -520,14 +520,16 @@ __global__ void __launch_bounds__(CLASS_THREADS) grad2e_bra_kernel(GradArgs a) {
         if (warp == 0) {
             const int sub = lane < NSUB ? lane : 0;
             plan_window<CX, CY, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], Q::NCD,
-                                    seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.i.nbp, sub, a.item_pq), f);
+                                    seg_groups<Q::KG, Q::NKG>(sub), bra_splits(st.i.nbp, sub, f.item_pq), f);
         }
         stage_bra_de<Q0::LA, Q0::LB>(st);
         if (!a.dglobal) {
             const int na = info.nA * Q::NA * n, nb = info.nB * Q::NB * n;
             for (int x = 0; x < a.nx; ++x) {
                 const double* X = a.Dx + (size_t)x * n * n;
+#pragma unroll 4
                 for (int i = threadIdx.x; i < na; i += blockDim.x) Dsm[(size_t)x * NF * n + i] = __ldg(X + (size_t)info.oA * n + i);
+#pragma unroll 4
                 for (int i = threadIdx.x; i < nb; i += blockDim.x) Dsm[((size_t)x * NF + NFA) * n + i] = __ldg(X + (size_t)info.oB * n + i);
             }
         }

@@ -167,7 +167,7 @@ struct aimd_ctx {
     double* bmax;           // [nblock][nblock] max |D| per block pair
     double* dmax;           // [1] max over bmax, behind the J/K accumulators (cleared with them)
     int* plan;              // work plans of the class kernels (LaunchEnv::plan_of)
-    int* plan_next;         // their chunk counters
+    int* plan_next;         // their chunk counters, then their split lengths
     int64_t* bra_work;      // [2 types][NCLS][npair] work units of each bra (bra_work_kernel)
     // launch shape (aimd_set_launch_shape): work-plan chunks per resident
     // CTA, primitive quartets per split column item
@@ -342,7 +342,7 @@ extern "C" int aimd_create(aimd_ctx** out, int natm, int nao, int nblock, const 
         CK(dalloc(&c->counts_hi, (size_t)NSEG * (np + 1)));
         CK(dalloc(&c->bmax, (size_t)nblock * nblock));
         CK(dalloc(&c->plan, (size_t)2 * NCLS * (np + NCLS)));
-        CK(dalloc(&c->plan_next, (size_t)2 * NCLS * NCLS));
+        CK(dalloc(&c->plan_next, (size_t)4 * NCLS * NCLS));
         CK(dalloc(&c->bra_work, (size_t)2 * NCLS * np));
         CK(dalloc(&c->bmc, (size_t)nblock * nblock));
         CK(dalloc(&c->bmx, (size_t)nblock * nblock));
@@ -635,9 +635,18 @@ __global__ void __launch_bounds__(128) bra_work_kernel(QuartetArgs q, int64_t* w
 // of class CX its chunk count ceil(W / target), target = max(total W /
 // parts, PLAN_MIN_WORK), as an exclusive prefix in off[0 .. nbra] (a bra is at
 // least one chunk: only the bras of many quartets are cut); the launch's chunk
-// counter is zeroed.
+// counter is zeroed. The minimum keeps a chunk's start (staging of the bra,
+// its ranges) small beside its items: 1024 units instead took the J/K build
+// of a UHF molecule of 24 functions from 473 to 641 us and the gradient of
+// (H2O)8 from 7.1 to 7.9 ms, 16384 took the former to 524.
 constexpr int PLAN_THREADS = 1024;
 constexpr int64_t PLAN_MIN_WORK = 4096;
+// Shortest split item. Launches of little work are bound by their longest
+// item, a chain of primitive quartets in one thread: shorter ones took the UHF
+// molecule's build from 550 to 473 us and the gradient of methanol from 696 to
+// 669, where items of 4 instead of 32 quartets everywhere cost the large
+// launches a digest each.
+constexpr int MIN_PQ = 4;
 
 template <typename T>
 __device__ T block_sum(T v, T* red) {
@@ -654,7 +663,8 @@ __device__ T block_sum(T v, T* red) {
 // one CTA per (bra class, ket class <= bra class, type): blockIdx.x = pair
 // index CX (CX + 1) / 2 + CY, blockIdx.y = type (0: FP64 ranges, 1: FP32)
 __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, const int64_t* work, int* plan,
-                                                            int* plan_next, int stride, int parts) {
+                                                            int* plan_next, int stride, int parts, int item_pq,
+                                                            int threads) {
     __shared__ int64_t red[PLAN_THREADS / 32];
     __shared__ int ired[PLAN_THREADS / 32];
     int cx = 0;
@@ -693,6 +703,11 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, const
     if (threadIdx.x == 0) {
         off[nbra] = base;
         plan_next[(rt * NCLS + cx) * NCLS + cy] = 0;
+        // a unit of work is half a primitive quartet of a column: items of
+        // item_pq quartets, or what gives two to each of the device's threads
+        const int64_t even_pq = W / (4 * (int64_t)threads);
+        plan_next[((2 + rt) * NCLS + cx) * NCLS + cy] =
+            even_pq >= item_pq ? item_pq : (even_pq < MIN_PQ ? min(MIN_PQ, item_pq) : static_cast<int>(even_pq));
     }
 }
 
@@ -704,7 +719,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, const
 void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, int per_sm, cudaStream_t st) {
     bra_work_kernel<<<dim3((c->npair + 127) / 128, NCLS), 128, 0, st>>>(q, c->bra_work);
     plan_kernel<<<dim3(NCLS * (NCLS + 1) / 2, mixed ? 2 : 1), PLAN_THREADS, 0, st>>>(
-        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, std::max(1, c->plan_chunks * per_sm * c->nsm / 8));
+        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, std::max(1, c->plan_chunks * per_sm * c->nsm / 8),
+        c->item_pq, CLASS_THREADS * c->nsm);
     c->launches += 2;
 }
 
@@ -903,7 +919,6 @@ extern "C" int aimd_jk(aimd_ctx* c, int nset, const double* D, double* J, double
         a.rbuf = 0;
         a.kglobal = c->jk_global_rows;
         a.dglobal = 0;
-        a.item_pq = c->item_pq;
         plan_launches(c, a.q, mixed, 2, st);
         if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
             return r;
@@ -977,7 +992,6 @@ extern "C" int aimd_jk_delta(aimd_ctx* c, int nset, const double* D, double* J, 
         a.rbuf = 0;
         a.kglobal = c->jk_global_rows;
         a.dglobal = 0;
-        a.item_pq = c->item_pq;
         plan_launches(c, a.q, mixed, 2, st);
         if (int r = run_concurrent(c, st, NSTREAM, "aimd_jk_delta", class_pair_launches(c, mixed), [&] { return launch_jks(e, a); }))
             return r;
@@ -1146,7 +1160,6 @@ extern "C" int aimd_grad2e(aimd_ctx* c, const double* Dc, int nx, const double* 
     a.bmx = c->bmx;
     a.nblock = c->nblock;
     a.dglobal = 0;
-    a.item_pq = c->item_pq;
     plan_launches(c, a.q, mixed, 4, st);
     const LaunchEnv e = launch_env(c);
     if (int r = run_concurrent(c, st, NSTREAM, "aimd_grad2e", class_pair_launches(c, mixed), [&] { return launch_grads(e, a); }))

@@ -36,7 +36,7 @@ struct LaunchEnv {
     int nsm;                 // SMs of the device
     // work plans of the class kernels: per (type, ket class) one [npair +
     // NCLS] array holding the [nbra + 1] prefix of each bra class in turn;
-    // chunk counters per (type, bra class, ket class)
+    // chunk counters per (type, bra class, ket class), then the split lengths
     int* plan;
     int* plan_next;
     int plan_stride;
@@ -46,7 +46,7 @@ struct LaunchEnv {
     cudaStream_t stream_of(int cx, int cy) const { return streams[(cx * (cx + 1) / 2 + cy) % NSTREAM]; }
     WorkPlan plan_of(int cx, int cy, int rt) const {
         return WorkPlan{plan + (size_t)(rt * NCLS + cy) * plan_stride + cls_start[cx] + cx,
-                        plan_next + (rt * NCLS + cx) * NCLS + cy};
+                        plan_next + (rt * NCLS + cx) * NCLS + cy, plan_next + ((2 + rt) * NCLS + cx) * NCLS + cy};
     }
 };
 

@@ -69,7 +69,8 @@ int aimd_set_fp32_cutoff(aimd_ctx *ctx, double cutoff);
  * turn, about chunks_per_cta / 4 an SM for J/K and chunks_per_cta / 2 for the
  * gradient, and at least one a bra pair (1..64, default 8), and a
  * column item of a pair with many primitive quartets is split over bra
- * primitives into items of about item_pq quartets (4..4096, default 32).
+ * primitives into items of about item_pq quartets (4..4096, default 32), and
+ * of fewer where a launch would not fill the device with items of that length.
  * Results change only by rounding; aimd_b200.engine.Engine.autotune picks
  * the shape by timing. AIMD_ERR_ARG outside the ranges. */
 int aimd_set_launch_shape(aimd_ctx *ctx, int chunks_per_cta, int item_pq);

@@ -158,3 +158,21 @@ def test_gradient_exchange_layouts_agree(n):
     none = I.two_electron_gradient_device(b, Dt, torch.empty((0, b.nao, b.nao), dtype=torch.float64, device="cuda"), 0.5)
     _close(two, one, "exchange densities")
     assert np.isfinite(none.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 9])
+def test_split_lengths_agree(n):
+    """Items split by the launch's work (1, 2 waters: the shortest, 9: the shape's own length) under several launch shapes."""
+    import torch
+    from aimd_b200.engine import Engine
+    b, D = _cluster(n)
+    Dt = torch.as_tensor(D[None], device="cuda")
+    out = []
+    for shape in ((8, 32), (8, 4), (64, 4096), (1, 5)):
+        eng = Engine(b)
+        eng.set_geometry(b.positions)
+        eng.set_launch_shape(*shape)
+        out.append([t.cpu().numpy() for t in (*eng.jk_acc(Dt, 1e-12), *eng.jk_delta_acc(Dt, 1e-12, 1e-15))])
+    for other in out[1:]:
+        for x, y in zip(out[0], other):
+            _close(y, x, "launch shape")
