@@ -73,7 +73,7 @@ __host__ __device__ constexpr double cart_norm(int lx, int ly, int lz) {
 // addition is associative, and wraps modulo 2^64, so only each addend and
 // the final total need to fit in 63 bits). The float value is restored once
 // at the end. Gradients: scale 2^44 (resolution 5.7e-14 Eh/bohr, range
-// +-5.2e5). J and K: scale jk_fix_for(max |D|), 2^44 for densities of
+// +-5.2e5). J and K: scale jk_fix_for(max |D|), 2^45 for densities of
 // magnitude 1, so that the builds of small difference densities keep the
 // relative resolution of a full build.
 typedef unsigned long long facc;
@@ -100,15 +100,18 @@ __device__ __forceinline__ facc join_planes(unsigned lo, unsigned hi) { return (
 __host__ __device__ __forceinline__ double from_fixed(facc u, double scale) {
     return static_cast<double>(static_cast<long long>(u)) / scale;
 }
-// J/K scale for a density of largest element m in [2^(e-1), 2^e): 2^(45-e)
-// (2^44 at m = 1), e clamped to [-60, 30]. J and K are linear in D, so their
-// elements stay below 2^18 m (far above any molecular Coulomb or exchange
-// element per unit density) and every sum fits; m = 0 or NaN gives e = 0.
+// J/K scale for a density of largest element m in [2^(e-1), 2^e): 2^(46-e)
+// (2^45 at m = 1), e clamped to [-60, 30]. Every sum below 2^17 m fits. J and
+// K are linear in D, and a density of all elements m gives 126 m at 200 AOs of
+// water and 189 m at 400 (growing as their number to the 0.6). The rounding of
+// the adds is the error of a small molecule's build, and items cut short
+// make more of them: with 2^(45-e), 2.4e-12 against 1.9e-12 before (relative,
+// UHF molecule of 24 functions). m = 0 or NaN gives e = 0.
 __device__ __forceinline__ double jk_fix_for(double m) {
     int e = 0;
     if (m > 0.0 && m <= 1.0e300) frexp(m, &e);
     e = e < -60 ? -60 : (e > 30 ? 30 : e);
-    return ldexp(1.0, 45 - e);
+    return ldexp(1.0, 46 - e);
 }
 
 // ---------------------------------------------------------------- Boys

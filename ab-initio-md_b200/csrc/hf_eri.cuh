@@ -28,7 +28,8 @@
 // 9.4, ps|ss 5.3 of 16.3): the bra functions' rows of D, read at the scattered
 // columns of a warp's ket pairs, were a cache line a lane and load. With the
 // rows in shared memory and the columns of an item digested together:
-// (H2O)32 93 -> 70 ms, (H2O)8 difference build 3.25 -> 1.95 ms.
+// (H2O)32 93 -> 70 ms, (H2O)8 difference build 3.25 -> 1.95 ms. Water now takes
+// 0.14 ms.
 #pragma once
 #include <type_traits>
 

@@ -28,7 +28,8 @@
 // in that step, against 180 here, and ten times the code: the kernels of a
 // small molecule are bound by fetching each instruction once. One B200, raised
 // form -> this one: methanol 6-31G** 16.4 -> 1.67 ms, (H2O)8 cc-pVDZ 73.1 ->
-// 10.2 ms, (H2O)32 1095 -> 178 ms.
+// 10.2 ms, (H2O)32 1095 -> 178 ms; with the Boys table, the rows of Dx in shared
+// memory and the pair data by sorted position 0.63, 7.1 and 155 ms.
 #pragma once
 #include "hf_eri.cuh"
 
