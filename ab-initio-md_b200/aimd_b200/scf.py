@@ -231,7 +231,9 @@ class _Orbitals:
     SCF loop. Up to ``EIGH_MAX`` orbitals by the one-CTA Jacobi kernel, started
     from the iteration before (from scratch every tenth call, so that the
     vectors' rounding does not add up); by torch.linalg.eigh above, and for
-    matrices that are not finite, which that refuses.
+    matrices that are not finite, which that refuses. The kernel reports a
+    failure by vectors of NaN; ``check`` raises for them, as torch.linalg.eigh
+    does, once the energy of their density is on the host.
     """
 
     def __init__(self, nspin: int) -> None:
@@ -253,6 +255,11 @@ class _Orbitals:
         _lib.check(_lib.load().aimd_eigh(n, F.data_ptr(), V.data_ptr(), w.data_ptr(), int(warm),
                                          torch.cuda.current_stream().cuda_stream), "aimd_eigh")
         return V
+
+    def check(self, energy: float) -> None:
+        if np.isnan(energy) and any(self.calls):
+            raise torch.linalg.LinAlgError("the eigenvectors of the Fock matrix are NaN: it holds a value that is not "
+                                           "finite, or the eigensolver did not converge")
 
 
 @dataclass(frozen=True, eq=False)
@@ -695,6 +702,7 @@ class SCFSolver:
         for it in range(1, opt.max_iter + 1):
             F = self._fock(Ik, Ds, inc)
             err, e_el, err_norm = evaluate(F)
+            orbitals.check(e_el)
             de = e_el - e_prev
             if (abs(de) < opt.conv_energy and err_norm < opt.conv_commutator and inc is not None and inc["n"] > 1
                     and opt.final_full_build):

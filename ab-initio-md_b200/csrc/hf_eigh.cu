@@ -33,7 +33,7 @@ struct Pair {
 };
 
 constexpr int EIGH_THREADS = 1024;     // one 2 x 2 block of rotations a thread at n = 64
-constexpr int EIGH_MAX_SWEEPS = 30;     // (a NaN matrix ends here)
+constexpr int EIGH_MAX_SWEEPS = 30;     // (random matrices of n = 64 take 8)
 constexpr double ROT_SMALL = 1e-5;      // sine of a rotation that does not disturb the others of its sweep
 
 __device__ double block_sum(double v, double* red) {
@@ -46,8 +46,20 @@ __device__ double block_sum(double v, double* red) {
     return t;
 }
 
+__device__ double block_max(double v, double* red) {
+    for (int d = 16; d > 0; d >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, d));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < EIGH_THREADS / 32; ++w) t = fmax(t, red[w]);
+    return t;
+}
+
 // A: lower triangle of the matrix [n][n]; V [n][n]: eigenvectors in columns,
 // ascending eigenvalues w; warm: V holds the starting vectors (orthonormal).
+// All of V and w are NaN if an element of A or of the starting vectors is not
+// finite, or if the sweeps do not end.
 __global__ void __launch_bounds__(EIGH_THREADS) jacobi_kernel(int n, const double* __restrict__ Ain, double* V, double* w,
                                                               int warm) {
     extern __shared__ double sm[];
@@ -62,12 +74,27 @@ __global__ void __launch_bounds__(EIGH_THREADS) jacobi_kernel(int n, const doubl
         u[q.j] = g.y * u0 + g.x * u1;
     };
     double *A = sm, *U = sm + m * ld, *T = sm + 2 * m * ld;
+    bool finite = true;
+    double big = 0.0;
     for (int e = threadIdx.x; e < m * m; e += EIGH_THREADS) {
         const int i = e / m, j = e % m;
         const bool in = i < n && j < n;
-        A[i * ld + j] = in ? Ain[(i > j ? i : j) * n + (i > j ? j : i)] : 0.0;
-        U[i * ld + j] = in && warm ? V[i * n + j] : (i == j ? 1.0 : 0.0);
+        const double a = in ? Ain[(i > j ? i : j) * n + (i > j ? j : i)] : 0.0;
+        const double u = in && warm ? V[i * n + j] : (i == j ? 1.0 : 0.0);
+        finite &= isfinite(a) && isfinite(u);
+        big = fmax(big, fabs(a));
+        A[i * ld + j] = a;
+        U[i * ld + j] = u;
     }
+    auto fail = [&] {
+        for (int e = threadIdx.x; e < n * n; e += EIGH_THREADS) V[e] = nan("");
+        for (int i = threadIdx.x; i < n; i += EIGH_THREADS) w[i] = nan("");
+    };
+    if (__syncthreads_or(!finite)) return fail();
+    // elements up to 1 by a power of two (exact): their squares stay in range
+    int ex;
+    frexp(block_max(big, red), &ex);
+    for (int e = threadIdx.x; e < m * m; e += EIGH_THREADS) A[e / m * ld + e % m] = scalbn(A[e / m * ld + e % m], -ex);
     __syncthreads();
     if (warm) {         // A <- U^T A U
         for (int e = threadIdx.x; e < n * n; e += EIGH_THREADS) {
@@ -89,7 +116,8 @@ __global__ void __launch_bounds__(EIGH_THREADS) jacobi_kernel(int n, const doubl
     double norm = 0.0;
     for (int e = threadIdx.x; e < m * m; e += EIGH_THREADS) norm += A[e / m * ld + e % m] * A[e / m * ld + e % m];
     norm = block_sum(norm, red);
-    for (int sweep = 0; sweep < EIGH_MAX_SWEEPS; ++sweep) {
+    for (int sweep = 0;; ++sweep) {
+        if (sweep == EIGH_MAX_SWEEPS) return fail();
         double off = 0.0;
         for (int e = threadIdx.x; e < m * m; e += EIGH_THREADS) {
             const int i = e / m, j = e % m;
@@ -155,7 +183,7 @@ __global__ void __launch_bounds__(EIGH_THREADS) jacobi_kernel(int n, const doubl
             rank += y < x || (y == x && k < i);
         }
         T[i] = rank;
-        w[rank] = x;
+        w[rank] = scalbn(x, ex);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < n * n; e += EIGH_THREADS) V[e / n * n + (int)T[e % n]] = U[e / n * ld + e % n];

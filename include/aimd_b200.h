@@ -146,8 +146,11 @@ int aimd_pair_data(aimd_ctx *ctx, int *npp_host, int *cls_host, int *sorted_host
  * symmetric matrix A[n][n] (its lower triangle is read), n <= AIMD_EIGH_MAX;
  * device memory, asynchronous on stream. warm != 0: V holds orthonormal
  * starting vectors, such as those of a nearby matrix (the SCF iteration
- * before). aimd/qc/scf.py (numpy.linalg.eigh of the orthogonalised Fock
- * matrix in SCFSolver._iterate, :863-923). AIMD_ERR_UNSUPPORTED above the size. */
+ * before). All of V and w are NaN if A or the starting vectors hold a value
+ * that is not finite, or if the iteration does not converge (the call is
+ * asynchronous and returns AIMD_OK). aimd/qc/scf.py (numpy.linalg.eigh of the
+ * orthogonalised Fock matrix in SCFSolver._iterate, :863-923).
+ * AIMD_ERR_UNSUPPORTED above the size. */
 #define AIMD_EIGH_MAX 64
 int aimd_eigh(int n, const double *A, double *V, double *w, int warm, void *stream);
 
