@@ -220,7 +220,10 @@ class Engine:
 
     @property
     def launch_shape(self) -> tuple[int, int]:
-        """(work-plan chunks per resident CTA, primitive quartets per split column item)."""
+        """
+        (work-plan chunks per CTA, counted as two an SM; primitive quartets per
+        split column item); (8, 32), the default, leaves both to the planner.
+        """
         c, q = ctypes.c_int(), ctypes.c_int()
         _lib.check(self.lib.aimd_get_launch_shape(self.handle, ctypes.byref(c), ctypes.byref(q)),
                    "aimd_get_launch_shape")
@@ -234,10 +237,9 @@ class Engine:
                  jk_weight: float = 10.0, reps: int = 2, fp32_cutoff: float = 0.0) -> dict:
         """
         Pick the launch shape of this context by timing, at the current
-        geometry: for every candidate (chunks per resident CTA, quartets per
-        split item) one warm J/K build of the densities D[nset, n, n] and,
-        if ``grad = (Dc, Dx, kfac, thr, gamma_bound)`` is given, one
-        two-electron gradient, timed with CUDA events on the current stream
+        geometry: for every candidate ``launch_shape`` one warm J/K build of
+        the densities D[nset, n, n] and, if ``grad = (Dc, Dx, kfac, thr,
+        gamma_bound)`` is given, one two-electron gradient, timed with CUDA events on the current stream
         (best of ``reps``); the score is jk_weight x J/K time + gradient
         time (an MD step runs about ten Fock builds per gradient). Sets and
         returns the fastest shape with every candidate's timings.

@@ -907,11 +907,9 @@ __device__ __forceinline__ int64_t ket_work(int sub) {
 // Bra-primitive splits of the column items of a ket segment: an item of a
 // pair of many primitive quartets would run them all in one thread while
 // the rest of the CTA waits at the next barrier, so such items are split
-// over ranges of the bra primitives (about item_pq quartets each: at most the
-// launch shape of the context, default ITEM_PQ, and fewer where the launch
-// would not fill the device with items of that length; the partial columns are
-// linear in the quartets and are digested one by one).
-constexpr int ITEM_PQ = 32;
+// over ranges of the bra primitives (about item_pq quartets each: split_length
+// of the launch; the partial columns are linear in the quartets and are
+// digested one by one).
 __device__ __forceinline__ int bra_splits(int nbp, int sub, int item_pq) {
     const int s = nbp * ket_prims2(sub / NCONB) / (2 * item_pq);
     return s < 1 ? 1 : (s > nbp ? nbp : s);

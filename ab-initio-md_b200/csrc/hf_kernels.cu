@@ -19,6 +19,7 @@
 #include "../../include/aimd_b200.h"
 #include "hf_eigh.h"
 #include "hf_launch.h"
+#include "hf_plan.h"
 
 using namespace hf;
 
@@ -169,10 +170,9 @@ struct aimd_ctx {
     int* plan;              // work plans of the class kernels (LaunchEnv::plan_of)
     int* plan_next;         // their chunk counters, then their split lengths
     int64_t* bra_work;      // [2 types][NCLS][npair] work units of each bra (bra_work_kernel)
-    // launch shape (aimd_set_launch_shape): work-plan chunks per resident
-    // CTA, primitive quartets per split column item
-    int plan_chunks = 8;
-    int item_pq = ITEM_PQ;
+    // launch shape (aimd_set_launch_shape): see hf_plan.h
+    int plan_chunks = DEFAULT_CHUNKS;
+    int item_pq = DEFAULT_ITEM_PQ;
     double* bmc;            // gradient: [nblock][nblock] max |Dc| and max over x of |Dx|
     double* bmx;
     cudaStream_t streams[NSTREAM] = {};
@@ -641,12 +641,6 @@ __global__ void __launch_bounds__(128) bra_work_kernel(QuartetArgs q, int64_t* w
 // (H2O)8 from 7.1 to 7.9 ms, 16384 took the former to 524.
 constexpr int PLAN_THREADS = 1024;
 constexpr int64_t PLAN_MIN_WORK = 4096;
-// Shortest split item. Launches of little work are bound by their longest
-// item, a chain of primitive quartets in one thread: shorter ones took the UHF
-// molecule's build from 550 to 473 us and the gradient of methanol from 696 to
-// 669, where items of 4 instead of 32 quartets everywhere cost the large
-// launches a digest each.
-constexpr int MIN_PQ = 4;
 
 template <typename T>
 __device__ T block_sum(T v, T* red) {
@@ -703,23 +697,16 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(QuartetArgs q, const
     if (threadIdx.x == 0) {
         off[nbra] = base;
         plan_next[(rt * NCLS + cx) * NCLS + cy] = 0;
-        // a unit of work is half a primitive quartet of a column: items of
-        // item_pq quartets, or what gives two to each of the device's threads
-        const int64_t even_pq = W / (4 * (int64_t)threads);
-        plan_next[((2 + rt) * NCLS + cx) * NCLS + cy] =
-            even_pq >= item_pq ? item_pq : (even_pq < MIN_PQ ? min(MIN_PQ, item_pq) : static_cast<int>(even_pq));
+        plan_next[((2 + rt) * NCLS + cx) * NCLS + cy] = split_length(W, item_pq, threads);
     }
 }
 
 // Plans of every class launch of one call (mixed: the FP32 ones too), on st
-// before the class streams fork; per_sm chunks an SM at the default launch
-// shape (two for J/K, four for the gradient: with 16, as many as the bras of a
-// large molecule make anyway, (H2O)32 J/K took 79 against 73 ms and the (H2O)8
-// difference build 5.6 against 2.8, in one CTA an SM).
+// before the class streams fork; per_sm: plan_parts.
 void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, int per_sm, cudaStream_t st) {
     bra_work_kernel<<<dim3((c->npair + 127) / 128, NCLS), 128, 0, st>>>(q, c->bra_work);
     plan_kernel<<<dim3(NCLS * (NCLS + 1) / 2, mixed ? 2 : 1), PLAN_THREADS, 0, st>>>(
-        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, std::max(1, c->plan_chunks * per_sm * c->nsm / 8),
+        q, c->bra_work, c->plan, c->plan_next, c->npair + NCLS, plan_parts(c->plan_chunks, per_sm, c->nsm),
         c->item_pq, CLASS_THREADS * c->nsm);
     c->launches += 2;
 }

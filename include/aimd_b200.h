@@ -65,12 +65,15 @@ int aimd_set_fp32_cutoff(aimd_ctx *ctx, double cutoff);
 
 /* Launch shape of the context's J/K and gradient kernels (no counterpart
  * in the reference, whose numba loops have no launch geometry): the work of
- * each class launch is cut into chunks that the persistent CTAs take in
- * turn, about chunks_per_cta / 4 an SM for J/K and chunks_per_cta / 2 for the
- * gradient, and at least one a bra pair (1..64, default 8), and a
- * column item of a pair with many primitive quartets is split over bra
- * primitives into items of about item_pq quartets (4..4096, default 32), and
- * of fewer where a launch would not fill the device with items of that length.
+ * each class launch is cut into chunks that the persistent CTAs take in turn,
+ * and a column item of a pair with many primitive quartets is split over bra
+ * primitives.
+ * chunks_per_cta (1..64): about that many chunks per CTA, counted as two CTAs
+ * an SM; 8, the default, leaves it to the planner (2 an SM for J/K, 4 for the
+ * gradient). A bra pair is at least one chunk.
+ * item_pq (4..4096): about that many primitive quartets a split item; 32, the
+ * default, leaves it to the planner (32, and fewer, down to 4, where a launch
+ * would not fill the device with items of that length).
  * Results change only by rounding; aimd_b200.engine.Engine.autotune picks
  * the shape by timing. AIMD_ERR_ARG outside the ranges. */
 int aimd_set_launch_shape(aimd_ctx *ctx, int chunks_per_cta, int item_pq);
