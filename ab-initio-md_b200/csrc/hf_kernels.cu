@@ -713,13 +713,23 @@ void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, int per_sm, cu
 
 int cls_size(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
 
-// all (X, Y <= X) gradient kernels, the costly classes first
-cudaError_t launch_grads(const LaunchEnv& e, const GradArgs& a) {
+// The status of a call's class launches and the bra class of the first that failed.
+struct ClassStatus {
     cudaError_t r = cudaSuccess;
+    int cls = -1;
+    void operator()(int cl, cudaError_t x) {
+        r = x;
+        if (x != cudaSuccess) cls = cl;
+    }
+};
+
+// all (X, Y <= X) gradient kernels, the costly classes first
+ClassStatus launch_grads(const LaunchEnv& e, const GradArgs& a) {
+    ClassStatus s;
     const bool mixed = a.q.counts_hi != nullptr;
 #define AIMD_G1(X, Y)                                                     \
-    if (r == cudaSuccess) r = launch_grad_c##X##_##Y(e, a);              \
-    if (r == cudaSuccess && mixed) r = launch_grad32_c##X##_##Y(e, a);
+    if (s.r == cudaSuccess) s(X, launch_grad_c##X##_##Y(e, a));          \
+    if (s.r == cudaSuccess && mixed) s(X, launch_grad32_c##X##_##Y(e, a));
     AIMD_G1(5, 5) AIMD_G1(5, 4) AIMD_G1(5, 3) AIMD_G1(5, 2) AIMD_G1(5, 1) AIMD_G1(5, 0)
     AIMD_G1(4, 4) AIMD_G1(4, 3) AIMD_G1(4, 2) AIMD_G1(4, 1) AIMD_G1(4, 0)
     AIMD_G1(3, 3) AIMD_G1(3, 2) AIMD_G1(3, 1) AIMD_G1(3, 0)
@@ -727,17 +737,17 @@ cudaError_t launch_grads(const LaunchEnv& e, const GradArgs& a) {
     AIMD_G1(1, 1) AIMD_G1(1, 0)
     AIMD_G1(0, 0)
 #undef AIMD_G1
-    return r;
+    return s;
 }
-cudaError_t launch_jks(const LaunchEnv& e, const JKArgs& a) {
-    cudaError_t r = cudaSuccess;
+ClassStatus launch_jks(const LaunchEnv& e, const JKArgs& a) {
+    ClassStatus s;
     const bool mixed = a.q.counts_hi != nullptr;
 #define AIMD_J1(X)                                            \
-    if (r == cudaSuccess) r = launch_jk_c##X(e, a);          \
-    if (r == cudaSuccess && mixed) r = launch_jk32_c##X(e, a);
+    if (s.r == cudaSuccess) s(X, launch_jk_c##X(e, a));      \
+    if (s.r == cudaSuccess && mixed) s(X, launch_jk32_c##X(e, a));
     AIMD_J1(5) AIMD_J1(4) AIMD_J1(3) AIMD_J1(2) AIMD_J1(1) AIMD_J1(0)
 #undef AIMD_J1
-    return r;
+    return s;
 }
 // kernel launches of launch_jks and launch_grads: one per non-empty (bra
 // class, ket class) and type
@@ -748,16 +758,16 @@ int class_pair_launches(aimd_ctx* c, bool mixed) {
     return mixed ? 2 * n : n;
 }
 
-int launch_status(aimd_ctx* c, cudaError_t r, const char* what, int nlaunch) {
-    if (r == cudaSuccess) {
+int launch_status(aimd_ctx* c, const ClassStatus& s, const char* what, int nlaunch) {
+    if (s.r == cudaSuccess) {
         c->launches += nlaunch;
         return AIMD_OK;
     }
-    if (r == cudaErrorInvalidConfiguration) {
-        snprintf(g_err, sizeof g_err, "%s: shared memory beyond the 227 KB per-CTA limit", what);
+    if (s.r == cudaErrorInvalidConfiguration) {
+        snprintf(g_err, sizeof g_err, "%s (pair class %d): shared memory beyond the 227 KB per-CTA limit", what, s.cls);
         return AIMD_ERR_UNSUPPORTED;
     }
-    snprintf(g_err, sizeof g_err, "%s: %s", what, cudaGetErrorString(r));
+    snprintf(g_err, sizeof g_err, "%s (pair class %d): %s", what, s.cls, cudaGetErrorString(s.r));
     return AIMD_ERR_CUDA;
 }
 
@@ -834,13 +844,12 @@ extern "C" int aimd_set_geometry(aimd_ctx* c, const double* pos, void* stream) {
         int n = 0;
         for (int cl = 0; cl < NCLS; ++cl) n += cls_size(c, cl) > 0;
         const int r = run_concurrent(c, st, NCLS, "aimd_set_geometry/schwarz", n, [&] {
-            cudaError_t x = launch_schwarz_c5(e, q, c->streams[5]);
-            if (x == cudaSuccess) x = launch_schwarz_c4(e, q, c->streams[4]);
-            if (x == cudaSuccess) x = launch_schwarz_c3(e, q, c->streams[3]);
-            if (x == cudaSuccess) x = launch_schwarz_c2(e, q, c->streams[2]);
-            if (x == cudaSuccess) x = launch_schwarz_c1(e, q, c->streams[1]);
-            if (x == cudaSuccess) x = launch_schwarz_c0(e, q, c->streams[0]);
-            return x;
+            ClassStatus s;
+#define AIMD_S1(X) \
+    if (s.r == cudaSuccess) s(X, launch_schwarz_c##X(e, q, c->streams[X]));
+            AIMD_S1(5) AIMD_S1(4) AIMD_S1(3) AIMD_S1(2) AIMD_S1(1) AIMD_S1(0)
+#undef AIMD_S1
+            return s;
         });
         if (r) return r;
     }
@@ -1191,10 +1200,10 @@ extern "C" int aimd_onee(aimd_ctx* c, const double* origin, double* S, double* T
     const LaunchEnv e = launch_env(c);
     const ShellView sv = shell_view(c);
     if (int r = run_concurrent(c, st, NCLS, "aimd_onee", shell_classes(c), [&] {
-            cudaError_t x = cudaSuccess;
-            for (int cl = NCLS - 1; cl >= 0 && x == cudaSuccess; --cl)
-                x = launch_onee(e, sv, cl, c->sp_cls_start, origin, S, T, M, V, c->streams[cl]);
-            return x;
+            ClassStatus s;
+            for (int cl = NCLS - 1; cl >= 0 && s.r == cudaSuccess; --cl)
+                s(cl, launch_onee(e, sv, cl, c->sp_cls_start, origin, S, T, M, V, c->streams[cl]));
+            return s;
         }))
         return r;
     return AIMD_OK;
@@ -1211,10 +1220,10 @@ extern "C" int aimd_onee_grad(aimd_ctx* c, const double* W, const double* D, dou
     const LaunchEnv e = launch_env(c);
     const ShellView sv = shell_view(c);
     if (int r = run_concurrent(c, st, NCLS, "aimd_onee_grad", shell_classes(c), [&] {
-            cudaError_t x = cudaSuccess;
-            for (int cl = NCLS - 1; cl >= 0 && x == cudaSuccess; --cl)
-                x = launch_onee_grad(e, sv, cl, c->sp_cls_start, W, D, c->gacc, c->streams[cl]);
-            return x;
+            ClassStatus s;
+            for (int cl = NCLS - 1; cl >= 0 && s.r == cudaSuccess; --cl)
+                s(cl, launch_onee_grad(e, sv, cl, c->sp_cls_start, W, D, c->gacc, c->streams[cl]));
+            return s;
         }))
         return r;
     from_fixed(st, 3 * (size_t)c->natm, c->gacc, FIX_G, grad, 1);
