@@ -110,11 +110,16 @@ __device__ __forceinline__ void stage_bra_scalars(const BraStageT<RT>& st) {
     }
 }
 
-// Fill the shared stage (E tables and scalars) for all bra primitives.
+// Fill the shared stage (E tables and scalars) for all bra primitives. An ss
+// bra has no table: E^{00}_0 = 1 (K is in the scalars), which bra_rows knows.
+// Without it the longest s contraction that a J/K launch takes beside the Boys
+// table is 45 primitives (41 with it).
+template <int LA, int LB>
+constexpr int bra_e_size() { return LA + LB > 0 ? BraE<LA, LB, 0>::SIZE : 0; }
 template <int LA, int LB, int G, typename RT>
 __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
     using BE = BraE<LA, LB, G>;
-    for (int w = threadIdx.x; w < st.i.nbp * 3; w += blockDim.x) {
+    for (int w = threadIdx.x; w < (LA + LB > 0 ? st.i.nbp * 3 : 0); w += blockDim.x) {
         const int ib = w / 3, d = w % 3;
         const double* b = st.i.rec + (size_t)ib * PPW;
         const double p = b[0] + b[1];
@@ -1280,7 +1285,7 @@ struct JKKernel {
     using Q0 = QClass<CX, 0>;
     static constexpr int NROW = Q0::NROW;
     static constexpr int NF = Q0::KA * Q0::NA + Q0::KB * Q0::NB;
-    static constexpr int ESIZE = BraE<Q0::LA, Q0::LB, 0>::SIZE;
+    static constexpr int ESIZE = bra_e_size<Q0::LA, Q0::LB>();
     // bra classes above ss: one kernel per ket class, so that each kernel
     // holds the code of one ket class only and the CTAs resident on an SM
     // share their instructions; dd bras accumulate K in global memory
@@ -1446,7 +1451,7 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS) schwarz_kernel(QuartetArgs a,
         qmax = 0ull;
     }
     __syncthreads();
-    const BraStageT<double> st = stage_view(info, smem, BraE<Q::LA, Q::LB, 0>::SIZE);
+    const BraStageT<double> st = stage_view(info, smem, bra_e_size<Q::LA, Q::LB>());
     stage_bra_e<Q::LA, Q::LB, 0>(st);
     __syncthreads();
     static_assert(Q::KG == Q::KCD, "diagonal quartets keep all contraction combinations in one item");
