@@ -13,6 +13,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "hf_boys.h"
+
 namespace hf {
 
 constexpr int LMAX = 2;            // s, p, d: every built-in basis set
@@ -227,33 +229,8 @@ __device__ __forceinline__ void boys_scaled(float alpha, float T, float (&g)[L +
     }
 }
 
-// FP64 F_N from a table, for the J/K and gradient kernels: below x = 36 + 3N
-// one interval of width 1/8 gives F_N as a polynomial of degree 7 in the
-// distance d from its middle c (interpolated at the Chebyshev nodes in
-// extended precision on the host), and e^-x = e^-c e^-d with e^-d by its Taylor
-// series to d^8 (|d| <= 1/16); the lower orders follow by the downward
-// recursion. From 36 + 3N on, F_n = (2n - 1)!! / (2x)^n F_0 with
-// F_0 = sqrt(pi / x) / 2 holds to 1e-16 (the neglected part is of order
-// x^(N - 1/2) e^-x / Gamma(N + 1/2)). Nine loads and some 25 operations, where
-// the series and erf branches above take 50 and 150 and a warp that holds both
-// kinds of x pays for both. The table of one order (9 coefficient columns of
-// 288 + 24N rows, 21 to 36 KB) is staged in shared memory: the rows of a warp's
-// lanes are scattered, which columns of coefficients spread over the banks.
-// Largest relative error over all orders and x <= 300 (mean): N = 4 8.9e-16
-// (1.0e-16) against 1.0e-15 (1.8e-16) of the branches above, N = 9 1.4e-15
-// (1.2e-16) against 1.8e-15 (3.2e-16). One B200, branches -> table: (H2O)32
-// J/K 118 -> 106 ms and gradient 176 -> 160 ms, (H2O)8 difference build
-// 4.2 -> 3.5 ms.
-constexpr int BOYS_MAX_N = 9, BOYS_COLS = 9;
-__host__ __device__ constexpr int boys_rows(int N) { return 8 * (36 + 3 * N); }
-__host__ __device__ constexpr int boys_offset(int N) {      // first element of order N in the table of all orders
-    int o = 0;
-    for (int m = 0; m < N; ++m) o += BOYS_COLS * boys_rows(m);
-    return o;
-}
-
 // How hermite_r gets g[n] = scale (-2 alpha)^n F_n(T): evaluated, or (FP64) from the
-// shared table of order N.
+// shared table of order L (BoysShared, hf_boys.h).
 struct BoysSeries {
     template <int L, typename RT>
     __device__ __forceinline__ void operator()(RT alpha, RT T, RT scale, RT (&g)[L + 1]) const {
@@ -262,55 +239,6 @@ struct BoysSeries {
         for (int n = 0; n <= L; ++n) g[n] *= scale;
     }
 };
-struct BoysShared {
-    const double* t;
-    template <int L>
-    __device__ __forceinline__ void operator()(double alpha, double T, double scale, double (&g)[L + 1]) const {
-        constexpr int NR = boys_rows(L);
-        if (!(T < 36 + 3 * L)) {        // (NaN too)
-            const double r = rsqrt(T);
-            double s = r * r;
-            s = fma(s, fma(-T, s, 1.0), s) * -alpha;        // 1 / T to rounding
-            g[0] = 0.88622692545275801365 * r * scale;
-#pragma unroll
-            for (int n = 1; n <= L; ++n) g[n] = g[n - 1] * ((2 * n - 1) * s);
-            return;
-        }
-        // row floor(8 T), as the integer nearest to 8 T - 1/2: adding 1.5 2^52
-        // leaves it in the low word (no conversion instructions)
-        const double m = fma(T, 8.0, -0.5) + 6755399441055744.0;
-        const double d = fma(-0.125, m - 6755399441055744.0, T - 0.0625);
-        const double* c = t + __double2loint(m);
-        double f = c[7 * NR];
-#pragma unroll
-        for (int j = 6; j >= 0; --j) f = fma(f, d, c[j * NR]);
-        if constexpr (L == 0) {
-            g[0] = f * scale;
-        } else {
-            double e = 1.0 / 40320;
-            e = fma(e, d, -1.0 / 5040);
-            e = fma(e, d, 1.0 / 720);
-            e = fma(e, d, -1.0 / 120);
-            e = fma(e, d, 1.0 / 24);
-            e = fma(e, d, -1.0 / 6);
-            e = fma(e, d, 0.5);
-            e = fma(e, d, -1.0);
-            const double e0 = c[8 * NR], ex = fma(e * d, e0, e0);
-            const double m2a = -2.0 * alpha, T2 = 2.0 * T;
-            double pw[L + 1];
-            pw[0] = scale;
-#pragma unroll
-            for (int n = 1; n <= L; ++n) pw[n] = pw[n - 1] * m2a;
-            g[L] = pw[L] * f;
-#pragma unroll
-            for (int n = L - 1; n >= 0; --n) {
-                f = fma(T2, f, ex) * (1.0 / (2 * n + 1));
-                g[n] = pw[n] * f;
-            }
-        }
-    }
-};
-
 // scale * R_tuv(alpha, PQ) for all t+u+v <= L, in place: levels n = L..0,
 // each level overwriting the previous one in decreasing Hermite index
 // (entries h only read lower indices of the level above). R[0] of level n

@@ -710,6 +710,7 @@ __host__ __device__ constexpr size_t fours(size_t n) { return (n + 3) & ~(size_t
 template <int L, typename RT, bool TABLE>
 struct BoysOf {
     static constexpr bool table = TABLE && sizeof(RT) == sizeof(double);
+    static_assert(!table || L <= BOYS_MAX_N, "order without a table");
     using type = std::conditional_t<table, BoysShared, BoysSeries>;
     static constexpr int elems = table ? BOYS_COLS * boys_rows(L) : 0;      // doubles of shared memory
     __device__ static type get(const double* shared) {

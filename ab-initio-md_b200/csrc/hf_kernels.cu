@@ -39,49 +39,7 @@ thread_local char g_err[512] = "";
 template <typename T>
 cudaError_t dalloc(T** p, size_t n) { return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T)); }
 
-// The tables of BoysShared for orders 0 .. BOYS_MAX_N, made once per process:
-// per interval of width 1/8 the polynomial in d = x - c that interpolates F_N
-// at the eight Chebyshev nodes, and e^-c. F_N at a node: the ascending series
-// of the top order in extended precision, then the downward recursion.
-std::vector<double> make_boys_tables() {
-    constexpr int K = BOYS_COLS - 1, M = BOYS_MAX_N;
-    const long double pi = 3.14159265358979323846264338327950288L, half = 1.0L / 16;    // half the interval
-    std::vector<double> out(boys_offset(M + 1));
-    long double node[4 * K];                        // cos(pi m / 2K)
-    for (int m = 0; m < 4 * K; ++m) node[m] = cosl(pi * m / (2 * K));
-    // monomial coefficients of the Chebyshev polynomials T_j
-    long double tc[K][K] = {};
-    tc[0][0] = tc[1][1] = 1.0L;
-    for (int j = 2; j < K; ++j)
-        for (int k = 0; k <= j; ++k) tc[j][k] = (k > 0 ? 2.0L * tc[j - 1][k - 1] : 0.0L) - tc[j - 2][k];
-    for (int i = 0; i < boys_rows(M); ++i) {
-        const long double c = (i + 0.5L) / 8;
-        long double f[M + 1][K];
-        for (int k = 0; k < K; ++k) {
-            const long double x = c + half * node[2 * k + 1], ex = expl(-x);
-            long double term = 1.0L / (2 * M + 1), sum = term;
-            for (int n = 1; term > 1e-22L * sum; ++n) sum += term *= 2.0L * x / (2 * M + 2 * n + 1);
-            f[M][k] = ex * sum;
-            for (int n = M - 1; n >= 0; --n) f[n][k] = (2.0L * x * f[n + 1][k] + ex) / (2 * n + 1);
-        }
-        for (int n = 0; n <= M; ++n) {
-            const int rows = boys_rows(n);
-            if (i >= rows) continue;
-            long double mono[K] = {};
-            for (int j = 0; j < K; ++j) {
-                long double a = 0.0L;
-                for (int k = 0; k < K; ++k) a += f[n][k] * node[j * (2 * k + 1) % (4 * K)];
-                a *= (j == 0 ? 1.0L : 2.0L) / K;
-                for (int k = 0; k <= j; ++k) mono[k] += a * tc[j][k];
-            }
-            double* t = out.data() + boys_offset(n) + i;
-            long double s = 1.0L;
-            for (int k = 0; k < K; ++k, s /= half) t[k * rows] = static_cast<double>(mono[k] * s);
-            t[K * rows] = static_cast<double>(expl(-c));
-        }
-    }
-    return out;
-}
+// made once per process
 const std::vector<double>& boys_tables() {
     static const std::vector<double> t = make_boys_tables();
     return t;
