@@ -41,7 +41,7 @@ using RT = float;
 template <int X, int YK, typename T>
 size_t jk_bytes(const LaunchEnv& e, const LaunchSlot& s) {
     constexpr int Y = YK < 0 ? 0 : YK;
-    return jk_smem_bytes<X, 1, Y, T>(s.threads, e.nao, e.maxbp[X], jk_rbuf_elems<X, YK, T>(e.maxbp[X], e.maxbp[Y]),
+    return jk_smem_bytes<X, Y, T>(s.threads, e.nao, e.maxbp[X], jk_rbuf_elems<X, YK, T>(e.maxbp[X], e.maxbp[Y]),
                                      s.kglobal != 0, s.dglobal != 0);
 }
 template <int X, int YK, typename T>
@@ -50,7 +50,7 @@ cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0) {
     constexpr int rt = sizeof(T) == sizeof(double) ? 0 : 1;
     JKArgs a = a0;
     a.rbuf = jk_rbuf_elems<X, YK, T>(e.maxbp[X], e.maxbp[Y]);
-    const void* kernel = (const void*)jk_bra_kernel<X, 1, T, YK>;
+    const void* kernel = (const void*)jk_bra_kernel<X, T, YK>;
     LaunchSlot& slot = e.slot(0, rt, X, Y);
     if (slot.grid == 0) {
         slot.kglobal = a.kglobal;
@@ -60,16 +60,16 @@ cudaError_t launch_one(const LaunchEnv& e, const JKArgs& a0) {
     a.kglobal = slot.kglobal;
     a.dglobal = slot.dglobal;
     a.plan = e.plan_of(X, Y, rt);
-    jk_bra_kernel<X, 1, T, YK><<<slot.grid, slot.threads, slot.smem, e.stream_of(X, Y)>>>(a);
+    jk_bra_kernel<X, T, YK><<<slot.grid, slot.threads, slot.smem, e.stream_of(X, Y)>>>(a);
     return cudaGetLastError();
 }
 
-// split bra classes: one launch per non-empty ket class (largest first); the
-// others: one launch over all ket classes
+// split bra classes: one launch per non-empty ket class (largest first); ss: one
+// launch, whose only ket class is ss
 cudaError_t AIMD_JK_NAME(const LaunchEnv& e, const JKArgs& a) {
     const int cnt = e.cls_count[CX];
     if (cnt == 0) return cudaSuccess;
-    if constexpr (!JKKernel<CX, 1>::SPLIT) {
+    if constexpr (!JKKernel<CX>::SPLIT) {
         return launch_one<CX, -1, RT>(e, a);
     } else {
         cudaError_t r = cudaSuccess;

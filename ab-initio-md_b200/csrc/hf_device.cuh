@@ -1,9 +1,11 @@
 // Device building blocks of the McMurchie-Davidson integrals (sm_100a).
 //
-// Boys function F_n(x): positive power series (small x) or erf + upward
-// recursion (x >= n + 1.5), without tables (Helgaker, Jorgensen & Olsen
-// 2000, sec. 9.8; the reference tabulates, aimd/qc/boys.py:88-114). Hermite expansion coefficients E^{ij}_t by the
-// Obara-Saika-type recursion of McMurchie & Davidson (aimd/qc/hermite.py:110),
+// Boys function F_n(x): from a table (hf_boys.h; the reference tabulates too,
+// aimd/qc/boys.py:88-114), or, where that is not staged and in FP32, by the
+// positive power series (small x) or erf and upward recursion (x >= n + 1.5;
+// Helgaker, Jorgensen & Olsen 2000, sec. 9.8). Hermite expansion coefficients
+// E^{ij}_t by the Obara-Saika-type recursion of McMurchie & Davidson
+// (aimd/qc/hermite.py:110),
 // Hermite Coulomb integrals R_tuv by the level recursion, evaluated in place
 // (aimd/qc/hermite.py:145).
 //
@@ -126,14 +128,15 @@ __host__ __device__ constexpr double boys_series_coef(int N, int k) {
     return a;
 }
 
-// F_N(x) without tables (no memory traffic in the integral loops):
+// F_N(x) without a table (Schwarz bounds, two-stage classes, gradient orders
+// above 5):
 //   x <  N + 1.5: the positive series above in Horner form, 22 + 2N terms
 //                 (relative truncation < 1e-15 on the whole interval);
 //   x >= N + 1.5: F_0 = sqrt(pi/x) erf(sqrt(x)) / 2 and the upward recursion
 //                 F_{m+1} = ((2m+1) F_m - e^{-x}) / (2x), stable there
 //                 (measured relative error < 1.5e-15 for N <= 10).
 // Both are standard evaluations of F_N (Helgaker, Jorgensen & Olsen 2000,
-// sec. 9.8); the reference tabulates instead (aimd/qc/boys.py:88-114).
+// sec. 9.8).
 // ex = e^{-x} is passed in by the caller, which needs it anyway.
 template <int N>
 __device__ __forceinline__ double boys_top(double x, double ex) {

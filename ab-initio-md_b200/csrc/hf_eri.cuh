@@ -66,10 +66,10 @@ struct QClass {
     static constexpr int NITEM = NCD / NCB;         // column items per ket pair and contraction group
 };
 
-// Bra-side E tables with an extra +G in i and j (G = 1 for gradients).
-template <int LA, int LB, int G>
+// E table of one bra primitive.
+template <int LA, int LB>
 struct BraE {
-    static constexpr int I = LA + 1 + G, J = LB + 1 + G, T = LA + LB + 1 + 2 * G;
+    static constexpr int I = LA + 1, J = LB + 1, T = LA + LB + 1;
     static constexpr int SIZE = 3 * I * J * T;
     __device__ static int at(int d, int i, int j, int t) { return ((d * I + i) * J + j) * T + t; }
 };
@@ -115,23 +115,23 @@ __device__ __forceinline__ void stage_bra_scalars(const BraStageT<RT>& st) {
 // Without it the longest s contraction that a J/K launch takes beside the Boys
 // table is 45 primitives (41 with it).
 template <int LA, int LB>
-constexpr int bra_e_size() { return LA + LB > 0 ? BraE<LA, LB, 0>::SIZE : 0; }
-template <int LA, int LB, int G, typename RT>
+constexpr int bra_e_size() { return LA + LB > 0 ? BraE<LA, LB>::SIZE : 0; }
+template <int LA, int LB, typename RT>
 __device__ __forceinline__ void stage_bra_e(const BraStageT<RT>& st) {
-    using BE = BraE<LA, LB, G>;
+    using BE = BraE<LA, LB>;
     for (int w = threadIdx.x; w < (LA + LB > 0 ? st.i.nbp * 3 : 0); w += blockDim.x) {
         const int ib = w / 3, d = w % 3;
         const double* b = st.i.rec + (size_t)ib * PPW;
         const double p = b[0] + b[1];
-        double e[LA + 1 + G][LB + 1 + G][LA + LB + 1 + 2 * G];
-        hermite_e<LA + G, LB + G>(b[6 + d], b[9 + d], 0.5 / p, 1.0, e);      // K is in the scalars
+        double e[LA + 1][LB + 1][LA + LB + 1];
+        hermite_e<LA, LB>(b[6 + d], b[9 + d], 0.5 / p, 1.0, e);      // K is in the scalars
         RT* out = st.E + (size_t)ib * BE::SIZE;
 #pragma unroll
-        for (int i = 0; i < LA + 1 + G; ++i)
+        for (int i = 0; i < LA + 1; ++i)
 #pragma unroll
-            for (int j = 0; j < LB + 1 + G; ++j)
+            for (int j = 0; j < LB + 1; ++j)
 #pragma unroll
-                for (int t = 0; t < LA + LB + 1 + 2 * G; ++t) out[BE::at(d, i, j, t)] = static_cast<RT>(e[i][j][t]);
+                for (int t = 0; t < LA + LB + 1; ++t) out[BE::at(d, i, j, t)] = static_cast<RT>(e[i][j][t]);
     }
     stage_bra_scalars(st);
 }
@@ -211,7 +211,7 @@ __device__ __forceinline__ void select_j(const RT (&e)[IM + 1][JM + 1][T + 1], i
 // the rows' boxes.
 template <int LA, int LB, int KG, typename RT, typename Row>
 __device__ __forceinline__ void bra_rows(const RT* E, const RT (&X)[KG][nherm(LA + LB)], Row row) {
-    using BE = BraE<LA, LB, 0>;
+    using BE = BraE<LA, LB>;
 #pragma unroll
     for (int az = 0; az <= LA; ++az)
 #pragma unroll
@@ -277,7 +277,7 @@ __device__ __forceinline__ void eri_column_bra_outer(const BraStageT<RT>& st, co
                                            int id, int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
                                            const RT* __restrict__ Rs, int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 0>;
+    using BE = BraE<Q::LA, Q::LB>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
     const int cx = cart_x(LC, ic), cy = cart_y(LC, ic), cz = cart_z(LC, ic);
     const int dx = cart_x(LD, id), dy = cart_y(LD, id), dz = cart_z(LD, id);
@@ -388,7 +388,7 @@ __device__ __forceinline__ void eri_column_ket_outer(const BraStageT<RT>& st, co
                                                      int kg, RT (&v)[QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
                                                      int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 0>;
+    using BE = BraE<Q::LA, Q::LB>;
     constexpr int LA = Q::LA, LB = Q::LB, L = Q::L;
     static_assert(Q::LCD == 0, "ket ss");
     const int nab = st.i.nA * st.i.nB;
@@ -439,7 +439,7 @@ __device__ __forceinline__ void eri_cols_ket_outer(const BraStageT<RT>& st, cons
                                                    RT (&v)[QClass<CX, CY>::NC][QClass<CX, CY>::NROW][QClass<CX, CY>::KG],
                                                    int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 0>;
+    using BE = BraE<Q::LA, Q::LB>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L;
     const int dx = LD ? cart_x(LD, id) : 0, dy = LD ? cart_y(LD, id) : 0, dz = LD ? cart_z(LD, id) : 0;
     const RT fd = static_cast<RT>(cart_norm(dx, dy, dz));
@@ -543,7 +543,6 @@ __device__ __forceinline__ void eri_column(const BraStageT<RT>& st, const double
 struct QuartetArgs {
     PairView pv;
     BlockView bv;
-    const int* sorted;          // [npair] pair index at sorted position
     const double* sortedQ;      // [npair]
     const int64_t* counts;      // [NSEG][npair + 1] kept ket prefix length per (ket segment, bra position)
     // mixed precision: [NSEG][npair + 1] prefix with Q1 Q2 >= the FP32
@@ -665,7 +664,7 @@ __device__ __forceinline__ void next_chunk(const WorkPlan& plan, int nbra, int t
     b = lo;
 }
 
-__device__ __forceinline__ void load_info(const QuartetArgs& a, const PairMeta& m, BraInfo& st) {
+__device__ __forceinline__ void load_info(const PairMeta& m, BraInfo& st) {
     st.P1 = m.P;
     st.A = m.A;
     st.B = m.B;
@@ -736,7 +735,7 @@ constexpr int CLASS_THREADS = 256;      // the largest
 
 struct JKArgs {
     QuartetArgs q;
-    const double* D;    // [nset][nao][nao], symmetric
+    const double* D;    // [nao][nao], symmetric
     facc* J;            // un-symmetrised accumulators, same shape (fixed point)
     facc* K;
     const double* dmax; // device scalar max |D|: the fixed-point scale of J and K is jk_fix_for(*dmax)
@@ -755,24 +754,23 @@ struct JKArgs {
     WorkPlan plan;      // chunks of the launch (set per launch)
 };
 
-// Digest the NCB columns (ic0 + c, id) of a quartet (all ket contractions kk)
-// for NS densities. Each tensor element the block reaches is visited
+// Digest the NCB columns (ic0 + c, id) of a quartet (all ket contractions kk).
+// Each tensor element the block reaches is visited
 // n_gen = (A==B ? 2:1)(C==D ? 2:1)(P1==P2 ? 2:1) times under the 8 index maps,
 // so each image carries g = 1/n_gen:
 //   J[m,n] += 2g v D[l,s],  J[l,s] += 2g v D[m,n]
 //   K[m,l] += g v D[n,s],   K[n,l] += g v D[m,s],  K[m,s] += g v D[n,l],  K[n,s] += g v D[m,l]
 // (m in A, n in B, l in C, s in D); the host forms J + J^T and K + K^T.
-// K rows m, n belong to the bra pair: Ksm[set][slot][col], slot < KA*NA for
+// K rows m, n belong to the bra pair: Ksm[slot][col], slot < KA*NA for
 // A's functions, then B's; so do the rows of D that K needs, which DA and DB
 // point to (staged in shared memory, or D itself where they do not fit). The
 // columns of one block of an item share their s: their parts of K[., s] and
 // J_ab are summed first.
-template <int CX, int CY, int NS, bool KGLOBAL, int NCB, typename ST, typename RT>
+template <int CX, int CY, bool KGLOBAL, int NCB, typename ST, typename RT>
 __device__ __forceinline__ void jk_digest(const JKArgs& a, const ST& st, const PairMeta& ket, int ic0, int id, int kg,
                                           const RT (&v)[NCB][QClass<CX, CY>::NROW][QClass<CX, CY>::KG], double* Jt,
                                           unsigned* Ksm, const double* DA, const double* DB, double fx) {
     using Q = QClass<CX, CY>;
-    static_assert(NS == 1, "one density a pass");
     const int nC = ket.nA, nD = ket.nB, oC = ket.oA, oD = ket.oB;
     const double g = (st.i.A == st.i.B ? 0.5 : 1.0) * (ket.A == ket.B ? 0.5 : 1.0) * (st.i.P1 == ket.P ? 0.5 : 1.0);
     const double gf = g * fx;               // scaled to fixed point (a power of two: exact)
@@ -1083,8 +1081,8 @@ __device__ __forceinline__ void flat_items(FlatItems& f, bool queued, int* queue
 // ---- Two-stage items: R_tuv staged in shared memory
 // A ket pair of class Y carries NCD Cartesian columns (x contraction
 // groups), each one work item; R_tuv of a primitive quartet is the same for
-// all of them. For the classes where recomputing it per item costs (RSmem
-// below), each queue chunk is cut into sub-chunks whose primitive quartets
+// all of them. For the classes where recomputing it per item costs
+// (QClass::RSMEM), each queue chunk is cut into sub-chunks whose primitive quartets
 // fit RB_PQ slots of a shared buffer (plus the largest single ket pair),
 // and per sub-chunk:
 //   stage 1: one thread per primitive quartet (ket pair i, ket primitive ik,
@@ -1155,8 +1153,9 @@ __device__ __forceinline__ void stage_r(const BraStageT<RT>& st, int ib, const d
     }
 }
 
-// ket_items with R staged per sub-chunk; work(pos, r, Rs) receives the ket
-// pair's staged R ([ik][ib][NH(L)]). Rbuf holds rsmem_bytes(...) bytes.
+// The column items of a segment's ket pairs [j0, j0 + cnt) that pass keep(pos),
+// r < nper of each; work(pos, r, Rs) receives the ket pair's staged R
+// ([ik][ib][NH(L)]). Rbuf holds rsmem_bytes(...) bytes.
 template <int L, typename RT, typename Keep, typename Work>
 __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQueueR& q, int& rot,
                                             const BraStageT<RT>& st, const QuartetArgs& qa, RT* Rbuf, Keep keep,
@@ -1217,7 +1216,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
                 stage_r<L>(st, ib, load_meta(qa, q.pos[i]).rec + (size_t)ik * PPW, Rbuf + (size_t)w * NH);
             }
             __syncthreads();
-            // stage 2: the column items of the sub-chunk, column-major as in ket_items
+            // stage 2: the column items of the sub-chunk, column-major as in flat_items
             const int nsc = l - f;
             const int items = nsc * nper;
             int it = static_cast<int>(threadIdx.x) - rot;
@@ -1233,7 +1232,7 @@ __device__ __forceinline__ void ket_items_r(int nper, int j0, int64_t cnt, KetQu
 }
 
 // The items of the staged bra pair (position spos) in the window that f holds.
-template <int CX, int CY, int NS, bool KGLOBAL, typename RT, typename Boys>
+template <int CX, int CY, bool KGLOBAL, typename RT, typename Boys>
 __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT>& st, int spos, double* Jt,
                                              unsigned* Ksm, FlatItems& f, KetQueueR* kq, int* queue, RT* Rbuf,
                                              Boys boys, const double* DA, const double* DB, double fx) {
@@ -1262,11 +1261,11 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
             // item = the NC columns of one id
             RT v[Q::NC][Q::NROW][Q::KG];
             eri_cols_ket_outer<CX, CY, RT>(st, k.rec, k.npp, cd, kg, v, ib0, ib1, nk, boys);
-            jk_digest<CX, CY, NS, KGLOBAL, Q::NC>(a, st, k, 0, cd, kg, v, Jt, Ksm, DA, DB, fx);
+            jk_digest<CX, CY, KGLOBAL, Q::NC>(a, st, k, 0, cd, kg, v, Jt, Ksm, DA, DB, fx);
         } else {
             RT v[1][Q::NROW][Q::KG];
             eri_column<CX, CY, RT, Q::RSMEM>(st, k.rec, k.npp, cd / Q::ND, cd % Q::ND, kg, v[0], Rs, ib0, ib1, nk, boys);
-            jk_digest<CX, CY, NS, KGLOBAL, 1>(a, st, k, cd / Q::ND, cd % Q::ND, kg, v, Jt, Ksm, DA, DB, fx);
+            jk_digest<CX, CY, KGLOBAL, 1>(a, st, k, cd / Q::ND, cd % Q::ND, kg, v, Jt, Ksm, DA, DB, fx);
         }
     };
     if constexpr (Q::RSMEM) {
@@ -1281,7 +1280,7 @@ __device__ __forceinline__ void jk_ket_class(const JKArgs& a, const BraStageT<RT
     }
 }
 
-template <int CX, int NS>
+template <int CX>
 struct JKKernel {
     using Q0 = QClass<CX, 0>;
     static constexpr int NROW = Q0::NROW;
@@ -1291,9 +1290,8 @@ struct JKKernel {
     // holds the code of one ket class only and the CTAs resident on an SM
     // share their instructions; dd bras accumulate K in global memory
     static constexpr bool SPLIT = CX >= 1;
-    static constexpr int NY = SPLIT ? CX + 1 : 1;
     static constexpr bool KGLOBAL = CX == 5;
-    static constexpr int KROWS = KGLOBAL ? 0 : NS * NF;
+    static constexpr int KROWS = KGLOBAL ? 0 : NF;
 };
 
 // The Boys function of the (CX, Y) J/K kernel: from the table, except for the
@@ -1302,30 +1300,29 @@ template <int CX, int Y, typename RT>
 using JKBoys = BoysOf<QClass<CX, Y>::L, RT, !QClass<CX, Y>::RSMEM>;
 
 // Dynamic shared memory: Boys table, per-thread J_ab slots
-// [NS][NROW][blockDim], K rows [NS][NF][nao] (unless KGLOBAL), D rows
+// [NROW][blockDim], K rows [NF][nao] (unless KGLOBAL), D rows
 // [NF][nao] (unless dglobal), staged R, bra stage.
 
 // RT = double: the FP64 quartets; RT = float: the FP32 quartets of the
 // mixed-precision path (their J/K contributions still accumulate in FP64).
 // YK = ket class of this kernel (-1: the ss bras, whose only ket class is ss).
 // Persistent: a CTA runs chunks of the launch's work plan until it is used up.
-template <int CX, int NS, typename RT, int YK>
+template <int CX, typename RT, int YK>
 __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
-    using KK = JKKernel<CX, NS>;
+    using KK = JKKernel<CX>;
     using Q0 = QClass<CX, 0>;
     constexpr int Y = YK < 0 ? 0 : YK;      // the unsplit kernel (CX = 0) has one ket class too
     static_assert(YK >= 0 || CX == 0, "bra classes above ss are split by ket class");
     extern __shared__ __align__(16) double smem[];
     const int n = a.q.nao;
-    const size_t nn = (size_t)n * n;
     const int krows = a.kglobal ? 0 : KK::KROWS;
     using QY = QClass<CX, Y>;
     using Boys = JKBoys<CX, Y, RT>;
     const int nt = blockDim.x;
     double* btab = smem;                                    // Boys table
     double* Jt = btab + Boys::elems;                        // per-thread J_ab slots
-    unsigned* Ksm = reinterpret_cast<unsigned*>(Jt + NS * KK::NROW * nt);   // low words of the K rows, then the high words
-    double* Dsm = Jt + NS * KK::NROW * nt + even((size_t)krows * n);       // the bra functions' rows of D
+    unsigned* Ksm = reinterpret_cast<unsigned*>(Jt + KK::NROW * nt);   // low words of the K rows, then the high words
+    double* Dsm = Jt + KK::NROW * nt + even((size_t)krows * n);       // the bra functions' rows of D
     RT* Rbuf = reinterpret_cast<RT*>(Dsm + (a.dglobal ? 0 : even((size_t)KK::NF * n)));
     RT* Esm = Rbuf + a.rbuf;
     __shared__ BraInfo info;
@@ -1345,7 +1342,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
             if (lane == 0) {
                 sh[0] = c;
                 sh[1] = b;
-                if (c >= 0) load_info(a.q, load_meta(a.q, a.q.cls_start[CX] + b), info);
+                if (c >= 0) load_info(load_meta(a.q, a.q.cls_start[CX] + b), info);
             }
         }
         __syncthreads();
@@ -1354,7 +1351,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
         const int spos = a.q.cls_start[CX] + b;
         if (!staged) {
             Boys::stage(a.q.boys, btab);
-            for (int i = threadIdx.x; i < krows * n + NS * KK::NROW * nt; i += blockDim.x) Jt[i] = 0.0;
+            for (int i = threadIdx.x; i < krows * n + KK::NROW * nt; i += blockDim.x) Jt[i] = 0.0;
             staged = true;
         }
         const BraStageT<RT> st = stage_view(info, Esm, KK::ESIZE);
@@ -1363,7 +1360,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
             plan_window<CX, Y, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], QY::NITEM,
                                    seg_groups<QY::KG, QY::NKG>(sub), bra_splits(st.i.nbp, sub, f.item_pq), f);
         }
-        stage_bra_e<Q0::LA, Q0::LB, 0>(st);
+        stage_bra_e<Q0::LA, Q0::LB>(st);
         const double *DA = a.D + (size_t)info.oA * n, *DB = a.D + (size_t)info.oB * n;
         if (!a.dglobal) {
             constexpr int NFA = Q0::KA * Q0::NA;
@@ -1376,25 +1373,24 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
             DB = Dsm + NFA * n;
         }
         __syncthreads();
-        jk_ket_class<CX, Y, NS, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf,
+        jk_ket_class<CX, Y, KK::KGLOBAL, RT>(a, st, spos, Jt, Ksm, f, kq.r(), kq.flat(), Rbuf,
                                                  Boys::get(btab), DA, DB, fx);
         __syncthreads();
-        // flush J_ab: a warp a (set, row) sums the threads' slots (in a fixed
+        // flush J_ab: a warp a row sums the threads' slots (in a fixed
         // order) and clears them
-        for (int i = warp; i < NS * KK::NROW; i += nt / 32) {
+        for (int r = warp; r < KK::NROW; r += nt / 32) {
             double val = 0.0;
             for (int t = 0; t < nt; t += 32) {
-                val += Jt[i * nt + t + lane];
-                Jt[i * nt + t + lane] = 0.0;
+                val += Jt[r * nt + t + lane];
+                Jt[r * nt + t + lane] = 0.0;
             }
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) val += __shfl_xor_sync(0xffffffffu, val, d);
             if (lane != 0 || val == 0.0) continue;
-            const int s = i / KK::NROW, r = i % KK::NROW;
             const int kab = r / Q0::NAB, ab = r % Q0::NAB;
             const int ka = kab / st.i.nB, kb = kab % st.i.nB;
             const int m = st.i.oA + ka * Q0::NA + ab / Q0::NB, nb_ = st.i.oB + kb * Q0::NB + ab % Q0::NB;
-            fadd(a.J + s * nn + (size_t)m * n + nb_, val, fx);
+            fadd(a.J + (size_t)m * n + nb_, val, fx);
         }
         // flush and clear the K rows
         if (krows > 0) {
@@ -1403,9 +1399,9 @@ __global__ void __launch_bounds__(CLASS_THREADS) jk_bra_kernel(JKArgs a) {
                 const facc val = join_planes(Ksm[i], Ksm[krows * n + i]);
                 if (val == 0) continue;
                 Ksm[i] = Ksm[krows * n + i] = 0u;
-                const int col = i % n, f_ = (i / n) % KK::NF, s = i / (n * KK::NF);
+                const int col = i % n, f_ = i / n;
                 const int row = f_ < NFA ? st.i.oA + f_ : st.i.oB + (f_ - NFA);
-                atomicAdd(a.K + s * nn + (size_t)row * n + col, val);     // integer: order-independent
+                atomicAdd(a.K + (size_t)row * n + col, val);     // integer: order-independent
             }
         }
         __syncthreads();
@@ -1422,12 +1418,12 @@ size_t jk_rbuf_elems(int max_bra_prims, int max_ket_prims) {
     return 0;
 }
 
-template <int CX, int NS, int Y, typename RT>
+template <int CX, int Y, typename RT>
 size_t jk_smem_bytes(int threads, int nao, int max_bra_prims, size_t rbuf_elems, bool kglobal, bool dglobal) {
-    using KK = JKKernel<CX, NS>;
+    using KK = JKKernel<CX>;
     const size_t krows = kglobal ? 0 : KK::KROWS;
     return sizeof(double) * (even(krows * nao) + (dglobal ? 0 : even((size_t)KK::NF * nao)) +
-                             (size_t)NS * KK::NROW * threads + JKBoys<CX, Y, RT>::elems) +
+                             (size_t)KK::NROW * threads + JKBoys<CX, Y, RT>::elems) +
            sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (KK::ESIZE + SBW));
 }
 
@@ -1453,7 +1449,7 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS) schwarz_kernel(QuartetArgs a,
     }
     __syncthreads();
     const BraStageT<double> st = stage_view(info, smem, bra_e_size<Q::LA, Q::LB>());
-    stage_bra_e<Q::LA, Q::LB, 0>(st);
+    stage_bra_e<Q::LA, Q::LB>(st);
     __syncthreads();
     static_assert(Q::KG == Q::KCD, "diagonal quartets keep all contraction combinations in one item");
     constexpr int NSP = SCHWARZ_THREADS / Q::NCD;       // ranges of the bra primitives

@@ -1,6 +1,6 @@
 // Integral-direct two-electron gradient 1/2 sum Gamma d(mn|ls)/dR.
 //
-// Same decomposition as the J/K build: one CTA per bra block pair, one
+// Same decomposition as the J/K build: chunks of one bra block pair each, one
 // thread item per (ket pair, ket component pair cd). The quartet list is
 // enumerated at thr / Gamma_bound, so every quartet the exact test can keep
 // is visited; each item applies the reference's test Q1 Q2 max|Gamma| < thr
@@ -52,7 +52,6 @@ struct GradArgs {
     WorkPlan plan;          // chunks of the launch (set per launch)
 };
 
-
 // Two-stage items (R_tuv to L + 1 staged per primitive quartet) for the
 // gradient of class pair (CX, CY): the same classes as the J/K build.
 template <int CX, int CY>
@@ -63,7 +62,7 @@ constexpr bool grad_rsmem() { return QClass<CX, CY>::RSMEM; }
 // the gradient body, and in registers it pushes the body into local memory.
 // Up to 84 values (L + 1 = 6, 172 KB for the eight warps of an SM); an odd
 // stride, so that a warp's accesses to one element spread over the banks.
-template <int CX, int CY, typename RT>
+template <int CX, int CY>
 constexpr bool grad_rcol() {
     constexpr int NH = nherm(QClass<CX, CY>::L + 1);
     return !grad_rsmem<CX, CY>() && NH > 20 && NH <= 84;
@@ -74,7 +73,7 @@ constexpr int grad_rstride() { return nherm(QClass<CX, CY>::L + 1) | 1; }
 // E and dE/dX_AB of one bra pair's primitives, in the same layout (st.E, st.D).
 template <int LA, int LB, typename RT>
 __device__ __forceinline__ void stage_bra_de(const BraStageT<RT>& st) {
-    using BE = BraE<LA, LB, 0>;
+    using BE = BraE<LA, LB>;
     for (int w = threadIdx.x; w < st.i.nbp * 3; w += blockDim.x) {
         const int ib = w / 3, d = w % 3;
         const double* b = st.i.rec + (size_t)ib * PPW;
@@ -108,7 +107,7 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                                            RT (&dA)[3], RT (&dB)[3], RT (&dC)[3], const RT* __restrict__ Rs,
                                            RT* Rcol, int ib0, int ib1, int nk, Boys boys) {
     using Q = QClass<CX, CY>;
-    using BE = BraE<Q::LA, Q::LB, 0>;
+    using BE = BraE<Q::LA, Q::LB>;
     constexpr int LA = Q::LA, LB = Q::LB, LC = Q::LC, LD = Q::LD, LAB = Q::LAB, LCD = Q::LCD, L = Q::L + 1;
     constexpr int NHB = Q::NHB, NH1 = nherm(LAB + 1);
     constexpr int KG = Q::KG;
@@ -284,7 +283,7 @@ __device__ __forceinline__ void grad_prims(const BraStageT<RT>& st, const RT (&G
                 const RT rs = rsqrt_t(b.p + q);
                 RT R[nherm(L)];
                 hermite_r_scaled<L>(b.p * q * (rs * rs), b.X - k.Qx, b.Y - k.Qy, b.Z - k.Qz, rs, R, boys);
-                if constexpr (grad_rcol<CX, CY, RT>()) {
+                if constexpr (grad_rcol<CX, CY>()) {
 #pragma unroll
                     for (int i = 0; i < nherm(L); ++i) Rcol[i] = R[i];
                     body(Rcol);
@@ -472,7 +471,7 @@ using GradBoys = BoysOf<QClass<CX, CY>::L + 1, RT, (QClass<CX, CY>::L + 1 <= 5)>
 // (bra pair of class CX, window of its ket pairs of class CY) of the
 // launch's work plan until it is used up. Dynamic shared memory: gradient
 // accumulator [natm][3] (one per CTA, flushed at the end), Boys table, D rows, staged R, bra E
-// tables (+1).
+// and dE/dX_AB tables.
 // RT = double: the FP64 quartets; RT = float: the FP32 quartets of the
 // mixed-precision path (accumulated in FP64).
 template <int CX, int CY, typename RT>
@@ -506,7 +505,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) grad2e_bra_kernel(GradArgs a) {
             if (lane == 0) {
                 sh[0] = c;
                 sh[1] = b;
-                if (c >= 0) load_info(a.q, load_meta(a.q, a.q.cls_start[CX] + b), info);
+                if (c >= 0) load_info(load_meta(a.q, a.q.cls_start[CX] + b), info);
             }
         }
         __syncthreads();                                        // (also orders the zeroing)
@@ -517,7 +516,7 @@ __global__ void __launch_bounds__(CLASS_THREADS) grad2e_bra_kernel(GradArgs a) {
             Boys::stage(a.q.boys, btab);
             staged = true;
         }
-        const BraStageT<RT> st = stage_view(info, Esm, BraE<Q0::LA, Q0::LB, 0>::SIZE);
+        const BraStageT<RT> st = stage_view(info, Esm, BraE<Q0::LA, Q0::LB>::SIZE);
         if (warp == 0) {
             const int sub = lane < NSUB ? lane : 0;
             plan_window<CX, CY, RT>(a.q, spos, st.i.nbp, c - a.plan.off[b], a.plan.off[b + 1] - a.plan.off[b], Q::NCD,
@@ -556,7 +555,7 @@ template <int CX, int CY, typename RT>
 size_t grad_rbuf_elems(int threads, int max_bra_prims, int max_ket_prims) {
     if constexpr (grad_rsmem<CX, CY>())
         return fours(rsmem_bytes<QClass<CX, CY>::L + 1, RT>(max_bra_prims, max_ket_prims) / sizeof(RT));
-    if constexpr (grad_rcol<CX, CY, RT>()) return fours((size_t)grad_rstride<CX, CY>() * threads);
+    if constexpr (grad_rcol<CX, CY>()) return fours((size_t)grad_rstride<CX, CY>() * threads);
     return 0;
 }
 
@@ -565,7 +564,7 @@ size_t grad_smem_bytes(int natm, int nx, int nao, int max_bra_prims, size_t rbuf
     using Q0 = QClass<CX, 0>;
     constexpr size_t NF = Q0::KA * Q0::NA + Q0::KB * Q0::NB;
     return sizeof(double) * (even(3 * (size_t)natm) + GradBoys<CX, CY, RT>::elems + (dglobal ? 0 : even(nx * NF * nao))) +
-           sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (2 * BraE<Q0::LA, Q0::LB, 0>::SIZE + SBW));
+           sizeof(RT) * (rbuf_elems + (size_t)max_bra_prims * (2 * BraE<Q0::LA, Q0::LB>::SIZE + SBW));
 }
 
 }  // namespace hf

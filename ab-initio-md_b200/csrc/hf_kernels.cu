@@ -518,7 +518,6 @@ QuartetArgs quartet_args(aimd_ctx* c, const int64_t* counts) {
     QuartetArgs q;
     q.pv = pair_view(c);
     q.bv = block_view(c);
-    q.sorted = c->sorted;
     q.sortedQ = c->sortedQ;
     q.counts = counts;
     q.counts_hi = nullptr;
@@ -543,12 +542,12 @@ int build_counts(aimd_ctx* c, double thr, int64_t* counts, cudaStream_t st, cons
     return AIMD_OK;
 }
 
-int ncls_pairs(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
+int cls_size(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
 
 LaunchEnv launch_env(aimd_ctx* c) {
     LaunchEnv e;
     for (int cl = 0; cl < NCLS; ++cl) {
-        e.cls_count[cl] = ncls_pairs(c, cl);
+        e.cls_count[cl] = cls_size(c, cl);
         e.maxbp[cl] = c->maxbp[cl];
     }
     for (int cl = 0; cl <= NCLS; ++cl) e.cls_start[cl] = c->cls_start[cl];
@@ -668,8 +667,6 @@ void plan_launches(aimd_ctx* c, const QuartetArgs& q, bool mixed, int per_sm, cu
         c->item_pq, CLASS_THREADS * c->nsm);
     c->launches += 2;
 }
-
-int cls_size(aimd_ctx* c, int cl) { return c->cls_start[cl + 1] - c->cls_start[cl]; }
 
 // The status of a call's class launches and the bra class of the first that failed.
 struct ClassStatus {
