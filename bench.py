@@ -29,8 +29,8 @@ gradient, Verlet update. ``--workload methanol``: CH3OH RHF/6-31G**
          2 sum NH(L-n) + 2 NH(Lab) NH(Lcd) n_cd n_kc + 2 NH(Lab) n_ab n_cd n_kc
          over the Schwarz-kept unique block quartets) / average duration,
          against the FP64 peak measured in the same run by a cuBLAS DGEMM;
-         the two-electron gradient likewise (bra Hermite order + 1, two
-         passes); the mixed-precision build and gradient against the
+         the two-electron gradient likewise (flop_model_device, as its
+         kernels evaluate it); the mixed-precision build and gradient against the
          measured FP32 SGEMM peak.
   cpu_baseline  the oracle (C + OpenMP restatement of the reference's numba
          path) on the host cores, on the workload itself at the converged
@@ -220,10 +220,11 @@ def flop_model_device(eng, basis, thr: float = 1e-12, grad: bool = False) -> tup
     FP64 flop model of one ERI pass and its primitive-quartet count, from the
     engine's pairs (unique block quartets p1 >= p2 in block-pair index
     order, p1 as bra, Q1 Q2 >= thr), evaluated on the device in row chunks.
-    grad=True: the two-electron gradient's model, the same sum with the bra
-    Hermite order raised by one (the derivative expansions, R to L + 1),
-    counted twice (the bra pass for centres A, B and the ket pass for C; D
-    follows by translational invariance).
+    grad=True: what the two-electron gradient evaluates, with the same dense
+    boxes: per primitive quartet R to L + 1 and, for each ket column, X to the
+    bra order + 1, Z, and the three sums of G; per bra primitive and column the
+    bra expansion Y and the three sums of U (D follows by translational
+    invariance).
     """
     import torch
     Q = eng.schwarz()
@@ -252,15 +253,17 @@ def flop_model_device(eng, basis, thr: float = 1e-12, grad: bool = False) -> tup
     for r0 in range(0, npair, chunk):
         p1 = idx[r0:r0 + chunk]
         keep = (Q[p1][:, None] * Q[None, :] >= thr) & (idx[None, :] <= p1[:, None])
-        dl = 1 if grad else 0
         Lb = Lp[p1][:, None]
         Lk = Lp[None, :]
-        per = (2 * rs[Lb + Lk + dl] + 2 * NH(Lb + dl) * NH(Lk) * nab[None, :] * ncon[None, :]
-               + 2 * NH(Lb + dl) * nab[p1][:, None] * nab[None, :] * ncon[None, :])
+        cols = nab[None, :] * ncon[None, :]
         if grad:
-            per = 2 * per
+            per = 2 * rs[Lb + Lk + 1] + cols * (2 * (NH(Lb + 1) + NH(Lb)) * NH(Lk) + 6 * NH(Lb))
+            once = cols * 8 * NH(Lb) * nab[p1][:, None]
+        else:
+            per = 2 * rs[Lb + Lk] + cols * (2 * NH(Lb) * NH(Lk) + 2 * NH(Lb) * nab[p1][:, None])
+            once = torch.zeros_like(per)
         ww = w[p1][:, None] * w[None, :]
-        total += float((per * ww * keep).sum())
+        total += float(((per * ww + once * w[p1][:, None]) * keep).sum())
         nq += float((ww * keep).sum())
     return total, nq
 
