@@ -16,8 +16,8 @@ runs molecules concurrently instead:
     copies; both release the Python GIL, so the streams keep the GPU busy
     with the kernels of several molecules at the same time.
 
-Results are those of running each molecule alone (same kernels, same
-screening; only the summation order of the FP64 atomics may differ).
+Results are those of running each molecule alone: same kernels, same
+screening, sums in fixed point.
 """
 
 from __future__ import annotations

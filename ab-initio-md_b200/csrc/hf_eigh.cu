@@ -7,11 +7,13 @@
 // 6-31G**, where the Fock build takes 0.3 ms). Here the matrix and the vectors
 // stay in shared memory for all sweeps, and an iteration may start from the
 // eigenvectors of the one before, in whose basis the matrix is nearly diagonal:
-// two or three sweeps then, six or seven from scratch: SCF and gradient of
-// methanol at two frames, 20 iterations, 39.5 -> 28.2 ms on one B200. Bound by the latency of
-// a round (two barriers, a square root, shared-memory passes over both
-// matrices). Above n = 64 a round's passes grow past what one SM does faster
-// than the library.
+// two or three sweeps then, seven or eight from scratch: SCF and gradient of
+// methanol at two frames, 20 iterations, 39.5 -> 28.2 ms on one B200. Bound by the
+// latency of a round (two barriers, a square root, shared-memory passes over both
+// matrices). The limit of 64 is where a start from scratch meets the library, and
+// one block of rotations a thread fills the CTA (us, one B200, from nearby vectors
+// / from scratch / library): n = 16 56 / 98 / 198, 32 113 / 236 / 283,
+// 48 217 / 461 / 776, 64 354 / 846 / 936.
 #include <cstdio>
 
 #include "../../include/aimd_b200.h"
